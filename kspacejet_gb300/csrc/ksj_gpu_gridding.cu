@@ -56,6 +56,7 @@ namespace {
 
 constexpr int kChunk = 16;        // grid columns per binning list (<= 32 lists per row)
 constexpr int kMaxWidth = 8;      // largest Kaiser-Bessel width
+constexpr int kWarpSortMax = 512; // longest list a warp sorts (16 registers a lane); longer ones take a block
 constexpr int kMaxGrid = 512;
 constexpr int kMaxThreads = 512;
 constexpr int kColsThreads = 256;  // k_cols block size
@@ -130,7 +131,7 @@ struct Shape {
 };
 
 struct Layout {
-  size_t flags, frame_flags, records, counts, cursor, offsets, entries, expanded, long_lists, samples_t, inter,
+  size_t flags, frame_flags, records, counts, cursor, offsets, entries, expanded, long_lists, mid_lists, samples_t, inter,
       coil_last, tables, total;
 };
 
@@ -259,7 +260,7 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   s->coil_group = cg;
   s->column_block = cb;
-  s->list_capacity = cap;
+  s->list_capacity = std::min(cap, kWarpSortMax);
   // frames per k_rows/k_cols pass: keep one pass's row-transformed grid
   // (channels x grid_rows x out_cols complex) within ~64 MB of L2
   // fields appended to the tuning struct are read only when the caller's
@@ -308,6 +309,7 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
   l.expanded = take(static_cast<size_t>(s.frames) * s.entries_per_frame * meta_vecs(s.width) * 16);
   l.long_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / (s.list_capacity + 1)) * 4);
+  l.mid_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / 33) * 4);
   l.samples_t = take(fm * s.channels * sample_bytes(d->sample_format));
   l.inter = take(static_cast<size_t>(s.frames) * s.grid_rows * s.out_cols * s.cpitch * sizeof(float2));
   l.coil_last = d->output == KSJ_GPU_OUTPUT_COIL_MAJOR
@@ -540,27 +542,65 @@ __global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, c
   }
 }
 
-// Warp-cooperative ascending sort of buf[0, n) (shared or global memory):
-// the bitonic network in its all-ascending form (first comparator of each
-// merge flipped), so positions >= n behave as +infinity and are never
-// touched -- no padding is needed.
-__device__ __forceinline__ void warp_sort(uint32_t* buf, int n, int lane) {
-  int p = 1;
-  while (p < n) p <<= 1;
-  for (int k = 2; k <= p; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < p; i += 32) {
-        const int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-        if (partner > i && partner < n) {
-          const uint32_t a = buf[i], b = buf[partner];
-          if (a > b) {
-            buf[i] = b;
-            buf[partner] = a;
-          }
-        }
-      }
-      __syncwarp();
+// Ascending sort of R * 32 keys held by a warp, key e = 32 r + lane in v[r]:
+// the bitonic network in its all-ascending form (the first comparator of each
+// merge flipped), so absent keys padded with 0xffffffff stay at the end and no
+// merge needs a direction.  Comparators between lanes are one shuffle and one
+// min or max per key, those between registers one min and one max per pair, and
+// the R keys of a lane are independent: the chain is the network's depth (45
+// comparators for 512 keys), where the same network over a buffer in shared
+// memory waits out a load, a compare and a store 45 * 16 times over.
+__device__ __forceinline__ uint32_t keep_min(uint32_t a, uint32_t b, bool low) { return low ? min(a, b) : max(a, b); }
+
+// The comparators at distances 16, 8, 4, 2, 1 (between lanes).
+template <int R>
+__device__ __forceinline__ void warp_merge_lanes(uint32_t (&v)[R], int lane, int from) {
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    if (j > from) continue;
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = keep_min(v[r], __shfl_xor_sync(0xffffffffu, v[r], j), (lane & j) == 0);
+  }
+}
+
+// The comparators at distances 32 * from_r, ..., 32 (between registers), then 16 ... 1.
+template <int R>
+__device__ __forceinline__ void warp_merge(uint32_t (&v)[R], int lane, int from_r) {
+#pragma unroll
+  for (int jr = R / 2; jr > 0; jr >>= 1) {
+    if (jr > from_r) continue;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r & jr) continue;
+      const uint32_t a = v[r], b = v[r + jr];
+      v[r] = min(a, b);
+      v[r + jr] = max(a, b);
     }
+  }
+  warp_merge_lanes<R>(v, lane, 16);
+}
+
+template <int R>
+__device__ __forceinline__ void warp_sort(uint32_t (&v)[R], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      v[r] = keep_min(v[r], __shfl_xor_sync(0xffffffffu, v[r], k - 1), (lane & (k >> 1)) == 0);
+    warp_merge_lanes<R>(v, lane, k >> 2);
+  }
+#pragma unroll
+  for (int kr = 2; kr <= R; kr <<= 1) {
+    // flipped: key e meets e ^ (32 kr - 1), i.e. register r ^ (kr - 1) of lane ^ 31
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int q = r ^ (kr - 1);
+      if (q < r) continue;
+      const uint32_t a = __shfl_xor_sync(0xffffffffu, v[q], 31), b = __shfl_xor_sync(0xffffffffu, v[r], 31);
+      v[r] = min(v[r], a);
+      v[q] = max(v[q], b);
+    }
+    warp_merge<R>(v, lane, kr >> 2);
   }
 }
 
@@ -654,8 +694,10 @@ struct SortArgs {
   uint32_t* entries;
   const unsigned char* records;
   float4* expanded;
-  uint32_t* long_lists;  // lists longer than `capacity`, left to k_sort_long
+  uint32_t* long_lists;  // lists longer than `capacity`, left to the blocks of k_sort_long
   uint32_t* long_count;
+  uint32_t* mid_lists;   // lists of 33 .. `capacity` entries, left to the warps of k_sort_long
+  uint32_t* mid_count;
   int frames, samples, lists_per_frame, nchunks, grid_rows, grid_cols, capacity;
   size_t entries_per_frame;  // 0 when the offsets are absolute (3-D: one entry array for all planes)
   int dim3;                  // 3-D: frames are grid planes and the records are per sample (SampleRecord3)
@@ -681,52 +723,64 @@ __device__ __forceinline__ void expand_at(const SortArgs& a, int f, int l, uint3
 }
 
 // Expanded entries of list l of frame f, entries i = first, first + step, ...
+// (four at a time: their record loads are all in flight before the first store).
 template <int W>
 __device__ __forceinline__ void expand_list(const SortArgs& a, int f, int l, uint32_t begin, int n,
                                             const uint32_t* sorted, int first, int step) {
+#pragma unroll 4
   for (int i = first; i < n; i += step) expand_at<W>(a, f, l, begin, i, sorted[i]);
 }
 
 constexpr int kSortGroup = 4;  // consecutive lists per warp in k_sort
 
+// A list of 33 .. 32 R entries: sorted in registers, then written back or expanded.
+template <int W, int R>
+__device__ __forceinline__ void sort_list_regs(const SortArgs& a, int f, int l, uint32_t begin, int n, int lane,
+                                               uint32_t* ent) {
+  uint32_t v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = 32 * r + lane < n ? ent[32 * r + lane] : 0xffffffffu;
+  warp_sort<R>(v, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = 32 * r + lane;
+    if (i < n) {
+      if (a.expanded == nullptr)
+        ent[i] = v[r];
+      else
+        expand_at<W>(a, f, l, begin, i, v[r]);
+    }
+  }
+}
+
 // One list (one warp): sort the sample indices ascending, then write every
 // entry in its expanded form (the dependent record loads happen here, across
 // many lists in flight, not in the row pass).  A list of at most 32 entries
 // is ranked on registers: its sample indices are distinct, so the number of
-// smaller indices is each entry's sorted position.  Longer lists are sorted
-// in the warp's shared buffer; lists longer than the buffer are queued for
+// smaller indices is each entry's sorted position.  Longer lists are queued for
 // k_sort_long.  The sorted indices themselves are written back only for the
 // density-weight path (no expansion), the one reader of them.
 template <int W>
-__device__ __forceinline__ void sort_list(const SortArgs& a, int f, int l, uint32_t begin, int n, int lane,
-                                          uint32_t* buf) {
+__device__ __forceinline__ void sort_list(const SortArgs& a, int f, int l, uint32_t begin, int n, int lane) {
   if (n == 0) return;
-  if (n > a.capacity) {
-    if (lane == 0)
-      a.long_lists[atomicAdd(a.long_count, 1u)] = static_cast<uint32_t>(static_cast<size_t>(f) * a.lists_per_frame + l);
-    return;
-  }
-  uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
-  if (n <= 32) {
-    const uint32_t key = lane < n ? ent[lane] : 0xffffffffu;
-    int rank = 0;
-    for (int j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key ? 1 : 0;
-    if (lane < n) {
-      if (a.expanded == nullptr)
-        ent[rank] = key;  // every lane read its key before the shuffles
-      else
-        expand_at<W>(a, f, l, begin, rank, key);
+  if (n > 32) {
+    if (lane == 0) {
+      const bool mid = n <= a.capacity;
+      (mid ? a.mid_lists : a.long_lists)[atomicAdd(mid ? a.mid_count : a.long_count, 1u)] =
+          static_cast<uint32_t>(static_cast<size_t>(f) * a.lists_per_frame + l);
     }
     return;
   }
-  for (int i = lane; i < n; i += 32) buf[i] = ent[i];
-  __syncwarp();
-  warp_sort(buf, n, lane);
-  if (a.expanded == nullptr) {
-    for (int i = lane; i < n; i += 32) ent[i] = buf[i];
-    return;
+  uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+  const uint32_t key = lane < n ? ent[lane] : 0xffffffffu;
+  int rank = 0;
+  for (int j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key ? 1 : 0;
+  if (lane < n) {
+    if (a.expanded == nullptr)
+      ent[rank] = key;  // every lane read its key before the shuffles
+    else
+      expand_at<W>(a, f, l, begin, rank, key);
   }
-  expand_list<W>(a, f, l, begin, n, buf, lane, 32);
 }
 
 // kSortGroup consecutive lists of one frame per warp.  Their entries are
@@ -735,7 +789,6 @@ __device__ __forceinline__ void sort_list(const SortArgs& a, int f, int l, uint3
 // entries (same order as sort_list), so tiny and empty lists share one warp.
 template <int W>
 __global__ void __launch_bounds__(256) k_sort(SortArgs a) {
-  extern __shared__ uint32_t sort_buf[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = (a.lists_per_frame + kSortGroup - 1) / kSortGroup;
   const size_t gg = static_cast<size_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
@@ -749,11 +802,10 @@ __global__ void __launch_bounds__(256) k_sort(SortArgs a) {
   const int total = static_cast<int>(__shfl_sync(0xffffffffu, my_off, ng) - begin);
   if (total == 0) return;
   if (total > 32) {
-    uint32_t* buf = sort_buf + static_cast<size_t>(warp) * a.capacity;
     for (int s = 0; s < ng; ++s) {
       const uint32_t b = __shfl_sync(0xffffffffu, my_off, s);
       const uint32_t e = __shfl_sync(0xffffffffu, my_off, s + 1);
-      sort_list<W>(a, f, l0 + s, b, static_cast<int>(e - b), lane, buf);
+      sort_list<W>(a, f, l0 + s, b, static_cast<int>(e - b), lane);
       __syncwarp();
     }
     return;
@@ -783,91 +835,105 @@ __global__ void __launch_bounds__(256) k_sort(SortArgs a) {
 }
 
 constexpr int kLongSortThreads = 1024;
+constexpr int kLongSortBlocks = 152;    // one per SM
 constexpr int kLongSortSmem = 16384;  // entries sorted in shared memory; longer lists in place in L2/HBM
 
-// The same bitonic network over a whole block.
+constexpr int kLongRegs = kWarpSortMax / 32;
+
+// The keys of each kWarpSortMax-key chunk of buf[0, n) sorted (first, whole
+// chunks from scratch) or merged (the comparators at distances below
+// kWarpSortMax) by a warp in registers.  buf holds n rounded up to whole
+// chunks, the padding 0xffffffff.  Synchronises the block.
+template <bool kWhole>
+__device__ __forceinline__ void block_chunks(uint32_t* buf, int n) {
+  const int lane = threadIdx.x & 31;
+  for (int c = (threadIdx.x >> 5) * kWarpSortMax; c < n; c += (kLongSortThreads / 32) * kWarpSortMax) {
+    uint32_t v[kLongRegs];
+#pragma unroll
+    for (int r = 0; r < kLongRegs; ++r) v[r] = buf[c + 32 * r + lane];
+    if constexpr (kWhole)
+      warp_sort<kLongRegs>(v, lane);
+    else
+      warp_merge<kLongRegs>(v, lane, kLongRegs / 2);
+#pragma unroll
+    for (int r = 0; r < kLongRegs; ++r) buf[c + 32 * r + lane] = v[r];
+  }
+  __syncthreads();
+}
+
+// One comparator stage over buf[0, n) (shared or global memory), thread per
+// pair: the flipped first stage of the merge into runs of k (i and its mirror
+// in the run), or the pairs at distance j.  Keys at or beyond n are absent
+// (they are the largest, and stay).  Synchronises the block.
+__device__ __forceinline__ void compare_pair(uint32_t* buf, int i, int partner, int n) {
+  if (partner < n) {
+    const uint32_t x = buf[i], y = buf[partner];
+    if (x > y) {
+      buf[i] = y;
+      buf[partner] = x;
+    }
+  }
+}
+__device__ __forceinline__ void block_flip(uint32_t* buf, int n, int k) {
+  const int lg = __ffs(k >> 1) - 1, pairs = ((n + k - 1) / k) << lg;
+  for (int p = threadIdx.x; p < pairs; p += kLongSortThreads) {
+    const int i = ((p >> lg) << (lg + 1)) + (p & ((1 << lg) - 1));
+    compare_pair(buf, i, i ^ (k - 1), n);
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void block_step(uint32_t* buf, int n, int j) {
+  const int lg = __ffs(j) - 1, pairs = ((n + 2 * j - 1) >> (lg + 1)) << lg;
+  for (int p = threadIdx.x; p < pairs; p += kLongSortThreads) {
+    const int i = ((p >> lg) << (lg + 1)) + (p & (j - 1));
+    compare_pair(buf, i, i + j, n);
+  }
+  __syncthreads();
+}
+
+// n keys of global memory into buf, padded to whole chunks, and back.
+__device__ __forceinline__ void chunk_load(uint32_t* buf, const uint32_t* ent, int n) {
+  const int padded = (n + kWarpSortMax - 1) / kWarpSortMax * kWarpSortMax;
+  for (int t = threadIdx.x; t < padded; t += kLongSortThreads) buf[t] = t < n ? ent[t] : 0xffffffffu;
+  __syncthreads();
+}
+__device__ __forceinline__ void chunk_store(const uint32_t* buf, uint32_t* ent, int n) {
+  for (int t = threadIdx.x; t < n; t += kLongSortThreads) ent[t] = buf[t];
+  __syncthreads();
+}
+
+// buf[0, n), n <= kLongSortSmem, sorted by the block: the network of warp_sort
+// over chunks in registers, only the comparators at distance kWarpSortMax and
+// above over shared memory (15 stages for 16384 keys instead of 105).
 __device__ __forceinline__ void block_sort(uint32_t* buf, int n) {
-  int p = 1;
-  while (p < n) p <<= 1;
-  for (int k = 2; k <= p; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < p; i += blockDim.x) {
-        const int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-        if (partner > i && partner < n) {
-          const uint32_t x = buf[i], y = buf[partner];
-          if (x > y) {
-            buf[i] = y;
-            buf[partner] = x;
-          }
-        }
-      }
-      __syncthreads();
-    }
+  block_chunks<true>(buf, n);
+  for (int k = 2 * kWarpSortMax; (k >> 1) < n; k <<= 1) {
+    block_flip(buf, n, k);
+    for (int j = k >> 2; j >= kWarpSortMax; j >>= 1) block_step(buf, n, j);
+    block_chunks<false>(buf, n);
   }
 }
 
-// Stages (k, j) for j = j0, j0 / 2, ..., 1 of that network on the chunk of
-// list elements [base, base + kLongSortSmem) held in buf (elements at or
-// beyond n are absent).  Every pair of these stages lies inside the chunk:
-// j < kLongSortSmem, and the mirrored partner of stage j = k / 2 only when
-// k <= kLongSortSmem.
-__device__ __forceinline__ void chunk_stages(uint32_t* buf, int base, int n, int k, int j0) {
-  for (int j = j0; j > 0; j >>= 1) {
-    for (int t = threadIdx.x; t < kLongSortSmem && base + t < n; t += blockDim.x) {
-      const int i = base + t;
-      const int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-      if (partner > i && partner < n) {
-        const uint32_t x = buf[t], y = buf[partner - base];
-        if (x > y) {
-          buf[t] = y;
-          buf[partner - base] = x;
-        }
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// The network of block_sort on a list longer than the shared buffer, in
-// place in global memory, with every stage whose pairs lie inside one
-// kLongSortSmem-entry chunk run on that chunk in shared memory: first each
-// chunk sorted whole (k up to the chunk size), then per larger k the stages
-// with j >= the chunk size over global memory and the rest chunk by chunk.
-// Same comparisons in the same stage order as block_sort: the same result.
-__device__ __forceinline__ void chunk_load(uint32_t* buf, const uint32_t* ent, int base, int n) {
-  for (int t = threadIdx.x; t < kLongSortSmem && base + t < n; t += blockDim.x) buf[t] = ent[base + t];
-  __syncthreads();
-}
-__device__ __forceinline__ void chunk_store(const uint32_t* buf, uint32_t* ent, int base, int n) {
-  for (int t = threadIdx.x; t < kLongSortSmem && base + t < n; t += blockDim.x) ent[base + t] = buf[t];
-  __syncthreads();
-}
+// The same network on a list longer than the shared buffer, in place in global
+// memory: chunks of kLongSortSmem keys sorted in the buffer, then per merge the
+// comparators at distance kLongSortSmem and above over global memory and the
+// rest chunk by chunk in the buffer.
 __device__ __forceinline__ void block_sort_chunked(uint32_t* ent, int n, uint32_t* buf) {
-  int p = 1;
-  while (p < n) p <<= 1;
   for (int base = 0; base < n; base += kLongSortSmem) {
-    chunk_load(buf, ent, base, n);
-    for (int k = 2; k <= kLongSortSmem; k <<= 1) chunk_stages(buf, base, n, k, k >> 1);
-    chunk_store(buf, ent, base, n);
+    const int cnt = min(kLongSortSmem, n - base);
+    chunk_load(buf, ent + base, cnt);
+    block_sort(buf, cnt);
+    chunk_store(buf, ent + base, cnt);
   }
-  for (int k = 2 * kLongSortSmem; k <= p; k <<= 1) {
-    for (int j = k >> 1; j >= kLongSortSmem; j >>= 1) {
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int partner = (j == (k >> 1)) ? (i ^ (k - 1)) : (i ^ j);
-        if (partner > i && partner < n) {
-          const uint32_t x = ent[i], y = ent[partner];
-          if (x > y) {
-            ent[i] = y;
-            ent[partner] = x;
-          }
-        }
-      }
-      __syncthreads();
-    }
+  for (int k = 2 * kLongSortSmem; (k >> 1) < n; k <<= 1) {
+    block_flip(ent, n, k);
+    for (int j = k >> 2; j >= kLongSortSmem; j >>= 1) block_step(ent, n, j);
     for (int base = 0; base < n; base += kLongSortSmem) {
-      chunk_load(buf, ent, base, n);
-      chunk_stages(buf, base, n, k, kLongSortSmem >> 1);
-      chunk_store(buf, ent, base, n);
+      const int cnt = min(kLongSortSmem, n - base);
+      chunk_load(buf, ent + base, cnt);
+      for (int j = kLongSortSmem >> 1; j >= kWarpSortMax; j >>= 1) block_step(buf, cnt, j);
+      block_chunks<false>(buf, cnt);
+      chunk_store(buf, ent + base, cnt);
     }
   }
 }
@@ -882,11 +948,10 @@ __device__ __forceinline__ void sort_long_list(const SortArgs& a, size_t gl, uin
   uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
   const uint32_t* sorted = ent;
   if (n <= kLongSortSmem) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) long_buf[i] = ent[i];
-    __syncthreads();
+    chunk_load(long_buf, ent, n);
     block_sort(long_buf, n);
     if (a.expanded == nullptr)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) ent[i] = long_buf[i];
+      for (int i = threadIdx.x; i < n; i += kLongSortThreads) ent[i] = long_buf[i];
     sorted = long_buf;
   } else {
     block_sort_chunked(ent, n, long_buf);
@@ -895,9 +960,12 @@ __device__ __forceinline__ void sort_long_list(const SortArgs& a, size_t gl, uin
   if (a.expanded != nullptr) expand_list<W>(a, f, l, begin, n, sorted, threadIdx.x, blockDim.x);
 }
 
-// Blocks take the queued long lists in turn: sort (in shared memory up to
-// kLongSortSmem entries, else in place with chunk-local stages in shared
-// memory) and expand.
+// The lists k_sort queued.  Blocks take the long ones in turn (sorted in shared
+// memory up to kLongSortSmem entries, else in place with chunk-local stages in
+// shared memory), then every warp the ones of 33 .. capacity entries, 2 to 16
+// keys a lane in registers.  A kernel of its own, because the networks' registers
+// would halve the warps that k_sort has in flight on the short lists: both in
+// one kernel measured 426 us on the lists of 96 radial frames, 202 us apart.
 template <int W>
 __global__ void __launch_bounds__(kLongSortThreads, 1) k_sort_long(SortArgs a) {
   extern __shared__ uint32_t long_buf[];
@@ -906,27 +974,45 @@ __global__ void __launch_bounds__(kLongSortThreads, 1) k_sort_long(SortArgs a) {
     sort_long_list<W>(a, a.long_lists[q], long_buf);
     __syncthreads();
   }
+  const uint32_t mids = *a.mid_count;
+  const int lane = threadIdx.x & 31;
+  for (uint32_t q = blockIdx.x * (kLongSortThreads / 32) + (threadIdx.x >> 5); q < mids;
+       q += gridDim.x * (kLongSortThreads / 32)) {
+    const uint32_t gl = a.mid_lists[q];
+    const int f = static_cast<int>(gl / a.lists_per_frame);
+    const int l = static_cast<int>(gl - static_cast<uint32_t>(f) * a.lists_per_frame);
+    const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
+    const uint32_t begin = off[l];
+    const int n = static_cast<int>(off[l + 1] - begin);
+    uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+    if (n <= 64)
+      sort_list_regs<W, 2>(a, f, l, begin, n, lane, ent);
+    else if (n <= 128)
+      sort_list_regs<W, 4>(a, f, l, begin, n, lane, ent);
+    else if (n <= 256)
+      sort_list_regs<W, 8>(a, f, l, begin, n, lane, ent);
+    else
+      sort_list_regs<W, 16>(a, f, l, begin, n, lane, ent);
+  }
 }
 
 // Launch k_sort and then k_sort_long for the lists it queued.
 template <int W>
-ksj_gpu_status launch_sort(SortArgs sa, size_t lists, size_t entries_total, int capacity, cudaStream_t stream) {
-  if (cudaMemsetAsync(sa.long_count, 0, sizeof(uint32_t), stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  const size_t smem = static_cast<size_t>(8) * capacity * 4;
-  if (cudaFuncSetAttribute(k_sort<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_sort_long<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSortSmem * 4) !=
-          cudaSuccess)
+ksj_gpu_status launch_sort(SortArgs sa, cudaStream_t stream) {
+  // both counts, in front of the queues
+  if (cudaMemsetAsync(sa.mid_count, 0, sizeof(uint32_t), stream) != cudaSuccess ||
+      cudaMemsetAsync(sa.long_count, 0, sizeof(uint32_t), stream) != cudaSuccess)
+    return KSJ_GPU_ERROR_CUDA;
+  if (cudaFuncSetAttribute(k_sort_long<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSortSmem * 4) !=
+      cudaSuccess)
     return KSJ_GPU_ERROR_CUDA;
   {
     LaunchScope scope("k_sort", stream);
     const size_t warps = static_cast<size_t>(sa.frames) * ((sa.lists_per_frame + kSortGroup - 1) / kSortGroup);
-    k_sort<W><<<static_cast<unsigned>((warps + 7) / 8), 256, smem, stream>>>(sa);
+    k_sort<W><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(sa);
   }
-  const size_t most = std::max<size_t>(1, entries_total / (static_cast<size_t>(capacity) + 1));
   LaunchScope scope("k_sort_long", stream);
-  k_sort_long<W><<<static_cast<unsigned>(std::min<size_t>(std::min<size_t>(most, lists), 1024)), kLongSortThreads,
-                   kLongSortSmem * 4, stream>>>(sa);
+  k_sort_long<W><<<kLongSortBlocks, kLongSortThreads, kLongSortSmem * 4, stream>>>(sa);
   return KSJ_GPU_OK;
 }
 
@@ -2131,7 +2217,7 @@ template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
                            uint32_t* offsets, uint32_t* entries, float4* expanded, uint32_t* long_lists,
-                           cudaStream_t stream, uint32_t* frame_flags = nullptr) {
+                           uint32_t* mid_lists, cudaStream_t stream, uint32_t* frame_flags = nullptr) {
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
   if (cudaMemsetAsync(counts, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   if (cudaMemsetAsync(cursor, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
@@ -2182,6 +2268,8 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     sa.expanded = expanded;
     sa.long_count = long_lists;
     sa.long_lists = long_lists + 1;
+    sa.mid_count = mid_lists;
+    sa.mid_lists = mid_lists + 1;
     sa.frames = s.frames;
     sa.samples = s.samples;
     sa.lists_per_frame = s.lists_per_frame;
@@ -2191,8 +2279,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     sa.capacity = s.list_capacity;
     sa.entries_per_frame = s.entries_per_frame;
     sa.dim3 = 0;
-    const ksj_gpu_status st = launch_sort<W>(sa, nl, static_cast<size_t>(s.frames) * s.entries_per_frame,
-                                             s.list_capacity, stream);
+    const ksj_gpu_status st = launch_sort<W>(sa, stream);
     if (st != KSJ_GPU_OK) return st;
   }
   return KSJ_GPU_OK;
@@ -2247,7 +2334,8 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   {
     const ksj_gpu_status st = build_lists<W>(s, d, d_traj, d_dcf, flags, records, counts, cursor, offsets, entries,
                                              reinterpret_cast<float4*>(ws + l.expanded),
-                                             reinterpret_cast<uint32_t*>(ws + l.long_lists), stream,
+                                             reinterpret_cast<uint32_t*>(ws + l.long_lists),
+                                             reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream,
                                              reinterpret_cast<uint32_t*>(ws + l.frame_flags));
     if (st != KSJ_GPU_OK) return st;
   }
@@ -2550,7 +2638,7 @@ __global__ void __launch_bounds__(256) k_pm_update(const PmRecord<W>* pm, const 
 }
 
 struct PmLayout {
-  size_t flags, records, counts, cursor, offsets, entries, long_lists, pm, w, grid, total;
+  size_t flags, records, counts, cursor, offsets, entries, long_lists, mid_lists, pm, w, grid, total;
 };
 
 PmLayout make_pm_layout(const Shape& s) {
@@ -2570,6 +2658,7 @@ PmLayout make_pm_layout(const Shape& s) {
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
   l.long_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / (s.list_capacity + 1)) * 4);
+  l.mid_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / 33) * 4);
   l.pm = take(fm * (8 + 16 * static_cast<size_t>(s.width)));
   l.w = take(fm * sizeof(double));
   l.grid = take(static_cast<size_t>(s.frames) * s.grid_rows * s.grid_cols * sizeof(double));
@@ -2590,7 +2679,8 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
       build_lists<W>(s, &dd, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
                      reinterpret_cast<uint32_t*>(ws + l.cursor), reinterpret_cast<uint32_t*>(ws + l.offsets),
                      reinterpret_cast<uint32_t*>(ws + l.entries), nullptr,
-                     reinterpret_cast<uint32_t*>(ws + l.long_lists), stream);
+                     reinterpret_cast<uint32_t*>(ws + l.long_lists), reinterpret_cast<uint32_t*>(ws + l.mid_lists),
+                     stream);
   if (st != KSJ_GPU_OK) return st;
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   PmRecord<W>* pm = reinterpret_cast<PmRecord<W>*>(ws + l.pm);
@@ -2758,7 +2848,7 @@ __global__ void __launch_bounds__(256) k_scatter3(const unsigned char* records, 
 }
 
 struct Layout3 {
-  size_t flags, records, counts, cursor, offsets, bases, entries, expanded, long_lists, samples_t, inter, inter2,
+  size_t flags, records, counts, cursor, offsets, bases, entries, expanded, long_lists, mid_lists, samples_t, inter, inter2,
       tables, total;
   size_t entries_total;
 };
@@ -2793,6 +2883,7 @@ Layout3 make_layout3(const Shape& s, uint32_t sample_format) {
   l.entries = take(l.entries_total * 4);
   l.expanded = take(l.entries_total * meta_vecs(s.width) * 16);
   l.long_lists = take((2 + l.entries_total / (s.list_capacity + 1)) * 4);
+  l.mid_lists = take((2 + l.entries_total / 33) * 4);
   l.samples_t = take(static_cast<size_t>(s.samples) * s.channels * sample_bytes(sample_format));
   l.inter = take(g * g * n * s.cpitch * sizeof(float2));
   l.inter2 = take(g * n * n * s.cpitch * sizeof(float2));
@@ -2834,7 +2925,7 @@ template <int W>
 ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_traj, const float* d_dcf,
                             uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
                             uint32_t* offsets, uint32_t* bases, uint32_t* entries, float4* expanded,
-                            uint32_t* long_lists, size_t entries_total, cudaStream_t stream) {
+                            uint32_t* long_lists, uint32_t* mid_lists, cudaStream_t stream) {
   const int g = s.grid_rows;
   const size_t nl = static_cast<size_t>(g) * s.lists_per_frame;
   if (cudaMemsetAsync(counts, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
@@ -2882,6 +2973,8 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     sa.expanded = expanded;
     sa.long_count = long_lists;
     sa.long_lists = sa.long_count + 1;
+    sa.mid_count = mid_lists;
+    sa.mid_lists = mid_lists + 1;
     sa.frames = g;
     sa.samples = s.samples;
     sa.lists_per_frame = s.lists_per_frame;
@@ -2891,7 +2984,7 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     sa.capacity = s.list_capacity;
     sa.entries_per_frame = 0;
     sa.dim3 = 1;
-    const ksj_gpu_status st = launch_sort<W>(sa, nl, entries_total, s.list_capacity, stream);
+    const ksj_gpu_status st = launch_sort<W>(sa, stream);
     if (st != KSJ_GPU_OK) return st;
   }
   return KSJ_GPU_OK;
@@ -2933,8 +3026,8 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
     const ksj_gpu_status st = build_lists3<W>(s, d->dcf_mode, d_traj, d_dcf, flags, ws + l.records, counts, cursor,
                                               offsets, reinterpret_cast<uint32_t*>(ws + l.bases), entries,
                                               reinterpret_cast<float4*>(ws + l.expanded),
-                                              reinterpret_cast<uint32_t*>(ws + l.long_lists), l.entries_total,
-                                              stream);
+                                              reinterpret_cast<uint32_t*>(ws + l.long_lists),
+                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream);
     if (st != KSJ_GPU_OK) return st;
   }
   {
@@ -3319,7 +3412,7 @@ __global__ void __launch_bounds__(256) k_pm_update3(const PmRecord3<W>* pm, cons
 }
 
 struct PmLayout3 {
-  size_t flags, records, counts, cursor, offsets, bases, entries, long_lists, pm, pmc, wzr, w, grid, part_base, partial,
+  size_t flags, records, counts, cursor, offsets, bases, entries, long_lists, mid_lists, pm, pmc, wzr, w, grid, part_base, partial,
       counters, total, entries_total, max_long;
 };
 
@@ -3342,6 +3435,7 @@ PmLayout3 make_pm_layout3(const Shape& s) {
   l.bases = take(g * 4);
   l.entries = take(l.entries_total * 4);
   l.long_lists = take((2 + l.entries_total / (s.list_capacity + 1)) * 4);
+  l.mid_lists = take((2 + l.entries_total / 33) * 4);
   l.pm = take(static_cast<size_t>(s.samples) * (16 + 24 * static_cast<size_t>(s.width)));
   l.pmc = take(static_cast<size_t>(s.samples) * (8 + 8 * static_cast<size_t>(s.width)));
   l.wzr = take(l.entries_total * sizeof(double));
@@ -3368,7 +3462,7 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
       s, KSJ_GPU_DCF_NONE, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
       reinterpret_cast<uint32_t*>(ws + l.cursor), reinterpret_cast<uint32_t*>(ws + l.offsets),
       reinterpret_cast<uint32_t*>(ws + l.bases), reinterpret_cast<uint32_t*>(ws + l.entries), nullptr,
-      reinterpret_cast<uint32_t*>(ws + l.long_lists), l.entries_total, stream);
+      reinterpret_cast<uint32_t*>(ws + l.long_lists), reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream);
   if (st != KSJ_GPU_OK) return st;
   static_assert(sizeof(PmCol3<W>) == 8 + 8 * W, "PmCol3 layout");
   PmRecord3<W>* pm = reinterpret_cast<PmRecord3<W>*>(ws + l.pm);
