@@ -12,12 +12,13 @@
 //   k_sort     per list (one warp): sort by sample index, so every cell later
 //              accumulates in sample order -- the reference's order -- and the
 //              result is deterministic whatever order the scatter produced
-//   k_samples_coil_last  [frame][coil][sample] -> [frame][sample][coil], so a
-//              warp reads one sample's coils as one coalesced segment
-//   k_rows     per (frame, grid row, coil group): each warp owns one
-//              32-column chunk of the row and its sorted list and accumulates
-//              lane-per-coil into shared memory with no atomics (a cell is
-//              only ever touched by its owning warp, in list order); the block
+//   k_samples_coil_last  [frame][coil][sample] -> [frame][sample][coil] times
+//              the sample's weight and phase, so the row pass reads one
+//              sample's coils as one coalesced segment
+//   k_rows     per (frame, grid row, coil group): groups of lanes (lane =
+//              coil) take the row's sorted lists, one 16-column chunk each,
+//              and sum its cells in registers with no atomics (a cell is
+//              only ever touched by its owning group, in list order); the block
 //              then runs the row inverse FFT of every coil line in place and
 //              writes only the columns the image keeps, coil-last
 //              ([frame][grid row][column][channel]), so the column pass
@@ -28,7 +29,7 @@
 //              in channel order (the reference RSS order and rounding)
 //   k_images_coil_major  coil-last -> coil-major transpose when asked for
 //
-// Binning lists are (frame, grid row, 32-column chunk); a sample is listed
+// Binning lists are (frame, grid row, 16-column chunk); a sample is listed
 // once per row its stencil covers and per chunk its W columns fall into
 // (one or two).  The "reference permutation" a list must equal is the
 // increasing sequence of sample indices whose stencil touches that row and
@@ -58,10 +59,9 @@ constexpr int kChunk = 16;        // grid columns per binning list (<= 32 lists 
 constexpr int kMaxWidth = 8;      // largest Kaiser-Bessel width
 constexpr int kWarpSortMax = 512; // longest list a warp sorts (16 registers a lane); longer ones take a block
 constexpr int kMaxGrid = 512;
-constexpr int kMaxThreads = 512;
 constexpr int kColsThreads = 256;  // k_cols block size
-constexpr int kAhead = 8;         // coil loads in flight per warp in k_rows
-constexpr int kAheadRegs = 2;     // the same for the register-cell form (its unrolled body grows with it: 2 measured best)
+constexpr int kRowsThreads = 384;  // most threads of a k_rows block (two such blocks per SM)
+constexpr int kRowsBatch = 8;      // list entries a lane group stages and loads samples for at once
 constexpr uint32_t kFlagBytes = 256;
 
 // Per (frame, sample) record written by k_prepare, read by k_rows.
@@ -85,20 +85,32 @@ struct alignas(16) SampleRecord3 {
   float wc[W];
 };
 
-// k_rows stages, per warp, the list entries of its current batch in shared
-// memory: {c0, sample, scale} and the W column weights times the row weight,
-// in 16-byte vectors read back as warp-wide broadcasts.
-__host__ __device__ constexpr int meta_vecs(int w) { return 1 + (w + 3) / 4; }
-__host__ __device__ constexpr int meta_batch(int w) { return w <= 4 ? 32 : 16; }
+// One sorted list entry as the row pass reads it: the first tap's column as
+// seen from the list's chunk (-7 .. 15; a row length lower when the taps reaching
+// the chunk wrapped past the last column), the sample index, and the W column
+// weights times the list's row (and plane) weight.
+__host__ __device__ constexpr int entry_bytes(int w) { return 8 + 4 * w; }
 
-// Shared memory of one k_rows block: accumulators, twiddles, the list
-// offsets of the row and the per-warp entry batches.
-inline size_t rows_smem_for(int grid_cols, int cg, int width, int threads) {
-  const int nchunks = (grid_cols + kChunk - 1) / kChunk;
-  const size_t head = static_cast<size_t>(grid_cols) * (cg + 1) * 8 + static_cast<size_t>(nchunks + 1) * 4;
-  return ((head + 15) & ~size_t{15}) + static_cast<size_t>(threads / 32) * meta_batch(width) * meta_vecs(width) * 16;
+// A staged entry in shared memory: the 16 weights of the chunk's columns (zero
+// where no tap falls), then the sample index.  80 bytes apart, so that lanes
+// writing or reading the same word of consecutive entries meet different banks.
+constexpr int kSlotFloats = 20;
+
+// Shared memory of one k_rows block: accumulators, twiddles and the staged
+// entries of every lane group.  Lane groups
+// are the lanes of a coil group's part: lanes = coil_group / coil_parts.
+inline size_t rows_smem_for(int grid_cols, int cg, int lanes, int threads) {
+  const size_t head = static_cast<size_t>(grid_cols) * (cg + 1) * 8;
+  return ((head + 15) & ~size_t{15}) + static_cast<size_t>(threads / lanes) * kRowsBatch * kSlotFloats * 4;
 }
-inline int rows_threads_for(int grid_cols) { return std::max(64, (grid_cols + 31) / 32 * 32); }
+// Threads of a k_rows block: enough for the transform's first step (n / 16
+// times cg of them) in two rounds, but no fewer than 8 warps, so that a row's
+// long lists, cut in segments, have warps to run on; narrow groups take 4, as
+// each of their many lane groups stages its own entries.
+inline int rows_threads_for(int grid_cols, int lanes, int cg) {
+  if (lanes < 4) return 128;
+  return grid_cols / 16 * cg > 512 ? kRowsThreads : 256;
+}
 
 constexpr uint32_t kWaitLimit = 1u << 22;  // polls before a bounded wait gives up
 
@@ -117,7 +129,7 @@ struct Shape {
   float beta, inv_i0_beta;
   float row_origin, col_origin;
   float phase_row, phase_col, phase_sign;  // origin-phase coefficients
-  int coil_group, column_block, list_capacity, frames_per_pass, rows_blocks, coil_parts;
+  int coil_group, column_block, list_capacity, frames_per_pass, coil_parts;
   uint32_t wait_fault;  // tests only: segment waits that cannot succeed, given up after this many polls
   int column_pass;      // 1 one CTA per tile (k_cols), 2 persistent ring (k_cols_ring)
   DifPlan plan_rows, plan_cols;
@@ -229,19 +241,23 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   if (cap == 0) cap = 512;
   if (cap < 64 || cap > 2048 || (cap & (cap - 1)) != 0) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   const size_t smem_limit = 200 * 1024;
+  const int parts = t && t->struct_size >= offsetof(ksj_gpu_gridding_tuning, coil_parts) + 4 && t->coil_parts
+                        ? static_cast<int>(t->coil_parts)
+                        : 1;
+  if (parts != 1 && parts != 2) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   auto rows_smem = [&](int g) {
-    return rows_smem_for(s->grid_cols, g, s->width, rows_threads_for(s->grid_cols));
+    const int lanes = std::max(1, g / parts);
+    return rows_smem_for(s->grid_cols, g, lanes, rows_threads_for(s->grid_cols, lanes, g));
   };
   if (cg == 0) {
     int want = 1;
     while (want < s->channels && want < 32) want <<= 1;
     cg = want;
-    // two row blocks per SM when they fit: (228 KiB - 2 x 1 KiB reserved) / 2;
-    // rows wider than 384 columns run one 512-thread block per SM whatever
-    // the group, and there the whole 32-coil register path wins (grid 512,
-    // 32 coils: 4.8 against 8.6 ms per 16-frame call with a 16-coil group)
-    const size_t per_block = rows_threads_for(s->grid_cols) <= 384 ? 115712 : smem_limit;
-    while (cg > 1 && rows_smem(cg) > per_block) cg >>= 1;
+    // two row blocks per SM at least ((228 KiB - 2 x 1 KiB reserved) / 2), so
+    // that one block's transform overlaps another's gridding; the whole coil
+    // array where it fits (32 coils on a 384 grid, 96 frames: groups of 32, 16, 8
+    // coils take 2488, 2640, 3621 us)
+    while (cg > 1 && rows_smem(cg) > 115712 - 1024) cg >>= 1;
   }
   if (cg < 1 || cg > 32 || (cg & (cg - 1)) != 0 || rows_smem(cg) > smem_limit) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   // column pass: cb columns x col_group coils per tile (a power of two
@@ -272,14 +288,8 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   if (fpp <= 0) fpp = s->frames >= 4 ? (s->frames + 1) / 2 : s->frames;
   s->frames_per_pass = std::min(fpp, s->frames);
   int rb = has(offsetof(ksj_gpu_gridding_tuning, rows_blocks_per_sm) + 4) ? static_cast<int>(t->rows_blocks_per_sm) : 0;
-  // default: two row CTAs per SM wherever the row kernel fits them (384
-  // threads; the coil group above was sized for two CTAs' shared memory)
-  if (rb == 0) rb = rows_threads_for(s->grid_cols) <= 384 && rows_smem(cg) <= 115712 ? 2 : 1;
-  if (rb != 1 && rb != 2) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  s->rows_blocks = rb;
-  int parts = has(offsetof(ksj_gpu_gridding_tuning, coil_parts) + 4) ? static_cast<int>(t->coil_parts) : 0;
-  if (parts == 0) parts = 1;
-  if ((parts != 1 && parts != 2) || parts > cg) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
+  if (rb < 0 || rb > 2) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
+  if (parts > cg) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   s->coil_parts = parts;
   s->wait_fault = has(offsetof(ksj_gpu_gridding_tuning, wait_fault_polls) + 4) ? t->wait_fault_polls : 0u;
   int cp = has(offsetof(ksj_gpu_gridding_tuning, column_pass) + 4) ? static_cast<int>(t->column_pass) : 0;
@@ -307,10 +317,10 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
   l.cursor = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
-  l.expanded = take(static_cast<size_t>(s.frames) * s.entries_per_frame * meta_vecs(s.width) * 16);
+  l.expanded = take(static_cast<size_t>(s.frames) * s.entries_per_frame * entry_bytes(s.width));
   l.long_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / (s.list_capacity + 1)) * 4);
   l.mid_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / 33) * 4);
-  l.samples_t = take(fm * s.channels * sample_bytes(d->sample_format));
+  l.samples_t = take(fm * s.channels * sizeof(float2));
   l.inter = take(static_cast<size_t>(s.frames) * s.grid_rows * s.out_cols * s.cpitch * sizeof(float2));
   l.coil_last = d->output == KSJ_GPU_OUTPUT_COIL_MAJOR
                     ? take(static_cast<size_t>(s.frames) * s.channels * s.out_rows * s.out_cols * sizeof(float2))
@@ -604,53 +614,20 @@ __device__ __forceinline__ void warp_sort(uint32_t (&v)[R], int lane) {
   }
 }
 
-// One list entry as k_rows consumes it (meta_vecs(W) 16-byte vectors):
-//   v0 = {tap word, sample index, scale.re, scale.im}, v1.. = the W column
-//   weights times this row's weight (zero padded).
-// The tap word holds the mask of taps that land in the list's column chunk
-// (bits 0-7) and the column of tap 0 as seen from the chunk (bits 9 up, one
-// row-length lower when the taps reaching the chunk wrapped past the last
-// column); bit 8 marks a one-chunk row that sees both ends of a wrap, whose
-// taps are wrapped one by one.
+// One list entry (entry_bytes(W)) from its sample's record.
 template <int W>
-__device__ __forceinline__ void expand_taps(uint32_t sidx, int c0, float sre, float sim, float wrow, const float* wc,
-                                            int col_lo, int col_hi, int grid_cols, float4* out) {
-  constexpr int kMV = meta_vecs(W);
-  const int cb0 = c0 >= col_hi ? c0 - grid_cols : c0;
-  uint32_t in_chunk = 0, straight = 0;
+__device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, const float* wc, int col_lo, int grid_cols,
+                                          unsigned char* out) {
+  float2* o = reinterpret_cast<float2*>(out);
+  const int t0 = c0 - col_lo >= kChunk ? c0 - col_lo - grid_cols : c0 - col_lo;
+  o[0] = make_float2(__int_as_float(t0), __uint_as_float(sidx));
 #pragma unroll
-  for (int j = 0; j < W; ++j) {
-    int col = c0 + j;
-    if (col >= grid_cols) col -= grid_cols;
-    if (col >= col_lo && col < col_hi) in_chunk |= 1u << j;
-    if (cb0 + j >= col_lo && cb0 + j < col_hi) straight |= 1u << j;
-  }
-  const int word0 = in_chunk == straight ? ((cb0 * 512) | static_cast<int>(in_chunk))
-                                         : ((c0 * 512) | 256 | static_cast<int>(in_chunk));
-  out[0] = make_float4(__int_as_float(word0), __uint_as_float(sidx), sre, sim);
-#pragma unroll
-  for (int v = 1; v < kMV; ++v) {
-    float t4[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = 4 * (v - 1) + u;
-      t4[u] = j < W ? wrow * wc[j] : 0.0f;
-    }
-    out[v] = make_float4(t4[0], t4[1], t4[2], t4[3]);
-  }
+  for (int j = 0; j < W; j += 2) o[1 + j / 2] = make_float2(wrow * wc[j], wrow * wc[j + 1]);
 }
 
-// One list entry as k_rows consumes it (meta_vecs(W) 16-byte vectors):
-//   v0 = {tap word, sample index, scale.re, scale.im}, v1.. = the W column
-//   weights times this row's weight (zero padded).
-// The tap word holds the mask of taps that land in the list's column chunk
-// (bits 0-7) and the column of tap 0 as seen from the chunk (bits 9 up, one
-// row-length lower when the taps reaching the chunk wrapped past the last
-// column); bit 8 marks a one-chunk row that sees both ends of a wrap, whose
-// taps are wrapped one by one.
 template <int W>
 __device__ __forceinline__ void expand_entry(const SampleRecord<W>* recs, uint32_t sidx, int row, int col_lo,
-                                             int col_hi, int grid_rows, int grid_cols, float4* out) {
+                                             int grid_rows, int grid_cols, unsigned char* out) {
   constexpr int kRV = static_cast<int>(sizeof(SampleRecord<W>) / 16);
   float4 q[kRV];
   const float4* rp = reinterpret_cast<const float4*>(recs + sidx);
@@ -663,13 +640,13 @@ __device__ __forceinline__ void expand_entry(const SampleRecord<W>* recs, uint32
 #pragma unroll
   for (int j = 0; j < W; ++j)
     if (j == ta) wr = w[4 + j];
-  expand_taps<W>(sidx, __float_as_int(w[1]), w[2], w[3], wr, w + 4 + W, col_lo, col_hi, grid_cols, out);
+  put_entry<W>(sidx, __float_as_int(w[1]), wr, w + 4 + W, col_lo, grid_cols, out);
 }
 
 // The 3-D form: the list's plane and row weights folded together.
 template <int W>
 __device__ __forceinline__ void expand_entry3(const SampleRecord3<W>* recs, uint32_t sidx, int plane, int row,
-                                              int col_lo, int col_hi, int grid, float4* out) {
+                                              int col_lo, int grid, unsigned char* out) {
   constexpr int kRV = static_cast<int>(sizeof(SampleRecord3<W>) / 16);
   float4 q[kRV];
   const float4* rp = reinterpret_cast<const float4*>(recs + sidx);
@@ -686,14 +663,14 @@ __device__ __forceinline__ void expand_entry3(const SampleRecord3<W>* recs, uint
     if (j == tz) wz = w[6 + j];
     if (j == ta) wr = w[6 + W + j];
   }
-  expand_taps<W>(sidx, __float_as_int(w[2]), w[4], w[5], wr * wz, w + 6 + 2 * W, col_lo, col_hi, grid, out);
+  put_entry<W>(sidx, __float_as_int(w[2]), wr * wz, w + 6 + 2 * W, col_lo, grid, out);
 }
 
 struct SortArgs {
   const uint32_t* offsets;
   uint32_t* entries;
   const unsigned char* records;
-  float4* expanded;
+  unsigned char* expanded;
   uint32_t* long_lists;  // lists longer than `capacity`, left to the blocks of k_sort_long
   uint32_t* long_count;
   uint32_t* mid_lists;   // lists of 33 .. `capacity` entries, left to the warps of k_sort_long
@@ -706,20 +683,15 @@ struct SortArgs {
 // Expanded entry i of list l of frame f (sample index sidx).
 template <int W>
 __device__ __forceinline__ void expand_at(const SortArgs& a, int f, int l, uint32_t begin, int i, uint32_t sidx) {
-  constexpr int kMV = meta_vecs(W);
   const int row = l / a.nchunks;
   const int col_lo = (l - row * a.nchunks) * kChunk;
-  const int col_hi = min(col_lo + kChunk, a.grid_cols);
-  float4* out = a.expanded + (static_cast<size_t>(f) * a.entries_per_frame + begin + i) * kMV;
-  float4 e[kMV];
+  unsigned char* out = a.expanded + (static_cast<size_t>(f) * a.entries_per_frame + begin + i) * entry_bytes(W);
   if (a.dim3)
-    expand_entry3<W>(reinterpret_cast<const SampleRecord3<W>*>(a.records), sidx, f, row, col_lo, col_hi, a.grid_cols,
-                     e);
+    expand_entry3<W>(reinterpret_cast<const SampleRecord3<W>*>(a.records), sidx, f, row, col_lo,
+                     a.grid_cols, out);
   else
     expand_entry<W>(reinterpret_cast<const SampleRecord<W>*>(a.records) + static_cast<size_t>(f) * a.samples, sidx, row,
-                    col_lo, col_hi, a.grid_rows, a.grid_cols, e);
-#pragma unroll
-  for (int v = 0; v < kMV; ++v) out[v] = e[v];
+                    col_lo, a.grid_rows, a.grid_cols, out);
 }
 
 // Expanded entries of list l of frame f, entries i = first, first + step, ...
@@ -1016,78 +988,96 @@ ksj_gpu_status launch_sort(SortArgs sa, cudaStream_t stream) {
   return KSJ_GPU_OK;
 }
 
-// [frame][channel][sample] -> [frame][sample][channel] through a 32x33
-// shared tile (launch (32, 8) threads, grid (ceil(samples/32),
+// [frame][channel][sample] -> [frame][sample][channel] complex64, each sample
+// times its weight and phase (dcf * exp(i * origin phase), in its record), through
+// a 32x33 shared tile (launch (32, 8) threads, grid (ceil(samples/32),
 // ceil(channels/32), frames)), checking every sample on the way: a
 // non-finite value (either component; bf16 exponent all ones) raises
-// KSJ_GPU_FLAG_NONFINITE_SAMPLE.
+// KSJ_GPU_FLAG_NONFINITE_SAMPLE.  The product is formed here, once, and not by
+// each of the W rows (W^2 in 3-D) that read the sample.
 //
 // Ragged batches (frame_channels / frame_samples / frame_src non-null):
 // frame f holds frame_channels[f] coils of frame_samples[f] samples, packed
 // [channel][sample] at address frame_src[f] (device memory, or host memory
 // the device reads in place); the padding up to the call's channels and
 // samples is written as zeros.
+struct CoilLastArgs {
+  const void* in;
+  float2* out;
+  const unsigned char* scales;  // the records' scale fields, `scale_stride` bytes apart
+  int scale_stride;
+  int channels, samples;
+  uint32_t* flags;
+  const uint32_t* frame_channels;
+  const uint32_t* frame_samples;
+  const uint64_t* frame_src;
+  int frame0;
+  uint32_t* frame_flags;
+};
+
 template <uint32_t kFormat>
-__global__ void __launch_bounds__(256) k_samples_coil_last(const void* in_raw, void* out_raw, int channels,
-                                                           int samples, uint32_t* flags,
-                                                           const uint32_t* frame_channels,
-                                                           const uint32_t* frame_samples,
-                                                           const uint64_t* frame_src, int frame0,
-                                                           uint32_t* frame_flags) {
+__global__ void __launch_bounds__(256) k_samples_coil_last(CoilLastArgs a) {
   using T = typename std::conditional<kFormat == KSJ_GPU_SAMPLES_BF16, uint32_t, unsigned long long>::type;
-  __shared__ T t[32][33];
-  const T* in = static_cast<const T*>(in_raw);
-  T* out = static_cast<T*>(out_raw);
-  const int f = blockIdx.z;
+  __shared__ float2 t[32][33];
+  const int channels = a.channels, samples = a.samples;
+  const int f = a.frame0 + blockIdx.z;
   const int s0 = blockIdx.x * 32;
   const int c0 = blockIdx.y * 32;
-  T* dst = out + static_cast<size_t>(f) * channels * samples;
-  const int live_c = frame_channels ? min(channels, static_cast<int>(__ldg(frame_channels + frame0 + f))) : channels;
-  const int live_s = frame_samples ? min(samples, static_cast<int>(__ldg(frame_samples + frame0 + f))) : samples;
+  float2* dst = a.out + static_cast<size_t>(f) * channels * samples;
+  const int live_c = a.frame_channels ? min(channels, static_cast<int>(__ldg(a.frame_channels + f))) : channels;
+  const int live_s = a.frame_samples ? min(samples, static_cast<int>(__ldg(a.frame_samples + f))) : samples;
   // ragged frames are packed at their own sample count
-  const T* src = frame_src ? reinterpret_cast<const T*>(__ldg(frame_src + frame0 + f))
-                           : in + static_cast<size_t>(f) * channels * samples;
-  const int pitch = frame_src ? live_s : samples;
+  const T* src = a.frame_src ? reinterpret_cast<const T*>(__ldg(a.frame_src + f))
+                             : static_cast<const T*>(a.in) + static_cast<size_t>(f) * channels * samples;
+  const int pitch = a.frame_src ? live_s : samples;
+  const int sm = s0 + threadIdx.x;
+  float2 scale = make_float2(0.0f, 0.0f);
+  if (sm < live_s)
+    scale = __ldg(reinterpret_cast<const float2*>(
+        a.scales + (static_cast<size_t>(f) * samples + sm) * static_cast<size_t>(a.scale_stride)));
   bool bad = false;
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const int c = c0 + y, sm = s0 + threadIdx.x;
+#pragma unroll
+  for (int y = threadIdx.y; y < 32; y += 8) {
+    const int c = c0 + y;
     if (c < channels && sm < samples) {
       if (c >= live_c || sm >= live_s) {
-        t[y][threadIdx.x] = T(0);
+        t[y][threadIdx.x] = make_float2(0.0f, 0.0f);
         continue;
       }
-      const T v = src[static_cast<size_t>(c) * pitch + sm];
-      if (kFormat == KSJ_GPU_SAMPLES_BF16) {
-        const uint32_t u = static_cast<uint32_t>(v);
-        bad |= (u & 0x7f80u) == 0x7f80u || (u & 0x7f800000u) == 0x7f800000u;
+      const T v = __ldg(src + static_cast<size_t>(c) * pitch + sm);
+      float2 x;
+      if constexpr (kFormat == KSJ_GPU_SAMPLES_BF16) {
+        bad |= (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u;
+        x = make_float2(bf16_to_float(static_cast<uint16_t>(v & 0xffffu)), bf16_to_float(static_cast<uint16_t>(v >> 16)));
       } else {
-        const uint64_t u = static_cast<uint64_t>(v);
-        bad |= (u & 0x7f800000ull) == 0x7f800000ull || (u & 0x7f80000000000000ull) == 0x7f80000000000000ull;
+        bad |= (v & 0x7f800000ull) == 0x7f800000ull || (v & 0x7f80000000000000ull) == 0x7f80000000000000ull;
+        x = make_float2(__uint_as_float(static_cast<uint32_t>(v)), __uint_as_float(static_cast<uint32_t>(v >> 32)));
       }
-      t[y][threadIdx.x] = v;
+      t[y][threadIdx.x] = cmul(x, scale);
     }
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0 && threadIdx.y == 0) {
-    atomicOr(flags, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
-    if (frame_flags) atomicOr(frame_flags + frame0 + f, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
+    atomicOr(a.flags, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
+    if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
   }
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const int sm = s0 + y, c = c0 + threadIdx.x;
-    if (c < channels && sm < samples) dst[static_cast<size_t>(sm) * channels + c] = t[threadIdx.x][y];
+#pragma unroll
+  for (int y = threadIdx.y; y < 32; y += 8) {
+    const int so = s0 + y, c = c0 + threadIdx.x;
+    if (c < channels && so < samples) dst[static_cast<size_t>(so) * channels + c] = t[threadIdx.x][y];
   }
 }
 
 struct RowsArgs {
   int frame0;             // first frame of this pass
-  const void* samples_t;  // [frame][sample][channel]
+  const float2* samples_t;     // [frame][sample][channel], weighted
   size_t sample_frame_stride;  // elements between frames of samples_t (0: one sample set for all frames)
   const uint32_t* offsets;
-  const float4* expanded;  // sorted list entries, expanded (meta_vecs(W) vectors each)
+  const unsigned char* expanded;  // sorted list entries (entry_bytes(width) each)
   const float2* tw_cols;
   const int* pos_cols;    // DIF output position of each kept column
   float2* inter;          // [frame][grid_row][out_col][cpitch]
   uint32_t* flags;
-  int frames, channels, samples, grid_rows, grid_cols, nchunks, lists_per_frame;
+  int frames, channels, samples, grid_rows, grid_cols, nchunks, lists_per_frame, width;
   size_t entries_per_frame;
   int coil_group, coil_parts;
   int out_cols, cpitch;
@@ -1097,77 +1087,13 @@ struct RowsArgs {
   DifPlan plan;
 };
 
-// Accumulator layout [column][coil]: gridding, the row FFT and the write-out
-// all put consecutive coils on consecutive lanes at one column, so every
-// shared-memory access of the block reads or writes contiguous float2s.
-struct AccAddr {
-  int cg;
-  __device__ __forceinline__ int operator()(int coil, int col) const { return col * cg + coil; }
-};
-
-// Register form of one column chunk (lane = coil): r[t] is the cell of column
-// col_lo + t.  A straight entry's taps are the columns cbase + j, so with the
-// warp-uniform d = cbase - col_lo every tap is a compile-time register index
-// (one switch case per d).  Taps at t < 0 or t >= kChunk belong to other
-// lists' chunks and are dropped; taps at width <= t < kChunk (a partial last
-// chunk) land in registers that are never stored.
-template <int W, int D, int J = 0>
-__device__ __forceinline__ void chunk_taps_at(float2 (&r)[kChunk], float2 v, const float* wt) {
-  if constexpr (J < W) {
-    if constexpr (D + J >= 0 && D + J < kChunk) {
-      r[D + J].x = fmaf(v.x, wt[J], r[D + J].x);
-      r[D + J].y = fmaf(v.y, wt[J], r[D + J].y);
-    }
-    chunk_taps_at<W, D, J + 1>(r, v, wt);
-  }
-}
-
-template <int W>
-__device__ __forceinline__ void chunk_taps(float2 (&r)[kChunk], int d, float2 v, const float* wt) {
-  static_assert(W <= 8 && kChunk == 16, "cases cover d in [-7, 15]");
-  switch (d) {
-#define KSJ_TAPS_CASE(D) \
-  case D:                \
-    chunk_taps_at<W, D>(r, v, wt); \
-    break;
-    KSJ_TAPS_CASE(-7) KSJ_TAPS_CASE(-6) KSJ_TAPS_CASE(-5) KSJ_TAPS_CASE(-4) KSJ_TAPS_CASE(-3) KSJ_TAPS_CASE(-2)
-    KSJ_TAPS_CASE(-1) KSJ_TAPS_CASE(0) KSJ_TAPS_CASE(1) KSJ_TAPS_CASE(2) KSJ_TAPS_CASE(3) KSJ_TAPS_CASE(4)
-    KSJ_TAPS_CASE(5) KSJ_TAPS_CASE(6) KSJ_TAPS_CASE(7) KSJ_TAPS_CASE(8) KSJ_TAPS_CASE(9) KSJ_TAPS_CASE(10)
-    KSJ_TAPS_CASE(11) KSJ_TAPS_CASE(12) KSJ_TAPS_CASE(13) KSJ_TAPS_CASE(14) KSJ_TAPS_CASE(15)
-#undef KSJ_TAPS_CASE
-    default:
-      break;
-  }
-}
-
-// Entries whose taps wrap around the grid inside one chunk (grids of at most
-// one chunk): the in-chunk taps of the mask, each at its wrapped column.
-template <int W>
-__device__ __forceinline__ void chunk_taps_wrapped(float2 (&r)[kChunk], int c0, uint32_t mask, int col_lo,
-                                                   int grid_cols, float2 v, const float* wt) {
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    if (!((mask >> j) & 1u)) continue;
-    int col = c0 + j;
-    if (col >= grid_cols) col -= grid_cols;
-    const int t = col - col_lo;
-#pragma unroll
-    for (int u = 0; u < kChunk; ++u) {
-      if (u == t) {
-        r[u].x = fmaf(v.x, wt[j], r[u].x);
-        r[u].y = fmaf(v.y, wt[j], r[u].y);
-      }
-    }
-  }
-}
-
 // Lists longer than kSegMin entries are gridded in segments (at most
-// kSegMax, all but the last of segment_length entries) that different warps
-// take at once, so that a row's long lists do not hold its CTA at the
+// kSegMax, all but the last of segment_length entries) that different lane
+// groups take at once, so that a row's long lists do not hold its CTA at the
 // barrier after the gridding while one warp works through each; a cell is then
 // the sum, in segment order, of its segments' partial sums, each partial sum
 // in sample order from zero.  Shorter lists are one segment: the cell is its
-// samples' sum in sample order.  Every row kernel uses the same segments.
+// samples' sum in sample order.  Every coil grouping uses the same segments.
 constexpr int kSegMin = 32;
 constexpr int kSegMax = 32;
 
@@ -1175,9 +1101,6 @@ __host__ __device__ inline int list_segments(int n) {
   return n <= kSegMin ? 1 : ((n + kSegMin - 1) / kSegMin < kSegMax ? (n + kSegMin - 1) / kSegMin : kSegMax);
 }
 static_assert(kSegMin * kSegMax <= (1 << 22), "segment counts are taken from lengths capped at 2^22");
-// First entry (absolute, within the frame's entries) of segment seg of a
-// list starting at `begin` with segments of sl entries.
-__host__ __device__ inline int seg_start(uint32_t begin, int seg, int sl) { return static_cast<int>(begin) + seg * sl; }
 
 __host__ __device__ inline int segment_length(int n) {
   if (n <= kSegMin) return n;  // one segment (most lists): no division
@@ -1185,83 +1108,62 @@ __host__ __device__ inline int segment_length(int n) {
   return (n + sg - 1) / sg;
 }
 
-// One column chunk's list entries (or one segment of them) gridded by a
-// warp, lane = coil: the chunk's 16 cells stay in registers, summed in entry
-// order from zero.  kWrap admits entries whose taps wrap around the grid
-// inside the chunk.  `meta` is the warp's staging buffer.
-//
-// have_sk: lane i's sk_first already holds the sample index of entry i (of
-// the first batch), loaded ahead by the caller; the first samples are then
-// requested before the batch's entries are staged, so the two loads overlap
-// instead of following each other.  Within the task, each batch loads the
-// next batch's sample indices the same way (one 4-byte load per lane, which
-// also brings the next batch's entries towards L1).
-template <int W, uint32_t kFormat, bool kWrap, int kAR>
-__device__ __forceinline__ void grid_entries_regs(float2 (&r)[kChunk], const RowsArgs& a, size_t sample_base,
-                                                  bool coil_ok, int lane, int col_lo, const float4* xent, int n,
-                                                  float4* meta, bool have_sk = false, uint32_t sk_first = 0u) {
-  constexpr int kMV = meta_vecs(W);
-  constexpr int kBatch = meta_batch(W);
-  const SampleRows<kFormat> sample_row(a.samples_t, sample_base, a.channels);
-#pragma unroll
-  for (int t = 0; t < kChunk; ++t) r[t] = make_float2(0.0f, 0.0f);
-  uint32_t sk_batch = sk_first;
-  bool sk_ready = have_sk;
-  for (int base = 0; base < n; base += kBatch) {
-    const int cnt = min(kBatch, n - base);
-    float2 yv[kAR];
-    const bool pre = sk_ready;
-    if (pre) {
-#pragma unroll
-      for (int k = 0; k < kAR; ++k) {
-        const uint32_t sk = __shfl_sync(0xffffffffu, sk_batch, k);
-        yv[k] = (coil_ok && k < cnt) ? sample_row(sk) : make_float2(0.0f, 0.0f);
-      }
+// Up to kRowsBatch entries of one list staged by their lane group (`lanes`
+// lanes, this one is `gl`): slot i gets entry i's weights spread over the
+// chunk's 16 columns, so that the lanes that apply them need no column
+// arithmetic and no branch per tap, and lane groups on different lists run in
+// step.  Slots from cnt on get no weights.  wrap: the grid's one chunk sees both
+// ends of a wrapped stencil (its length, else 0).  Returns this lane's share of the
+// halves its slots touch: bit 2 i the low, 2 i + 1 the high half of slot i.
+__device__ __forceinline__ uint32_t stage_entries(int w, float* slots, const unsigned char* ent, int cnt, int gl,
+                                                  int lanes, int wrap) {
+  uint32_t halves = 0;
+#pragma unroll 1
+  for (int i = gl; i < kRowsBatch; i += lanes) {
+    float* slot = slots + i * kSlotFloats;
+    float4* s4 = reinterpret_cast<float4*>(slot);
+    float2 h = make_float2(__int_as_float(-kMaxWidth), 0.0f), p0 = h, p1 = h;  // no tap, no sample
+    const float2* e = reinterpret_cast<const float2*>(ent + i * entry_bytes(w));
+    if (i < cnt) {
+      h = __ldg(e);
+      p0 = __ldg(e + 1);
+      if (w > 2) p1 = __ldg(e + 2);
     }
-    if (have_sk && base + kBatch < n) {
-      const int nb = base + kBatch;
-      sk_batch = lane < min(kBatch, n - nb) ? __float_as_uint(__ldg(&xent[static_cast<size_t>(nb + lane) * kMV].y)) : 0u;
-      sk_ready = true;
-    }
-    __syncwarp();  // the previous batch is read by every lane before it is replaced
-    if (lane < cnt) {
-      const float4* src = xent + static_cast<size_t>(base + lane) * kMV;
-      float4* m = meta + lane * kMV;
 #pragma unroll
-      for (int v = 0; v < kMV; ++v) m[v] = __ldg(src + v);
+    for (int q = 0; q < 4; ++q) s4[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    slot[kChunk] = h.y;
+    const int t0 = __float_as_int(h.x);
+    auto put = [&](int t, float v) {
+      if (wrap != 0 && t >= wrap) t -= wrap;
+      if (static_cast<uint32_t>(t) < kChunk) slot[t] = v;
+    };
+    put(t0, p0.x);
+    put(t0 + 1, p0.y);
+    if (w > 2) {
+      put(t0 + 2, p1.x);
+      put(t0 + 3, p1.y);
     }
-    __syncwarp();
-    auto fetch = [&](int i) { return sample_row(__float_as_uint(meta[i * kMV].y)); };
-    if (!pre) {
-#pragma unroll
-      for (int k = 0; k < kAR; ++k) yv[k] = (coil_ok && k < cnt) ? fetch(k) : make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (int j = 4; j < w; j += 2) {
+      const float2 p = i < cnt ? __ldg(e + 1 + j / 2) : make_float2(0.0f, 0.0f);
+      put(t0 + j, p.x);
+      put(t0 + j + 1, p.y);
     }
-    for (int i0 = 0; i0 < cnt; i0 += kAR) {
+    if (i < cnt) halves |= (wrap != 0 ? 3u : (t0 < 8 ? 1u : 0u) | (t0 + w > 8 ? 2u : 0u)) << (2 * i);
+  }
+  return halves;
+}
+
+// Eight columns of the chunk: the staged weights of one entry on its sample.
+template <int kFirst>
+__device__ __forceinline__ void half_taps(float2 (&r)[kChunk], const float* slot, float2 y) {
+  const float4 a = reinterpret_cast<const float4*>(slot)[kFirst / 4];
+  const float4 b = reinterpret_cast<const float4*>(slot)[kFirst / 4 + 1];
+  const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-      for (int k = 0; k < kAR; ++k) {
-        const int i = i0 + k;
-        if (i >= cnt) break;
-        const float2 y = yv[k];
-        yv[k] = (coil_ok && i + kAR < cnt) ? fetch(i + kAR) : make_float2(0.0f, 0.0f);
-        const float4 m0 = meta[i * kMV];
-        float wt[4 * (kMV - 1)];
-#pragma unroll
-        for (int v = 1; v < kMV; ++v) {
-          const float4 mv = meta[i * kMV + v];
-          wt[4 * (v - 1)] = mv.x;
-          wt[4 * (v - 1) + 1] = mv.y;
-          wt[4 * (v - 1) + 2] = mv.z;
-          wt[4 * (v - 1) + 3] = mv.w;
-        }
-        const int word0 = __float_as_int(m0.x);
-        const int cbase = word0 >> 9;  // arithmetic shift: may be negative
-        const float2 v = cmul(y, make_float2(m0.z, m0.w));
-        if (kWrap && (word0 & 256))
-          chunk_taps_wrapped<W>(r, cbase, static_cast<uint32_t>(word0) & 255u, col_lo, a.grid_cols, v, wt);
-        else
-          chunk_taps<W>(r, cbase - col_lo, v, wt);
-      }
-    }
+  for (int t = 0; t < 8; ++t) {
+    r[kFirst + t].x = fmaf(y.x, w[t], r[kFirst + t].x);
+    r[kFirst + t].y = fmaf(y.y, w[t], r[kFirst + t].y);
   }
 }
 
@@ -1269,25 +1171,23 @@ __device__ __forceinline__ void grid_entries_regs(float2 (&r)[kChunk], const Row
 // first cell of this lane's coil, cells `stride` apart).  A one-segment list
 // (counter null) stores them.  For a segmented list each lane works on its
 // own coil's cells alone: segment 0 stores, segment seg > 0 waits until the
-// list's counter shows all 32 lanes of segments 0 .. seg-1 in, then adds its
+// list's counter shows all `lanes` lanes of segments 0 .. seg-1 in, then adds its
 // partial sums; every lane then counts itself in.  Lanes wait on the counter
 // each for itself (no warp-wide sync), fenced on both sides.  The wait is
 // bounded: on a timeout the lane's partial sums are dropped, it still counts
 // itself in (the later segments do not wait out the limit as well) and
 // KSJ_GPU_FLAG_WAIT_TIMEOUT is raised.
-__device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst, int stride, int width, bool live,
-                                          int seg, int* counter, uint32_t* flags, uint32_t wait_limit,
+__device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst, int stride, int width, int seg,
+                                          int lanes, int* counter, uint32_t* flags, uint32_t wait_limit,
                                           int wait_beyond) {
   if (counter == nullptr) {
-    if (live) {
-      if (width == kChunk) {  // every chunk of the row but a partial last one
+    if (width == kChunk) {  // every chunk of the row but a partial last one
 #pragma unroll
-        for (int t = 0; t < kChunk; ++t) dst[t * stride] = r[t];
-      } else {
+      for (int t = 0; t < kChunk; ++t) dst[t * stride] = r[t];
+    } else {
 #pragma unroll
-        for (int t = 0; t < kChunk; ++t)
-          if (t < width) dst[t * stride] = r[t];
-      }
+      for (int t = 0; t < kChunk; ++t)
+        if (t < width) dst[t * stride] = r[t];
     }
     return;
   }
@@ -1295,7 +1195,7 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
   bool ok = true;
   if (seg > 0) {
     uint32_t polls = 0;
-    while (*reinterpret_cast<volatile int*>(counter) < 32 * seg + wait_beyond) {
+    while (*reinterpret_cast<volatile int*>(counter) < lanes * seg + wait_beyond) {
       if (++polls >= wait_limit) {
         ok = false;
         atomicOr(flags, KSJ_GPU_FLAG_WAIT_TIMEOUT);
@@ -1305,7 +1205,7 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
     }
     __threadfence_block();
   }
-  if (live && ok) {
+  if (ok) {
 #pragma unroll
     for (int t = 0; t < kChunk; ++t) {
       if (t < width) {
@@ -1322,133 +1222,65 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
   atomicAdd(counter, 1);
 }
 
-// The row's task table, built by warp 0: rank r is the r-th longest list
-// (chunk[r]), cut into list_segments(len) segments of segment_length(len)
-// entries; tasks base[r] .. base[r + 1] - 1 are its segments (times the coil
-// parts).
-struct RowTasks {
-  int* chunk;
-  int* base;      // nchunks + 1 entries
-  int* combined;  // per (chunk, part): lanes of finished segments
-  int* next;
-};
-
-// (rank, segment) of task q (parts folded out by the caller); a row without
-// segmented lists has task q = rank q.
-__device__ __forceinline__ void task_of(const RowTasks& t, int nchunks, int q, int lane, int* rank, int* seg) {
-  if (t.base[nchunks] == nchunks) {
-    *rank = q;
-    *seg = 0;
-    return;
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, lane < nchunks && t.base[lane] <= q);
-  *rank = __popc(m) - 1;
-  *seg = q - t.base[*rank];
-}
-
-// Gridding of one row by whole 32-coil warps (lane = coil): warps take the
-// row's tasks (list segments, longest lists first) from the shared counter.
-// Every chunk is at least one task, so every cell of the row is stored.
-template <int W, uint32_t kFormat, bool kWrap, int kAR>
-__device__ __forceinline__ void rows_grid_regs(const RowsArgs& a, int f, int cgi, int lane, float2* acc,
-                                               const uint32_t* offs, const RowTasks& tasks, float4* meta) {
-  constexpr int kMV = meta_vecs(W);
-  const int coil_global = cgi * 32 + lane;
-  const bool coil_ok = coil_global < a.channels;
-  const size_t sample_base = static_cast<size_t>(f) * a.sample_frame_stride + (coil_ok ? coil_global : 0);
-  const int ntasks = tasks.base[a.nchunks];
-  constexpr int kBatch = meta_batch(W);
-  // A warp claims one task at a time and loads its first sample indices
-  // before it grids it.  Tasks are claimed in increasing order, so the
-  // smallest unfinished task is always some warp's current one: a segment's
-  // wait for its predecessors always ends.  (Claiming the next task ahead,
-  // to hide that load behind the current task, measured slower: 1.34 vs 1.28
-  // ms on 96 radial frames, a claimed-ahead task waits behind its owner's
-  // current one while other warps idle.)
-  auto claim = [&]() {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(tasks.next, 1);
-    return __shfl_sync(0xffffffffu, q, 0);
-  };
-  struct Task {
-    int chunk, seg, n, e0, e1;
-  };
-  auto decode = [&](int q) {
-    Task t;
-    int rank;
-    task_of(tasks, a.nchunks, q, lane, &rank, &t.seg);
-    t.chunk = tasks.chunk[rank];
-    const uint32_t begin = offs[t.chunk];
-    t.n = static_cast<int>(offs[t.chunk + 1] - begin);
-    const int sl = segment_length(t.n);
-    t.e0 = seg_start(begin, t.seg, sl);
-    t.e1 = min(static_cast<int>(begin) + t.n, t.e0 + sl);
-    return t;
-  };
-  auto entries_of = [&](const Task& t) {
-    return a.expanded + (static_cast<size_t>(f) * a.entries_per_frame + static_cast<size_t>(t.e0)) * meta_vecs(W);
-  };
-  auto first_sk = [&](const Task& t) {
-    return lane < min(kBatch, t.e1 - t.e0) ? __float_as_uint(__ldg(&entries_of(t)[static_cast<size_t>(lane) * kMV].y))
-                                           : 0u;
-  };
-  for (;;) {
-    const int q = claim();
-    if (q >= ntasks) break;
-    const Task cur = decode(q);
-    float2 r[kChunk];
-    grid_entries_regs<W, kFormat, kWrap, kAR>(r, a, sample_base, coil_ok, lane, cur.chunk * kChunk, entries_of(cur),
-                                              cur.e1 - cur.e0, meta, true, first_sk(cur));
-    put_chunk(r, acc + static_cast<size_t>(cur.chunk * kChunk) * 32 + lane, 32,
-              min(kChunk, a.grid_cols - cur.chunk * kChunk), true, cur.seg,
-              list_segments(cur.n) > 1 ? tasks.combined + cur.chunk : nullptr, a.flags, a.wait_limit, a.wait_beyond);
-  }
-}
-
-// kBlocks CTAs per SM: 2 for rows of up to 384 columns (384 threads), 1
-// above; two resident CTAs let one block's FFT overlap another's gridding.
-// kCG = 32 fixes a 32-coil group taken whole by one warp (coil_parts 1):
-// lane = coil, no tap groups, every tap offset a constant; kCG = 0 reads the
-// group and the split from the arguments.
+// One CTA per (frame, grid row, coil group): the row's cells gridded into
+// shared memory [column][coil], then the row's inverse transform and the kept
+// columns written coil-last.
+//
+// Gridding.  A task is one segment of one list (times the coil parts); a lane
+// group (lane = coil, `lanes` of them) grids a task into registers, the 16
+// cells of its chunk, and a warp takes as many tasks at once as it has lane
+// groups, longest first, from a shared counter.  The groups of a warp run in step
+// on different lists (neighbours in length), because a staged entry's weights
+// are spread over the whole chunk: the same 8 or 16 multiply-adds whatever the
+// columns, where a tap switch would send every group its own way.  Tasks are
+// claimed in increasing order and a warp's groups are put in that order, so the
+// smallest unfinished segment is always some warp's current one: a segment's
+// wait for its predecessors always ends.
+//
+// Bound by issue slots (32 coils: two thirds of the cycles issue) and, for few
+// rows, by the longest row.  A call, before (a switch on the tap column for 32 coils, cells in
+// shared memory below) -> now: 96 frames x 384 rows x 32 coils 2597 -> 2488 us, one
+// such frame 141 -> 119, 8 coils on a 512 grid 585 -> 330, on a 128 grid 210 -> 115,
+// 11 coils, width 6, on a 300 grid 670 -> 385, 20 coils in 3-D 57.9 -> 46.7 ms.
+//
+// kN: the row length for the two-step transform (128 .. 512), or 0 for the
+// in-place mixed-radix form of any other length; one instance per length keeps
+// each kernel's code small.  kLgL (when nonzero) fixes log2 of the coil group.
 // kHalf: the sigma = 2 crop form of the row transform (out_cols =
 // grid_cols / 2, col_shift = out_cols / 2), whose kept columns are known at
 // compile time (fft_two_step_half); the same bytes as the general form.
-template <int W, uint32_t kFormat, int kThreads, int kBlocks, int kCG, bool kHalf = false>
-__global__ void __launch_bounds__(kThreads, kBlocks) k_rows(RowsArgs a) {
+template <int kN, int kLgL, bool kHalf>
+__global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int row = blockIdx.x;
   const int cgi = blockIdx.y;
   const int f = a.frame0 + blockIdx.z;
-  const int cg = kCG ? kCG : a.coil_group;
+  const int cg = kLgL ? (1 << kLgL) : a.coil_group;
   const int tid = threadIdx.x;
   const int nthreads = blockDim.x;
   const int lane = tid & 31;
+  const int warp = tid >> 5;
   float2* acc = reinterpret_cast<float2*>(smem_raw);
   float2* tw = acc + static_cast<size_t>(a.grid_cols) * cg;
-  uint32_t* offs = reinterpret_cast<uint32_t*>(tw + a.grid_cols);  // this row's list offsets
-  constexpr int kMV = meta_vecs(W);
-  constexpr int kBatch = meta_batch(W);
-  const int warp = tid >> 5;
   // offsets from the shared array itself keep every access a shared-memory one
-  const size_t meta_off = (static_cast<size_t>(a.grid_cols) * (cg + 1) * sizeof(float2) +
-                           static_cast<size_t>(a.nchunks + 1) * sizeof(uint32_t) + 15) & ~static_cast<size_t>(15);
-  float4* meta = reinterpret_cast<float4*>(smem_raw + meta_off) + warp * kBatch * kMV;
-  const AccAddr addr{cg};
+  const size_t slot_off = (static_cast<size_t>(a.grid_cols) * (cg + 1) * sizeof(float2) + 15) & ~static_cast<size_t>(15);
 
   const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1) + row * a.nchunks;
-  for (int i = tid; i <= a.nchunks; i += nthreads) offs[i] = __ldg(off + i);
-  // task order: the row's lists longest first (a bitonic sort across warp 0,
-  // one key per lane: length << 8 | chunk), each cut into its segments, taken
-  // from a shared counter
-  __shared__ int task_chunk[kMaxGrid / kChunk];
+  // the row's task table: rank r is the r-th longest list (a bitonic sort
+  // across warp 0, one key per lane: length << 8 | chunk), cut into
+  // list_segments(len) segments; tasks task_base[r] .. task_base[r + 1] - 1
+  // are its segments
+  __shared__ int4 task_list[kMaxGrid / kChunk];  // per rank: first entry, length, segment length, chunk
   __shared__ int task_base[kMaxGrid / kChunk + 1];
-  __shared__ int task_combined[2 * (kMaxGrid / kChunk)];
+  __shared__ int task_combined[2 * (kMaxGrid / kChunk)];  // per (part, chunk): lanes of finished segments
   __shared__ int task_next;
   if (warp == 0) {
     int key = -1;
+    uint32_t start = 0, length = 0;
     if (lane < a.nchunks) {
-      const uint32_t len = min(__ldg(off + lane + 1) - __ldg(off + lane), 1u << 22);
-      key = static_cast<int>(len << 8) | lane;
+      start = __ldg(off + lane);
+      length = __ldg(off + lane + 1) - start;
+      key = static_cast<int>(min(length, 1u << 22) << 8) | lane;
     }
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1) {
@@ -1471,200 +1303,123 @@ __global__ void __launch_bounds__(kThreads, kBlocks) k_rows(RowsArgs a) {
       const int v = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += v;
     }
+    const int chunk = key & 31;
+    start = __shfl_sync(0xffffffffu, start, chunk);
+    length = __shfl_sync(0xffffffffu, length, chunk);
     if (lane < a.nchunks) {
-      task_chunk[lane] = key & 255;
+      const int n = static_cast<int>(length);
+      task_list[lane] = make_int4(static_cast<int>(start), n, segment_length(n), chunk);
       task_base[lane] = incl - nseg;
     }
     if (lane == a.nchunks - 1) task_base[a.nchunks] = incl;
     if (lane == 0) task_next = 0;
   }
   for (int i = tid; i < 2 * (kMaxGrid / kChunk); i += nthreads) task_combined[i] = 0;
-  const RowTasks tasks{task_chunk, task_base, task_combined, &task_next};
-  // (the 32-coil path stores every cell of the row from registers)
-  if (kCG != 32)
-    for (int i = tid; i < a.grid_cols * cg; i += nthreads) acc[i] = make_float2(0.0f, 0.0f);
   for (int i = tid; i < a.grid_cols; i += nthreads) tw[i] = a.tw_cols[i];
   __syncthreads();
 
-  if constexpr (kCG == 32) {
-    constexpr int kAR = kAheadRegs;  // a deeper prefetch measured slower in both instances (code size)
-    // taps wrap around the grid inside one chunk only on grids narrower than
-    // kChunk + W - 1 columns; the loop for those keeps a per-tap form
-    if (a.grid_cols < kChunk + W - 1)
-      rows_grid_regs<W, kFormat, true, kAR>(a, f, cgi, lane, acc, offs, tasks, meta);
-    else
-      rows_grid_regs<W, kFormat, false, kAR>(a, f, cgi, lane, acc, offs, tasks, meta);
-  } else {
-  // ---- gridding.  A task is (column chunk, coil part): the chunk's sorted
-  // list applied to a subset of the coil group.  Cells of different coils are
-  // independent, so parts of one list may run on different warps with every
-  // cell still summed in sample order.  Warps take tasks round-robin.
-  //
-  // Per batch of list entries, lane i loads entry i's sample index and record
-  // (vector loads), folds the row weight into the W column weights and stages
-  // them in the warp's shared batch; then the warp walks the batch in order
-  // with the coil loads of the next kAhead samples always in flight.
-  // A list longer than kSegMin entries is gridded in segments like the
-  // 32-coil path's (lane = coil of the part, cells in registers, segments
-  // combined in order), so that every coil grouping gives the same cells.
-  const int parts = kCG ? 1 : a.coil_parts;
-  const int cpart = cg / parts;
-  const int ntasks = tasks.base[a.nchunks] * parts;
   {
-    // lanes: coil = lane % cpp, tap group = lane / cpp
-    int cpp = 1;
-    while (cpp < cpart) cpp <<= 1;
-    const int ngroups = 32 / cpp;
-    // taps j this lane applies: j mod ngroups equal to its tap group
-    uint32_t my_taps = 0;
-#pragma unroll
-    for (int j = 0; j < W; ++j)
-      if ((j & (ngroups - 1)) == lane / cpp) my_taps |= 1u << j;
-    const void* ks = a.samples_t;
+    const int lg_parts = a.coil_parts - 1;  // coil_parts is 1 or 2
+    const int lanes = cg >> lg_parts, groups = 32 / lanes;
+    const int g = lane / lanes, gl = lane - g * lanes;
+    float* slots = reinterpret_cast<float*>(smem_raw + slot_off) +
+                   static_cast<size_t>(warp * groups + g) * kRowsBatch * kSlotFloats;
+    const int ntasks = task_base[a.nchunks] << lg_parts;
+    const bool segmented_row = task_base[a.nchunks] != a.nchunks;
+    const int wrap = a.nchunks == 1 ? a.grid_cols : 0;
+    const float2* samples = a.samples_t + static_cast<size_t>(f) * a.sample_frame_stride;
+    const unsigned char* ents = a.expanded + static_cast<size_t>(f) * a.entries_per_frame * entry_bytes(a.width);
     for (;;) {
-      int task = 0;
-      if (lane == 0) task = atomicAdd(&task_next, 1);
-      task = __shfl_sync(0xffffffffu, task, 0);
-      if (task >= ntasks) break;
-      const int q = task / parts;
-      const int part = task - q * parts;
-      int rank, seg;
-      task_of(tasks, a.nchunks, q, lane, &rank, &seg);
-      const int chunk = task_chunk[rank];
-      const uint32_t begin = offs[chunk];
-      const int n = static_cast<int>(offs[chunk + 1] - begin);
-      const float4* xent = a.expanded + (static_cast<size_t>(f) * a.entries_per_frame + begin) * kMV;
-      const int col_lo = chunk * kChunk;
-      if (list_segments(n) > 1) {
-        const int sl = segment_length(n);
-        const int e0 = seg * sl, e1 = min(n, e0 + sl);
-        const bool lane_coil = lane < cpart;
-        const int rc = part * cpart + (lane_coil ? lane : 0);
-        const int rg = cgi * cg + rc;
-        const bool rok = lane_coil && rg < a.channels;
-        const size_t rbase = static_cast<size_t>(f) * a.sample_frame_stride + (rok ? rg : 0);
-        float2 r[kChunk];
-        grid_entries_regs<W, kFormat, true, kAheadRegs>(r, a, rbase, rok, lane, col_lo,
-                                                        xent + static_cast<size_t>(e0) * kMV, e1 - e0, meta);
-        put_chunk(r, acc + addr(rc, col_lo), cg, min(kChunk, a.grid_cols - col_lo), lane_coil, seg,
-                  tasks.combined + part * a.nchunks + chunk, a.flags, a.wait_limit, a.wait_beyond);
-        continue;
+      int q = 0;
+      if (lane == 0) q = atomicAdd(&task_next, groups);
+      q = __shfl_sync(0xffffffffu, q, 0);
+      if (q >= ntasks) break;
+      q += g;
+      const bool live = q < ntasks;
+      const int part = q & lg_parts;
+      q >>= lg_parts;
+      // (rank, segment) of the task; a row without segmented lists has task q = rank q
+      int rank = live ? q : 0, seg = 0;
+      if (segmented_row) {
+        rank = 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+          if (rank + d < a.nchunks && task_base[rank + d] <= q) rank += d;
+        seg = q - task_base[rank];
       }
-      const int col_hi = min(col_lo + kChunk, a.grid_cols);
-      const int my_coil = part * cpart + lane % cpp;  // coil index within the group
-      const int coil_global = cgi * cg + my_coil;
-      const bool coil_ok = (lane % cpp) < cpart && coil_global < a.channels;
-      const size_t sample_base = static_cast<size_t>(f) * a.sample_frame_stride + (coil_ok ? coil_global : 0);
-      for (int base = 0; base < n; base += kBatch) {
-        const int cnt = min(kBatch, n - base);
+      const int4 list = task_list[rank];
+      const int chunk = list.w;
+      const int first = seg * list.z;
+      const int cnt = live ? max(0, min(list.y - first, list.z)) : 0;
+      const unsigned char* ent = ents + (static_cast<size_t>(static_cast<uint32_t>(list.x)) + first) * entry_bytes(a.width);
+      const int coil = part * lanes + gl;
+      // (lanes past the channels read the first coil: their lines are not kept)
+      const SampleRows<KSJ_GPU_SAMPLES_CF32> sample_row(
+          samples, cgi * cg + coil < a.channels ? cgi * cg + coil : 0, a.channels);
+      float2 r[kChunk];
+#pragma unroll
+      for (int t = 0; t < kChunk; ++t) r[t] = make_float2(0.0f, 0.0f);
+      const int most = __reduce_max_sync(0xffffffffu, cnt);
+      for (int base = 0; base < most; base += kRowsBatch) {
         __syncwarp();  // the previous batch is read by every lane before it is replaced
-        if (lane < cnt) {
-          const float4* src = xent + static_cast<size_t>(base + lane) * kMV;
-          float4* m = meta + lane * kMV;
-#pragma unroll
-          for (int v = 0; v < kMV; ++v) m[v] = __ldg(src + v);
-        }
+        const uint32_t halves = __reduce_or_sync(
+            0xffffffffu, stage_entries(a.width, slots, ent + base * entry_bytes(a.width), cnt - base, gl, lanes, wrap));
         __syncwarp();
-        auto fetch = [&](int i) {
-          const uint32_t sk = __float_as_uint(meta[i * kMV].y);
-          return load_sample<kFormat>(ks, sample_base + static_cast<size_t>(sk) * a.channels);
-        };
-        float2 yv[kAhead];
+        // every sample of the batch is requested before the first is used
+        float2 y[kRowsBatch];
 #pragma unroll
-        for (int k = 0; k < kAhead; ++k) yv[k] = (coil_ok && k < cnt) ? fetch(k) : make_float2(0.0f, 0.0f);
-        for (int i0 = 0; i0 < cnt; i0 += kAhead) {
+        for (int i = 0; i < kRowsBatch; ++i) {
+          y[i] = make_float2(0.0f, 0.0f);
+          if (base + i < cnt)
+            y[i] = sample_row(reinterpret_cast<const uint32_t*>(slots + i * kSlotFloats)[kChunk]);
+        }
 #pragma unroll
-          for (int k = 0; k < kAhead; ++k) {
-            const int i = i0 + k;
-            if (i >= cnt) break;
-            const float2 y = yv[k];
-            yv[k] = (coil_ok && i + kAhead < cnt) ? fetch(i + kAhead) : make_float2(0.0f, 0.0f);
-            const float4 m0 = meta[i * kMV];
-            float wt[4 * (kMV - 1)];
-#pragma unroll
-            for (int v = 1; v < kMV; ++v) {
-              const float4 mv = meta[i * kMV + v];
-              wt[4 * (v - 1)] = mv.x;
-              wt[4 * (v - 1) + 1] = mv.y;
-              wt[4 * (v - 1) + 2] = mv.z;
-              wt[4 * (v - 1) + 3] = mv.w;
-            }
-            const int word0 = __float_as_int(m0.x);
-            const int cbase = word0 >> 9;  // arithmetic shift: may be negative
-            const uint32_t mask = static_cast<uint32_t>(word0) & my_taps;
-            if (coil_ok) {
-              const float2 v = cmul(y, make_float2(m0.z, m0.w));
-              if (!(word0 & 256)) {
-                // taps j of the mask are the consecutive cells cbase + j
-                const int base = addr(my_coil, cbase);
-#pragma unroll
-                for (int j = 0; j < W; ++j) {
-                  if (!((mask >> j) & 1u)) continue;
-                  float2* cell = acc + (base + j * cg);
-                  float2 c = *cell;
-                  c.x = fmaf(v.x, wt[j], c.x);
-                  c.y = fmaf(v.y, wt[j], c.y);
-                  *cell = c;
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < W; ++j) {
-                  if (!((mask >> j) & 1u)) continue;
-                  int col = cbase + j;
-                  if (col >= a.grid_cols) col -= a.grid_cols;
-                  float2* cell = acc + addr(my_coil, col);
-                  float2 c = *cell;
-                  c.x = fmaf(v.x, wt[j], c.x);
-                  c.y = fmaf(v.y, wt[j], c.y);
-                  *cell = c;
-                }
-              }
-            }
-            // tap groups of one lane set may meet in a cell across samples
-            if (ngroups > 1) __syncwarp();
-          }
+        for (int i = 0; i < kRowsBatch; ++i) {
+          if (halves & (1u << (2 * i))) half_taps<0>(r, slots + i * kSlotFloats, y[i]);
+          if (halves & (2u << (2 * i))) half_taps<8>(r, slots + i * kSlotFloats, y[i]);
+        }
+      }
+      float2* dst = acc + chunk * kChunk * cg + coil;
+      const int width = min(kChunk, a.grid_cols - chunk * kChunk);
+      const bool segmented = live && list.z < list.y;
+      if (!__any_sync(0xffffffffu, segmented)) {
+        if (live) put_chunk(r, dst, cg, width, 0, lanes, nullptr, a.flags, a.wait_limit, a.wait_beyond);
+      } else {
+        // in task order: a group may wait for the segment of an earlier one
+        for (int k = 0; k < groups; ++k) {
+          if (k == g && live)
+            put_chunk(r, dst, cg, width, seg, lanes, segmented ? task_combined + part * a.nchunks + chunk : nullptr,
+                      a.flags, a.wait_limit, a.wait_beyond);
+          __syncwarp();
         }
       }
     }
-  }
   }
   __syncthreads();
 
   // ---- row inverse FFT of every coil line; the kept columns are written
   // coil-last: [frame][grid_row][out_col][channel]
-  const int lg_cg = ilog2(cg);
+  const int lg_cg = kLgL ? kLgL : ilog2(cg);
   float2* dst_row = a.inter + (static_cast<size_t>(f) * a.grid_rows + row) * a.out_cols * a.cpitch + cgi * cg;
   const int live_lines = min(cg, a.channels - cgi * cg);
-  auto emit = [&](int k, int line, float2 v) {
-    int pc = k + a.col_shift;
-    if (pc >= a.grid_cols) pc -= a.grid_cols;
-    if (pc < a.out_cols && line < live_lines) dst_row[static_cast<size_t>(pc) * a.cpitch + line] = v;
-  };
-  if constexpr (kHalf) {
-    auto live = [&](int line) { return line < live_lines; };
-    auto emit_half = [&](int pc, int, int line, float2 v) { dst_row[static_cast<size_t>(pc) * a.cpitch + line] = v; };
-    switch (a.grid_cols) {
-      case 128: fft_two_step_half<16, 8>(acc, lg_cg, tw, tid, nthreads, live, emit_half); return;
-      case 192: fft_two_step_half<16, 12>(acc, lg_cg, tw, tid, nthreads, live, emit_half); return;
-      case 256: fft_two_step_half<16, 16>(acc, lg_cg, tw, tid, nthreads, live, emit_half); return;
-      case 384: fft_two_step_half<16, 24>(acc, lg_cg, tw, tid, nthreads, live, emit_half); return;
-      default:
-        if constexpr (kThreads >= 512) {
-          fft_two_step_half<16, 32>(acc, lg_cg, tw, tid, nthreads, live, emit_half);
-          return;
-        }
-        break;
+  if constexpr (kN != 0 && kHalf) {
+    fft_two_step_half<16, kN / 16>(
+        acc, lg_cg, tw, tid, nthreads, [&](int line) { return line < live_lines; },
+        [&](int pc, int, int line, float2 v) { dst_row[static_cast<size_t>(pc) * a.cpitch + line] = v; });
+  } else if constexpr (kN != 0) {
+    fft_two_step<16, kN / 16>(acc, lg_cg, tw, tid, nthreads, [&](int k, int line, float2 v) {
+      int pc = k + a.col_shift;
+      if (pc >= a.grid_cols) pc -= a.grid_cols;
+      if (pc < a.out_cols && line < live_lines) dst_row[static_cast<size_t>(pc) * a.cpitch + line] = v;
+    });
+  } else {
+    // other lengths: in place (output digit-reversed), then the kept columns
+    dif_lines(acc, lg_cg, a.plan, tw, tid, nthreads);
+    const int coil = tid & (cg - 1);
+    if (coil < live_lines) {
+      for (int pc = tid >> lg_cg; pc < a.out_cols; pc += nthreads >> lg_cg)
+        dst_row[static_cast<size_t>(pc) * a.cpitch + coil] = acc[(__ldg(a.pos_cols + pc) << lg_cg) + coil];
     }
-  }
-  // (blocks of kThreads threads take rows of up to kThreads columns)
-  if (fft_two_step_rows<kThreads>(a.grid_cols, acc, lg_cg, tw, tid, nthreads, emit)) return;
-
-  // other lengths: in place (output digit-reversed), then the kept columns
-  dif_lines(acc, lg_cg, a.plan, tw, tid, nthreads);
-  const int coil = tid & (cg - 1);
-  if (coil < live_lines) {
-    for (int pc = tid >> lg_cg; pc < a.out_cols; pc += nthreads >> lg_cg)
-      dst_row[static_cast<size_t>(pc) * a.cpitch + coil] = acc[(__ldg(a.pos_cols + pc) << lg_cg) + coil];
   }
 }
 
@@ -2033,26 +1788,40 @@ __global__ void __launch_bounds__(RingCfg<kN>::kThreads, RingCfg<kN>::kBlocks)
 
 // ------------------------------------------------------------------ driver
 
-// The row-pass kernel a shape selects (rows_blocks: k_rows with that many
-// CTAs per SM), its launch setup and launch.
+using RowsKernel = void (*)(RowsArgs);
+
+template <int kN>
+RowsKernel rows_kernel_two_step(int cg, bool half) {
+  switch (cg) {
+    case 32: return half ? k_rows<kN, 5, true> : k_rows<kN, 5, false>;
+    case 16: return half ? k_rows<kN, 4, true> : k_rows<kN, 4, false>;
+    case 8: return half ? k_rows<kN, 3, true> : k_rows<kN, 3, false>;
+    default: return half ? k_rows<kN, 0, true> : k_rows<kN, 0, false>;
+  }
+}
+
+RowsKernel rows_kernel_for(int n, int cg, bool half) {
+  switch (n) {
+    case 128: return rows_kernel_two_step<128>(cg, half);
+    case 192: return rows_kernel_two_step<192>(cg, half);
+    case 256: return rows_kernel_two_step<256>(cg, half);
+    case 384: return rows_kernel_two_step<384>(cg, half);
+    case 512: return rows_kernel_two_step<512>(cg, half);
+    default: return k_rows<0, 0, false>;
+  }
+}
+
+// The row-pass kernel a shape selects, its launch setup and launch.
 struct RowsLauncher {
-  void (*kernel)(RowsArgs) = nullptr;
+  RowsKernel kernel = nullptr;
   int threads = 0;
   size_t smem = 0;
 
-  template <int W, uint32_t kFormat>
   bool setup(const Shape& s) {
-    smem = rows_smem_for(s.grid_cols, s.coil_group, s.width, rows_threads_for(s.grid_cols));
-    threads = rows_threads_for(s.grid_cols);
-    const bool whole32 = s.coil_group == 32 && s.coil_parts == 1;
-    // the sigma = 2 crop form for the 32-coil register path
-    const bool half = whole32 && s.kb && s.out_cols * 2 == s.grid_cols && has_two_step_rows(s.grid_cols);
-    if (threads <= 384 && s.rows_blocks == 2)
-      kernel = half ? k_rows<W, kFormat, 384, 2, 32, true>
-                    : (whole32 ? k_rows<W, kFormat, 384, 2, 32> : k_rows<W, kFormat, 384, 2, 0>);
-    else
-      kernel = half ? k_rows<W, kFormat, kMaxThreads, 1, 32, true>
-                    : (whole32 ? k_rows<W, kFormat, kMaxThreads, 1, 32> : k_rows<W, kFormat, kMaxThreads, 1, 0>);
+    const int lanes = s.coil_group / s.coil_parts;
+    threads = rows_threads_for(s.grid_cols, lanes, s.coil_group);
+    smem = rows_smem_for(s.grid_cols, s.coil_group, lanes, threads);
+    kernel = rows_kernel_for(s.grid_cols, s.coil_group, s.kb && s.out_cols * 2 == s.grid_cols);
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
                cudaSuccess &&
            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
@@ -2216,7 +1985,7 @@ struct ColsPass {
 template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
-                           uint32_t* offsets, uint32_t* entries, float4* expanded, uint32_t* long_lists,
+                           uint32_t* offsets, uint32_t* entries, unsigned char* expanded, uint32_t* long_lists,
                            uint32_t* mid_lists, cudaStream_t stream, uint32_t* frame_flags = nullptr) {
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
   if (cudaMemsetAsync(counts, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
@@ -2333,29 +2102,27 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   }
   {
     const ksj_gpu_status st = build_lists<W>(s, d, d_traj, d_dcf, flags, records, counts, cursor, offsets, entries,
-                                             reinterpret_cast<float4*>(ws + l.expanded),
+                                             ws + l.expanded,
                                              reinterpret_cast<uint32_t*>(ws + l.long_lists),
                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream,
                                              reinterpret_cast<uint32_t*>(ws + l.frame_flags));
     if (st != KSJ_GPU_OK) return st;
   }
-  const size_t frame_samples = static_cast<size_t>(s.samples) * s.channels;  // elements per frame
   auto to_coil_last = [&](int f0, int nf, cudaStream_t st) {
-    const size_t eb = sample_bytes(d->sample_format);
     const dim3 tg((s.samples + 31) / 32, (s.channels + 31) / 32, nf);
     LaunchScope scope("k_samples_coil_last", st);
-    const unsigned char* in = s.frame_kspace ? nullptr : static_cast<const unsigned char*>(d_kspace) + f0 * frame_samples * eb;
-    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, st>>>(
-        in, ws + l.samples_t + f0 * frame_samples * eb,
-        s.channels, s.samples, flags, s.frame_channels, s.frame_samples, s.frame_kspace, f0,
-        reinterpret_cast<uint32_t*>(ws + l.frame_flags));
+    const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t), records + offsetof(SampleRecord<W>, scale),
+                         static_cast<int>(sizeof(SampleRecord<W>)), s.channels, s.samples, flags, s.frame_channels,
+                         s.frame_samples, s.frame_kspace, f0, reinterpret_cast<uint32_t*>(ws + l.frame_flags)};
+    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, st>>>(a);
   };
   if (io == nullptr || io->copy == nullptr) to_coil_last(0, s.frames, stream);
   RowsArgs r{};
-  r.samples_t = ws + l.samples_t;
+  r.samples_t = reinterpret_cast<const float2*>(ws + l.samples_t);
   r.sample_frame_stride = static_cast<size_t>(s.samples) * s.channels;
   r.offsets = offsets;
-  r.expanded = reinterpret_cast<const float4*>(ws + l.expanded);
+  r.expanded = ws + l.expanded;
+  r.width = s.width;
   r.tw_cols = tw_cols;
   r.pos_cols = pos_cols;
   r.inter = inter;
@@ -2377,7 +2144,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   r.plan = s.plan_cols;
   r.col_shift = s.kb ? s.out_cols / 2 : 0;
   RowsLauncher rows_launch;
-  if (!rows_launch.setup<W, kFormat>(s)) return KSJ_GPU_ERROR_CUDA;
+  if (!rows_launch.setup(s)) return KSJ_GPU_ERROR_CUDA;
 
   ColsArgs c{};
   c.tw_rows = tw_rows;
@@ -2863,7 +2630,7 @@ size_t record3_bytes(int width) {
 }
 
 // s: the 2-D shape of one plane with frames = planes (see make_shape3).
-Layout3 make_layout3(const Shape& s, uint32_t sample_format) {
+Layout3 make_layout3(const Shape& s) {
   Layout3 l{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -2881,10 +2648,10 @@ Layout3 make_layout3(const Shape& s, uint32_t sample_format) {
   l.offsets = take((nl + g) * 4);
   l.bases = take(g * 4);
   l.entries = take(l.entries_total * 4);
-  l.expanded = take(l.entries_total * meta_vecs(s.width) * 16);
+  l.expanded = take(l.entries_total * entry_bytes(s.width));
   l.long_lists = take((2 + l.entries_total / (s.list_capacity + 1)) * 4);
   l.mid_lists = take((2 + l.entries_total / 33) * 4);
-  l.samples_t = take(static_cast<size_t>(s.samples) * s.channels * sample_bytes(sample_format));
+  l.samples_t = take(static_cast<size_t>(s.samples) * s.channels * sizeof(float2));
   l.inter = take(g * g * n * s.cpitch * sizeof(float2));
   l.inter2 = take(g * n * n * s.cpitch * sizeof(float2));
   // twiddles (rows, cols), deapodisation (rows, cols), DIF positions (rows, cols), ones for the pixel axis
@@ -2924,7 +2691,7 @@ ksj_gpu_status make_shape3(const ksj_gpu_gridding3_desc* d, const ksj_gpu_griddi
 template <int W>
 ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_traj, const float* d_dcf,
                             uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
-                            uint32_t* offsets, uint32_t* bases, uint32_t* entries, float4* expanded,
+                            uint32_t* offsets, uint32_t* bases, uint32_t* entries, unsigned char* expanded,
                             uint32_t* long_lists, uint32_t* mid_lists, cudaStream_t stream) {
   const int g = s.grid_rows;
   const size_t nl = static_cast<size_t>(g) * s.lists_per_frame;
@@ -3025,7 +2792,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   {
     const ksj_gpu_status st = build_lists3<W>(s, d->dcf_mode, d_traj, d_dcf, flags, ws + l.records, counts, cursor,
                                               offsets, reinterpret_cast<uint32_t*>(ws + l.bases), entries,
-                                              reinterpret_cast<float4*>(ws + l.expanded),
+                                              ws + l.expanded,
                                               reinterpret_cast<uint32_t*>(ws + l.long_lists),
                                               reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream);
     if (st != KSJ_GPU_OK) return st;
@@ -3033,15 +2800,18 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   {
     const dim3 tg((s.samples + 31) / 32, (s.channels + 31) / 32, 1);
     LaunchScope scope("k_samples_coil_last", stream);
-    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, stream>>>(d_kspace, ws + l.samples_t, s.channels, s.samples,
-                                                                 flags, nullptr, nullptr, nullptr, 0, nullptr);
+    const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t),
+                         ws + l.records + offsetof(SampleRecord3<W>, scale), static_cast<int>(sizeof(SampleRecord3<W>)),
+                         s.channels, s.samples, flags, nullptr, nullptr, nullptr, 0, nullptr};
+    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, stream>>>(a);
   }
   // rows of every plane (x transformed, kept columns, coil-last)
   RowsArgs r{};
-  r.samples_t = ws + l.samples_t;
+  r.samples_t = reinterpret_cast<const float2*>(ws + l.samples_t);
   r.sample_frame_stride = 0;
   r.offsets = offsets;
-  r.expanded = reinterpret_cast<const float4*>(ws + l.expanded);
+  r.expanded = ws + l.expanded;
+  r.width = s.width;
   r.tw_cols = tw_cols;
   r.pos_cols = pos_cols;
   r.inter = inter;
@@ -3063,7 +2833,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   r.plan = s.plan_cols;
   r.col_shift = n / 2;
   RowsLauncher rows_launch;
-  if (!rows_launch.setup<W, kFormat>(s)) return KSJ_GPU_ERROR_CUDA;
+  if (!rows_launch.setup(s)) return KSJ_GPU_ERROR_CUDA;
   // columns of every plane (y transformed, cropped, y/x deapodised): [plane][pixel][cpitch]
   ColsArgs c{};
   c.tw_rows = tw_rows;
@@ -3982,11 +3752,11 @@ extern "C" ksj_gpu_status ksj_gpu_gridding_binning(const ksj_gpu_gridding_desc* 
     const uint32_t* fo = off.data() + static_cast<size_t>(f) * (s.lists_per_frame + 1);
     for (int i = 0; i < s.lists_per_frame; ++i)
       out_offsets[static_cast<size_t>(f) * s.lists_per_frame + i] = base + fo[i];
-    // the sample index of every expanded entry (second word of its first vector)
+    // the sample index of every expanded entry (its second word)
     const uint32_t n = fo[s.lists_per_frame];
-    const size_t entry_bytes = static_cast<size_t>(meta_vecs(s.width)) * 16;
-    if (n && cudaMemcpy2D(out_samples + base, 4, ws + l.expanded + static_cast<size_t>(f) * s.entries_per_frame * entry_bytes + 4,
-                          entry_bytes, 4, n, cudaMemcpyDeviceToHost) != cudaSuccess)
+    const size_t pitch = entry_bytes(s.width);
+    if (n && cudaMemcpy2D(out_samples + base, 4, ws + l.expanded + static_cast<size_t>(f) * s.entries_per_frame * pitch + 4,
+                          pitch, 4, n, cudaMemcpyDeviceToHost) != cudaSuccess)
       return KSJ_GPU_ERROR_CUDA;
     base += n;
   }
@@ -4125,7 +3895,7 @@ extern "C" ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* de
 extern "C" size_t ksj_gpu_gridding3_workspace_bytes(const ksj_gpu_gridding3_desc* desc) {
   Shape s{};
   if (make_shape3(desc, nullptr, &s) != KSJ_GPU_OK) return 0;
-  return make_layout3(s, desc->sample_format).total;
+  return make_layout3(s).total;
 }
 
 extern "C" ksj_gpu_status ksj_gpu_gridding3_adjoint(const ksj_gpu_gridding3_desc* desc,
@@ -4137,7 +3907,7 @@ extern "C" ksj_gpu_status ksj_gpu_gridding3_adjoint(const ksj_gpu_gridding3_desc
   if (st != KSJ_GPU_OK) return st;
   if (d_kspace == nullptr || d_traj == nullptr || d_out == nullptr) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   if (desc->dcf_mode == KSJ_GPU_DCF_EXTERNAL && d_dcf == nullptr) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  const Layout3 l = make_layout3(s, desc->sample_format);
+  const Layout3 l = make_layout3(s);
   if (l.entries_total > 0xffffffffull) return KSJ_GPU_ERROR_UNSUPPORTED;
   if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 || workspace_bytes < l.total)
     return KSJ_GPU_ERROR_WORKSPACE;
