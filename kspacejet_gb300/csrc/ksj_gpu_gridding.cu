@@ -2,12 +2,12 @@
 //
 // One call reconstructs `frames` independent frames of `channels` coils:
 //
-//   k_tables   quarter-turn-reduced FFT twiddles, FP64 Kaiser-Bessel
-//              deapodisation factors (per call, tiny)
 //   k_prepare  per (frame, sample): error-free grid coordinate, taps and
 //              weights (linear or Kaiser-Bessel), accurately reduced origin
 //              phase times the DCF, and a count per binning list
-//   k_scan     per frame: exclusive scan of the list counts
+//   k_scan     per frame: exclusive scan of the list counts; in further blocks
+//              the call's tables (quarter-turn-reduced FFT twiddles, FP64
+//              Kaiser-Bessel deapodisation factors)
 //   k_scatter  per (frame, sample): append the sample to each list it touches
 //   k_sort     per list (one warp): sort by sample index, so every cell later
 //              accumulates in sample order -- the reference's order -- and the
@@ -143,7 +143,7 @@ struct Shape {
 };
 
 struct Layout {
-  size_t flags, frame_flags, records, counts, cursor, offsets, entries, expanded, long_lists, mid_lists, samples_t, inter,
+  size_t flags, frame_flags, cleared, records, counts, cursor, offsets, entries, expanded, long_lists, mid_lists, samples_t, inter,
       coil_last, tables, total;
 };
 
@@ -310,10 +310,11 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
   };
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
-  l.flags = take(kFlagBytes);
+  l.flags = take(kFlagBytes);  // flags, frame flags and counts are cleared together
   l.frame_flags = take(static_cast<size_t>(s.frames) * 4);
-  l.records = take(fm * record_bytes(s.width));
   l.counts = take(nl * 4);
+  l.cleared = off;
+  l.records = take(fm * record_bytes(s.width));
   l.cursor = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
@@ -344,21 +345,43 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
 // index that kept image row / column p takes: p itself for the linear
 // operator (no oversampling), (p - n/2) mod g for Kaiser-Bessel (the image is
 // centred on q = p - n/2).
-__global__ void k_tables(float2* tw_rows, int grid_rows, float2* tw_cols, int grid_cols, float* inv_dr, int out_rows,
-                         float* inv_dc, int out_cols, int* pos_rows, int* pos_cols, DifPlan plan_rows,
-                         DifPlan plan_cols, int kb, int width, double beta, double i0_beta) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  auto source = [&](int p, int n, int g) { return kb ? (p - n / 2 + g) % g : p; };
-  if (i < out_rows) {
-    const int k = source(i, out_rows, grid_rows);
-    pos_rows[i] = has_two_step_rows(grid_rows) ? two_step_slot(k, grid_rows) : dif_position(plan_rows, k);
+struct TablesArgs {
+  float2* tw_rows;
+  float2* tw_cols;
+  float* inv_dr;
+  float* inv_dc;
+  int* pos_rows;
+  int* pos_cols;
+  int grid_rows, grid_cols, out_rows, out_cols;
+  DifPlan plan_rows, plan_cols;
+  int kb, width;
+  double beta, i0_beta;
+};
+
+// Entries of all tables; one thread each, see table_entry.
+__host__ __device__ inline int table_entries(const TablesArgs& t) {
+  return t.out_rows + t.out_cols + t.grid_rows + t.grid_cols;
+}
+
+__device__ __forceinline__ void table_entry(const TablesArgs& t, int i) {
+  auto source = [&](int p, int n, int g) { return t.kb ? (p - n / 2 + g) % g : p; };
+  if (i < t.out_rows) {
+    const int k = source(i, t.out_rows, t.grid_rows);
+    t.pos_rows[i] = has_two_step_rows(t.grid_rows) ? two_step_slot(k, t.grid_rows) : dif_position(t.plan_rows, k);
+    t.inv_dr[i] = t.kb ? kb_inv_deapod(i, t.out_rows, t.grid_rows, t.width, t.beta, t.i0_beta) : 1.0f;
+    return;
   }
-  if (i < out_cols) pos_cols[i] = dif_position(plan_cols, source(i, out_cols, grid_cols));
-  if (i < grid_rows) tw_rows[i] = twiddle(i, grid_rows);
-  if (i < grid_cols) tw_cols[i] = twiddle(i, grid_cols);
-  auto inv_psi = [&](int p, int n, int g) -> float { return kb ? kb_inv_deapod(p, n, g, width, beta, i0_beta) : 1.0f; };
-  if (i < out_rows) inv_dr[i] = inv_psi(i, out_rows, grid_rows);
-  if (i < out_cols) inv_dc[i] = inv_psi(i, out_cols, grid_cols);
+  i -= t.out_rows;
+  if (i < t.out_cols) {
+    t.pos_cols[i] = dif_position(t.plan_cols, source(i, t.out_cols, t.grid_cols));
+    t.inv_dc[i] = t.kb ? kb_inv_deapod(i, t.out_cols, t.grid_cols, t.width, t.beta, t.i0_beta) : 1.0f;
+    return;
+  }
+  i -= t.out_cols;
+  if (i < t.grid_rows)
+    t.tw_rows[i] = twiddle(i, t.grid_rows);
+  else if (i - t.grid_rows < t.grid_cols)
+    t.tw_cols[i - t.grid_rows] = twiddle(i - t.grid_rows, t.grid_cols);
 }
 
 __global__ void __launch_bounds__(256) k_fill(float* p, int n, float v) {
@@ -482,48 +505,82 @@ __global__ void __launch_bounds__(256) k_prepare(PrepareArgs a) {
   }
 }
 
-// Exclusive scan of one frame's list counts (one block per frame).
-__global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, int lists) {
+// Exclusive scan of one frame's list counts, one block per frame: list starts
+// into `offsets` and, as the scatter's running positions, into `cursor`.  Bound by latency (one block
+// for a single frame), so a warp holds its whole stretch of counts in registers,
+// 32 consecutive ones per load, all loads in flight at once (per-thread
+// stretches, read twice one count after another, took 24 us for 16384 lists, this 5).
+// Blocks from `frames` on fill the call's tables meanwhile, 64 entries each: their FP64
+// functions run at a few lanes per clock and SM, so they are spread over many
+// (a kernel of their own on one or two SMs took 7 to 20 us).
+constexpr int kScanPer = kMaxGrid * (kMaxGrid / kChunk) / 1024;  // counts per thread, at most
+constexpr int kTablesPerBlock = 64;
+
+__global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* cursor, int lists,
+                                               int frames, uint32_t* mid_count, uint32_t* long_count,
+                                               const __grid_constant__ TablesArgs tables) {
+  if (static_cast<int>(blockIdx.x) >= frames) {
+    const int i = (blockIdx.x - frames) * kTablesPerBlock + threadIdx.x;
+    if (threadIdx.x < kTablesPerBlock && i < table_entries(tables)) table_entry(tables, i);
+    return;
+  }
   __shared__ uint32_t warp_sums[32];
   const int f = blockIdx.x;
   const uint32_t* c = counts + static_cast<size_t>(f) * lists;
   uint32_t* o = offsets + static_cast<size_t>(f) * (lists + 1);
-  const int per = (lists + blockDim.x - 1) / blockDim.x;
-  const int begin = threadIdx.x * per;
-  const int end = min(begin + per, lists);
-  uint32_t local = 0;
-  for (int i = begin; i < end; ++i) local += c[i];
+  uint32_t* cur = cursor + static_cast<size_t>(f) * lists;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t incl = local;
+  const int per = (lists + 1023) / 1024;
+  const int base = warp * per * 32 + lane;
+  uint32_t v[kScanPer];
+  uint32_t local = 0;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
-  if (lane == 31) warp_sums[warp] = incl;
+  for (int k = 0; k < kScanPer; ++k) v[k] = k < per && base + 32 * k < lists ? __ldg(c + base + 32 * k) : 0u;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) local += v[k];
+  local = __reduce_add_sync(0xffffffffu, local);
+  if (lane == 0) warp_sums[warp] = local;
+  if (f == 0 && threadIdx.x == 0) *mid_count = *long_count = 0;  // the queues k_sort fills
   __syncthreads();
   if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    uint32_t ws = lane < nw ? warp_sums[lane] : 0u;
+    uint32_t ws = warp_sums[lane];
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, ws, d);
-      if (lane >= d) ws += v;
+      const uint32_t u = __shfl_up_sync(0xffffffffu, ws, d);
+      if (lane >= d) ws += u;
     }
-    if (lane < nw) warp_sums[lane] = ws;
+    warp_sums[lane] = ws;
   }
   __syncthreads();
-  uint32_t run = incl - local + (warp > 0 ? warp_sums[warp - 1] : 0u);
-  for (int i = begin; i < end; ++i) {
-    o[i] = run;
-    run += c[i];
+  uint32_t run = warp_sums[warp] - local;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) {
+    if (k >= per) break;
+    uint32_t incl = v[k];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (base + 32 * k < lists) o[base + 32 * k] = cur[base + 32 * k] = run + incl - v[k];
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  if (threadIdx.x == blockDim.x - 1) o[lists] = run;
+  if (threadIdx.x == 0) o[lists] = warp_sums[31];
+}
+
+// The scan of `frames` frames, with the tables where they are wanted.
+ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* cursor, int lists, int frames,
+                           uint32_t* mid_count, uint32_t* long_count, const TablesArgs* tables, cudaStream_t stream) {
+  const int extra = tables ? (table_entries(*tables) + kTablesPerBlock - 1) / kTablesPerBlock : 0;
+  LaunchScope scope("k_scan", stream);
+  k_scan<<<frames + extra, 1024, 0, stream>>>(counts, offsets, cursor, lists, frames, mid_count, long_count,
+                                              tables ? *tables : TablesArgs{});
+  return KSJ_GPU_OK;
 }
 
 template <int W>
-__global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, const uint32_t* offsets,
-                                                 uint32_t* cursor, uint32_t* entries, int frames, int samples,
+__global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, uint32_t* cursor, uint32_t* entries,
+                                                 int frames, int samples,
                                                  int grid_rows, int grid_cols, int nchunks, size_t entries_per_frame) {
   const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<size_t>(frames) * samples) return;
@@ -536,7 +593,6 @@ __global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, c
   int k0, k1;
   list_chunks<W>(c0, grid_cols, &k0, &k1);
   const int lists = grid_rows * nchunks;
-  const uint32_t* off = offsets + static_cast<size_t>(f) * (lists + 1);
   uint32_t* cur = cursor + static_cast<size_t>(f) * lists;
   uint32_t* ent = entries + static_cast<size_t>(f) * entries_per_frame;
 #pragma unroll
@@ -544,11 +600,8 @@ __global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, c
     int row = r0 + j;
     if (row >= grid_rows) row -= grid_rows;
     const int l0 = row * nchunks + k0;
-    ent[off[l0] + atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(s);
-    if (k1 != k0) {
-      const int l1 = row * nchunks + k1;
-      ent[off[l1] + atomicAdd(cur + l1, 1u)] = static_cast<uint32_t>(s);
-    }
+    ent[atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(s);
+    if (k1 != k0) ent[atomicAdd(cur + row * nchunks + k1, 1u)] = static_cast<uint32_t>(s);
   }
 }
 
@@ -971,10 +1024,6 @@ __global__ void __launch_bounds__(kLongSortThreads, 1) k_sort_long(SortArgs a) {
 // Launch k_sort and then k_sort_long for the lists it queued.
 template <int W>
 ksj_gpu_status launch_sort(SortArgs sa, cudaStream_t stream) {
-  // both counts, in front of the queues
-  if (cudaMemsetAsync(sa.mid_count, 0, sizeof(uint32_t), stream) != cudaSuccess ||
-      cudaMemsetAsync(sa.long_count, 0, sizeof(uint32_t), stream) != cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
   if (cudaFuncSetAttribute(k_sort_long<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSortSmem * 4) !=
       cudaSuccess)
     return KSJ_GPU_ERROR_CUDA;
@@ -1981,15 +2030,14 @@ struct ColsPass {
 
 // The binning lists of one call: per-sample records, list counts, offsets,
 // the scattered entries and their sort (and, when `expanded` is given, the
-// expanded entries the row pass reads).  `flags` must already be cleared.
+// expanded entries the row pass reads), and the call's tables where `tables`
+// names them.  The flags and counts must already be cleared.
 template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
                            uint32_t* offsets, uint32_t* entries, unsigned char* expanded, uint32_t* long_lists,
-                           uint32_t* mid_lists, cudaStream_t stream, uint32_t* frame_flags = nullptr) {
-  const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
-  if (cudaMemsetAsync(counts, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  if (cudaMemsetAsync(cursor, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+                           uint32_t* mid_lists, cudaStream_t stream, uint32_t* frame_flags = nullptr,
+                           const TablesArgs* tables = nullptr) {
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   {
     PrepareArgs p{};
@@ -2019,14 +2067,11 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     LaunchScope scope("k_prepare", stream);
     k_prepare<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(p);
   }
-  {
-    LaunchScope scope("k_scan", stream);
-    k_scan<<<s.frames, 1024, 0, stream>>>(counts, offsets, s.lists_per_frame);
-  }
+  launch_scan(counts, offsets, cursor, s.lists_per_frame, s.frames, mid_lists, long_lists, tables, stream);
   {
     LaunchScope scope("k_scatter", stream);
     k_scatter<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
-        records, offsets, cursor, entries, s.frames, s.samples, s.grid_rows, s.grid_cols, s.nchunks,
+        records, cursor, entries, s.frames, s.samples, s.grid_rows, s.grid_cols, s.nchunks,
         s.entries_per_frame);
   }
   {
@@ -2088,24 +2133,17 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   int* pos_rows = reinterpret_cast<int*>(inv_dc + s.out_cols);
   int* pos_cols = pos_rows + s.out_rows;
 
-  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess ||
-      cudaMemsetAsync(ws + l.frame_flags, 0, static_cast<size_t>(s.frames) * 4, stream) != cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
-  {
-    const int n = std::max(std::max(s.grid_rows, s.grid_cols), std::max(s.out_rows, s.out_cols));
-    const double beta = s.beta;
-    LaunchScope scope("k_tables", stream);
-    k_tables<<<(n + 255) / 256, 256, 0, stream>>>(tw_rows, s.grid_rows, tw_cols, s.grid_cols, inv_dr, s.out_rows,
-                                                  inv_dc, s.out_cols, pos_rows, pos_cols, s.plan_rows, s.plan_cols,
-                                                  s.kb ? 1 : 0, s.width, beta,
-                                                  s.kb ? std::cyl_bessel_i(0.0, beta) : 1.0);
-  }
+  if (cudaMemsetAsync(ws + l.flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  const double beta = s.beta;
+  const TablesArgs tables{tw_rows, tw_cols, inv_dr, inv_dc, pos_rows, pos_cols, s.grid_rows, s.grid_cols, s.out_rows,
+                          s.out_cols, s.plan_rows, s.plan_cols, s.kb ? 1 : 0, s.width, beta,
+                          s.kb ? std::cyl_bessel_i(0.0, beta) : 1.0};
   {
     const ksj_gpu_status st = build_lists<W>(s, d, d_traj, d_dcf, flags, records, counts, cursor, offsets, entries,
                                              ws + l.expanded,
                                              reinterpret_cast<uint32_t*>(ws + l.long_lists),
                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream,
-                                             reinterpret_cast<uint32_t*>(ws + l.frame_flags));
+                                             reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables);
     if (st != KSJ_GPU_OK) return st;
   }
   auto to_coil_last = [&](int f0, int nf, cudaStream_t st) {
@@ -2405,7 +2443,7 @@ __global__ void __launch_bounds__(256) k_pm_update(const PmRecord<W>* pm, const 
 }
 
 struct PmLayout {
-  size_t flags, records, counts, cursor, offsets, entries, long_lists, mid_lists, pm, w, grid, total;
+  size_t flags, cleared, records, counts, cursor, offsets, entries, long_lists, mid_lists, pm, w, grid, total;
 };
 
 PmLayout make_pm_layout(const Shape& s) {
@@ -2418,9 +2456,10 @@ PmLayout make_pm_layout(const Shape& s) {
   };
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
-  l.flags = take(kFlagBytes);
-  l.records = take(fm * record_bytes(s.width));
+  l.flags = take(kFlagBytes);  // flags and counts are cleared together
   l.counts = take(nl * 4);
+  l.cleared = off;
+  l.records = take(fm * record_bytes(s.width));
   l.cursor = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
@@ -2439,7 +2478,7 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
                                  cudaStream_t stream) {
   static_assert(sizeof(PmRecord<W>) == 8 + 16 * W, "PmRecord layout");
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   ksj_gpu_gridding_desc dd = *d;
   dd.dcf_mode = KSJ_GPU_DCF_NONE;
   const ksj_gpu_status st =
@@ -2581,16 +2620,19 @@ __global__ void __launch_bounds__(512) k_plane_bases(uint32_t* offsets, int plan
   if (t < planes) bases[t] = tot[t];
 }
 
-__global__ void __launch_bounds__(256) k_offsets_add(uint32_t* offsets, int planes, int lists, const uint32_t* bases) {
+__global__ void __launch_bounds__(256) k_offsets_add(uint32_t* offsets, uint32_t* cursor, int planes, int lists,
+                                                     const uint32_t* bases) {
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<size_t>(planes) * (lists + 1)) return;
-  offsets[i] += bases[i / (lists + 1)];
+  const size_t p = i / (lists + 1), l = i - p * (lists + 1);
+  const uint32_t at = offsets[i] + bases[p];
+  offsets[i] = at;
+  if (l < static_cast<size_t>(lists)) cursor[p * lists + l] = at;
 }
 
 template <int W>
-__global__ void __launch_bounds__(256) k_scatter3(const unsigned char* records, const uint32_t* offsets,
-                                                  uint32_t* cursor, uint32_t* entries, int samples, int grid,
-                                                  int nchunks, int lists_per_plane) {
+__global__ void __launch_bounds__(256) k_scatter3(const unsigned char* records, uint32_t* cursor, uint32_t* entries,
+                                                  int samples, int grid, int nchunks, int lists_per_plane) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= samples) return;
   const SampleRecord3<W>& rec = reinterpret_cast<const SampleRecord3<W>*>(records)[idx];
@@ -2599,23 +2641,19 @@ __global__ void __launch_bounds__(256) k_scatter3(const unsigned char* records, 
   for (int i = 0; i < W; ++i) {
     int plane = rec.z0 + i;
     if (plane >= grid) plane -= grid;
-    const uint32_t* off = offsets + static_cast<size_t>(plane) * (lists_per_plane + 1);
     uint32_t* cur = cursor + static_cast<size_t>(plane) * lists_per_plane;
     for (int j = 0; j < W; ++j) {
       int row = rec.r0 + j;
       if (row >= grid) row -= grid;
       const int l0 = row * nchunks + k0;
-      entries[off[l0] + atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(idx);
-      if (k1 != k0) {
-        const int l1 = row * nchunks + k1;
-        entries[off[l1] + atomicAdd(cur + l1, 1u)] = static_cast<uint32_t>(idx);
-      }
+      entries[atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(idx);
+      if (k1 != k0) entries[atomicAdd(cur + row * nchunks + k1, 1u)] = static_cast<uint32_t>(idx);
     }
   }
 }
 
 struct Layout3 {
-  size_t flags, records, counts, cursor, offsets, bases, entries, expanded, long_lists, mid_lists, samples_t, inter, inter2,
+  size_t flags, cleared, records, counts, cursor, offsets, bases, entries, expanded, long_lists, mid_lists, samples_t, inter, inter2,
       tables, total;
   size_t entries_total;
 };
@@ -2641,9 +2679,10 @@ Layout3 make_layout3(const Shape& s) {
   const size_t g = static_cast<size_t>(s.grid_rows), n = static_cast<size_t>(s.rows);
   const size_t nl = g * s.lists_per_frame;
   l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
-  l.flags = take(kFlagBytes);
-  l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
+  l.flags = take(kFlagBytes);  // flags and counts are cleared together
   l.counts = take(nl * 4);
+  l.cleared = off;
+  l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
   l.cursor = take(nl * 4);
   l.offsets = take((nl + g) * 4);
   l.bases = take(g * 4);
@@ -2687,16 +2726,15 @@ ksj_gpu_status make_shape3(const ksj_gpu_gridding3_desc* d, const ksj_gpu_griddi
 
 // The 3-D binning lists: per-sample records, (plane, row, chunk) counts, per-plane
 // scans made absolute, the scattered entries, their sort and (when `expanded`
-// is given) the expanded entries.  `flags` must already be cleared.
+// is given) the expanded entries, and the call's tables where `tables` names
+// them.  The flags and counts must already be cleared.
 template <int W>
 ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_traj, const float* d_dcf,
                             uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
                             uint32_t* offsets, uint32_t* bases, uint32_t* entries, unsigned char* expanded,
-                            uint32_t* long_lists, uint32_t* mid_lists, cudaStream_t stream) {
+                            uint32_t* long_lists, uint32_t* mid_lists, cudaStream_t stream,
+                            const TablesArgs* tables = nullptr) {
   const int g = s.grid_rows;
-  const size_t nl = static_cast<size_t>(g) * s.lists_per_frame;
-  if (cudaMemsetAsync(counts, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  if (cudaMemsetAsync(cursor, 0, nl * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   {
     Prepare3Args p{};
     p.traj = d_traj;
@@ -2716,21 +2754,18 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     LaunchScope scope("k_prepare3", stream);
     k_prepare3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(p);
   }
+  launch_scan(counts, offsets, cursor, s.lists_per_frame, g, mid_lists, long_lists, tables, stream);
   {
-    LaunchScope scope("k_scan", stream);
-    k_scan<<<g, 1024, 0, stream>>>(counts, offsets, s.lists_per_frame);
-  }
-  {
-        LaunchScope scope("k_plane_offsets", stream);
+    LaunchScope scope("k_plane_offsets", stream);
     k_plane_bases<<<1, 512, 0, stream>>>(offsets, g, s.lists_per_frame, bases);
     const size_t total = static_cast<size_t>(g) * (s.lists_per_frame + 1);
-    k_offsets_add<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(offsets, g, s.lists_per_frame,
-                                                                                bases);
+    k_offsets_add<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(offsets, cursor, g,
+                                                                                s.lists_per_frame, bases);
   }
   {
     LaunchScope scope("k_scatter3", stream);
-    k_scatter3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(records, offsets, cursor, entries, s.samples, g,
-                                                               s.nchunks, s.lists_per_frame);
+    k_scatter3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(records, cursor, entries, s.samples, g, s.nchunks,
+                                                               s.lists_per_frame);
   }
   {
     SortArgs sa{};
@@ -2777,14 +2812,9 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   int* pos_cols = pos_rows + n;
   float* ones = reinterpret_cast<float*>(pos_cols + n);
 
-  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  {
-    const int nt = std::max(g, n);
-    LaunchScope scope("k_tables", stream);
-    k_tables<<<(nt + 255) / 256, 256, 0, stream>>>(tw_rows, g, tw_cols, g, inv_dr, n, inv_dc, n, pos_rows, pos_cols,
-                                                   s.plan_rows, s.plan_cols, 1, s.width, s.beta,
-                                                   std::cyl_bessel_i(0.0, static_cast<double>(s.beta)));
-  }
+  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  const TablesArgs tables{tw_rows, tw_cols, inv_dr, inv_dc, pos_rows, pos_cols, g, g, n, n, s.plan_rows, s.plan_cols, 1,
+                          s.width, s.beta, std::cyl_bessel_i(0.0, static_cast<double>(s.beta))};
   {
     LaunchScope scope("k_fill_ones", stream);
     k_fill<<<(n * n + 255) / 256, 256, 0, stream>>>(ones, n * n, 1.0f);
@@ -2794,7 +2824,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
                                               offsets, reinterpret_cast<uint32_t*>(ws + l.bases), entries,
                                               ws + l.expanded,
                                               reinterpret_cast<uint32_t*>(ws + l.long_lists),
-                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream);
+                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream, &tables);
     if (st != KSJ_GPU_OK) return st;
   }
   {
@@ -3182,7 +3212,7 @@ __global__ void __launch_bounds__(256) k_pm_update3(const PmRecord3<W>* pm, cons
 }
 
 struct PmLayout3 {
-  size_t flags, records, counts, cursor, offsets, bases, entries, long_lists, mid_lists, pm, pmc, wzr, w, grid, part_base, partial,
+  size_t flags, cleared, records, counts, cursor, offsets, bases, entries, long_lists, mid_lists, pm, pmc, wzr, w, grid, part_base, partial,
       counters, total, entries_total, max_long;
 };
 
@@ -3197,9 +3227,10 @@ PmLayout3 make_pm_layout3(const Shape& s) {
   const size_t g = static_cast<size_t>(s.grid_rows);
   const size_t nl = g * s.lists_per_frame;
   l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
-  l.flags = take(kFlagBytes);
-  l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
+  l.flags = take(kFlagBytes);  // flags and counts are cleared together
   l.counts = take(nl * 4);
+  l.cleared = off;
+  l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
   l.cursor = take(nl * 4);
   l.offsets = take((nl + g) * 4);
   l.bases = take(g * 4);
@@ -3227,7 +3258,7 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
   static_assert(sizeof(PmRecord3<W>) == 16 + 24 * W, "PmRecord3 layout");
   const int g = s.grid_rows;
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   const ksj_gpu_status st = build_lists3<W>(
       s, KSJ_GPU_DCF_NONE, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
       reinterpret_cast<uint32_t*>(ws + l.cursor), reinterpret_cast<uint32_t*>(ws + l.offsets),
