@@ -4,14 +4,19 @@
 //
 //   k_prepare  per (frame, sample): error-free grid coordinate, taps and
 //              weights (linear or Kaiser-Bessel), accurately reduced origin
-//              phase times the DCF, and a count per binning list
-//   k_scan     per frame: exclusive scan of the list counts; in further blocks
+//              phase times the DCF; per block of consecutive samples a count
+//              for every binning list
+//   k_bin_prefix  per list: each block's start among the list's entries, and the
+//              list's length
+//   k_scan     per frame: exclusive scan of the list lengths; in further blocks
 //              the call's tables (quarter-turn-reduced FFT twiddles, FP64
 //              Kaiser-Bessel deapodisation factors)
-//   k_scatter  per (frame, sample): append the sample to each list it touches
-//   k_sort     per list (one warp): sort by sample index, so every cell later
-//              accumulates in sample order -- the reference's order -- and the
-//              result is deterministic whatever order the scatter produced
+//   k_place    per block of samples: every sample's entries straight into their
+//              places, in sample order, so every cell later accumulates in
+//              sample order -- the reference's order -- and the result is
+//              deterministic
+//   (3-D: k_prepare3 and k_scatter3 append to the lists with atomics, and
+//              k_sort and k_sort_long restore the sample order)
 //   k_samples_coil_last  [frame][coil][sample] -> [frame][sample][coil] times
 //              the sample's weight and phase, so the row pass reads one
 //              sample's coils as one coalesced segment
@@ -114,6 +119,13 @@ inline int rows_threads_for(int grid_cols, int lanes, int cg) {
 
 constexpr uint32_t kWaitLimit = 1u << 22;  // polls before a bounded wait gives up
 
+// Binning in sample order (k_prepare, k_place): a block takes bin_span
+// consecutive samples, kBinThreads at a time, with a word or two of shared
+// memory per binning list of the frame.
+constexpr int kBinThreads = 512;
+constexpr int kBinWarps = kBinThreads / 32;
+constexpr size_t kPlaceListBytes = 4;  // of k_place: the list's running position
+
 struct Shape {
   int frames, channels, samples;
   int rows, cols;          // image
@@ -129,6 +141,7 @@ struct Shape {
   float beta, inv_i0_beta;
   float row_origin, col_origin;
   float phase_row, phase_col, phase_sign;  // origin-phase coefficients
+  int bin_blocks, bin_span;  // 2-D binning: blocks per frame and samples per block
   int coil_group, column_block, list_capacity, frames_per_pass, coil_parts;
   uint32_t wait_fault;  // tests only: segment waits that cannot succeed, given up after this many polls
   int column_pass;      // 1 one CTA per tile (k_cols), 2 persistent ring (k_cols_ring)
@@ -143,7 +156,7 @@ struct Shape {
 };
 
 struct Layout {
-  size_t flags, frame_flags, cleared, records, counts, cursor, offsets, entries, expanded, long_lists, mid_lists, samples_t, inter,
+  size_t flags, frame_flags, cleared, records, counts, totals, offsets, expanded, samples_t, inter,
       coil_last, tables, total;
 };
 
@@ -195,6 +208,15 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   s->nchunks = (s->grid_cols + kChunk - 1) / kChunk;
   s->lists_per_frame = s->grid_rows * s->nchunks;
   s->entries_per_frame = static_cast<size_t>(s->samples) * s->width * 2;
+  {
+    // as many blocks as k_place has resident at once, over all frames: fewer
+    // leave SMs idle, more only add counts to scan
+    const int turns = (s->samples + kBinThreads - 1) / kBinThreads;
+    const int resident = 152 * std::min(4, std::max(1, static_cast<int>(220 * 1024 / (kPlaceListBytes * s->lists_per_frame))));
+    const int blocks = std::min(turns, std::max(1, resident / s->frames));
+    s->bin_span = (turns + blocks - 1) / blocks * kBinThreads;
+    s->bin_blocks = (s->samples + s->bin_span - 1) / s->bin_span;
+  }
   s->out_rows = s->rows;
   s->out_cols = s->cols;
   s->col_group = 2;
@@ -310,17 +332,14 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
   };
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
-  l.flags = take(kFlagBytes);  // flags, frame flags and counts are cleared together
+  l.flags = take(kFlagBytes);  // flags and frame flags are cleared together
   l.frame_flags = take(static_cast<size_t>(s.frames) * 4);
-  l.counts = take(nl * 4);
   l.cleared = off;
   l.records = take(fm * record_bytes(s.width));
-  l.cursor = take(nl * 4);
+  l.counts = take(nl * s.bin_blocks * 4);
+  l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
-  l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
   l.expanded = take(static_cast<size_t>(s.frames) * s.entries_per_frame * entry_bytes(s.width));
-  l.long_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / (s.list_capacity + 1)) * 4);
-  l.mid_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / 33) * 4);
   l.samples_t = take(fm * s.channels * sizeof(float2));
   l.inter = take(static_cast<size_t>(s.frames) * s.grid_rows * s.out_cols * s.cpitch * sizeof(float2));
   l.coil_last = d->output == KSJ_GPU_OUTPUT_COIL_MAJOR
@@ -398,9 +417,10 @@ struct PrepareArgs {
   uint32_t dcf_mode;
   uint32_t require_nyquist;
   unsigned char* records;
-  uint32_t* counts;
+  uint32_t* counts;               // [frame][block][list]: entries of the block's samples in the list
   uint32_t* flags;
   int frames, samples, grid_rows, grid_cols, nchunks, lists_per_frame;
+  int bin_span;                   // samples per block
   int kb;
   float beta, two_over_w, inv_i0_beta;
   float phase_row, phase_col, phase_sign;
@@ -413,21 +433,18 @@ __device__ __forceinline__ void list_chunks(int c0, int grid_cols, int* k0, int*
   *k1 = last / kChunk;
 }
 
+// One sample's record, and its entries counted in `counts` (shared memory, per list).
 template <int W>
-__global__ void __launch_bounds__(256) k_prepare(PrepareArgs a) {
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t total = static_cast<size_t>(a.frames) * a.samples;
-  if (idx >= total) return;
-  const int f = static_cast<int>(idx / a.samples);
-  if (a.frame_samples != nullptr &&
-      idx - static_cast<size_t>(f) * a.samples >= static_cast<size_t>(__ldg(a.frame_samples + f))) {
+__device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int sample, uint32_t* counts) {
+  const size_t idx = static_cast<size_t>(f) * a.samples + sample;
+  if (a.frame_samples != nullptr && static_cast<uint32_t>(sample) >= __ldg(a.frame_samples + f)) {
     // a padding sample of a ragged batch: in no list (its trajectory is not read)
     reinterpret_cast<SampleRecord<W>*>(a.records)[idx].r0 = -1;
     return;
   }
   const float2 k =
       a.frame_traj != nullptr
-          ? reinterpret_cast<const float2*>(__ldg(a.frame_traj + f))[idx - static_cast<size_t>(f) * a.samples]
+          ? reinterpret_cast<const float2*>(__ldg(a.frame_traj + f))[sample]
           : __ldg(reinterpret_cast<const float2*>(a.traj) + idx);
   bool ok = isfinite(k.x) && isfinite(k.y);
   if (ok && a.require_nyquist) ok = k.x >= -kPiF && k.x <= kPiF && k.y >= -kPiF && k.y <= kPiF;
@@ -495,7 +512,6 @@ __global__ void __launch_bounds__(256) k_prepare(PrepareArgs a) {
   reinterpret_cast<SampleRecord<W>*>(a.records)[idx] = rec;
   int k0, k1;
   list_chunks<W>(rec.c0, a.grid_cols, &k0, &k1);
-  uint32_t* counts = a.counts + static_cast<size_t>(f) * a.lists_per_frame;
 #pragma unroll
   for (int j = 0; j < W; ++j) {
     int row = rec.r0 + j;
@@ -505,11 +521,50 @@ __global__ void __launch_bounds__(256) k_prepare(PrepareArgs a) {
   }
 }
 
-// Exclusive scan of one frame's list counts, one block per frame: list starts
-// into `offsets` and, as the scatter's running positions, into `cursor`.  Bound by latency (one block
+// One block per (block of samples, frame).  The counts go to shared memory: as atomics on
+// global memory the samples of a radial scan's centre, all in the same few
+// lists, were serialised (25 us for 205824 samples on a 512 grid, this 17).
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
+  extern __shared__ uint32_t prepare_counts[];
+  const int f = blockIdx.y;
+  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) prepare_counts[l] = 0;
+  __syncthreads();
+  const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
+  for (int sample = s0 + threadIdx.x; sample < s1; sample += kBinThreads)
+    prepare_sample<W>(a, f, sample, prepare_counts);
+  __syncthreads();
+  uint32_t* out = a.counts + (static_cast<size_t>(f) * gridDim.x + blockIdx.x) * a.lists_per_frame;
+  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) out[l] = prepare_counts[l];
+}
+
+// Thread per list: the blocks' counts of the list become each block's start
+// among the list's entries; their sum is the list's length.  Eight blocks'
+// counts are in flight at once.
+__global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* totals, int blocks, int lists) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= lists) return;
+  uint32_t* c = counts + static_cast<size_t>(blockIdx.y) * blocks * lists + l;
+  uint32_t run = 0;
+  for (int b0 = 0; b0 < blocks; b0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = b0 + k < blocks ? c[static_cast<size_t>(b0 + k) * lists] : 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (b0 + k < blocks) c[static_cast<size_t>(b0 + k) * lists] = run;
+      run += v[k];
+    }
+  }
+  totals[static_cast<size_t>(blockIdx.y) * lists + l] = run;
+}
+
+// Exclusive scan of one frame's list lengths, one block per frame: list starts
+// into `offsets` and, as a scatter's running positions, into `cursor` (3-D; null otherwise).  Bound by latency (one block
 // for a single frame), so a warp holds its whole stretch of counts in registers,
 // 32 consecutive ones per load, all loads in flight at once (per-thread
-// stretches, read twice one count after another, took 24 us for 16384 lists, this 5).
+// stretches, read twice one count after another, took 24 us for 16384 lists, this
+// and the tables 10).
 // Blocks from `frames` on fill the call's tables meanwhile, 64 entries each: their FP64
 // functions run at a few lanes per clock and SM, so they are spread over many
 // (a kernel of their own on one or two SMs took 7 to 20 us).
@@ -540,7 +595,7 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t*
   for (int k = 0; k < kScanPer; ++k) local += v[k];
   local = __reduce_add_sync(0xffffffffu, local);
   if (lane == 0) warp_sums[warp] = local;
-  if (f == 0 && threadIdx.x == 0) *mid_count = *long_count = 0;  // the queues k_sort fills
+  if (f == 0 && threadIdx.x == 0 && mid_count != nullptr) *mid_count = *long_count = 0;  // the queues k_sort fills
   __syncthreads();
   if (warp == 0) {
     uint32_t ws = warp_sums[lane];
@@ -562,7 +617,10 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t*
       const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += u;
     }
-    if (base + 32 * k < lists) o[base + 32 * k] = cur[base + 32 * k] = run + incl - v[k];
+    if (base + 32 * k < lists) {
+      o[base + 32 * k] = run + incl - v[k];
+      if (cursor != nullptr) cur[base + 32 * k] = run + incl - v[k];
+    }
     run += __shfl_sync(0xffffffffu, incl, 31);
   }
   if (threadIdx.x == 0) o[lists] = warp_sums[31];
@@ -576,33 +634,6 @@ ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* 
   k_scan<<<frames + extra, 1024, 0, stream>>>(counts, offsets, cursor, lists, frames, mid_count, long_count,
                                               tables ? *tables : TablesArgs{});
   return KSJ_GPU_OK;
-}
-
-template <int W>
-__global__ void __launch_bounds__(256) k_scatter(const unsigned char* records, uint32_t* cursor, uint32_t* entries,
-                                                 int frames, int samples,
-                                                 int grid_rows, int grid_cols, int nchunks, size_t entries_per_frame) {
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<size_t>(frames) * samples) return;
-  const int f = static_cast<int>(idx / samples);
-  const int s = static_cast<int>(idx - static_cast<size_t>(f) * samples);
-  const SampleRecord<W>* rec = reinterpret_cast<const SampleRecord<W>*>(records) + idx;
-  const int r0 = rec->r0;
-  if (r0 < 0) return;  // padding sample of a ragged batch
-  const int c0 = rec->c0;
-  int k0, k1;
-  list_chunks<W>(c0, grid_cols, &k0, &k1);
-  const int lists = grid_rows * nchunks;
-  uint32_t* cur = cursor + static_cast<size_t>(f) * lists;
-  uint32_t* ent = entries + static_cast<size_t>(f) * entries_per_frame;
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    int row = r0 + j;
-    if (row >= grid_rows) row -= grid_rows;
-    const int l0 = row * nchunks + k0;
-    ent[atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(s);
-    if (k1 != k0) ent[atomicAdd(cur + row * nchunks + k1, 1u)] = static_cast<uint32_t>(s);
-  }
 }
 
 // Ascending sort of R * 32 keys held by a warp, key e = 32 r + lane in v[r]:
@@ -678,22 +709,155 @@ __device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, con
   for (int j = 0; j < W; j += 2) o[1 + j / 2] = make_float2(wrow * wc[j], wrow * wc[j + 1]);
 }
 
+struct PlaceArgs {
+  const unsigned char* records;
+  const uint32_t* offsets;  // [frame][list + 1]
+  const uint32_t* starts;   // [frame][block][list]: the block's start in the list (k_bin_prefix)
+  unsigned char* expanded;  // entries in their places, or null:
+  uint32_t* entries;        // the sample indices alone
+  int samples, grid_rows, grid_cols, nchunks, lists_per_frame, bin_span;
+  size_t entries_per_frame;
+};
+
+// A warp's samples, one per lane: how many lanes below this one join each of this
+// lane's lists (rows r0 + j wrapped, chunks k0 and k1), and whether one above does.
+// Byte j of below[h] is the count for (row r0 + j, chunk k0 or k1); bit j of
+// above[h].  r0 < 0: no sample.  Every lane's rows and chunks go round the warp once.
 template <int W>
-__device__ __forceinline__ void expand_entry(const SampleRecord<W>* recs, uint32_t sidx, int row, int col_lo,
-                                             int grid_rows, int grid_cols, unsigned char* out) {
-  constexpr int kRV = static_cast<int>(sizeof(SampleRecord<W>) / 16);
-  float4 q[kRV];
-  const float4* rp = reinterpret_cast<const float4*>(recs + sidx);
+struct WarpRanks {
+  static constexpr int kWords = (W + 3) / 4;
+  uint32_t below[2][kWords], above[2];
+};
+
+template <int W>
+__device__ __forceinline__ WarpRanks<W> warp_ranks(int r0, int k0, int k1, int grid_rows) {
+  constexpr uint32_t kRows = (1u << W) - 1u;
+  WarpRanks<W> out;
 #pragma unroll
-  for (int v = 0; v < kRV; ++v) q[v] = __ldg(rp + v);
-  const float* w = reinterpret_cast<const float*>(q);
-  int ta = row - __float_as_int(w[0]);
-  if (ta < 0) ta += grid_rows;
-  float wr = 0.0f;
+  for (int h = 0; h < 2; ++h) {
+    out.above[h] = 0;
+#pragma unroll
+    for (int q = 0; q < WarpRanks<W>::kWords; ++q) out.below[h][q] = 0;
+  }
+  const int lane = threadIdx.x & 31;
+  // row, chunk, chunk (63, 63: no sample)
+  const uint32_t mine = r0 < 0 ? 0xfffu : static_cast<uint32_t>(r0) << 12 | static_cast<uint32_t>(k0) << 6 | static_cast<uint32_t>(k1);
+#pragma unroll 4
+  for (int i = 0; i < 32; ++i) {
+    const uint32_t other = __shfl_sync(0xffffffffu, mine, i);
+    // this lane's rows that the other sample's stencil covers: its rows start
+    // d before ours, or (across the wrap) grid_rows - d after
+    int d = r0 - static_cast<int>(other >> 12);
+    if (d < 0) d += grid_rows;
+    const uint32_t rows = (kRows >> min(d, 31)) | ((kRows << min(grid_rows - d, 31)) & kRows);
+    const uint32_t o0 = (other >> 6) & 63u, o1 = other & 63u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t k = static_cast<uint32_t>(h ? k1 : k0);
+      const uint32_t m = k == o0 || k == o1 ? rows : 0u;
+      if (i < lane) {
+#pragma unroll
+        for (int q = 0; q < WarpRanks<W>::kWords; ++q)  // bit j of a nibble to byte j
+          out.below[h][q] += (((m >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
+      } else if (i > lane) {
+        out.above[h] |= m;
+      }
+    }
+  }
+  return out;
+}
+
+// Places of one sample per thread in the lists of rows r0 .. r0 + W - 1
+// (wrapped) and chunks k0 and k1 (r0 < 0: no sample), in thread order: a list's
+// entries have to stand in sample order.  at: running position of each list.  The
+// ranks within the warps are found first, by all warps at once; then the warps take
+// turns, passed on by named barriers: each reads its lists' positions, adds the ranks,
+// and the last lane of a list moves its position on.  Called by the whole block;
+// synchronises it first.
+template <int W>
+__device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1, int nchunks, int grid_rows,
+                                           uint32_t (&pos)[W][2]) {
+  const int warp = threadIdx.x >> 5;
+  const WarpRanks<W> ranks = warp_ranks<W>(r0, k0, k1, grid_rows);
+  int first[2];  // list of row r0 and each chunk, -1: none
+  first[0] = r0 >= 0 ? r0 * nchunks + k0 : -1;
+  first[1] = r0 >= 0 && k1 != k0 ? r0 * nchunks + k1 : -1;
+  const int wrap = grid_rows - r0;  // rows from here on wrap
+  auto list_of = [&](int j, int h) { return first[h] + (j >= wrap ? j - grid_rows : j) * nchunks; };
+  __syncthreads();  // the positions are loaded, and every warp's last turn is over
+  if (warp > 0) asm volatile("bar.sync %0, 64;" ::"r"(warp) : "memory");
 #pragma unroll
   for (int j = 0; j < W; ++j)
-    if (j == ta) wr = w[4 + j];
-  put_entry<W>(sidx, __float_as_int(w[1]), wr, w + 4 + W, col_lo, grid_cols, out);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (first[h] >= 0) pos[j][h] = at[list_of(j, h)];
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (first[h] >= 0) {
+        pos[j][h] += (ranks.below[h][j / 4] >> (8 * (j & 3))) & 255u;
+        if (!((ranks.above[h] >> j) & 1u)) at[list_of(j, h)] = pos[j][h] + 1;
+      }
+    }
+  }
+  __syncwarp();
+  if (warp + 1 < kBinWarps) asm volatile("bar.arrive %0, 64;" ::"r"(warp + 1) : "memory");
+}
+
+// One block per (block of samples, frame): kBinThreads samples at a time, their
+// places in turn (place_turn), their entries written outside the turns.
+//
+// Bound by the chain of turns and, for one frame, by launches: appending to the
+// lists with atomics and sorting each
+// afterwards took three kernels (scatter, sort, long sort: 40 us of a 128-grid
+// slice, 92 us of 205824 samples on a 512 grid, 219 us of 96 frames of 13056
+// samples) where this and k_bin_prefix take 21, 60 and 144.  (Finding the ranks inside the
+// turns, by lane masks per list in shared memory, took 203 of the 144.)
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
+  extern __shared__ uint32_t place_smem[];
+  uint32_t* at = place_smem;  // running position of each list
+  const int f = blockIdx.y;
+  {
+    const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
+    const uint32_t* st = a.starts + (static_cast<size_t>(f) * gridDim.x + blockIdx.x) * a.lists_per_frame;
+#pragma unroll 4
+    for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) at[l] = __ldg(off + l) + __ldg(st + l);
+  }
+  const SampleRecord<W>* recs = reinterpret_cast<const SampleRecord<W>*>(a.records) + static_cast<size_t>(f) * a.samples;
+  const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
+  for (int base = s0; base < s1; base += kBinThreads) {
+    const int sample = base + threadIdx.x;
+    constexpr int kRV = static_cast<int>(sizeof(SampleRecord<W>) / 16);
+    float4 q[kRV];
+    if (sample < s1) {
+#pragma unroll
+      for (int v = 0; v < kRV; ++v) q[v] = __ldg(reinterpret_cast<const float4*>(recs + sample) + v);
+    }
+    const float* w = reinterpret_cast<const float*>(q);
+    const int r0 = sample < s1 ? __float_as_int(w[0]) : -1;  // -1: also a padding sample of a ragged batch
+    const int c0 = r0 >= 0 ? __float_as_int(w[1]) : 0;
+    int k0, k1;
+    list_chunks<W>(c0, a.grid_cols, &k0, &k1);
+    uint32_t pos[W][2];
+    place_turn<W>(at, r0, k0, k1, a.nchunks, a.grid_rows, pos);
+    if (r0 < 0) continue;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h && k1 == k0) continue;
+        const size_t slot = static_cast<size_t>(f) * a.entries_per_frame + pos[j][h];
+        if (a.expanded != nullptr)
+          put_entry<W>(static_cast<uint32_t>(sample), c0, w[4 + j], w + 4 + W, (h ? k1 : k0) * kChunk, a.grid_cols,
+                       a.expanded + slot * entry_bytes(W));
+        else
+          a.entries[slot] = static_cast<uint32_t>(sample);
+      }
+    }
+  }
 }
 
 // The 3-D form: the list's plane and row weights folded together.
@@ -719,6 +883,8 @@ __device__ __forceinline__ void expand_entry3(const SampleRecord3<W>* recs, uint
   put_entry<W>(sidx, __float_as_int(w[2]), wr * wz, w + 6 + 2 * W, col_lo, grid, out);
 }
 
+// The lists of a 3-D call: a frame f is a grid plane, offsets are absolute (one
+// entry array for all planes).
 struct SortArgs {
   const uint32_t* offsets;
   uint32_t* entries;
@@ -729,8 +895,6 @@ struct SortArgs {
   uint32_t* mid_lists;   // lists of 33 .. `capacity` entries, left to the warps of k_sort_long
   uint32_t* mid_count;
   int frames, samples, lists_per_frame, nchunks, grid_rows, grid_cols, capacity;
-  size_t entries_per_frame;  // 0 when the offsets are absolute (3-D: one entry array for all planes)
-  int dim3;                  // 3-D: frames are grid planes and the records are per sample (SampleRecord3)
 };
 
 // Expanded entry i of list l of frame f (sample index sidx).
@@ -738,13 +902,8 @@ template <int W>
 __device__ __forceinline__ void expand_at(const SortArgs& a, int f, int l, uint32_t begin, int i, uint32_t sidx) {
   const int row = l / a.nchunks;
   const int col_lo = (l - row * a.nchunks) * kChunk;
-  unsigned char* out = a.expanded + (static_cast<size_t>(f) * a.entries_per_frame + begin + i) * entry_bytes(W);
-  if (a.dim3)
-    expand_entry3<W>(reinterpret_cast<const SampleRecord3<W>*>(a.records), sidx, f, row, col_lo,
-                     a.grid_cols, out);
-  else
-    expand_entry<W>(reinterpret_cast<const SampleRecord<W>*>(a.records) + static_cast<size_t>(f) * a.samples, sidx, row,
-                    col_lo, a.grid_rows, a.grid_cols, out);
+  unsigned char* out = a.expanded + (static_cast<size_t>(begin) + i) * entry_bytes(W);
+  expand_entry3<W>(reinterpret_cast<const SampleRecord3<W>*>(a.records), sidx, f, row, col_lo, a.grid_cols, out);
 }
 
 // Expanded entries of list l of frame f, entries i = first, first + step, ...
@@ -796,7 +955,7 @@ __device__ __forceinline__ void sort_list(const SortArgs& a, int f, int l, uint3
     }
     return;
   }
-  uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+  uint32_t* ent = a.entries + begin;
   const uint32_t key = lane < n ? ent[lane] : 0xffffffffu;
   int rank = 0;
   for (int j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key ? 1 : 0;
@@ -835,7 +994,7 @@ __global__ void __launch_bounds__(256) k_sort(SortArgs a) {
     }
     return;
   }
-  uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+  uint32_t* ent = a.entries + begin;
   const bool live = lane < total;
   const uint32_t key = live ? ent[lane] : 0xffffffffu;
   int seg = 0;  // list of entry `lane` within the group (empty lists are skipped over)
@@ -970,7 +1129,7 @@ __device__ __forceinline__ void sort_long_list(const SortArgs& a, size_t gl, uin
   const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
   const uint32_t begin = off[l];
   const int n = static_cast<int>(off[l + 1] - begin);
-  uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+  uint32_t* ent = a.entries + begin;
   const uint32_t* sorted = ent;
   if (n <= kLongSortSmem) {
     chunk_load(long_buf, ent, n);
@@ -1009,7 +1168,7 @@ __global__ void __launch_bounds__(kLongSortThreads, 1) k_sort_long(SortArgs a) {
     const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
     const uint32_t begin = off[l];
     const int n = static_cast<int>(off[l + 1] - begin);
-    uint32_t* ent = a.entries + static_cast<size_t>(f) * a.entries_per_frame + begin;
+    uint32_t* ent = a.entries + begin;
     if (n <= 64)
       sort_list_regs<W, 2>(a, f, l, begin, n, lane, ent);
     else if (n <= 128)
@@ -2028,17 +2187,21 @@ struct ColsPass {
   }
 };
 
-// The binning lists of one call: per-sample records, list counts, offsets,
-// the scattered entries and their sort (and, when `expanded` is given, the
-// expanded entries the row pass reads), and the call's tables where `tables`
-// names them.  The flags and counts must already be cleared.
+// The binning lists of one call: per-sample records, list offsets, and the lists'
+// entries in sample order, as the row pass reads them (`expanded`) or as sample
+// indices alone (`entries`); and the call's tables where `tables` names them.  The
+// flags must already be cleared.
 template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
-                           uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
-                           uint32_t* offsets, uint32_t* entries, unsigned char* expanded, uint32_t* long_lists,
-                           uint32_t* mid_lists, cudaStream_t stream, uint32_t* frame_flags = nullptr,
-                           const TablesArgs* tables = nullptr) {
-  const size_t fm = static_cast<size_t>(s.frames) * s.samples;
+                           uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* totals,
+                           uint32_t* offsets, uint32_t* entries, unsigned char* expanded, cudaStream_t stream,
+                           uint32_t* frame_flags = nullptr, const TablesArgs* tables = nullptr) {
+  const int count_smem = s.lists_per_frame * 4;
+  const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
+  if (cudaFuncSetAttribute(k_prepare<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, count_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_place<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
+    return KSJ_GPU_ERROR_CUDA;
+  const dim3 blocks(s.bin_blocks, s.frames);
   {
     PrepareArgs p{};
     p.traj = d_traj;
@@ -2057,6 +2220,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.grid_cols = s.grid_cols;
     p.nchunks = s.nchunks;
     p.lists_per_frame = s.lists_per_frame;
+    p.bin_span = s.bin_span;
     p.kb = s.kb ? 1 : 0;
     p.beta = s.beta;
     p.two_over_w = 2.0f / static_cast<float>(s.width);
@@ -2065,36 +2229,30 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.phase_col = s.phase_col;
     p.phase_sign = s.phase_sign;
     LaunchScope scope("k_prepare", stream);
-    k_prepare<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(p);
-  }
-  launch_scan(counts, offsets, cursor, s.lists_per_frame, s.frames, mid_lists, long_lists, tables, stream);
-  {
-    LaunchScope scope("k_scatter", stream);
-    k_scatter<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
-        records, cursor, entries, s.frames, s.samples, s.grid_rows, s.grid_cols, s.nchunks,
-        s.entries_per_frame);
+    k_prepare<W><<<blocks, kBinThreads, count_smem, stream>>>(p);
   }
   {
-    SortArgs sa{};
-    sa.offsets = offsets;
-    sa.entries = entries;
-    sa.records = records;
-    sa.expanded = expanded;
-    sa.long_count = long_lists;
-    sa.long_lists = long_lists + 1;
-    sa.mid_count = mid_lists;
-    sa.mid_lists = mid_lists + 1;
-    sa.frames = s.frames;
-    sa.samples = s.samples;
-    sa.lists_per_frame = s.lists_per_frame;
-    sa.nchunks = s.nchunks;
-    sa.grid_rows = s.grid_rows;
-    sa.grid_cols = s.grid_cols;
-    sa.capacity = s.list_capacity;
-    sa.entries_per_frame = s.entries_per_frame;
-    sa.dim3 = 0;
-    const ksj_gpu_status st = launch_sort<W>(sa, stream);
-    if (st != KSJ_GPU_OK) return st;
+    LaunchScope scope("k_bin_prefix", stream);
+    k_bin_prefix<<<dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream>>>(counts, totals, s.bin_blocks,
+                                                                                    s.lists_per_frame);
+  }
+  launch_scan(totals, offsets, nullptr, s.lists_per_frame, s.frames, nullptr, nullptr, tables, stream);
+  {
+    PlaceArgs p{};
+    p.records = records;
+    p.offsets = offsets;
+    p.starts = counts;
+    p.expanded = expanded;
+    p.entries = entries;
+    p.samples = s.samples;
+    p.grid_rows = s.grid_rows;
+    p.grid_cols = s.grid_cols;
+    p.nchunks = s.nchunks;
+    p.lists_per_frame = s.lists_per_frame;
+    p.bin_span = s.bin_span;
+    p.entries_per_frame = s.entries_per_frame;
+    LaunchScope scope("k_place", stream);
+    k_place<W><<<blocks, kBinThreads, place_smem, stream>>>(p);
   }
   return KSJ_GPU_OK;
 }
@@ -2121,10 +2279,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
                           cudaStream_t stream, const HostIo* io = nullptr) {
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
   unsigned char* records = ws + l.records;
-  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + l.counts);
-  uint32_t* cursor = reinterpret_cast<uint32_t*>(ws + l.cursor);
   uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + l.offsets);
-  uint32_t* entries = reinterpret_cast<uint32_t*>(ws + l.entries);
   float2* inter = reinterpret_cast<float2*>(ws + l.inter);
   float2* tw_rows = reinterpret_cast<float2*>(ws + l.tables);
   float2* tw_cols = tw_rows + s.grid_rows;
@@ -2139,11 +2294,10 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
                           s.out_cols, s.plan_rows, s.plan_cols, s.kb ? 1 : 0, s.width, beta,
                           s.kb ? std::cyl_bessel_i(0.0, beta) : 1.0};
   {
-    const ksj_gpu_status st = build_lists<W>(s, d, d_traj, d_dcf, flags, records, counts, cursor, offsets, entries,
-                                             ws + l.expanded,
-                                             reinterpret_cast<uint32_t*>(ws + l.long_lists),
-                                             reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream,
-                                             reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables);
+    const ksj_gpu_status st =
+        build_lists<W>(s, d, d_traj, d_dcf, flags, records, reinterpret_cast<uint32_t*>(ws + l.counts),
+                       reinterpret_cast<uint32_t*>(ws + l.totals), offsets, nullptr, ws + l.expanded, stream,
+                       reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables);
     if (st != KSJ_GPU_OK) return st;
   }
   auto to_coil_last = [&](int f0, int nf, cudaStream_t st) {
@@ -2443,7 +2597,7 @@ __global__ void __launch_bounds__(256) k_pm_update(const PmRecord<W>* pm, const 
 }
 
 struct PmLayout {
-  size_t flags, cleared, records, counts, cursor, offsets, entries, long_lists, mid_lists, pm, w, grid, total;
+  size_t flags, records, counts, totals, offsets, entries, pm, w, grid, total;
 };
 
 PmLayout make_pm_layout(const Shape& s) {
@@ -2456,15 +2610,12 @@ PmLayout make_pm_layout(const Shape& s) {
   };
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
-  l.flags = take(kFlagBytes);  // flags and counts are cleared together
-  l.counts = take(nl * 4);
-  l.cleared = off;
+  l.flags = take(kFlagBytes);
   l.records = take(fm * record_bytes(s.width));
-  l.cursor = take(nl * 4);
+  l.counts = take(nl * s.bin_blocks * 4);
+  l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
-  l.long_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / (s.list_capacity + 1)) * 4);
-  l.mid_lists = take((2 + static_cast<size_t>(s.frames) * s.entries_per_frame / 33) * 4);
   l.pm = take(fm * (8 + 16 * static_cast<size_t>(s.width)));
   l.w = take(fm * sizeof(double));
   l.grid = take(static_cast<size_t>(s.frames) * s.grid_rows * s.grid_cols * sizeof(double));
@@ -2478,15 +2629,13 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
                                  cudaStream_t stream) {
   static_assert(sizeof(PmRecord<W>) == 8 + 16 * W, "PmRecord layout");
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   ksj_gpu_gridding_desc dd = *d;
   dd.dcf_mode = KSJ_GPU_DCF_NONE;
   const ksj_gpu_status st =
       build_lists<W>(s, &dd, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
-                     reinterpret_cast<uint32_t*>(ws + l.cursor), reinterpret_cast<uint32_t*>(ws + l.offsets),
-                     reinterpret_cast<uint32_t*>(ws + l.entries), nullptr,
-                     reinterpret_cast<uint32_t*>(ws + l.long_lists), reinterpret_cast<uint32_t*>(ws + l.mid_lists),
-                     stream);
+                     reinterpret_cast<uint32_t*>(ws + l.totals), reinterpret_cast<uint32_t*>(ws + l.offsets),
+                     reinterpret_cast<uint32_t*>(ws + l.entries), nullptr, stream);
   if (st != KSJ_GPU_OK) return st;
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   PmRecord<W>* pm = reinterpret_cast<PmRecord<W>*>(ws + l.pm);
@@ -2784,8 +2933,6 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     sa.grid_rows = g;
     sa.grid_cols = g;
     sa.capacity = s.list_capacity;
-    sa.entries_per_frame = 0;
-    sa.dim3 = 1;
     const ksj_gpu_status st = launch_sort<W>(sa, stream);
     if (st != KSJ_GPU_OK) return st;
   }
