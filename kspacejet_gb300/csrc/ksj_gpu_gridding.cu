@@ -1295,24 +1295,27 @@ struct RowsArgs {
   DifPlan plan;
 };
 
-// Lists longer than kSegMin entries are gridded in segments (at most
+// Lists longer than a row's unit are gridded in segments (at most
 // kSegMax, all but the last of segment_length entries) that different lane
 // groups take at once, so that a row's long lists do not hold its CTA at the
 // barrier after the gridding while one warp works through each; a cell is then
 // the sum, in segment order, of its segments' partial sums, each partial sum
 // in sample order from zero.  Shorter lists are one segment: the cell is its
-// samples' sum in sample order.  Every coil grouping uses the same segments.
-constexpr int kSegMin = 32;
+// samples' sum in sample order.  The unit is kSegMin entries, or a 32nd of the
+// row's where that is more (a row with that many has lists enough to share out,
+// and every segment pays for putting its 16 cells in turn): it depends on the
+// lists alone, so every coil grouping gives the same cells.  Units of 32, 64, 128 entries
+// and this rule measured, us of the row pass: 8 coils on a 128 grid 35, 29, 33,
+// 28, on a 512 grid 131, 107, 99, 95; a 32-coil frame 35, 31, 37, 32.
+constexpr int kSegMin = 64;
 constexpr int kSegMax = 32;
 
-__host__ __device__ inline int list_segments(int n) {
-  return n <= kSegMin ? 1 : ((n + kSegMin - 1) / kSegMin < kSegMax ? (n + kSegMin - 1) / kSegMin : kSegMax);
+__device__ __forceinline__ int list_segments(int n, int unit) {
+  return n <= unit ? 1 : min((n + unit - 1) / unit, kSegMax);
 }
-static_assert(kSegMin * kSegMax <= (1 << 22), "segment counts are taken from lengths capped at 2^22");
-
-__host__ __device__ inline int segment_length(int n) {
-  if (n <= kSegMin) return n;  // one segment (most lists): no division
-  const int sg = list_segments(n);
+__device__ __forceinline__ int segment_length(int n, int unit) {
+  if (n <= unit) return n;  // one segment (most lists): no division
+  const int sg = list_segments(n, unit);
   return (n + sg - 1) / sg;
 }
 
@@ -1504,7 +1507,8 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
     // capped at 2^22 entries: the same count, since kSegMin * kSegMax entries
     // already take the most segments)
     const int len = lane < a.nchunks ? (key >> 8) : 0;
-    const int nseg = lane < a.nchunks ? list_segments(len) : 0;
+    const int unit = max(kSegMin, (__reduce_add_sync(0xffffffffu, len) + 32 - 1) / 32);
+    const int nseg = lane < a.nchunks ? list_segments(len, unit) : 0;
     int incl = nseg;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -1516,7 +1520,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
     length = __shfl_sync(0xffffffffu, length, chunk);
     if (lane < a.nchunks) {
       const int n = static_cast<int>(length);
-      task_list[lane] = make_int4(static_cast<int>(start), n, segment_length(n), chunk);
+      task_list[lane] = make_int4(static_cast<int>(start), n, segment_length(n, unit), chunk);
       task_base[lane] = incl - nseg;
     }
     if (lane == a.nchunks - 1) task_base[a.nchunks] = incl;
