@@ -177,59 +177,31 @@ extern "C" ksj_gpu_status ksj_gpu_walsh_combine(uint32_t rows, uint32_t cols, ui
 // element of A is split as hi + lo (both bf16, hi = bf16(a), lo = bf16(a - hi))
 // and G ~= hi hi^T + lo hi^T + (lo hi^T)^T, every product accumulated in FP32
 // by the tensor cores:
-//   k_cov_split   X -> the operand [hi(Re); hi(Im); lo(Re); lo(Im)] (128 rows of bf16, samples contiguous)
-//   k_cov_mma     per block a range of 64-sample tiles: TMA (128-byte swizzle) into a 4-stage ring,
-//                 one thread issues tcgen05.mma M=128 (the whole operand), N=64 (its hi rows, the same
-//                 shared memory), K=16; the 128 x 64 FP32 accumulator lives in tensor memory and is
-//                 read out once by the four warps
-//   k_cov_sum / k_cov_form  sum the blocks' accumulators in block order and form R (deterministic)
+//   k_cov_mma     per block a range of 64-sample tiles of X: split in registers into the operand
+//                 [hi(Re); hi(Im); lo(Re); lo(Im)] (128 rows of bf16) and stored to one of two
+//                 shared-memory stages in the 128-byte swizzle, the next tile's samples already
+//                 requested; one thread issues tcgen05.mma M=128 (the whole operand), N=64 (its hi
+//                 rows, the same shared memory), K=16; the 128 x 64 FP32 accumulator lives in tensor
+//                 memory and is read out once by four warps
+//   k_cov_form    sums the blocks' accumulators in a fixed order; its last block forms R or the
+//                 noise covariance (deterministic)
 
 namespace ksj_gpu {
 namespace {
 
 constexpr int kCovRows = 128;
 constexpr int kCovKTile = 64;  // samples per stage: 128 bytes of bf16 per operand row
-constexpr int kCovStages = 4;
+constexpr int kCovStages = 2;
 constexpr uint32_t kCovStageBytes = kCovRows * kCovKTile * 2;
-constexpr int kCovThreads = 128;
+constexpr int kCovThreads = 256;
 constexpr uint32_t kCovWaitLimit = 1u << 22;
-constexpr int kCovMaxBlocks = 304;
+constexpr int kCovMaxBlocks = 304;  // two per SM
 
-// Four consecutive samples of one coil per thread: four 8-byte loads (a
-// warp reads 1 KiB contiguous) and one 8-byte store per operand row.
-constexpr int kSplitPerThread = 4;
-static_assert(kCovKTile % kSplitPerThread == 0, "padded sample count is a multiple of the per-thread samples");
-
-__global__ void __launch_bounds__(256) k_cov_split(const float2* __restrict__ x, uint16_t* a, int channels,
-                                                   int samples, int kpad) {
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int quads = kpad / kSplitPerThread;
-  if (idx >= static_cast<size_t>(32) * quads) return;
-  const int c = static_cast<int>(idx / quads);
-  const int s0 = static_cast<int>(idx - static_cast<size_t>(c) * quads) * kSplitPerThread;
-  uint16_t h[2][kSplitPerThread], l[2][kSplitPerThread];
-#pragma unroll
-  for (int i = 0; i < kSplitPerThread; ++i) {
-    const int sm = s0 + i;
-    float2 v = make_float2(0.0f, 0.0f);
-    if (c < channels && sm < samples) v = __ldg(x + static_cast<size_t>(c) * samples + sm);
-    const __nv_bfloat16 hr = __float2bfloat16_rn(v.x);
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v.y);
-    h[0][i] = __bfloat16_as_ushort(hr);
-    h[1][i] = __bfloat16_as_ushort(hi);
-    l[0][i] = __bfloat16_as_ushort(__float2bfloat16_rn(v.x - __bfloat162float(hr)));
-    l[1][i] = __bfloat16_as_ushort(__float2bfloat16_rn(v.y - __bfloat162float(hi)));
-  }
-  auto pack = [](const uint16_t (&v)[kSplitPerThread]) {
-    return make_uint2(static_cast<uint32_t>(v[0]) | (static_cast<uint32_t>(v[1]) << 16),
-                      static_cast<uint32_t>(v[2]) | (static_cast<uint32_t>(v[3]) << 16));
-  };
-  const size_t k = static_cast<size_t>(kpad);
-  *reinterpret_cast<uint2*>(a + static_cast<size_t>(c) * k + s0) = pack(h[0]);
-  *reinterpret_cast<uint2*>(a + static_cast<size_t>(32 + c) * k + s0) = pack(h[1]);
-  *reinterpret_cast<uint2*>(a + static_cast<size_t>(64 + c) * k + s0) = pack(l[0]);
-  *reinterpret_cast<uint2*>(a + static_cast<size_t>(96 + c) * k + s0) = pack(l[1]);
-}
+// Four consecutive samples of one coil per thread and turn, two turns per tile
+// (32 coils x 64 samples): eight 8-byte loads in flight, one 8-byte store per
+// operand row and turn (a half-warp stores one row's 128 bytes).
+constexpr int kCovQuad = 4;
+constexpr int kCovTurns = 32 * kCovKTile / kCovQuad / kCovThreads;
 
 // Shared-memory matrix descriptor of a K-major operand in the 128-byte swizzle
 // layout (8-row x 128-byte atoms stacked 1024 bytes apart along M/N).
@@ -245,13 +217,6 @@ __device__ __forceinline__ uint64_t sw128_kmajor_desc(uint32_t saddr) {
 // Instruction descriptor, kind::f16: FP32 accumulator, bf16 A and B, both
 // K-major, N = 64, M = 128.
 constexpr uint32_t kCovIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const void* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_addr(bar))
-      : "memory");
-}
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
@@ -282,16 +247,62 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 }
 
 struct CovArgs {
+  const float2* x;  // [channels][samples]
   float* partials;  // [blocks][128][64]
   uint32_t* flags;
-  int ktiles;
+  int channels, samples, ktiles;
 };
 
-__global__ void __launch_bounds__(kCovThreads) k_cov_mma(const __grid_constant__ CUtensorMap amap, CovArgs a) {
+// One tile's samples of this thread's quads (zero past the channels and samples).
+__device__ __forceinline__ void cov_load(const CovArgs& a, int tile, float2 (&v)[kCovTurns][kCovQuad]) {
+#pragma unroll
+  for (int u = 0; u < kCovTurns; ++u) {
+    const int q = threadIdx.x + u * kCovThreads;
+    const int c = q / (kCovKTile / kCovQuad);
+    const int s0 = tile * kCovKTile + (q % (kCovKTile / kCovQuad)) * kCovQuad;
+    const float2* src = a.x + static_cast<size_t>(c) * a.samples + s0;
+#pragma unroll
+    for (int i = 0; i < kCovQuad; ++i)
+      v[u][i] = c < a.channels && s0 + i < a.samples ? __ldg(src + i) : make_float2(0.0f, 0.0f);
+  }
+}
+
+// Split into hi and lo and stored: operand row r at r * 128 bytes, its 16-byte
+// chunk k at k ^ (r mod 8) (the 128-byte swizzle of a 1024-byte aligned stage).
+__device__ __forceinline__ void cov_store(unsigned char* stage, const float2 (&v)[kCovTurns][kCovQuad]) {
+#pragma unroll
+  for (int u = 0; u < kCovTurns; ++u) {
+    const int q = threadIdx.x + u * kCovThreads;
+    const int c = q / (kCovKTile / kCovQuad), quad = q % (kCovKTile / kCovQuad);
+    uint32_t h[2][2], l[2][2];  // [Re, Im][pair of samples]
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 p = v[u][2 * i], n = v[u][2 * i + 1];
+      const __nv_bfloat162 hr = __floats2bfloat162_rn(p.x, n.x), hi = __floats2bfloat162_rn(p.y, n.y);
+      const __nv_bfloat162 lr = __floats2bfloat162_rn(p.x - __low2float(hr), n.x - __high2float(hr));
+      const __nv_bfloat162 li = __floats2bfloat162_rn(p.y - __low2float(hi), n.y - __high2float(hi));
+      h[0][i] = *reinterpret_cast<const uint32_t*>(&hr);
+      h[1][i] = *reinterpret_cast<const uint32_t*>(&hi);
+      l[0][i] = *reinterpret_cast<const uint32_t*>(&lr);
+      l[1][i] = *reinterpret_cast<const uint32_t*>(&li);
+    }
+    // rows c, 32 + c, 64 + c and 96 + c: the same row mod 8
+    unsigned char* dst = stage + c * 128 + (((quad >> 1) ^ (c & 7)) << 4) + ((quad & 1) << 3);
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      *reinterpret_cast<uint2*>(dst + part * 32 * 128) = make_uint2(h[part][0], h[part][1]);
+      *reinterpret_cast<uint2*>(dst + (2 + part) * 32 * 128) = make_uint2(l[part][0], l[part][1]);
+    }
+  }
+}
+
+// Bound by reading X once: 412160 samples x 32 coils (105 MB) in 27 us; splitting into a
+// bf16 operand in memory first (another 105 MB written and read) took 58.
+__global__ void __launch_bounds__(kCovThreads, 2) k_cov_mma(CovArgs a) {
   extern __shared__ __align__(16) unsigned char cov_smem[];
   // stage buffers on a 1024-byte boundary (128-byte swizzle atoms)
   unsigned char* base = cov_smem + ((1024u - (smem_addr(cov_smem) & 1023u)) & 1023u);
-  __shared__ __align__(8) uint64_t full[kCovStages], empty[kCovStages], done;
+  __shared__ __align__(8) uint64_t empty[kCovStages], done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed;
   const int tid = threadIdx.x;
@@ -300,10 +311,7 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_mma(const __grid_constant__
   const int t1 = static_cast<int>(static_cast<long long>(a.ktiles) * (blockIdx.x + 1) / gridDim.x);
   const int n = t1 - t0;
   if (tid == 0) {
-    for (int s = 0; s < kCovStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
-    }
+    for (int s = 0; s < kCovStages; ++s) mbar_init(&empty[s], 1);
     mbar_init(&done, 1);
     mbar_init_fence();
     failed = 0;
@@ -318,29 +326,22 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_mma(const __grid_constant__
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_base;
 
-  if (tid == 0) {
-    int issued = 0;  // tiles whose copy was started
-    auto stage_ptr = [&](int s) { return base + static_cast<size_t>(s) * kCovStageBytes; };
-    auto load = [&](int j) {
-      const int s = j % kCovStages;
-      mbar_arrive_expect_tx(&full[s], kCovStageBytes);
-      tma_load_2d(stage_ptr(s), &amap, (t0 + j) * kCovKTile, 0, &full[s]);
-      ++issued;
-    };
-    bool ok = true;
-    for (int j = 0; j < kCovStages - 1 && j < n; ++j) load(j);
-    for (int i = 0; i < n && ok; ++i) {
-      const int j = i + kCovStages - 1;
-      if (j < n) {
-        // the slot's previous tile (j - stages) must have been consumed by its MMAs
-        if (j >= kCovStages) ok = mbar_wait_bounded(&empty[j % kCovStages], ((j / kCovStages) - 1) & 1, kCovWaitLimit);
-        if (!ok) break;
-        load(j);
-      }
-      const int s = i % kCovStages;
-      ok = mbar_wait_bounded(&full[s], (i / kCovStages) & 1, kCovWaitLimit);
-      if (!ok) break;
-      const uint32_t sa = smem_addr(stage_ptr(s));
+  float2 v[kCovTurns][kCovQuad];
+  if (n > 0) cov_load(a, t0, v);
+  bool ok = true;
+  for (int i = 0; i < n; ++i) {
+    const int s = i & 1;
+    unsigned char* stage = base + s * kCovStageBytes;
+    // the stage's previous tile must have been consumed by its MMAs
+    if (i >= kCovStages) ok = mbar_wait_bounded(&empty[s], ((i >> 1) - 1) & 1, kCovWaitLimit);
+    if (ok) cov_store(stage, v);
+    if (i + 1 < n) cov_load(a, t0 + i + 1, v);
+    fence_proxy_async_shared();  // the stores, before the MMAs read them
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t sa = smem_addr(stage);
 #pragma unroll
       for (int k = 0; k < kCovKTile / 16; ++k) {
         const uint64_t d = sw128_kmajor_desc(sa + k * 32);
@@ -348,34 +349,34 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_mma(const __grid_constant__
       }
       umma_commit(&empty[s]);
     }
+  }
+  if (tid == 0) {
     // every MMA issued so far completes before `done` fires
     umma_commit(&done);
     const bool fin = mbar_wait_bounded(&done, 0, kCovWaitLimit);
     if (!ok || !fin) {
       failed = 1;
       atomicOr(a.flags, KSJ_GPU_FLAG_WAIT_TIMEOUT);
-      // let every copy this block started land before its shared memory goes
-      for (int j = 0; j < issued; ++j) mbar_wait_bounded(&full[j % kCovStages], (j / kCovStages) & 1, kCovWaitLimit);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!failed) {
+  if (!failed && warp < 4) {
     // accumulator row 32*warp + lane, 64 FP32 columns
     const int row = warp * 32 + (tid & 31);
     float* dst = a.partials + (static_cast<size_t>(blockIdx.x) * kCovRows + row) * 64;
 #pragma unroll
     for (int c = 0; c < 64; c += 16) {
-      float v[16];
-      tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + c, v);
+      float w[16];
+      tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + c, w);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (n == 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+        for (int i = 0; i < 16; ++i) w[i] = 0.0f;
       }
 #pragma unroll
-      for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(dst + c + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(dst + c + i) = make_float4(w[i], w[i + 1], w[i + 2], w[i + 3]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -383,31 +384,68 @@ __global__ void __launch_bounds__(kCovThreads) k_cov_mma(const __grid_constant__
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
 }
 
-// Sum of the blocks' accumulators, one thread per accumulator element (the
-// blocks' copies of an element are 32 KiB apart: coalesced across threads),
-// in block order.
-__global__ void __launch_bounds__(256) k_cov_sum(const float* partials, int blocks, float* sum) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= kCovRows * 64) return;
-  float s = 0.0f;
-#pragma unroll 8
-  for (int b = 0; b < blocks; ++b) s += partials[static_cast<size_t>(b) * kCovRows * 64 + e];
-  sum[e] = s;
-}
+// The covariance from the blocks' accumulators.  Each block sums 32
+// accumulator elements, eight threads an element over an eighth of the blocks'
+// copies each (in block order, the eighths then added in order: deterministic,
+// and eight short chains of loads where one per element waited out all of
+// them); the last block to finish forms the elements of R or of the noise covariance.
+//
+// G = hi hi^T + lo hi^T + (lo hi^T)^T, R = G times 1/M (in float, as the
+// reference scales its sums).  The lower triangle is computed and the upper
+// mirrored (conjugate), as the reference stores it, so R is Hermitian bit for bit.
+//
+// means non-null: the noise covariance of noise_model_estimate.cpp:161-162
+// (covariance_channel_major_with_workspace, population normalisation,
+// moments.hpp:99-140), C(r, c) = (1/M) sum_s conj(x_r - mu_r) (x_c - mu_c)
+// = conj(R(r, c) - mu_r conj(mu_c)); lower triangle computed, upper mirrored.
+constexpr int kCovSumElems = 32, kCovSumSlices = 8;
+static_assert(kCovRows * 64 % kCovSumElems == 0, "whole blocks of elements");
 
-// One thread per covariance element: G = hi hi^T + lo hi^T + (lo hi^T)^T from
-// the summed accumulator, then R times 1/M (in float, as the reference scales
-// its sums).  The lower triangle is computed and the upper mirrored
-// (conjugate), as the reference stores it, so R is Hermitian bit for bit.
-__global__ void __launch_bounds__(256) k_cov_form(const float* d, int channels, float inv_m, float2* cov) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= channels * channels) return;
-  const int i = idx / channels, j = idx - (idx / channels) * channels;
-  auto g = [&](int r, int c) { return d[r * 64 + c] + d[(64 + r) * 64 + c] + d[(64 + c) * 64 + r]; };
-  const int r = i >= j ? i : j, c = i >= j ? j : i;
-  const float re = g(r, c) + g(32 + r, 32 + c);
-  const float im = r == c ? 0.0f : g(32 + r, c) - g(r, 32 + c);
-  cov[idx] = make_float2(re * inv_m, (i >= j ? im : -im) * inv_m);
+__global__ void __launch_bounds__(kCovSumElems * kCovSumSlices) k_cov_form(const float* partials, int blocks, float* sum,
+                                                                           uint32_t* finished, int channels,
+                                                                           float inv_m,
+                                                                           const float2* __restrict__ means,
+                                                                           float2* cov) {
+  __shared__ float part[kCovSumSlices][kCovSumElems];
+  __shared__ bool last;
+  const int el = threadIdx.x % kCovSumElems, slice = threadIdx.x / kCovSumElems;
+  const int e = blockIdx.x * kCovSumElems + el;
+  const int b0 = blocks * slice / kCovSumSlices, b1 = blocks * (slice + 1) / kCovSumSlices;
+  float s = 0.0f;
+#pragma unroll 20
+  for (int b = b0; b < b1; ++b) s += __ldg(partials + static_cast<size_t>(b) * kCovRows * 64 + e);
+  part[slice][el] = s;
+  __syncthreads();
+  if (slice == 0) {
+    for (int k = 1; k < kCovSumSlices; ++k) s += part[k][el];
+    sum[e] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(finished, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  auto g = [&](int r, int c) {
+    return __ldcg(sum + r * 64 + c) + __ldcg(sum + (64 + r) * 64 + c) + __ldcg(sum + (64 + c) * 64 + r);
+  };
+  for (int idx = threadIdx.x; idx < channels * channels; idx += blockDim.x) {
+    const int i = idx / channels, j = idx - (idx / channels) * channels;
+    const int r = i >= j ? i : j, c = i >= j ? j : i;
+    const float re = (g(r, c) + g(32 + r, 32 + c)) * inv_m;
+    const float im = r == c ? 0.0f : (g(32 + r, c) - g(r, 32 + c)) * inv_m;
+    if (means == nullptr) {
+      cov[idx] = make_float2(re, i >= j ? im : -im);
+    } else {
+      const float2 mr = means[r], mc = means[c];
+      // d = R(r, c) - mu_r conj(mu_c); C(r, c) = conj(d), C(c, r) = d
+      const float dre = re - (mr.x * mc.x + mr.y * mc.y);
+      const float dim = r == c ? 0.0f : im - (mr.y * mc.x - mr.x * mc.y);
+      cov[idx] = make_float2(dre, i >= j ? -dim : dim);
+    }
+  }
 }
 
 // Per-channel mean of channel-major X [channels][samples] (one block per
@@ -437,53 +475,14 @@ __global__ void __launch_bounds__(256) k_channel_means(const float2* __restrict_
   }
 }
 
-// The noise covariance of noise_model_estimate.cpp:161-162
-// (covariance_channel_major_with_workspace, population normalisation,
-// moments.hpp:99-140): C(r, c) = (1/M) sum_s conj(x_r - mu_r) (x_c - mu_c)
-// = conj(R(r, c) - mu_r conj(mu_c)) with R = (1/M) X X^H as k_cov_form
-// forms it.  The lower triangle is computed and the upper mirrored, so C is
-// Hermitian bit for bit.
-__global__ void __launch_bounds__(256) k_noise_form(const float* d, int channels, float inv_m,
-                                                    const float2* __restrict__ means, float2* cov) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= channels * channels) return;
-  const int i = idx / channels, j = idx - (idx / channels) * channels;
-  auto g = [&](int r, int c) { return d[r * 64 + c] + d[(64 + r) * 64 + c] + d[(64 + c) * 64 + r]; };
-  const int r = i >= j ? i : j, c = i >= j ? j : i;
-  const float rre = (g(r, c) + g(32 + r, 32 + c)) * inv_m;
-  const float rim = r == c ? 0.0f : (g(32 + r, c) - g(r, 32 + c)) * inv_m;
-  const float2 mr = means[r], mc = means[c];
-  // d = R(r, c) - mu_r conj(mu_c)
-  const float dre = rre - (mr.x * mc.x + mr.y * mc.y);
-  const float dim = r == c ? 0.0f : rim - (mr.y * mc.x - mr.x * mc.y);
-  cov[idx] = make_float2(dre, i >= j ? -dim : dim);  // C(r, c) = conj(d); C(c, r) = d
-}
-
-using EncodeTiled2Fn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled2Fn cov_encode() {
-  static EncodeTiled2Fn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<EncodeTiled2Fn>(p);
-  }();
-  return fn;
-}
-
 struct CovLayout {
-  size_t flags, operand, partials, sum, means, total;
-  int kpad, ktiles, blocks;
+  size_t flags, partials, sum, means, total;
+  int ktiles, blocks;
 };
 
 CovLayout cov_layout(uint32_t samples) {
   CovLayout l{};
-  l.kpad = static_cast<int>((samples + kCovKTile - 1) / kCovKTile * kCovKTile);
-  l.ktiles = l.kpad / kCovKTile;
+  l.ktiles = static_cast<int>((samples + kCovKTile - 1) / kCovKTile);
   l.blocks = std::min(l.ktiles, kCovMaxBlocks);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -491,8 +490,7 @@ CovLayout cov_layout(uint32_t samples) {
     off = align_up(off + bytes, 256);
     return at;
   };
-  l.flags = take(16);
-  l.operand = take(static_cast<size_t>(kCovRows) * l.kpad * 2);
+  l.flags = take(16);  // check flags, then the count of finished k_cov_form blocks
   l.partials = take(static_cast<size_t>(l.blocks) * kCovRows * 64 * sizeof(float));
   l.sum = take(static_cast<size_t>(kCovRows) * 64 * sizeof(float));
   l.means = take(32 * sizeof(float2));
@@ -523,60 +521,28 @@ ksj_gpu_status covariance_run(uint32_t channels, uint32_t samples, const void* d
   const CovLayout l = cov_layout(samples);
   if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 || workspace_bytes < l.total)
     return KSJ_GPU_ERROR_WORKSPACE;
-  EncodeTiled2Fn enc = cov_encode();
-  if (enc == nullptr) return KSJ_GPU_ERROR_CUDA;
   unsigned char* ws = static_cast<unsigned char*>(d_workspace);
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  uint16_t* operand = reinterpret_cast<uint16_t*>(ws + l.operand);
   float* partials = reinterpret_cast<float*>(ws + l.partials);
   if (cudaMemsetAsync(flags, 0, 16, cs) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  {
-    const size_t n = static_cast<size_t>(32) * (l.kpad / kSplitPerThread);
-    LaunchScope scope("k_cov_split", cs);
-    k_cov_split<<<static_cast<unsigned>((n + 255) / 256), 256, 0, cs>>>(static_cast<const float2*>(d_kspace),
-                                                                        operand, static_cast<int>(channels),
-                                                                        static_cast<int>(samples), l.kpad);
-  }
-  CUtensorMap map;
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(l.kpad), static_cast<cuuint64_t>(kCovRows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(l.kpad) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kCovKTile), static_cast<cuuint32_t>(kCovRows)};
-  const cuuint32_t estr[2] = {1, 1};
-  if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, operand, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return KSJ_GPU_ERROR_CUDA;
   const size_t smem = 1024 + static_cast<size_t>(kCovStages) * kCovStageBytes;
-  if (cudaFuncSetAttribute(k_cov_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-      cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
   {
-    CovArgs args{partials, flags, l.ktiles};
+    const CovArgs args{static_cast<const float2*>(d_kspace), partials, flags, static_cast<int>(channels),
+                       static_cast<int>(samples), l.ktiles};
     LaunchScope scope("k_cov_mma", cs);
-    k_cov_mma<<<l.blocks, kCovThreads, smem, cs>>>(map, args);
+    k_cov_mma<<<l.blocks, kCovThreads, smem, cs>>>(args);
   }
-  float* sum = reinterpret_cast<float*>(ws + l.sum);
-  {
-    LaunchScope scope("k_cov_sum", cs);
-    k_cov_sum<<<kCovRows * 64 / 256, 256, 0, cs>>>(partials, l.blocks, sum);
-  }
-  const int n = static_cast<int>(channels * channels);
-  const float inv_m = 1.0f / static_cast<float>(samples);
+  float2* means = nullptr;
   if (noise) {
-    float2* means = reinterpret_cast<float2*>(ws + l.means);
-    {
-      LaunchScope scope("k_channel_means", cs);
-      k_channel_means<<<channels, 256, 0, cs>>>(static_cast<const float2*>(d_kspace), static_cast<int>(samples),
-                                                means);
-    }
-    LaunchScope scope("k_noise_form", cs);
-    k_noise_form<<<(n + 255) / 256, 256, 0, cs>>>(sum, static_cast<int>(channels), inv_m, means,
-                                                  static_cast<float2*>(d_cov));
-  } else {
-    LaunchScope scope("k_cov_form", cs);
-    k_cov_form<<<(n + 255) / 256, 256, 0, cs>>>(sum, static_cast<int>(channels), inv_m, static_cast<float2*>(d_cov));
+    means = reinterpret_cast<float2*>(ws + l.means);
+    LaunchScope scope("k_channel_means", cs);
+    k_channel_means<<<channels, 256, 0, cs>>>(static_cast<const float2*>(d_kspace), static_cast<int>(samples), means);
   }
+  LaunchScope scope("k_cov_form", cs);
+  k_cov_form<<<kCovRows * 64 / kCovSumElems, kCovSumElems * kCovSumSlices, 0, cs>>>(
+      partials, l.blocks, reinterpret_cast<float*>(ws + l.sum), flags + 1, static_cast<int>(channels),
+      1.0f / static_cast<float>(samples), means, static_cast<float2*>(d_cov));
   return check_launch();
 }
 
