@@ -527,6 +527,7 @@ __device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int 
 template <int W>
 __global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
   extern __shared__ uint32_t prepare_counts[];
+  chain_begin();
   const int f = blockIdx.y;
   for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) prepare_counts[l] = 0;
   __syncthreads();
@@ -542,6 +543,7 @@ __global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
 // among the list's entries; their sum is the list's length.  Eight blocks'
 // counts are in flight at once.
 __global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* totals, int blocks, int lists) {
+  chain_begin();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= lists) return;
   uint32_t* c = counts + static_cast<size_t>(blockIdx.y) * blocks * lists + l;
@@ -574,6 +576,7 @@ constexpr int kTablesPerBlock = 64;
 __global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* cursor, int lists,
                                                int frames, uint32_t* mid_count, uint32_t* long_count,
                                                const __grid_constant__ TablesArgs tables) {
+  chain_begin();
   if (static_cast<int>(blockIdx.x) >= frames) {
     const int i = (blockIdx.x - frames) * kTablesPerBlock + threadIdx.x;
     if (threadIdx.x < kTablesPerBlock && i < table_entries(tables)) table_entry(tables, i);
@@ -631,8 +634,7 @@ ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* 
                            uint32_t* mid_count, uint32_t* long_count, const TablesArgs* tables, cudaStream_t stream) {
   const int extra = tables ? (table_entries(*tables) + kTablesPerBlock - 1) / kTablesPerBlock : 0;
   LaunchScope scope("k_scan", stream);
-  k_scan<<<frames + extra, 1024, 0, stream>>>(counts, offsets, cursor, lists, frames, mid_count, long_count,
-                                              tables ? *tables : TablesArgs{});
+  launch_chained(k_scan, frames + extra, 1024, 0, stream, counts, offsets, cursor, lists, frames, mid_count, long_count, tables ? *tables : TablesArgs{});
   return KSJ_GPU_OK;
 }
 
@@ -818,6 +820,7 @@ __device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1,
 template <int W>
 __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
   extern __shared__ uint32_t place_smem[];
+  chain_begin();
   uint32_t* at = place_smem;  // running position of each list
   const int f = blockIdx.y;
   {
@@ -1227,6 +1230,7 @@ template <uint32_t kFormat>
 __global__ void __launch_bounds__(256) k_samples_coil_last(CoilLastArgs a) {
   using T = typename std::conditional<kFormat == KSJ_GPU_SAMPLES_BF16, uint32_t, unsigned long long>::type;
   __shared__ float2 t[32][33];
+  chain_wait();  // (row-pass blocks waiting beside these would hold shared memory their cache uses)
   const int channels = a.channels, samples = a.samples;
   const int f = a.frame0 + blockIdx.z;
   const int s0 = blockIdx.x * 32;
@@ -1463,6 +1467,7 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
 template <int kN, int kLgL, bool kHalf>
 __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  chain_begin();
   const int row = blockIdx.x;
   const int cgi = blockIdx.y;
   const int f = a.frame0 + blockIdx.z;
@@ -1681,6 +1686,7 @@ struct ColsArgs {
 template <int kN, int kLgL = 0, bool kHalf = false>
 __global__ void __launch_bounds__(kColsThreads) k_cols(const __grid_constant__ CUtensorMap inter_map, ColsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_cols[];
+  chain_begin();
   unsigned char* smem_raw = smem_cols;
   const int cb = a.column_block;
   const int cgc = a.col_group;
@@ -1879,6 +1885,7 @@ __global__ void __launch_bounds__(RingCfg<kN>::kThreads, RingCfg<kN>::kBlocks)
   constexpr int kLgL = kRingLgLines;
   extern __shared__ __align__(16) unsigned char smem_cols[];
   unsigned char* smem_raw = smem_cols;
+  chain_begin();
   const int tc = a.tile_coils;
   const int lg_tc = ilog2(tc);
   const int cb = kL / tc;  // columns per tile
@@ -2042,7 +2049,7 @@ struct RowsLauncher {
   // One pass of nf frames of grid_rows rows and `groups` coil groups.
   void launch(const RowsArgs& r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
     LaunchScope scope("k_rows", stream);
-    kernel<<<dim3(grid_rows, groups, nf), threads, smem, stream>>>(r);
+    launch_chained(kernel, dim3(grid_rows, groups, nf), threads, smem, stream, r);
   }
 };
 
@@ -2184,9 +2191,9 @@ struct ColsPass {
     LaunchScope scope(name, stream);
     if (ring) {
       c.units = nf * c.col_blocks;
-      kernel<<<std::min(ctas, c.units), threads, smem, stream>>>(map, c);
+      launch_chained(kernel, std::min(ctas, c.units), threads, smem, stream, map, c);
     } else {
-      kernel<<<dim3((out_cols + column_block - 1) / column_block, nf), kColsThreads, smem, stream>>>(map, c);
+      launch_chained(kernel, dim3((out_cols + column_block - 1) / column_block, nf), kColsThreads, smem, stream, map, c);
     }
   }
 };
@@ -2233,12 +2240,12 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.phase_col = s.phase_col;
     p.phase_sign = s.phase_sign;
     LaunchScope scope("k_prepare", stream);
-    k_prepare<W><<<blocks, kBinThreads, count_smem, stream>>>(p);
+    launch_chained(k_prepare<W>, blocks, kBinThreads, count_smem, stream, p);
   }
   {
     LaunchScope scope("k_bin_prefix", stream);
-    k_bin_prefix<<<dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream>>>(counts, totals, s.bin_blocks,
-                                                                                    s.lists_per_frame);
+    launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream, counts, totals,
+                   s.bin_blocks, s.lists_per_frame);
   }
   launch_scan(totals, offsets, nullptr, s.lists_per_frame, s.frames, nullptr, nullptr, tables, stream);
   {
@@ -2256,7 +2263,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.bin_span = s.bin_span;
     p.entries_per_frame = s.entries_per_frame;
     LaunchScope scope("k_place", stream);
-    k_place<W><<<blocks, kBinThreads, place_smem, stream>>>(p);
+    launch_chained(k_place<W>, blocks, kBinThreads, place_smem, stream, p);
   }
   return KSJ_GPU_OK;
 }
@@ -2310,7 +2317,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
     const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t), records + offsetof(SampleRecord<W>, scale),
                          static_cast<int>(sizeof(SampleRecord<W>)), s.channels, s.samples, flags, s.frame_channels,
                          s.frame_samples, s.frame_kspace, f0, reinterpret_cast<uint32_t*>(ws + l.frame_flags)};
-    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, st>>>(a);
+    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, st, a);
   };
   if (io == nullptr || io->copy == nullptr) to_coil_last(0, s.frames, stream);
   RowsArgs r{};
@@ -2984,7 +2991,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
     const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t),
                          ws + l.records + offsetof(SampleRecord3<W>, scale), static_cast<int>(sizeof(SampleRecord3<W>)),
                          s.channels, s.samples, flags, nullptr, nullptr, nullptr, 0, nullptr};
-    k_samples_coil_last<kFormat><<<tg, dim3(32, 8), 0, stream>>>(a);
+    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, stream, a);
   }
   // rows of every plane (x transformed, kept columns, coil-last)
   RowsArgs r{};

@@ -34,6 +34,36 @@ class LaunchScope {
   cudaEvent_t start_ = nullptr;
 };
 
+// A launch that may begin while the stream's previous kernel ends (programmatic
+// dependent launch): its blocks take the places that kernel's last blocks leave
+// and wait there, so that the launch itself costs nothing between the two.  The
+// kernel must begin with chain_wait() or chain_begin(), before it touches memory that earlier
+// kernels write or read.
+template <typename... Params, typename... Args>
+inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                           Args&&... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute{};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// The wait for all earlier kernels of the stream (and their memory).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// The same, and the word that the next kernel may take this one's places.
+__device__ __forceinline__ void chain_begin() {
+  chain_wait();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // ------------------------------------------------------------------- complex
