@@ -79,7 +79,6 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
-__device__ __forceinline__ float2 cmul_i(float2 a) { return make_float2(-a.y, a.x); }  // a * i
 // a + i b and a - i b (the parts of b swapped: scalar)
 __device__ __forceinline__ float2 cadd_i(float2 a, float2 b) { return make_float2(a.x - b.y, a.y + b.x); }
 __device__ __forceinline__ float2 csub_i(float2 a, float2 b) { return make_float2(a.x + b.y, a.y - b.x); }
@@ -593,24 +592,79 @@ __device__ __forceinline__ void fft_two_step_half(float2* smem, int lg_lines, co
   }
 }
 
-// Row lengths up to kMaxN with a two-step form (N1 = 16): false for any other n.
-template <int kMaxN, int kBarId = 0, typename Emit>
-__device__ __forceinline__ bool fft_two_step_rows(int n, float2* smem, int lg_lines, const float2* tw, int tid,
-                                                  int nthreads, Emit&& emit) {
-  switch (n) {
-    case 128: fft_two_step<16, 8, kBarId>(smem, lg_lines, tw, tid, nthreads, emit); return true;
-    case 192: fft_two_step<16, 12, kBarId>(smem, lg_lines, tw, tid, nthreads, emit); return true;
-    case 256: fft_two_step<16, 16, kBarId>(smem, lg_lines, tw, tid, nthreads, emit); return true;
-    case 384: fft_two_step<16, 24, kBarId>(smem, lg_lines, tw, tid, nthreads, emit); return true;
-    case 512:
-      if constexpr (kMaxN >= 512) {
-        fft_two_step<16, 32, kBarId>(smem, lg_lines, tw, tid, nthreads, emit);
-        return true;
-      }
-      return false;
-    default: return false;
+// 16-point inverse DFT of inputs of which only 0-3 and 12-15 are nonzero.
+__device__ __forceinline__ void dft16_outer(float2* v) {
+  float2 t[4][4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    // 4-point DFT of (a, 0, 0, d)
+    const float2 a = v[q], d = v[12 + q];
+    t[q][0] = cadd(a, d);
+    t[q][1] = csub_i(a, d);
+    t[q][2] = csub(a, d);
+    t[q][3] = cadd_i(a, d);
+  }
+#pragma unroll
+  for (int q = 1; q < 4; ++q) {
+#pragma unroll
+    for (int k1 = 1; k1 < 4; ++k1) t[q][k1] = cmul(t[q][k1], omega96(q * k1 * 6));
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1) {
+    float2 u[4] = {t[0][k1], t[1][k1], t[2][k1], t[3][k1]};
+    dft_inverse<4>(u);
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = u[k2];
   }
 }
+
+// The two-step transform (N1 = 16) of lines that are not in shared memory yet:
+// step A takes its inputs from load(n, line), straight from global memory into
+// registers, all 16 (or 8) of a task in flight together, so shared memory holds
+// only the values between the steps, [column][line] with `pitch` elements per
+// column.  kOuter: only the inputs n < N/4 and n >= 3N/4 are nonzero (an image
+// of N/2 pixels placed around frequency 0); the others are neither loaded nor
+// summed.  kLinesFast: a warp's lanes are consecutive lines in step A (inputs
+// line-contiguous), else consecutive n (inputs n-contiguous; an odd pitch then
+// keeps the stores apart).  Lines from `live` on are skipped.
+template <int N2, bool kOuter, bool kLinesFast, typename Load, typename Emit>
+__device__ __forceinline__ void fft_two_step_from(float2* smem, int lg_lines, int pitch, int live,
+                                                  const float2* __restrict__ tw, int tid, int nthreads, Load&& load,
+                                                  Emit&& emit) {
+  constexpr int N1 = 16;
+  const int lines = 1 << lg_lines;
+  for (int u = tid; u < N2 * lines; u += nthreads) {
+    const int line = kLinesFast ? u & (lines - 1) : u / N2;
+    const int n2 = kLinesFast ? u >> lg_lines : u - line * N2;
+    if (line >= live) continue;
+    float2 v[N1];
+#pragma unroll
+    for (int n1 = 0; n1 < N1; ++n1)
+      if (!kOuter || n1 < N1 / 4 || n1 >= 3 * N1 / 4) v[n1] = load(N2 * n1 + n2, line);
+    if constexpr (kOuter)
+      dft16_outer(v);
+    else
+      dft_reg<N1>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], tw[n2 * k1]);
+    float2* e = smem + n2 * pitch + line;
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) e[N2 * k1 * pitch] = v[k1];
+  }
+  __syncthreads();
+  for (int u = tid; u < N1 * lines; u += nthreads) {
+    const int line = u & (lines - 1), k1 = u >> lg_lines;
+    if (line >= live) continue;
+    const float2* e = smem + N2 * k1 * pitch + line;
+    float2 v[N2];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) v[n2] = e[n2 * pitch];
+    dft_reg<N2>(v);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) emit(k1 + N1 * k2, line, v[k2]);
+  }
+}
+
 __host__ __device__ constexpr bool has_two_step_rows(int n) {
   return n == 128 || n == 192 || n == 256 || n == 384 || n == 512;
 }
