@@ -3503,9 +3503,9 @@ ksj_gpu_status dispatch_width(const Shape& s, const Layout& l, const ksj_gpu_gri
 // with Direction::inverse and Normalization::inverse: 1/cols on the row pass,
 // 1/rows on the column pass, libs/numerics/kspacejet-fft/src/eigen/
 // eigen_fft_transforms.cpp:148-205), no shift; channel-major k-space in,
-// coil-last images out.  Here: [frame][channel][pixel] ->
-// [frame][pixel][channel] (k_transpose), the row transform per (frame, row,
-// coil group) (k_cart_rows), then the column pass k_cols with its
+// coil-last images out.  Here: the row transform per (frame, row, coil group)
+// (k_cart_rows), which reads the channel-major rows as they are and writes
+// them coil-last, then the column pass k_cols with its
 // deapodisation factors set to 1/rows and 1/cols and no crop or shift.
 // An axis whose length has a prime factor above 7 (no mixed-radix plan; the
 // reference's transform takes every length 2..512) is transformed by a
@@ -3572,33 +3572,48 @@ __global__ void k_cart_tables(float2* tw_rows, int rows, float2* tw_cols, int co
 }
 
 // One block per (frame, row, coil group of cg): the row's cg coil lines
-// [column][coil] from the coil-last samples, transformed along the row; every
-// column written to [frame][row][column][cpitch].  kN > 0: the two-step
-// transform of that length; 0: the mixed-radix plan; -1: the direct DFT.
+// transformed along the row and every column written to
+// [frame][row][column][cpitch].  kN > 0: the two-step transform of that
+// length, its inputs straight from the channel-major rows (a warp takes
+// consecutive columns of a coil) and its steps exchanged through shared memory of an
+// odd pitch, cg + 1, so that lanes on consecutive columns store to different
+// banks; 0: the mixed-radix plan; -1: the direct DFT, both on a copy of the
+// rows in shared memory.  Bound by HBM: a separate pass that made the k-space
+// coil-last first moved it twice more (8 frames x 32 coils x 256^2: 46 + 120 us, now 57).
 template <int kN>
-__global__ void __launch_bounds__(kCartThreads) k_cart_rows(const float2* __restrict__ coil_last, float2* inter,
+__global__ void __launch_bounds__(kCartThreads) k_cart_rows(const float2* __restrict__ kspace, float2* inter,
                                                             const float2* __restrict__ tw_cols,
                                                             const int* __restrict__ pos_cols, DifPlan plan, int rows,
                                                             int cols, int channels, int cg, int cpitch) {
   extern __shared__ __align__(16) float2 cart_smem[];
   float2* acc = cart_smem;
-  float2* tw = cart_smem + static_cast<size_t>(cols) * cg;
+  float2* tw = cart_smem + static_cast<size_t>(cols) * (kN > 0 ? cg + 1 : cg);
   const int row = blockIdx.x, cgi = blockIdx.y, f = blockIdx.z;
   const int lg = ilog2(cg);
-  const float2* src = coil_last + (static_cast<size_t>(f) * rows + row) * cols * channels;
-  for (int i = threadIdx.x; i < cols * cg; i += blockDim.x) {
-    const int col = i >> lg, gc = cgi * cg + (i & (cg - 1));
-    acc[i] = gc < channels ? __ldg(src + static_cast<size_t>(col) * channels + gc) : make_float2(0.0f, 0.0f);
-  }
+  const size_t plane = static_cast<size_t>(rows) * cols;
+  const float2* src = kspace + (static_cast<size_t>(f) * channels + cgi * cg) * plane + static_cast<size_t>(row) * cols;
+  const int live = min(cg, channels - cgi * cg);
   for (int i = threadIdx.x; i < cols; i += blockDim.x) tw[i] = tw_cols[i];
+  if constexpr (kN <= 0) {
+    // four columns of eight coils per warp (or as many as make 32): whole
+    // 32-byte sectors, and the stores meet a bank four times
+    const int lg_c = min(lg, 3);
+    for (int i = threadIdx.x; i < ((cols + 31) / 32 * 32) << lg; i += blockDim.x) {
+      const int l = i & 31, block = i >> 5;                 // blocks: coils first, then columns
+      const int coil = ((block & ((1 << (lg - lg_c)) - 1)) << lg_c) + (l >> (5 - lg_c));
+      const int col = ((block >> (lg - lg_c)) << (5 - lg_c)) + (l & ((1 << (5 - lg_c)) - 1));
+      if (col < cols) acc[(col << lg) + coil] = coil < live ? __ldg(src + coil * plane + col) : make_float2(0.0f, 0.0f);
+    }
+  }
   __syncthreads();
   float2* dst = inter + (static_cast<size_t>(f) * rows + row) * cols * cpitch + cgi * cg;
-  const int live = min(cg, channels - cgi * cg);
   auto emit = [&](int k, int line, float2 v) {
     if (line < live) dst[static_cast<size_t>(k) * cpitch + line] = v;
   };
   if constexpr (kN > 0) {
-    fft_two_step<16, kN / 16>(acc, lg, tw, threadIdx.x, blockDim.x, emit);
+    fft_two_step_from<kN / 16, false, false>(
+        acc, lg, cg + 1, live, tw, threadIdx.x, blockDim.x,
+        [&](int col, int coil) { return __ldg(src + coil * plane + col); }, emit);
   } else if constexpr (kN < 0) {
     dft_direct_lines(acc, lg, cols, tw, threadIdx.x, blockDim.x, emit);
   } else {
@@ -3695,7 +3710,8 @@ ksj_gpu_status make_cart_shape(uint32_t rows, uint32_t cols, uint32_t channels, 
   };
   const size_t px = static_cast<size_t>(frames) * rows * cols;
   c->flags = take(kFlagBytes);
-  c->coil_last = take(px * channels * sizeof(float2));
+  // coil images on their way to the RSS of the direct-DFT column form
+  c->coil_last = is_fft_size(rows) ? off : take(px * channels * sizeof(float2));
   c->inter = take(px * s.cpitch * sizeof(float2));
   c->tables = take((static_cast<size_t>(rows) + cols) * (sizeof(float2) + sizeof(float) + sizeof(int)));
   c->total = off;
@@ -4186,27 +4202,18 @@ extern "C" ksj_gpu_status ksj_gpu_cartesian_ifft2(uint32_t rows, uint32_t cols, 
                                                        s.plan_rows, s.plan_cols);
   }
   {
-    // [frame][channel][pixel] -> [frame][pixel][channel]
-    const int pixels = static_cast<int>(rows * cols);
-    const dim3 tg((pixels + 31) / 32, (channels + 31) / 32, frames);
-    LaunchScope scope("k_kspace_coil_last", cstream);
-    k_transpose<unsigned long long><<<tg, dim3(32, 8), 0, cstream>>>(
-        static_cast<const unsigned long long*>(d_kspace), reinterpret_cast<unsigned long long*>(coil_last),
-        static_cast<int>(channels), pixels);
-  }
-  {
     const CartRowsKernel rk = cart_rows_for(static_cast<int>(cols));
-    const size_t smem = (static_cast<size_t>(cols) * cs.cg + cols) * sizeof(float2);
+    const size_t smem = (static_cast<size_t>(cols) * (cs.cg + 1) + cols) * sizeof(float2);
     if (cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
       return KSJ_GPU_ERROR_CUDA;
     const dim3 grid(rows, (channels + cs.cg - 1) / cs.cg, frames);
     LaunchScope scope("k_cart_rows", cstream);
-    rk<<<grid, kCartThreads, smem, cstream>>>(coil_last, inter, tw_cols, pos_cols, s.plan_cols, static_cast<int>(rows),
+    rk<<<grid, kCartThreads, smem, cstream>>>(static_cast<const float2*>(d_kspace), inter, tw_cols, pos_cols, s.plan_cols, static_cast<int>(rows),
                                              static_cast<int>(cols), static_cast<int>(channels), cs.cg, s.cpitch);
   }
   if (!is_fft_size(rows)) {
     // direct DFT along the columns, coil-last into the output (or into the
-    // consumed coil-last buffer, then its RSS)
+    // workspace, then its RSS)
     float2* dst = output == KSJ_GPU_OUTPUT_COIL_LAST ? static_cast<float2*>(d_out) : coil_last;
     const size_t smem = (static_cast<size_t>(rows) * cs.cg + rows) * sizeof(float2);
     if (cudaFuncSetAttribute(k_cart_cols_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
