@@ -15,8 +15,8 @@
 //              places, in sample order, so every cell later accumulates in
 //              sample order -- the reference's order -- and the result is
 //              deterministic
-//   (3-D: k_prepare3 and k_scatter3 append to the lists with atomics, and
-//              k_sort and k_sort_long restore the sample order)
+//   (3-D: the same twice over, first the samples of every grid plane, then
+//              each plane's samples as a frame's)
 //   k_samples_coil_last  [frame][coil][sample] -> [frame][sample][coil] times
 //              the sample's weight and phase, so the row pass reads one
 //              sample's coils as one coalesced segment
@@ -62,7 +62,6 @@ namespace {
 
 constexpr int kChunk = 16;        // grid columns per binning list (<= 32 lists per row)
 constexpr int kMaxWidth = 8;      // largest Kaiser-Bessel width
-constexpr int kWarpSortMax = 512; // longest list a warp sorts (16 registers a lane); longer ones take a block
 constexpr int kMaxGrid = 512;
 constexpr int kColsThreads = 256;  // k_cols block size
 constexpr int kRowsThreads = 384;  // most threads of a k_rows block (two such blocks per SM)
@@ -142,7 +141,7 @@ struct Shape {
   float row_origin, col_origin;
   float phase_row, phase_col, phase_sign;  // origin-phase coefficients
   int bin_blocks, bin_span;  // 2-D binning: blocks per frame and samples per block
-  int coil_group, column_block, list_capacity, frames_per_pass, coil_parts;
+  int coil_group, column_block, frames_per_pass, coil_parts;
   uint32_t wait_fault;  // tests only: segment waits that cannot succeed, given up after this many polls
   int column_pass;      // 1 one CTA per tile (k_cols), 2 persistent ring (k_cols_ring)
   DifPlan plan_rows, plan_cols;
@@ -298,7 +297,6 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   s->coil_group = cg;
   s->column_block = cb;
-  s->list_capacity = std::min(cap, kWarpSortMax);
   // frames per k_rows/k_cols pass: keep one pass's row-transformed grid
   // (channels x grid_rows x out_cols complex) within ~64 MB of L2
   // fields appended to the tuning struct are read only when the caller's
@@ -433,294 +431,6 @@ __device__ __forceinline__ void list_chunks(int c0, int grid_cols, int* k0, int*
   *k1 = last / kChunk;
 }
 
-// One sample's record, and its entries counted in `counts` (shared memory, per list).
-template <int W>
-__device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int sample, uint32_t* counts) {
-  const size_t idx = static_cast<size_t>(f) * a.samples + sample;
-  if (a.frame_samples != nullptr && static_cast<uint32_t>(sample) >= __ldg(a.frame_samples + f)) {
-    // a padding sample of a ragged batch: in no list (its trajectory is not read)
-    reinterpret_cast<SampleRecord<W>*>(a.records)[idx].r0 = -1;
-    return;
-  }
-  const float2 k =
-      a.frame_traj != nullptr
-          ? reinterpret_cast<const float2*>(__ldg(a.frame_traj + f))[sample]
-          : __ldg(reinterpret_cast<const float2*>(a.traj) + idx);
-  bool ok = isfinite(k.x) && isfinite(k.y);
-  if (ok && a.require_nyquist) ok = k.x >= -kPiF && k.x <= kPiF && k.y >= -kPiF && k.y <= kPiF;
-  // a coordinate far outside the grid would overflow the int tap arithmetic
-  if (ok && !a.require_nyquist) ok = fabsf(k.x) < 1.0e4f && fabsf(k.y) < 1.0e4f;
-  float w = 1.0f;
-  if (a.dcf_mode == KSJ_GPU_DCF_ANALYTIC_RAMP) {
-    w = hypotf(k.x, k.y);
-  } else if (a.dcf_mode == KSJ_GPU_DCF_EXTERNAL) {
-    w = __ldg(a.dcf + idx);
-    if (!(isfinite(w) && w >= 0.0f)) {
-      atomicOr(a.flags, KSJ_GPU_FLAG_BAD_DCF);
-      if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_BAD_DCF);
-      w = 0.0f;
-    }
-  }
-  SampleRecord<W> rec;
-  if (!ok) {
-    atomicOr(a.flags, KSJ_GPU_FLAG_BAD_TRAJECTORY);
-    if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_BAD_TRAJECTORY);
-    rec.r0 = 0;
-    rec.c0 = 0;
-    rec.scale = make_float2(0.0f, 0.0f);
-#pragma unroll
-    for (int j = 0; j < W; ++j) {
-      rec.wr[j] = 0.0f;
-      rec.wc[j] = 0.0f;
-    }
-  } else {
-    const dfloat ur = grid_coordinate(k.x, static_cast<float>(a.grid_rows));
-    const dfloat uc = grid_coordinate(k.y, static_cast<float>(a.grid_cols));
-    float fr, fc;
-    const int lr = dfloor(ur, &fr);
-    const int lc = dfloor(uc, &fc);
-    if (!a.kb) {
-      // periodic 2x2 linear stencil (eigen_radial_gridding.cpp:325-342)
-      rec.r0 = wrap_index(lr, a.grid_rows);
-      rec.c0 = wrap_index(lc, a.grid_cols);
-      rec.wr[0] = 1.0f - fr;
-      rec.wr[1] = fr;
-      rec.wc[0] = 1.0f - fc;
-      rec.wc[1] = fc;
-#pragma unroll
-      for (int j = 2; j < W; ++j) {
-        rec.wr[j] = 0.0f;
-        rec.wc[j] = 0.0f;
-      }
-    } else {
-      const int sr = lr - W / 2 + 1;
-      const int sc = lc - W / 2 + 1;
-      rec.r0 = wrap_index(sr, a.grid_rows);
-      rec.c0 = wrap_index(sc, a.grid_cols);
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        // offset (tap - u), exact in its high part
-        const float dr = __fsub_rn(__fsub_rn(static_cast<float>(sr + j), ur.hi), ur.lo);
-        const float dc = __fsub_rn(__fsub_rn(static_cast<float>(sc + j), uc.hi), uc.lo);
-        rec.wr[j] = kb_weight(dr, a.two_over_w, a.beta, a.inv_i0_beta);
-        rec.wc[j] = kb_weight(dc, a.two_over_w, a.beta, a.inv_i0_beta);
-      }
-    }
-    const float2 e = exp_i_dot(k.x, a.phase_row, k.y, a.phase_col, a.phase_sign);
-    rec.scale = cscale(e, w);
-  }
-  reinterpret_cast<SampleRecord<W>*>(a.records)[idx] = rec;
-  int k0, k1;
-  list_chunks<W>(rec.c0, a.grid_cols, &k0, &k1);
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    int row = rec.r0 + j;
-    if (row >= a.grid_rows) row -= a.grid_rows;
-    atomicAdd(counts + row * a.nchunks + k0, 1u);
-    if (k1 != k0) atomicAdd(counts + row * a.nchunks + k1, 1u);
-  }
-}
-
-// One block per (block of samples, frame).  The counts go to shared memory: as atomics on
-// global memory the samples of a radial scan's centre, all in the same few
-// lists, were serialised (25 us for 205824 samples on a 512 grid, this 17).
-template <int W>
-__global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
-  extern __shared__ uint32_t prepare_counts[];
-  chain_begin();
-  const int f = blockIdx.y;
-  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) prepare_counts[l] = 0;
-  __syncthreads();
-  const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
-  for (int sample = s0 + threadIdx.x; sample < s1; sample += kBinThreads)
-    prepare_sample<W>(a, f, sample, prepare_counts);
-  __syncthreads();
-  uint32_t* out = a.counts + (static_cast<size_t>(f) * gridDim.x + blockIdx.x) * a.lists_per_frame;
-  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) out[l] = prepare_counts[l];
-}
-
-// Thread per list: the blocks' counts of the list become each block's start
-// among the list's entries; their sum is the list's length.  Eight blocks'
-// counts are in flight at once.
-__global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* totals, int blocks, int lists) {
-  chain_begin();
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= lists) return;
-  uint32_t* c = counts + static_cast<size_t>(blockIdx.y) * blocks * lists + l;
-  uint32_t run = 0;
-  for (int b0 = 0; b0 < blocks; b0 += 8) {
-    uint32_t v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = b0 + k < blocks ? c[static_cast<size_t>(b0 + k) * lists] : 0u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (b0 + k < blocks) c[static_cast<size_t>(b0 + k) * lists] = run;
-      run += v[k];
-    }
-  }
-  totals[static_cast<size_t>(blockIdx.y) * lists + l] = run;
-}
-
-// Exclusive scan of one frame's list lengths, one block per frame: list starts
-// into `offsets` and, as a scatter's running positions, into `cursor` (3-D; null otherwise).  Bound by latency (one block
-// for a single frame), so a warp holds its whole stretch of counts in registers,
-// 32 consecutive ones per load, all loads in flight at once (per-thread
-// stretches, read twice one count after another, took 24 us for 16384 lists, this
-// and the tables 10).
-// Blocks from `frames` on fill the call's tables meanwhile, 64 entries each: their FP64
-// functions run at a few lanes per clock and SM, so they are spread over many
-// (a kernel of their own on one or two SMs took 7 to 20 us).
-constexpr int kScanPer = kMaxGrid * (kMaxGrid / kChunk) / 1024;  // counts per thread, at most
-constexpr int kTablesPerBlock = 64;
-
-__global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* cursor, int lists,
-                                               int frames, uint32_t* mid_count, uint32_t* long_count,
-                                               const __grid_constant__ TablesArgs tables) {
-  chain_begin();
-  if (static_cast<int>(blockIdx.x) >= frames) {
-    const int i = (blockIdx.x - frames) * kTablesPerBlock + threadIdx.x;
-    if (threadIdx.x < kTablesPerBlock && i < table_entries(tables)) table_entry(tables, i);
-    return;
-  }
-  __shared__ uint32_t warp_sums[32];
-  const int f = blockIdx.x;
-  const uint32_t* c = counts + static_cast<size_t>(f) * lists;
-  uint32_t* o = offsets + static_cast<size_t>(f) * (lists + 1);
-  uint32_t* cur = cursor + static_cast<size_t>(f) * lists;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (lists + 1023) / 1024;
-  const int base = warp * per * 32 + lane;
-  uint32_t v[kScanPer];
-  uint32_t local = 0;
-#pragma unroll
-  for (int k = 0; k < kScanPer; ++k) v[k] = k < per && base + 32 * k < lists ? __ldg(c + base + 32 * k) : 0u;
-#pragma unroll
-  for (int k = 0; k < kScanPer; ++k) local += v[k];
-  local = __reduce_add_sync(0xffffffffu, local);
-  if (lane == 0) warp_sums[warp] = local;
-  if (f == 0 && threadIdx.x == 0 && mid_count != nullptr) *mid_count = *long_count = 0;  // the queues k_sort fills
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t ws = warp_sums[lane];
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, ws, d);
-      if (lane >= d) ws += u;
-    }
-    warp_sums[lane] = ws;
-  }
-  __syncthreads();
-  uint32_t run = warp_sums[warp] - local;
-#pragma unroll
-  for (int k = 0; k < kScanPer; ++k) {
-    if (k >= per) break;
-    uint32_t incl = v[k];
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += u;
-    }
-    if (base + 32 * k < lists) {
-      o[base + 32 * k] = run + incl - v[k];
-      if (cursor != nullptr) cur[base + 32 * k] = run + incl - v[k];
-    }
-    run += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (threadIdx.x == 0) o[lists] = warp_sums[31];
-}
-
-// The scan of `frames` frames, with the tables where they are wanted.
-ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, uint32_t* cursor, int lists, int frames,
-                           uint32_t* mid_count, uint32_t* long_count, const TablesArgs* tables, cudaStream_t stream) {
-  const int extra = tables ? (table_entries(*tables) + kTablesPerBlock - 1) / kTablesPerBlock : 0;
-  LaunchScope scope("k_scan", stream);
-  launch_chained(k_scan, frames + extra, 1024, 0, stream, counts, offsets, cursor, lists, frames, mid_count, long_count, tables ? *tables : TablesArgs{});
-  return KSJ_GPU_OK;
-}
-
-// Ascending sort of R * 32 keys held by a warp, key e = 32 r + lane in v[r]:
-// the bitonic network in its all-ascending form (the first comparator of each
-// merge flipped), so absent keys padded with 0xffffffff stay at the end and no
-// merge needs a direction.  Comparators between lanes are one shuffle and one
-// min or max per key, those between registers one min and one max per pair, and
-// the R keys of a lane are independent: the chain is the network's depth (45
-// comparators for 512 keys), where the same network over a buffer in shared
-// memory waits out a load, a compare and a store 45 * 16 times over.
-__device__ __forceinline__ uint32_t keep_min(uint32_t a, uint32_t b, bool low) { return low ? min(a, b) : max(a, b); }
-
-// The comparators at distances 16, 8, 4, 2, 1 (between lanes).
-template <int R>
-__device__ __forceinline__ void warp_merge_lanes(uint32_t (&v)[R], int lane, int from) {
-#pragma unroll
-  for (int j = 16; j > 0; j >>= 1) {
-    if (j > from) continue;
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = keep_min(v[r], __shfl_xor_sync(0xffffffffu, v[r], j), (lane & j) == 0);
-  }
-}
-
-// The comparators at distances 32 * from_r, ..., 32 (between registers), then 16 ... 1.
-template <int R>
-__device__ __forceinline__ void warp_merge(uint32_t (&v)[R], int lane, int from_r) {
-#pragma unroll
-  for (int jr = R / 2; jr > 0; jr >>= 1) {
-    if (jr > from_r) continue;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (r & jr) continue;
-      const uint32_t a = v[r], b = v[r + jr];
-      v[r] = min(a, b);
-      v[r + jr] = max(a, b);
-    }
-  }
-  warp_merge_lanes<R>(v, lane, 16);
-}
-
-template <int R>
-__device__ __forceinline__ void warp_sort(uint32_t (&v)[R], int lane) {
-#pragma unroll
-  for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      v[r] = keep_min(v[r], __shfl_xor_sync(0xffffffffu, v[r], k - 1), (lane & (k >> 1)) == 0);
-    warp_merge_lanes<R>(v, lane, k >> 2);
-  }
-#pragma unroll
-  for (int kr = 2; kr <= R; kr <<= 1) {
-    // flipped: key e meets e ^ (32 kr - 1), i.e. register r ^ (kr - 1) of lane ^ 31
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int q = r ^ (kr - 1);
-      if (q < r) continue;
-      const uint32_t a = __shfl_xor_sync(0xffffffffu, v[q], 31), b = __shfl_xor_sync(0xffffffffu, v[r], 31);
-      v[r] = min(v[r], a);
-      v[q] = max(v[q], b);
-    }
-    warp_merge<R>(v, lane, kr >> 2);
-  }
-}
-
-// One list entry (entry_bytes(W)) from its sample's record.
-template <int W>
-__device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, const float* wc, int col_lo, int grid_cols,
-                                          unsigned char* out) {
-  float2* o = reinterpret_cast<float2*>(out);
-  const int t0 = c0 - col_lo >= kChunk ? c0 - col_lo - grid_cols : c0 - col_lo;
-  o[0] = make_float2(__int_as_float(t0), __uint_as_float(sidx));
-#pragma unroll
-  for (int j = 0; j < W; j += 2) o[1 + j / 2] = make_float2(wrow * wc[j], wrow * wc[j + 1]);
-}
-
-struct PlaceArgs {
-  const unsigned char* records;
-  const uint32_t* offsets;  // [frame][list + 1]
-  const uint32_t* starts;   // [frame][block][list]: the block's start in the list (k_bin_prefix)
-  unsigned char* expanded;  // entries in their places, or null:
-  uint32_t* entries;        // the sample indices alone
-  int samples, grid_rows, grid_cols, nchunks, lists_per_frame, bin_span;
-  size_t entries_per_frame;
-};
-
 // A warp's samples, one per lane: how many lanes below this one join each of this
 // lane's lists (rows r0 + j wrapped, chunks k0 and k1), and whether one above does.
 // Byte j of below[h] is the count for (row r0 + j, chunk k0 or k1); bit j of
@@ -808,6 +518,232 @@ __device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1,
   if (warp + 1 < kBinWarps) asm volatile("bar.arrive %0, 64;" ::"r"(warp + 1) : "memory");
 }
 
+// One sample counted in its lists (shared memory).
+template <int W>
+__device__ __forceinline__ void count_lists(uint32_t* counts, int r0, int k0, int k1, int nchunks, int grid_rows) {
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    int row = r0 + j;
+    if (row >= grid_rows) row -= grid_rows;
+    atomicAdd(counts + row * nchunks + k0, 1u);
+    if (k1 != k0) atomicAdd(counts + row * nchunks + k1, 1u);
+  }
+}
+
+// One sample's record, and its entries counted in `counts` (shared memory, per list).
+template <int W>
+__device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int sample, uint32_t* counts) {
+  const size_t idx = static_cast<size_t>(f) * a.samples + sample;
+  if (a.frame_samples != nullptr && static_cast<uint32_t>(sample) >= __ldg(a.frame_samples + f)) {
+    // a padding sample of a ragged batch: in no list (its trajectory is not read)
+    reinterpret_cast<SampleRecord<W>*>(a.records)[idx].r0 = -1;
+    return;
+  }
+  const float2 k =
+      a.frame_traj != nullptr
+          ? reinterpret_cast<const float2*>(__ldg(a.frame_traj + f))[sample]
+          : __ldg(reinterpret_cast<const float2*>(a.traj) + idx);
+  bool ok = isfinite(k.x) && isfinite(k.y);
+  if (ok && a.require_nyquist) ok = k.x >= -kPiF && k.x <= kPiF && k.y >= -kPiF && k.y <= kPiF;
+  // a coordinate far outside the grid would overflow the int tap arithmetic
+  if (ok && !a.require_nyquist) ok = fabsf(k.x) < 1.0e4f && fabsf(k.y) < 1.0e4f;
+  float w = 1.0f;
+  if (a.dcf_mode == KSJ_GPU_DCF_ANALYTIC_RAMP) {
+    w = hypotf(k.x, k.y);
+  } else if (a.dcf_mode == KSJ_GPU_DCF_EXTERNAL) {
+    w = __ldg(a.dcf + idx);
+    if (!(isfinite(w) && w >= 0.0f)) {
+      atomicOr(a.flags, KSJ_GPU_FLAG_BAD_DCF);
+      if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_BAD_DCF);
+      w = 0.0f;
+    }
+  }
+  SampleRecord<W> rec;
+  if (!ok) {
+    atomicOr(a.flags, KSJ_GPU_FLAG_BAD_TRAJECTORY);
+    if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_BAD_TRAJECTORY);
+    rec.r0 = 0;
+    rec.c0 = 0;
+    rec.scale = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      rec.wr[j] = 0.0f;
+      rec.wc[j] = 0.0f;
+    }
+  } else {
+    const dfloat ur = grid_coordinate(k.x, static_cast<float>(a.grid_rows));
+    const dfloat uc = grid_coordinate(k.y, static_cast<float>(a.grid_cols));
+    float fr, fc;
+    const int lr = dfloor(ur, &fr);
+    const int lc = dfloor(uc, &fc);
+    if (!a.kb) {
+      // periodic 2x2 linear stencil (eigen_radial_gridding.cpp:325-342)
+      rec.r0 = wrap_index(lr, a.grid_rows);
+      rec.c0 = wrap_index(lc, a.grid_cols);
+      rec.wr[0] = 1.0f - fr;
+      rec.wr[1] = fr;
+      rec.wc[0] = 1.0f - fc;
+      rec.wc[1] = fc;
+#pragma unroll
+      for (int j = 2; j < W; ++j) {
+        rec.wr[j] = 0.0f;
+        rec.wc[j] = 0.0f;
+      }
+    } else {
+      const int sr = lr - W / 2 + 1;
+      const int sc = lc - W / 2 + 1;
+      rec.r0 = wrap_index(sr, a.grid_rows);
+      rec.c0 = wrap_index(sc, a.grid_cols);
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        // offset (tap - u), exact in its high part
+        const float dr = __fsub_rn(__fsub_rn(static_cast<float>(sr + j), ur.hi), ur.lo);
+        const float dc = __fsub_rn(__fsub_rn(static_cast<float>(sc + j), uc.hi), uc.lo);
+        rec.wr[j] = kb_weight(dr, a.two_over_w, a.beta, a.inv_i0_beta);
+        rec.wc[j] = kb_weight(dc, a.two_over_w, a.beta, a.inv_i0_beta);
+      }
+    }
+    const float2 e = exp_i_dot(k.x, a.phase_row, k.y, a.phase_col, a.phase_sign);
+    rec.scale = cscale(e, w);
+  }
+  reinterpret_cast<SampleRecord<W>*>(a.records)[idx] = rec;
+  int k0, k1;
+  list_chunks<W>(rec.c0, a.grid_cols, &k0, &k1);
+  count_lists<W>(counts, rec.r0, k0, k1, a.nchunks, a.grid_rows);
+}
+
+// One block per (block of samples, frame).  The counts go to shared memory: as atomics on
+// global memory the samples of a radial scan's centre, all in the same few
+// lists, were serialised (25 us for 205824 samples on a 512 grid, this 17).
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
+  extern __shared__ uint32_t prepare_counts[];
+  chain_begin();
+  const int f = blockIdx.y;
+  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) prepare_counts[l] = 0;
+  __syncthreads();
+  const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
+  for (int sample = s0 + threadIdx.x; sample < s1; sample += kBinThreads)
+    prepare_sample<W>(a, f, sample, prepare_counts);
+  __syncthreads();
+  uint32_t* out = a.counts + (static_cast<size_t>(f) * gridDim.x + blockIdx.x) * a.lists_per_frame;
+  for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) out[l] = prepare_counts[l];
+}
+
+// Thread per list: the blocks' counts of the list become each block's start
+// among the list's entries; their sum is the list's length.  Eight blocks'
+// counts are in flight at once.
+__global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* totals, int blocks, int lists) {
+  chain_begin();
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= lists) return;
+  uint32_t* c = counts + static_cast<size_t>(blockIdx.y) * blocks * lists + l;
+  uint32_t run = 0;
+  for (int b0 = 0; b0 < blocks; b0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = b0 + k < blocks ? c[static_cast<size_t>(b0 + k) * lists] : 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (b0 + k < blocks) c[static_cast<size_t>(b0 + k) * lists] = run;
+      run += v[k];
+    }
+  }
+  totals[static_cast<size_t>(blockIdx.y) * lists + l] = run;
+}
+
+// Exclusive scan of one frame's list lengths, one block per frame.  Bound by latency (one block
+// for a single frame), so a warp holds its whole stretch of counts in registers,
+// 32 consecutive ones per load, all loads in flight at once (per-thread
+// stretches, read twice one count after another, took 24 us for 16384 lists, this
+// and the tables 10).
+// Blocks from `frames` on fill the call's tables meanwhile, 64 entries each: their FP64
+// functions run at a few lanes per clock and SM, so they are spread over many
+// (a kernel of their own on one or two SMs took 7 to 20 us).
+constexpr int kScanPer = kMaxGrid * (kMaxGrid / kChunk) / 1024;  // counts per thread, at most
+constexpr int kTablesPerBlock = 64;
+
+__global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, int lists,
+                                               int frames,
+                                               const __grid_constant__ TablesArgs tables) {
+  chain_begin();
+  if (static_cast<int>(blockIdx.x) >= frames) {
+    const int i = (blockIdx.x - frames) * kTablesPerBlock + threadIdx.x;
+    if (threadIdx.x < kTablesPerBlock && i < table_entries(tables)) table_entry(tables, i);
+    return;
+  }
+  __shared__ uint32_t warp_sums[32];
+  const int f = blockIdx.x;
+  const uint32_t* c = counts + static_cast<size_t>(f) * lists;
+  uint32_t* o = offsets + static_cast<size_t>(f) * (lists + 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (lists + 1023) / 1024;
+  const int base = warp * per * 32 + lane;
+  uint32_t v[kScanPer];
+  uint32_t local = 0;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) v[k] = k < per && base + 32 * k < lists ? __ldg(c + base + 32 * k) : 0u;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) local += v[k];
+  local = __reduce_add_sync(0xffffffffu, local);
+  if (lane == 0) warp_sums[warp] = local;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t ws = warp_sums[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, ws, d);
+      if (lane >= d) ws += u;
+    }
+    warp_sums[lane] = ws;
+  }
+  __syncthreads();
+  uint32_t run = warp_sums[warp] - local;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) {
+    if (k >= per) break;
+    uint32_t incl = v[k];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += u;
+    }
+    if (base + 32 * k < lists) o[base + 32 * k] = run + incl - v[k];
+    run += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (threadIdx.x == 0) o[lists] = warp_sums[31];
+}
+
+// The scan of `frames` frames, with the tables where they are wanted.
+ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, int lists, int frames,
+                           const TablesArgs* tables, cudaStream_t stream) {
+  const int extra = tables ? (table_entries(*tables) + kTablesPerBlock - 1) / kTablesPerBlock : 0;
+  LaunchScope scope("k_scan", stream);
+  launch_chained(k_scan, frames + extra, 1024, 0, stream, counts, offsets, lists, frames, tables ? *tables : TablesArgs{});
+  return KSJ_GPU_OK;
+}
+
+// One list entry (entry_bytes(W)) from its sample's record.
+template <int W>
+__device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, const float* wc, int col_lo, int grid_cols,
+                                          unsigned char* out) {
+  float2* o = reinterpret_cast<float2*>(out);
+  const int t0 = c0 - col_lo >= kChunk ? c0 - col_lo - grid_cols : c0 - col_lo;
+  o[0] = make_float2(__int_as_float(t0), __uint_as_float(sidx));
+#pragma unroll
+  for (int j = 0; j < W; j += 2) o[1 + j / 2] = make_float2(wrow * wc[j], wrow * wc[j + 1]);
+}
+
+struct PlaceArgs {
+  const unsigned char* records;
+  const uint32_t* offsets;  // [frame][list + 1]
+  const uint32_t* starts;   // [frame][block][list]: the block's start in the list (k_bin_prefix)
+  unsigned char* expanded;  // entries in their places, or null:
+  uint32_t* entries;        // the sample indices alone
+  int samples, grid_rows, grid_cols, nchunks, lists_per_frame, bin_span;
+  size_t entries_per_frame;
+};
+
 // One block per (block of samples, frame): kBinThreads samples at a time, their
 // places in turn (place_turn), their entries written outside the turns.
 //
@@ -861,342 +797,6 @@ __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
       }
     }
   }
-}
-
-// The 3-D form: the list's plane and row weights folded together.
-template <int W>
-__device__ __forceinline__ void expand_entry3(const SampleRecord3<W>* recs, uint32_t sidx, int plane, int row,
-                                              int col_lo, int grid, unsigned char* out) {
-  constexpr int kRV = static_cast<int>(sizeof(SampleRecord3<W>) / 16);
-  float4 q[kRV];
-  const float4* rp = reinterpret_cast<const float4*>(recs + sidx);
-#pragma unroll
-  for (int v = 0; v < kRV; ++v) q[v] = __ldg(rp + v);
-  const float* w = reinterpret_cast<const float*>(q);
-  int tz = plane - __float_as_int(w[0]);
-  if (tz < 0) tz += grid;
-  int ta = row - __float_as_int(w[1]);
-  if (ta < 0) ta += grid;
-  float wz = 0.0f, wr = 0.0f;
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    if (j == tz) wz = w[6 + j];
-    if (j == ta) wr = w[6 + W + j];
-  }
-  put_entry<W>(sidx, __float_as_int(w[2]), wr * wz, w + 6 + 2 * W, col_lo, grid, out);
-}
-
-// The lists of a 3-D call: a frame f is a grid plane, offsets are absolute (one
-// entry array for all planes).
-struct SortArgs {
-  const uint32_t* offsets;
-  uint32_t* entries;
-  const unsigned char* records;
-  unsigned char* expanded;
-  uint32_t* long_lists;  // lists longer than `capacity`, left to the blocks of k_sort_long
-  uint32_t* long_count;
-  uint32_t* mid_lists;   // lists of 33 .. `capacity` entries, left to the warps of k_sort_long
-  uint32_t* mid_count;
-  int frames, samples, lists_per_frame, nchunks, grid_rows, grid_cols, capacity;
-};
-
-// Expanded entry i of list l of frame f (sample index sidx).
-template <int W>
-__device__ __forceinline__ void expand_at(const SortArgs& a, int f, int l, uint32_t begin, int i, uint32_t sidx) {
-  const int row = l / a.nchunks;
-  const int col_lo = (l - row * a.nchunks) * kChunk;
-  unsigned char* out = a.expanded + (static_cast<size_t>(begin) + i) * entry_bytes(W);
-  expand_entry3<W>(reinterpret_cast<const SampleRecord3<W>*>(a.records), sidx, f, row, col_lo, a.grid_cols, out);
-}
-
-// Expanded entries of list l of frame f, entries i = first, first + step, ...
-// (four at a time: their record loads are all in flight before the first store).
-template <int W>
-__device__ __forceinline__ void expand_list(const SortArgs& a, int f, int l, uint32_t begin, int n,
-                                            const uint32_t* sorted, int first, int step) {
-#pragma unroll 4
-  for (int i = first; i < n; i += step) expand_at<W>(a, f, l, begin, i, sorted[i]);
-}
-
-constexpr int kSortGroup = 4;  // consecutive lists per warp in k_sort
-
-// A list of 33 .. 32 R entries: sorted in registers, then written back or expanded.
-template <int W, int R>
-__device__ __forceinline__ void sort_list_regs(const SortArgs& a, int f, int l, uint32_t begin, int n, int lane,
-                                               uint32_t* ent) {
-  uint32_t v[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) v[r] = 32 * r + lane < n ? ent[32 * r + lane] : 0xffffffffu;
-  warp_sort<R>(v, lane);
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int i = 32 * r + lane;
-    if (i < n) {
-      if (a.expanded == nullptr)
-        ent[i] = v[r];
-      else
-        expand_at<W>(a, f, l, begin, i, v[r]);
-    }
-  }
-}
-
-// One list (one warp): sort the sample indices ascending, then write every
-// entry in its expanded form (the dependent record loads happen here, across
-// many lists in flight, not in the row pass).  A list of at most 32 entries
-// is ranked on registers: its sample indices are distinct, so the number of
-// smaller indices is each entry's sorted position.  Longer lists are queued for
-// k_sort_long.  The sorted indices themselves are written back only for the
-// density-weight path (no expansion), the one reader of them.
-template <int W>
-__device__ __forceinline__ void sort_list(const SortArgs& a, int f, int l, uint32_t begin, int n, int lane) {
-  if (n == 0) return;
-  if (n > 32) {
-    if (lane == 0) {
-      const bool mid = n <= a.capacity;
-      (mid ? a.mid_lists : a.long_lists)[atomicAdd(mid ? a.mid_count : a.long_count, 1u)] =
-          static_cast<uint32_t>(static_cast<size_t>(f) * a.lists_per_frame + l);
-    }
-    return;
-  }
-  uint32_t* ent = a.entries + begin;
-  const uint32_t key = lane < n ? ent[lane] : 0xffffffffu;
-  int rank = 0;
-  for (int j = 0; j < n; ++j) rank += __shfl_sync(0xffffffffu, key, j) < key ? 1 : 0;
-  if (lane < n) {
-    if (a.expanded == nullptr)
-      ent[rank] = key;  // every lane read its key before the shuffles
-    else
-      expand_at<W>(a, f, l, begin, rank, key);
-  }
-}
-
-// kSortGroup consecutive lists of one frame per warp.  Their entries are
-// contiguous; when there are at most 32 of them, lane i takes entry i of the
-// group, finds its list from the list starts and ranks it among that list's
-// entries (same order as sort_list), so tiny and empty lists share one warp.
-template <int W>
-__global__ void __launch_bounds__(256) k_sort(SortArgs a) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int groups = (a.lists_per_frame + kSortGroup - 1) / kSortGroup;
-  const size_t gg = static_cast<size_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  if (gg >= static_cast<size_t>(a.frames) * groups) return;
-  const int f = static_cast<int>(gg / groups);
-  const int l0 = static_cast<int>(gg - static_cast<size_t>(f) * groups) * kSortGroup;
-  const int ng = min(kSortGroup, a.lists_per_frame - l0);
-  const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1) + l0;
-  const uint32_t my_off = lane <= ng ? off[lane] : 0u;  // lane s: start of list l0 + s
-  const uint32_t begin = __shfl_sync(0xffffffffu, my_off, 0);
-  const int total = static_cast<int>(__shfl_sync(0xffffffffu, my_off, ng) - begin);
-  if (total == 0) return;
-  if (total > 32) {
-    for (int s = 0; s < ng; ++s) {
-      const uint32_t b = __shfl_sync(0xffffffffu, my_off, s);
-      const uint32_t e = __shfl_sync(0xffffffffu, my_off, s + 1);
-      sort_list<W>(a, f, l0 + s, b, static_cast<int>(e - b), lane);
-      __syncwarp();
-    }
-    return;
-  }
-  uint32_t* ent = a.entries + begin;
-  const bool live = lane < total;
-  const uint32_t key = live ? ent[lane] : 0xffffffffu;
-  int seg = 0;  // list of entry `lane` within the group (empty lists are skipped over)
-#pragma unroll
-  for (int s = 1; s < kSortGroup; ++s) {
-    const uint32_t st = __shfl_sync(0xffffffffu, my_off, s);
-    if (s < ng && begin + lane >= st) seg = s;
-  }
-  int rank = 0;
-  for (int j = 0; j < total; ++j) {
-    const uint32_t kj = __shfl_sync(0xffffffffu, key, j);
-    const int sj = __shfl_sync(0xffffffffu, seg, j);
-    rank += (sj == seg && kj < key) ? 1 : 0;
-  }
-  const uint32_t lbegin = __shfl_sync(0xffffffffu, my_off, seg);
-  if (live) {
-    if (a.expanded == nullptr)
-      ent[lbegin - begin + rank] = key;  // every lane read its key before the shuffles
-    else
-      expand_at<W>(a, f, l0 + seg, lbegin, rank, key);
-  }
-}
-
-constexpr int kLongSortThreads = 1024;
-constexpr int kLongSortBlocks = 152;    // one per SM
-constexpr int kLongSortSmem = 16384;  // entries sorted in shared memory; longer lists in place in L2/HBM
-
-constexpr int kLongRegs = kWarpSortMax / 32;
-
-// The keys of each kWarpSortMax-key chunk of buf[0, n) sorted (first, whole
-// chunks from scratch) or merged (the comparators at distances below
-// kWarpSortMax) by a warp in registers.  buf holds n rounded up to whole
-// chunks, the padding 0xffffffff.  Synchronises the block.
-template <bool kWhole>
-__device__ __forceinline__ void block_chunks(uint32_t* buf, int n) {
-  const int lane = threadIdx.x & 31;
-  for (int c = (threadIdx.x >> 5) * kWarpSortMax; c < n; c += (kLongSortThreads / 32) * kWarpSortMax) {
-    uint32_t v[kLongRegs];
-#pragma unroll
-    for (int r = 0; r < kLongRegs; ++r) v[r] = buf[c + 32 * r + lane];
-    if constexpr (kWhole)
-      warp_sort<kLongRegs>(v, lane);
-    else
-      warp_merge<kLongRegs>(v, lane, kLongRegs / 2);
-#pragma unroll
-    for (int r = 0; r < kLongRegs; ++r) buf[c + 32 * r + lane] = v[r];
-  }
-  __syncthreads();
-}
-
-// One comparator stage over buf[0, n) (shared or global memory), thread per
-// pair: the flipped first stage of the merge into runs of k (i and its mirror
-// in the run), or the pairs at distance j.  Keys at or beyond n are absent
-// (they are the largest, and stay).  Synchronises the block.
-__device__ __forceinline__ void compare_pair(uint32_t* buf, int i, int partner, int n) {
-  if (partner < n) {
-    const uint32_t x = buf[i], y = buf[partner];
-    if (x > y) {
-      buf[i] = y;
-      buf[partner] = x;
-    }
-  }
-}
-__device__ __forceinline__ void block_flip(uint32_t* buf, int n, int k) {
-  const int lg = __ffs(k >> 1) - 1, pairs = ((n + k - 1) / k) << lg;
-  for (int p = threadIdx.x; p < pairs; p += kLongSortThreads) {
-    const int i = ((p >> lg) << (lg + 1)) + (p & ((1 << lg) - 1));
-    compare_pair(buf, i, i ^ (k - 1), n);
-  }
-  __syncthreads();
-}
-__device__ __forceinline__ void block_step(uint32_t* buf, int n, int j) {
-  const int lg = __ffs(j) - 1, pairs = ((n + 2 * j - 1) >> (lg + 1)) << lg;
-  for (int p = threadIdx.x; p < pairs; p += kLongSortThreads) {
-    const int i = ((p >> lg) << (lg + 1)) + (p & (j - 1));
-    compare_pair(buf, i, i + j, n);
-  }
-  __syncthreads();
-}
-
-// n keys of global memory into buf, padded to whole chunks, and back.
-__device__ __forceinline__ void chunk_load(uint32_t* buf, const uint32_t* ent, int n) {
-  const int padded = (n + kWarpSortMax - 1) / kWarpSortMax * kWarpSortMax;
-  for (int t = threadIdx.x; t < padded; t += kLongSortThreads) buf[t] = t < n ? ent[t] : 0xffffffffu;
-  __syncthreads();
-}
-__device__ __forceinline__ void chunk_store(const uint32_t* buf, uint32_t* ent, int n) {
-  for (int t = threadIdx.x; t < n; t += kLongSortThreads) ent[t] = buf[t];
-  __syncthreads();
-}
-
-// buf[0, n), n <= kLongSortSmem, sorted by the block: the network of warp_sort
-// over chunks in registers, only the comparators at distance kWarpSortMax and
-// above over shared memory (15 stages for 16384 keys instead of 105).
-__device__ __forceinline__ void block_sort(uint32_t* buf, int n) {
-  block_chunks<true>(buf, n);
-  for (int k = 2 * kWarpSortMax; (k >> 1) < n; k <<= 1) {
-    block_flip(buf, n, k);
-    for (int j = k >> 2; j >= kWarpSortMax; j >>= 1) block_step(buf, n, j);
-    block_chunks<false>(buf, n);
-  }
-}
-
-// The same network on a list longer than the shared buffer, in place in global
-// memory: chunks of kLongSortSmem keys sorted in the buffer, then per merge the
-// comparators at distance kLongSortSmem and above over global memory and the
-// rest chunk by chunk in the buffer.
-__device__ __forceinline__ void block_sort_chunked(uint32_t* ent, int n, uint32_t* buf) {
-  for (int base = 0; base < n; base += kLongSortSmem) {
-    const int cnt = min(kLongSortSmem, n - base);
-    chunk_load(buf, ent + base, cnt);
-    block_sort(buf, cnt);
-    chunk_store(buf, ent + base, cnt);
-  }
-  for (int k = 2 * kLongSortSmem; (k >> 1) < n; k <<= 1) {
-    block_flip(ent, n, k);
-    for (int j = k >> 2; j >= kLongSortSmem; j >>= 1) block_step(ent, n, j);
-    for (int base = 0; base < n; base += kLongSortSmem) {
-      const int cnt = min(kLongSortSmem, n - base);
-      chunk_load(buf, ent + base, cnt);
-      for (int j = kLongSortSmem >> 1; j >= kWarpSortMax; j >>= 1) block_step(buf, cnt, j);
-      block_chunks<false>(buf, cnt);
-      chunk_store(buf, ent + base, cnt);
-    }
-  }
-}
-
-template <int W>
-__device__ __forceinline__ void sort_long_list(const SortArgs& a, size_t gl, uint32_t* long_buf) {
-  const int f = static_cast<int>(gl / a.lists_per_frame);
-  const int l = static_cast<int>(gl - static_cast<size_t>(f) * a.lists_per_frame);
-  const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
-  const uint32_t begin = off[l];
-  const int n = static_cast<int>(off[l + 1] - begin);
-  uint32_t* ent = a.entries + begin;
-  const uint32_t* sorted = ent;
-  if (n <= kLongSortSmem) {
-    chunk_load(long_buf, ent, n);
-    block_sort(long_buf, n);
-    if (a.expanded == nullptr)
-      for (int i = threadIdx.x; i < n; i += kLongSortThreads) ent[i] = long_buf[i];
-    sorted = long_buf;
-  } else {
-    block_sort_chunked(ent, n, long_buf);
-  }
-  __syncthreads();
-  if (a.expanded != nullptr) expand_list<W>(a, f, l, begin, n, sorted, threadIdx.x, blockDim.x);
-}
-
-// The lists k_sort queued.  Blocks take the long ones in turn (sorted in shared
-// memory up to kLongSortSmem entries, else in place with chunk-local stages in
-// shared memory), then every warp the ones of 33 .. capacity entries, 2 to 16
-// keys a lane in registers.  A kernel of its own, because the networks' registers
-// would halve the warps that k_sort has in flight on the short lists: both in
-// one kernel measured 426 us on the lists of 96 radial frames, 202 us apart.
-template <int W>
-__global__ void __launch_bounds__(kLongSortThreads, 1) k_sort_long(SortArgs a) {
-  extern __shared__ uint32_t long_buf[];
-  const uint32_t queued = *a.long_count;
-  for (uint32_t q = blockIdx.x; q < queued; q += gridDim.x) {
-    sort_long_list<W>(a, a.long_lists[q], long_buf);
-    __syncthreads();
-  }
-  const uint32_t mids = *a.mid_count;
-  const int lane = threadIdx.x & 31;
-  for (uint32_t q = blockIdx.x * (kLongSortThreads / 32) + (threadIdx.x >> 5); q < mids;
-       q += gridDim.x * (kLongSortThreads / 32)) {
-    const uint32_t gl = a.mid_lists[q];
-    const int f = static_cast<int>(gl / a.lists_per_frame);
-    const int l = static_cast<int>(gl - static_cast<uint32_t>(f) * a.lists_per_frame);
-    const uint32_t* off = a.offsets + static_cast<size_t>(f) * (a.lists_per_frame + 1);
-    const uint32_t begin = off[l];
-    const int n = static_cast<int>(off[l + 1] - begin);
-    uint32_t* ent = a.entries + begin;
-    if (n <= 64)
-      sort_list_regs<W, 2>(a, f, l, begin, n, lane, ent);
-    else if (n <= 128)
-      sort_list_regs<W, 4>(a, f, l, begin, n, lane, ent);
-    else if (n <= 256)
-      sort_list_regs<W, 8>(a, f, l, begin, n, lane, ent);
-    else
-      sort_list_regs<W, 16>(a, f, l, begin, n, lane, ent);
-  }
-}
-
-// Launch k_sort and then k_sort_long for the lists it queued.
-template <int W>
-ksj_gpu_status launch_sort(SortArgs sa, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(k_sort_long<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSortSmem * 4) !=
-      cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
-  {
-    LaunchScope scope("k_sort", stream);
-    const size_t warps = static_cast<size_t>(sa.frames) * ((sa.lists_per_frame + kSortGroup - 1) / kSortGroup);
-    k_sort<W><<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(sa);
-  }
-  LaunchScope scope("k_sort_long", stream);
-  k_sort_long<W><<<kLongSortBlocks, kLongSortThreads, kLongSortSmem * 4, stream>>>(sa);
-  return KSJ_GPU_OK;
 }
 
 // [frame][channel][sample] -> [frame][sample][channel] complex64, each sample
@@ -2247,7 +1847,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream, counts, totals,
                    s.bin_blocks, s.lists_per_frame);
   }
-  launch_scan(totals, offsets, nullptr, s.lists_per_frame, s.frames, nullptr, nullptr, tables, stream);
+  launch_scan(totals, offsets, s.lists_per_frame, s.frames, tables, stream);
   {
     PlaceArgs p{};
     p.records = records;
@@ -2689,16 +2289,15 @@ struct Prepare3Args {
   const float* dcf;
   uint32_t dcf_mode;
   unsigned char* records;
-  uint32_t* counts;  // [plane][row * nchunks + chunk]
+  uint32_t* counts;  // [block][plane]: samples of the block on the plane
   uint32_t* flags;
-  int samples, grid, nchunks, lists_per_plane;
+  int samples, grid, bin_span;
   float beta, two_over_w, inv_i0_beta, phase;
 };
 
+// One sample's record; its first tap plane.
 template <int W>
-__global__ void __launch_bounds__(256) k_prepare3(Prepare3Args a) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= a.samples) return;
+__device__ __forceinline__ int prepare_sample3(const Prepare3Args& a, int idx) {
   const float kz = __ldg(a.traj + 3 * static_cast<size_t>(idx));
   const float ky = __ldg(a.traj + 3 * static_cast<size_t>(idx) + 1);
   const float kx = __ldg(a.traj + 3 * static_cast<size_t>(idx) + 2);
@@ -2744,19 +2343,150 @@ __global__ void __launch_bounds__(256) k_prepare3(Prepare3Args a) {
     rec.scale = cscale(exp_i_dot3(kz, a.phase, ky, a.phase, kx, a.phase), w);
   }
   reinterpret_cast<SampleRecord3<W>*>(a.records)[idx] = rec;
-  int k0, k1;
-  list_chunks<W>(rec.c0, a.grid, &k0, &k1);
+  return rec.z0;
+}
+
+// Binning in 3-D, in sample order: a sample is first placed in the lists of its W
+// planes (k_prepare3 counts, k_plane_place), then a plane's samples, in that
+// order, in the plane's row and chunk lists as a frame's (k_count3, k_place3,
+// kPlaneBlocks blocks a plane).  Appending to the (plane, row, chunk) lists with
+// atomics and sorting them took 15 ms of a call on 10.24 M samples, 384^3 (the
+// centre's lists hold up to 1.5e5 entries), these take 5.7.
+constexpr int kPlaneBlocks = 16;
+
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_prepare3(Prepare3Args a) {
+  __shared__ uint32_t counts[kMaxGrid];
+  for (int p = threadIdx.x; p < a.grid; p += kBinThreads) counts[p] = 0;
+  __syncthreads();
+  const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
+  for (int base = s0; base < s1; base += kBinThreads) {
+    const int sample = base + threadIdx.x;
+    if (sample < s1) count_lists<W>(counts, prepare_sample3<W>(a, sample), 0, 0, 1, a.grid);
+  }
+  __syncthreads();
+  for (int p = threadIdx.x; p < a.grid; p += kBinThreads) a.counts[blockIdx.x * a.grid + p] = counts[p];
+}
+
+// The samples of every plane, in order.  starts: [block][plane].
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_plane_place(const unsigned char* records, const uint32_t* offsets,
+                                                             const uint32_t* starts, uint32_t* plane_samples,
+                                                             int samples, int grid, int bin_span) {
+  __shared__ uint32_t at[kMaxGrid];
+  for (int p = threadIdx.x; p < grid; p += kBinThreads)
+    at[p] = __ldg(offsets + p) + __ldg(starts + blockIdx.x * grid + p);
+  const int s0 = blockIdx.x * bin_span, s1 = min(s0 + bin_span, samples);
+  for (int base = s0; base < s1; base += kBinThreads) {
+    const int sample = base + threadIdx.x;
+    const int z0 = sample < s1 ? reinterpret_cast<const SampleRecord3<W>*>(records)[sample].z0 : -1;
+    uint32_t pos[W][2];
+    place_turn<W>(at, z0, 0, 0, 1, grid, pos);
+    if (z0 < 0) continue;
 #pragma unroll
-  for (int i = 0; i < W; ++i) {
-    int plane = rec.z0 + i;
-    if (plane >= a.grid) plane -= a.grid;
-    uint32_t* counts = a.counts + static_cast<size_t>(plane) * a.lists_per_plane;
+    for (int j = 0; j < W; ++j) plane_samples[pos[j][0]] = static_cast<uint32_t>(sample);
+  }
+}
+
+// Items [*i0, *i1) of plane p's samples that block b of kPlaneBlocks takes, as
+// positions in plane_samples.
+__device__ __forceinline__ void plane_span(const uint32_t* plane_offsets, int p, int b, uint32_t* i0, uint32_t* i1) {
+  const uint32_t begin = __ldg(plane_offsets + p), end = __ldg(plane_offsets + p + 1);
+  const uint32_t turns = (end - begin + kBinThreads - 1) / kBinThreads;
+  const uint32_t span = (turns + kPlaneBlocks - 1) / kPlaneBlocks * kBinThreads;
+  *i0 = min(begin + b * span, end);
+  *i1 = min(*i0 + span, end);
+}
+
+// One block per (block of a plane's samples, plane): their counts per list.
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_count3(const unsigned char* records, const uint32_t* plane_offsets,
+                                                        const uint32_t* plane_samples, uint32_t* counts, int grid,
+                                                        int nchunks, int lists_per_plane) {
+  extern __shared__ uint32_t list_counts[];
+  for (int l = threadIdx.x; l < lists_per_plane; l += kBinThreads) list_counts[l] = 0;
+  __syncthreads();
+  uint32_t i0, i1;
+  plane_span(plane_offsets, blockIdx.y, blockIdx.x, &i0, &i1);
+  for (uint32_t base = i0; base < i1; base += kBinThreads) {
+    const uint32_t i = base + threadIdx.x;
+    int r0 = -1, c0 = 0;
+    if (i < i1) {
+      const SampleRecord3<W>* rec = reinterpret_cast<const SampleRecord3<W>*>(records) + __ldg(plane_samples + i);
+      const int4 first = __ldg(reinterpret_cast<const int4*>(rec));  // z0, r0, c0
+      r0 = first.y;
+      c0 = first.z;
+    }
+    int k0, k1;
+    list_chunks<W>(c0, grid, &k0, &k1);
+    if (r0 >= 0) count_lists<W>(list_counts, r0, k0, k1, nchunks, grid);
+  }
+  __syncthreads();
+  uint32_t* out = counts + (static_cast<size_t>(blockIdx.y) * kPlaneBlocks + blockIdx.x) * lists_per_plane;
+  for (int l = threadIdx.x; l < lists_per_plane; l += kBinThreads) out[l] = list_counts[l];
+}
+
+struct Place3Args {
+  const unsigned char* records;
+  const uint32_t* plane_offsets;
+  const uint32_t* plane_samples;
+  const uint32_t* offsets;  // [plane][list + 1], absolute
+  const uint32_t* starts;   // [plane][block][list]
+  unsigned char* expanded;  // entries in their places, or null:
+  uint32_t* entries;        // the sample indices alone
+  int grid, nchunks, lists_per_plane;
+};
+
+// One block per (block of a plane's samples, plane): the entries of its lists.
+template <int W>
+__global__ void __launch_bounds__(kBinThreads) k_place3(Place3Args a) {
+  extern __shared__ uint32_t place_smem[];
+  uint32_t* at = place_smem;
+  const int plane = blockIdx.y;
+  uint32_t i0, i1;
+  plane_span(a.plane_offsets, plane, blockIdx.x, &i0, &i1);
+  if (i0 >= i1) return;
+  {
+    const uint32_t* off = a.offsets + static_cast<size_t>(plane) * (a.lists_per_plane + 1);
+    const uint32_t* st = a.starts + (static_cast<size_t>(plane) * kPlaneBlocks + blockIdx.x) * a.lists_per_plane;
+#pragma unroll 4
+    for (int l = threadIdx.x; l < a.lists_per_plane; l += kBinThreads) at[l] = __ldg(off + l) + __ldg(st + l);
+  }
+  for (uint32_t base = i0; base < i1; base += kBinThreads) {
+    const uint32_t i = base + threadIdx.x;
+    constexpr int kRV = static_cast<int>(sizeof(SampleRecord3<W>) / 16);
+    float4 q[kRV];
+    uint32_t sample = 0;
+    if (i < i1) {
+      sample = __ldg(a.plane_samples + i);
+      const float4* rp = reinterpret_cast<const float4*>(reinterpret_cast<const SampleRecord3<W>*>(a.records) + sample);
+#pragma unroll
+      for (int v = 0; v < kRV; ++v) q[v] = __ldg(rp + v);
+    }
+    const float* w = reinterpret_cast<const float*>(q);
+    const int r0 = i < i1 ? __float_as_int(w[1]) : -1, c0 = i < i1 ? __float_as_int(w[2]) : 0;
+    int k0, k1;
+    list_chunks<W>(c0, a.grid, &k0, &k1);
+    uint32_t pos[W][2];
+    place_turn<W>(at, r0, k0, k1, a.nchunks, a.grid, pos);
+    if (r0 < 0) continue;
+    int tz = plane - __float_as_int(w[0]);
+    if (tz < 0) tz += a.grid;
+    float wz = 0.0f;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (j == tz) wz = w[6 + j];
 #pragma unroll
     for (int j = 0; j < W; ++j) {
-      int row = rec.r0 + j;
-      if (row >= a.grid) row -= a.grid;
-      atomicAdd(counts + row * a.nchunks + k0, 1u);
-      if (k1 != k0) atomicAdd(counts + row * a.nchunks + k1, 1u);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h && k1 == k0) continue;
+        if (a.expanded != nullptr)
+          put_entry<W>(sample, c0, w[6 + W + j] * wz, w + 6 + 2 * W, (h ? k1 : k0) * kChunk, a.grid,
+                       a.expanded + static_cast<size_t>(pos[j][h]) * entry_bytes(W));
+        else
+          a.entries[pos[j][h]] = sample;
+      }
     }
   }
 }
@@ -2780,41 +2510,35 @@ __global__ void __launch_bounds__(512) k_plane_bases(uint32_t* offsets, int plan
   if (t < planes) bases[t] = tot[t];
 }
 
-__global__ void __launch_bounds__(256) k_offsets_add(uint32_t* offsets, uint32_t* cursor, int planes, int lists,
-                                                     const uint32_t* bases) {
+__global__ void __launch_bounds__(256) k_offsets_add(uint32_t* offsets, int planes, int lists, const uint32_t* bases) {
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= static_cast<size_t>(planes) * (lists + 1)) return;
-  const size_t p = i / (lists + 1), l = i - p * (lists + 1);
-  const uint32_t at = offsets[i] + bases[p];
-  offsets[i] = at;
-  if (l < static_cast<size_t>(lists)) cursor[p * lists + l] = at;
+  offsets[i] += bases[i / (lists + 1)];
 }
 
-template <int W>
-__global__ void __launch_bounds__(256) k_scatter3(const unsigned char* records, uint32_t* cursor, uint32_t* entries,
-                                                  int samples, int grid, int nchunks, int lists_per_plane) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= samples) return;
-  const SampleRecord3<W>& rec = reinterpret_cast<const SampleRecord3<W>*>(records)[idx];
-  int k0, k1;
-  list_chunks<W>(rec.c0, grid, &k0, &k1);
-  for (int i = 0; i < W; ++i) {
-    int plane = rec.z0 + i;
-    if (plane >= grid) plane -= grid;
-    uint32_t* cur = cursor + static_cast<size_t>(plane) * lists_per_plane;
-    for (int j = 0; j < W; ++j) {
-      int row = rec.r0 + j;
-      if (row >= grid) row -= grid;
-      const int l0 = row * nchunks + k0;
-      entries[atomicAdd(cur + l0, 1u)] = static_cast<uint32_t>(idx);
-      if (k1 != k0) entries[atomicAdd(cur + row * nchunks + k1, 1u)] = static_cast<uint32_t>(idx);
-    }
-  }
+// Workspace of the 3-D binning.
+struct Lists3 {
+  size_t plane_counts, plane_totals, plane_offsets, plane_samples, counts, totals, offsets, bases;
+};
+
+template <class Take>
+Lists3 take_lists3(const Shape& s, Take&& take) {
+  const size_t g = static_cast<size_t>(s.grid_rows), nl = g * s.lists_per_frame;
+  Lists3 l{};
+  l.plane_counts = take(static_cast<size_t>(s.bin_blocks) * g * 4);
+  l.plane_totals = take(g * 4);
+  l.plane_offsets = take((g + 1) * 4);
+  l.plane_samples = take(static_cast<size_t>(s.samples) * s.width * 4);
+  l.counts = take(nl * kPlaneBlocks * 4);
+  l.totals = take(nl * 4);
+  l.offsets = take((nl + g) * 4);
+  l.bases = take(g * 4);
+  return l;
 }
 
 struct Layout3 {
-  size_t flags, cleared, records, counts, cursor, offsets, bases, entries, expanded, long_lists, mid_lists, samples_t, inter, inter2,
-      tables, total;
+  size_t flags, records, expanded, samples_t, inter, inter2, tables, total;
+  Lists3 lists;
   size_t entries_total;
 };
 
@@ -2837,19 +2561,11 @@ Layout3 make_layout3(const Shape& s) {
     return at;
   };
   const size_t g = static_cast<size_t>(s.grid_rows), n = static_cast<size_t>(s.rows);
-  const size_t nl = g * s.lists_per_frame;
   l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
-  l.flags = take(kFlagBytes);  // flags and counts are cleared together
-  l.counts = take(nl * 4);
-  l.cleared = off;
+  l.flags = take(kFlagBytes);
   l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
-  l.cursor = take(nl * 4);
-  l.offsets = take((nl + g) * 4);
-  l.bases = take(g * 4);
-  l.entries = take(l.entries_total * 4);
+  l.lists = take_lists3(s, take);
   l.expanded = take(l.entries_total * entry_bytes(s.width));
-  l.long_lists = take((2 + l.entries_total / (s.list_capacity + 1)) * 4);
-  l.mid_lists = take((2 + l.entries_total / 33) * 4);
   l.samples_t = take(static_cast<size_t>(s.samples) * s.channels * sizeof(float2));
   l.inter = take(g * g * n * s.cpitch * sizeof(float2));
   l.inter2 = take(g * n * n * s.cpitch * sizeof(float2));
@@ -2881,71 +2597,82 @@ ksj_gpu_status make_shape3(const ksj_gpu_gridding3_desc* d, const ksj_gpu_griddi
   const ksj_gpu_status st = make_shape(&d2, t, s);
   if (st != KSJ_GPU_OK) return st;
   s->entries_per_frame = 0;  // absolute offsets into one entry array
+  // the plane stage of the binning: one frame, planes for lists (four blocks per SM)
+  const int turns = (s->samples + kBinThreads - 1) / kBinThreads;
+  const int blocks = std::min(turns, 152 * 4);
+  s->bin_span = (turns + blocks - 1) / blocks * kBinThreads;
+  s->bin_blocks = (s->samples + s->bin_span - 1) / s->bin_span;
   return KSJ_GPU_OK;
 }
 
-// The 3-D binning lists: per-sample records, (plane, row, chunk) counts, per-plane
-// scans made absolute, the scattered entries, their sort and (when `expanded`
-// is given) the expanded entries, and the call's tables where `tables` names
-// them.  The flags and counts must already be cleared.
+// The 3-D binning lists: per-sample records, the samples of every plane, the
+// (plane, row, chunk) list offsets, and the lists' entries as the row pass reads them
+// (`expanded`) or as sample indices alone (`entries`); and the call's tables where
+// `tables` names them.  The flags must already be cleared.
 template <int W>
 ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_traj, const float* d_dcf,
-                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* cursor,
-                            uint32_t* offsets, uint32_t* bases, uint32_t* entries, unsigned char* expanded,
-                            uint32_t* long_lists, uint32_t* mid_lists, cudaStream_t stream,
+                            uint32_t* flags, unsigned char* records, unsigned char* ws, const Lists3& l,
+                            uint32_t* entries, unsigned char* expanded, cudaStream_t stream,
                             const TablesArgs* tables = nullptr) {
   const int g = s.grid_rows;
+  auto at = [&](size_t offset) { return reinterpret_cast<uint32_t*>(ws + offset); };
+  const int count_smem = s.lists_per_frame * 4;
+  const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
+  if (cudaFuncSetAttribute(k_count3<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, count_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_place3<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
+    return KSJ_GPU_ERROR_CUDA;
   {
     Prepare3Args p{};
     p.traj = d_traj;
     p.dcf = d_dcf;
     p.dcf_mode = dcf_mode;
     p.records = records;
-    p.counts = counts;
+    p.counts = at(l.plane_counts);
     p.flags = flags;
     p.samples = s.samples;
     p.grid = g;
-    p.nchunks = s.nchunks;
-    p.lists_per_plane = s.lists_per_frame;
+    p.bin_span = s.bin_span;
     p.beta = s.beta;
     p.two_over_w = 2.0f / static_cast<float>(s.width);
     p.inv_i0_beta = s.inv_i0_beta;
     p.phase = s.phase_row;
     LaunchScope scope("k_prepare3", stream);
-    k_prepare3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(p);
+    k_prepare3<W><<<s.bin_blocks, kBinThreads, 0, stream>>>(p);
   }
-  launch_scan(counts, offsets, cursor, s.lists_per_frame, g, mid_lists, long_lists, tables, stream);
+  {
+    LaunchScope scope("k_bin_prefix", stream);
+    launch_chained(k_bin_prefix, (g + 127) / 128, 128, 0, stream, at(l.plane_counts), at(l.plane_totals), s.bin_blocks, g);
+  }
+  launch_scan(at(l.plane_totals), at(l.plane_offsets), g, 1, tables, stream);
+  {
+    LaunchScope scope("k_plane_place", stream);
+    k_plane_place<W><<<s.bin_blocks, kBinThreads, 0, stream>>>(records, at(l.plane_offsets), at(l.plane_counts),
+                                                              at(l.plane_samples), s.samples, g, s.bin_span);
+  }
+  const dim3 blocks(kPlaneBlocks, g);
+  {
+    LaunchScope scope("k_count3", stream);
+    k_count3<W><<<blocks, kBinThreads, count_smem, stream>>>(records, at(l.plane_offsets), at(l.plane_samples),
+                                                            at(l.counts), g, s.nchunks, s.lists_per_frame);
+  }
+  {
+    LaunchScope scope("k_bin_prefix", stream);
+    launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, g), 128, 0, stream, at(l.counts), at(l.totals),
+                   kPlaneBlocks, s.lists_per_frame);
+  }
+  launch_scan(at(l.totals), at(l.offsets), s.lists_per_frame, g, nullptr, stream);
   {
     LaunchScope scope("k_plane_offsets", stream);
-    k_plane_bases<<<1, 512, 0, stream>>>(offsets, g, s.lists_per_frame, bases);
+    k_plane_bases<<<1, 512, 0, stream>>>(at(l.offsets), g, s.lists_per_frame, at(l.bases));
     const size_t total = static_cast<size_t>(g) * (s.lists_per_frame + 1);
-    k_offsets_add<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(offsets, cursor, g,
-                                                                                s.lists_per_frame, bases);
+    k_offsets_add<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(at(l.offsets), g, s.lists_per_frame,
+                                                                                at(l.bases));
   }
   {
-    LaunchScope scope("k_scatter3", stream);
-    k_scatter3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(records, cursor, entries, s.samples, g, s.nchunks,
-                                                               s.lists_per_frame);
-  }
-  {
-    SortArgs sa{};
-    sa.offsets = offsets;
-    sa.entries = entries;
-    sa.records = records;
-    sa.expanded = expanded;
-    sa.long_count = long_lists;
-    sa.long_lists = sa.long_count + 1;
-    sa.mid_count = mid_lists;
-    sa.mid_lists = mid_lists + 1;
-    sa.frames = g;
-    sa.samples = s.samples;
-    sa.lists_per_frame = s.lists_per_frame;
-    sa.nchunks = s.nchunks;
-    sa.grid_rows = g;
-    sa.grid_cols = g;
-    sa.capacity = s.list_capacity;
-    const ksj_gpu_status st = launch_sort<W>(sa, stream);
-    if (st != KSJ_GPU_OK) return st;
+    const Place3Args p{records, at(l.plane_offsets), at(l.plane_samples), at(l.offsets), at(l.counts), expanded, entries,
+                       g, s.nchunks, s.lists_per_frame};
+    LaunchScope scope("k_place3", stream);
+    k_place3<W><<<blocks, kBinThreads, place_smem, stream>>>(p);
   }
   return KSJ_GPU_OK;
 }
@@ -2956,10 +2683,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
                            cudaStream_t stream) {
   const int g = s.grid_rows, n = s.rows;
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + l.counts);
-  uint32_t* cursor = reinterpret_cast<uint32_t*>(ws + l.cursor);
-  uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + l.offsets);
-  uint32_t* entries = reinterpret_cast<uint32_t*>(ws + l.entries);
+  uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + l.lists.offsets);
   float2* inter = reinterpret_cast<float2*>(ws + l.inter);
   float2* inter2 = reinterpret_cast<float2*>(ws + l.inter2);
   float2* tw_rows = reinterpret_cast<float2*>(ws + l.tables);
@@ -2970,7 +2694,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   int* pos_cols = pos_rows + n;
   float* ones = reinterpret_cast<float*>(pos_cols + n);
 
-  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   const TablesArgs tables{tw_rows, tw_cols, inv_dr, inv_dc, pos_rows, pos_cols, g, g, n, n, s.plan_rows, s.plan_cols, 1,
                           s.width, s.beta, std::cyl_bessel_i(0.0, static_cast<double>(s.beta))};
   {
@@ -2978,11 +2702,8 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
     k_fill<<<(n * n + 255) / 256, 256, 0, stream>>>(ones, n * n, 1.0f);
   }
   {
-    const ksj_gpu_status st = build_lists3<W>(s, d->dcf_mode, d_traj, d_dcf, flags, ws + l.records, counts, cursor,
-                                              offsets, reinterpret_cast<uint32_t*>(ws + l.bases), entries,
-                                              ws + l.expanded,
-                                              reinterpret_cast<uint32_t*>(ws + l.long_lists),
-                                              reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream, &tables);
+    const ksj_gpu_status st = build_lists3<W>(s, d->dcf_mode, d_traj, d_dcf, flags, ws + l.records, ws, l.lists, nullptr,
+                                              ws + l.expanded, stream, &tables);
     if (st != KSJ_GPU_OK) return st;
   }
   {
@@ -3175,7 +2896,7 @@ __device__ __forceinline__ void pm3_accumulate(const uint32_t* entries, uint32_t
 
 // The 3-D grid step for lists of at most `capacity` entries: the
 // lanes-per-list form of k_pm_grid, with the entry's plane weight in u.
-// Longer lists (queued by the list sort) are left to k_pm_long3.
+// Longer lists (queued by k_pm_queue) are left to k_pm_long3.
 template <int W, bool kFirst>
 __global__ void __launch_bounds__(kPmThreads) k_pm_grid3(const uint32_t* offsets, const uint32_t* entries,
                                                          const PmRecord3<W>* pm, const PmCol3<W>* pmc, const double* w,
@@ -3204,7 +2925,18 @@ __global__ void __launch_bounds__(kPmThreads) k_pm_grid3(const uint32_t* offsets
   if (active) pm_reduce_store(cells, threadIdx.x - q, q, grid + (static_cast<size_t>(plane) * g + row) * g, lo, g);
 }
 
-// The queued long lists (count at long_lists[0], global list ids after it)
+// The lists longer than kPmLong entries, queued: count at long_lists[0]
+// (cleared before), global list ids after it.
+constexpr int kPmLong = 512;
+
+__global__ void __launch_bounds__(256) k_pm_queue(const uint32_t* offsets, int planes, int lists, uint32_t* long_lists) {
+  const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= static_cast<size_t>(planes) * lists) return;
+  const uint32_t* off = offsets + i + i / lists;  // lists + 1 offsets per plane
+  if (off[1] - off[0] > kPmLong) long_lists[1 + atomicAdd(long_lists, 1u)] = static_cast<uint32_t>(i);
+}
+
+// The queued long lists
 // are cut into parts of kPmPart entries: part_base[i] is the first part of
 // queued list i (an exclusive scan, the total at part_base[count]).
 constexpr uint32_t kPmPart = 512;
@@ -3370,8 +3102,9 @@ __global__ void __launch_bounds__(256) k_pm_update3(const PmRecord3<W>* pm, cons
 }
 
 struct PmLayout3 {
-  size_t flags, cleared, records, counts, cursor, offsets, bases, entries, long_lists, mid_lists, pm, pmc, wzr, w, grid, part_base, partial,
-      counters, total, entries_total, max_long;
+  size_t flags, records, entries, long_lists, pm, pmc, wzr, w, grid, part_base, partial, counters, total, entries_total,
+      max_long;
+  Lists3 lists;
 };
 
 PmLayout3 make_pm_layout3(const Shape& s) {
@@ -3383,18 +3116,13 @@ PmLayout3 make_pm_layout3(const Shape& s) {
     return at;
   };
   const size_t g = static_cast<size_t>(s.grid_rows);
-  const size_t nl = g * s.lists_per_frame;
   l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
-  l.flags = take(kFlagBytes);  // flags and counts are cleared together
-  l.counts = take(nl * 4);
-  l.cleared = off;
+  l.max_long = l.entries_total / (kPmLong + 1) + 2;
+  l.flags = take(kFlagBytes);
   l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
-  l.cursor = take(nl * 4);
-  l.offsets = take((nl + g) * 4);
-  l.bases = take(g * 4);
+  l.lists = take_lists3(s, take);
   l.entries = take(l.entries_total * 4);
-  l.long_lists = take((2 + l.entries_total / (s.list_capacity + 1)) * 4);
-  l.mid_lists = take((2 + l.entries_total / 33) * 4);
+  l.long_lists = take(l.max_long * 4);
   l.pm = take(static_cast<size_t>(s.samples) * (16 + 24 * static_cast<size_t>(s.width)));
   l.pmc = take(static_cast<size_t>(s.samples) * (8 + 8 * static_cast<size_t>(s.width)));
   l.wzr = take(l.entries_total * sizeof(double));
@@ -3402,7 +3130,6 @@ PmLayout3 make_pm_layout3(const Shape& s) {
   l.grid = take(g * g * g * sizeof(double));
   // the long lists' parts of kPmPart entries: first part of each list, the
   // parts' sums, one counter per list
-  l.max_long = l.entries_total / (static_cast<size_t>(s.list_capacity) + 1) + 2;
   l.part_base = take((l.max_long + 1) * 4);
   l.partial = take((l.entries_total / kPmPart + l.max_long) * kChunk * sizeof(double));
   l.counters = take(l.max_long * 4);
@@ -3416,12 +3143,11 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
   static_assert(sizeof(PmRecord3<W>) == 16 + 24 * W, "PmRecord3 layout");
   const int g = s.grid_rows;
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  if (cudaMemsetAsync(flags, 0, l.cleared - l.flags, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-  const ksj_gpu_status st = build_lists3<W>(
-      s, KSJ_GPU_DCF_NONE, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
-      reinterpret_cast<uint32_t*>(ws + l.cursor), reinterpret_cast<uint32_t*>(ws + l.offsets),
-      reinterpret_cast<uint32_t*>(ws + l.bases), reinterpret_cast<uint32_t*>(ws + l.entries), nullptr,
-      reinterpret_cast<uint32_t*>(ws + l.long_lists), reinterpret_cast<uint32_t*>(ws + l.mid_lists), stream);
+  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess ||
+      cudaMemsetAsync(ws + l.long_lists, 0, 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  const ksj_gpu_status st =
+      build_lists3<W>(s, KSJ_GPU_DCF_NONE, d_traj, nullptr, flags, ws + l.records, ws, l.lists,
+                      reinterpret_cast<uint32_t*>(ws + l.entries), nullptr, stream);
   if (st != KSJ_GPU_OK) return st;
   static_assert(sizeof(PmCol3<W>) == 8 + 8 * W, "PmCol3 layout");
   PmRecord3<W>* pm = reinterpret_cast<PmRecord3<W>*>(ws + l.pm);
@@ -3434,13 +3160,19 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
     k_pm_prepare3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(d_traj, pm, pmc, w, s.samples, g, s.beta,
                                                                  1.0 / std::cyl_bessel_i(0.0, static_cast<double>(s.beta)));
   }
-  const uint32_t* offsets = reinterpret_cast<const uint32_t*>(ws + l.offsets);
+  const uint32_t* offsets = reinterpret_cast<const uint32_t*>(ws + l.lists.offsets);
   const uint32_t* entries = reinterpret_cast<const uint32_t*>(ws + l.entries);
   const uint32_t* long_lists = reinterpret_cast<const uint32_t*>(ws + l.long_lists);
   uint32_t* part_base = reinterpret_cast<uint32_t*>(ws + l.part_base);
   uint32_t* counters = reinterpret_cast<uint32_t*>(ws + l.counters);
   double* partial = reinterpret_cast<double*>(ws + l.partial);
   if (cudaMemsetAsync(counters, 0, l.max_long * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  {
+    LaunchScope scope("k_pm_queue", stream);
+    const size_t lists = static_cast<size_t>(g) * s.lists_per_frame;
+    k_pm_queue<<<static_cast<unsigned>((lists + 255) / 256), 256, 0, stream>>>(
+        offsets, g, s.lists_per_frame, reinterpret_cast<uint32_t*>(ws + l.long_lists));
+  }
   {
     LaunchScope scope("k_pm_long_parts", stream);
     k_pm_long_parts<<<1, 1024, 0, stream>>>(long_lists, offsets, s.lists_per_frame, part_base);
@@ -3459,7 +3191,7 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
       LaunchScope scope("k_pm_grid3", stream);
       auto kernel = it == 0 ? k_pm_grid3<W, true> : k_pm_grid3<W, false>;
       kernel<<<grid_blocks, kPmThreads, 0, stream>>>(offsets, entries, pm, pmc, w, wzr, grid, g, s.nchunks,
-                                                     s.lists_per_frame, s.list_capacity);
+                                                     s.lists_per_frame, kPmLong);
     }
     {
       LaunchScope scope("k_pm_long3", stream);
