@@ -94,6 +94,9 @@ struct alignas(16) SampleRecord3 {
 // the chunk wrapped past the last column), the sample index, and the W column
 // weights times the list's row (and plane) weight.
 __host__ __device__ constexpr int entry_bytes(int w) { return 8 + 4 * w; }
+// Widths 2 and 6 are stored and loaded in 16-byte vectors (24-byte entries padded
+// to 32 for the same cost the row pass 2 % more than they saved).
+__host__ __device__ constexpr bool entry_vectors(int w) { return entry_bytes(w) % 16 == 0; }
 
 // A staged entry in shared memory: the 16 weights of the chunk's columns (zero
 // where no tap falls), then the sample index.  80 bytes apart, so that lanes
@@ -208,13 +211,24 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   s->lists_per_frame = s->grid_rows * s->nchunks;
   s->entries_per_frame = static_cast<size_t>(s->samples) * s->width * 2;
   {
-    // as many blocks as k_place has resident at once, over all frames: fewer
-    // leave SMs idle, more only add counts to scan
+    // Samples per block of the binning, in turns of kBinThreads: the time is about
+    // the turns an SM gets, with the loading of the list positions (one turn per
+    // 4608 lists) for each block and half as much again where it has one block
+    // alone; so the blocks of all frames should fill whole rounds of SMs (96 frames x
+    // 26 turns: 3, 4, 6 blocks a frame take 108, 161, 132 us of k_place).
     const int turns = (s->samples + kBinThreads - 1) / kBinThreads;
-    const int resident = 152 * std::min(4, std::max(1, static_cast<int>(220 * 1024 / (kPlaceListBytes * s->lists_per_frame))));
-    const int blocks = std::min(turns, std::max(1, resident / s->frames));
-    s->bin_span = (turns + blocks - 1) / blocks * kBinThreads;
-    s->bin_blocks = (s->samples + s->bin_span - 1) / s->bin_span;
+    const double load = s->lists_per_frame / 4608.0;
+    double best = 0.0;
+    for (int t = 1; t <= turns; t += 1 + t / 16) {
+      const int blocks = (turns + t - 1) / t;
+      const double rounds = std::ceil(static_cast<double>(blocks) * s->frames / 152.0);
+      const double cost = (t + load) * std::max(rounds, 1.5);
+      if (t == 1 || cost <= best) {
+        best = cost;
+        s->bin_span = t * kBinThreads;
+        s->bin_blocks = blocks;
+      }
+    }
   }
   s->out_rows = s->rows;
   s->out_cols = s->cols;
@@ -727,11 +741,19 @@ ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, int lists,
 template <int W>
 __device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, const float* wc, int col_lo, int grid_cols,
                                           unsigned char* out) {
-  float2* o = reinterpret_cast<float2*>(out);
-  const int t0 = c0 - col_lo >= kChunk ? c0 - col_lo - grid_cols : c0 - col_lo;
-  o[0] = make_float2(__int_as_float(t0), __uint_as_float(sidx));
+  float v[entry_bytes(W) / 4];
+  v[0] = __int_as_float(c0 - col_lo >= kChunk ? c0 - col_lo - grid_cols : c0 - col_lo);
+  v[1] = __uint_as_float(sidx);
 #pragma unroll
-  for (int j = 0; j < W; j += 2) o[1 + j / 2] = make_float2(wrow * wc[j], wrow * wc[j + 1]);
+  for (int j = 0; j < W; ++j) v[2 + j] = wrow * wc[j];
+  if constexpr (entry_vectors(W)) {
+#pragma unroll
+    for (int q = 0; q < entry_bytes(W) / 16; ++q)
+      reinterpret_cast<float4*>(out)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < entry_bytes(W) / 8; ++q) reinterpret_cast<float2*>(out)[q] = make_float2(v[2 * q], v[2 * q + 1]);
+  }
 }
 
 struct PlaceArgs {
@@ -940,8 +962,14 @@ __device__ __forceinline__ uint32_t stage_entries(int w, float* slots, const uns
     float2 h = make_float2(__int_as_float(-kMaxWidth), 0.0f), p0 = h, p1 = h;  // no tap, no sample
     const float2* e = reinterpret_cast<const float2*>(ent + i * entry_bytes(w));
     if (i < cnt) {
-      h = __ldg(e);
-      p0 = __ldg(e + 1);
+      if (entry_vectors(w)) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(e));
+        h = make_float2(q.x, q.y);
+        p0 = make_float2(q.z, q.w);
+      } else {
+        h = __ldg(e);
+        p0 = __ldg(e + 1);
+      }
       if (w > 2) p1 = __ldg(e + 2);
     }
 #pragma unroll
