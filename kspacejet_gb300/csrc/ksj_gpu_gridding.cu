@@ -914,6 +914,7 @@ struct RowsArgs {
   int frames, channels, samples, grid_rows, grid_cols, nchunks, lists_per_frame, width;
   size_t entries_per_frame;
   int coil_group, coil_parts;
+  int both_ends;  // block x takes rows in from both ends
   int out_cols, cpitch;
   int col_shift;  // kept column of frequency k: (k + col_shift) mod grid_cols, when below out_cols
   uint32_t wait_limit;   // polls before a segment wait gives up
@@ -1096,7 +1097,9 @@ template <int kN, int kLgL, bool kHalf>
 __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   chain_begin();
-  const int row = blockIdx.x;
+  const int row = !a.both_ends ? blockIdx.x
+                  : (blockIdx.x & 1) ? a.grid_rows - 1 - static_cast<int>(blockIdx.x >> 1)
+                                     : static_cast<int>(blockIdx.x >> 1);
   const int cgi = blockIdx.y;
   const int f = a.frame0 + blockIdx.z;
   const int cg = kLgL ? (1 << kLgL) : a.coil_group;
@@ -1675,7 +1678,11 @@ struct RowsLauncher {
   }
 
   // One pass of nf frames of grid_rows rows and `groups` coil groups.
-  void launch(const RowsArgs& r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
+  // A launch of few waves takes the rows in from both ends: frequency 0, where radial
+  // scans crowd, is at row 0, and the rows before it, at the end, should not be the
+  // last to start (a 32-coil frame 72 -> 65 us; 48 frames, 61 waves, 1 % slower).
+  void launch(RowsArgs r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
+    r.both_ends = static_cast<long long>(grid_rows) * groups * nf <= 16 * 304;
     LaunchScope scope("k_rows", stream);
     launch_chained(kernel, dim3(grid_rows, groups, nf), threads, smem, stream, r);
   }
