@@ -1089,7 +1089,8 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
 //
 // kN: the row length for the two-step transform (128 .. 512), or 0 for the
 // in-place mixed-radix form of any other length; one instance per length keeps
-// each kernel's code small.  kLgL (when nonzero) fixes log2 of the coil group.
+// each kernel's code small.  kLgL (when nonzero) fixes log2 of the coil group, taken
+// whole (coil_parts 1), and with it the lane groups (3 % of the row pass at 32 coils).
 // kHalf: the sigma = 2 crop form of the row transform (out_cols =
 // grid_cols / 2, col_shift = out_cols / 2), whose kept columns are known at
 // compile time (fft_two_step_half); the same bytes as the general form.
@@ -1167,9 +1168,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
   __syncthreads();
 
   {
-    const int lg_parts = a.coil_parts - 1;  // coil_parts is 1 or 2
+    const int lg_parts = kLgL ? 0 : a.coil_parts - 1;  // coil_parts is 1 or 2
     const int lanes = cg >> lg_parts, groups = 32 / lanes;
-    const int g = lane / lanes, gl = lane - g * lanes;
+    const int g = lane / lanes, gl = lane & (lanes - 1);
     float* slots = reinterpret_cast<float*>(smem_raw + slot_off) +
                    static_cast<size_t>(warp * groups + g) * kRowsBatch * kSlotFloats;
     const int ntasks = task_base[a.nchunks] << lg_parts;
@@ -1646,10 +1647,12 @@ RowsKernel rows_kernel_two_step(int cg, bool half) {
     case 32: return half ? k_rows<kN, 5, true> : k_rows<kN, 5, false>;
     case 16: return half ? k_rows<kN, 4, true> : k_rows<kN, 4, false>;
     case 8: return half ? k_rows<kN, 3, true> : k_rows<kN, 3, false>;
+    case 4: return half ? k_rows<kN, 2, true> : k_rows<kN, 2, false>;
     default: return half ? k_rows<kN, 0, true> : k_rows<kN, 0, false>;
   }
 }
 
+// The instance for rows of n columns; cg 0: a coil group and parts known at run time.
 RowsKernel rows_kernel_for(int n, int cg, bool half) {
   switch (n) {
     case 128: return rows_kernel_two_step<128>(cg, half);
@@ -1671,7 +1674,7 @@ struct RowsLauncher {
     const int lanes = s.coil_group / s.coil_parts;
     threads = rows_threads_for(s.grid_cols, lanes, s.coil_group);
     smem = rows_smem_for(s.grid_cols, s.coil_group, lanes, threads);
-    kernel = rows_kernel_for(s.grid_cols, s.coil_group, s.kb && s.out_cols * 2 == s.grid_cols);
+    kernel = rows_kernel_for(s.grid_cols, s.coil_parts == 1 ? s.coil_group : 0, s.kb && s.out_cols * 2 == s.grid_cols);
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
                cudaSuccess &&
            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
