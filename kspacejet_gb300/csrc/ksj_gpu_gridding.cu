@@ -756,12 +756,28 @@ __device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, con
   }
 }
 
+// Density weights (2-D): a sample's double-precision taps, and one sorted list
+// entry as the grid step streams it.
+template <int W>
+struct PmRecord {
+  int r0, c0;  // first tap row and column (wrapped)
+  double wr[W];
+  double wc[W];
+};
+template <int W>
+struct alignas(16) PmEntry {
+  double wr;     // the list's row weight (0: the taps miss the row)
+  int t0;        // first tap's column as seen from the chunk, as in the float entries
+  uint32_t sample;
+  double wc[W];
+};
+
 struct PlaceArgs {
   const unsigned char* records;
   const uint32_t* offsets;  // [frame][list + 1]
   const uint32_t* starts;   // [frame][block][list]: the block's start in the list (k_bin_prefix)
-  unsigned char* expanded;  // entries in their places, or null:
-  uint32_t* entries;        // the sample indices alone
+  unsigned char* expanded;  // entries in their places
+  const void* pm;           // density weights: the samples' PmRecords, and `expanded` takes PmEntry
   int samples, grid_rows, grid_cols, nchunks, lists_per_frame, bin_span;
   size_t entries_per_frame;
 };
@@ -769,13 +785,15 @@ struct PlaceArgs {
 // One block per (block of samples, frame): kBinThreads samples at a time, their
 // places in turn (place_turn), their entries written outside the turns.
 //
+// kPm: the entries are the density weights' (PmEntry).
+//
 // Bound by the chain of turns and, for one frame, by launches: appending to the
 // lists with atomics and sorting each
 // afterwards took three kernels (scatter, sort, long sort: 40 us of a 128-grid
 // slice, 92 us of 205824 samples on a 512 grid, 219 us of 96 frames of 13056
 // samples) where this and k_bin_prefix take 21, 60 and 144.  (Finding the ranks inside the
 // turns, by lane masks per list in shared memory, took 203 of the 144.)
-template <int W>
+template <int W, bool kPm>
 __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
   extern __shared__ uint32_t place_smem[];
   chain_begin();
@@ -805,17 +823,33 @@ __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
     uint32_t pos[W][2];
     place_turn<W>(at, r0, k0, k1, a.nchunks, a.grid_rows, pos);
     if (r0 < 0) continue;
+    PmRecord<W> pm;
+    if constexpr (kPm) pm = static_cast<const PmRecord<W>*>(a.pm)[static_cast<size_t>(f) * a.samples + sample];
 #pragma unroll
     for (int j = 0; j < W; ++j) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (h && k1 == k0) continue;
         const size_t slot = static_cast<size_t>(f) * a.entries_per_frame + pos[j][h];
-        if (a.expanded != nullptr)
-          put_entry<W>(static_cast<uint32_t>(sample), c0, w[4 + j], w + 4 + W, (h ? k1 : k0) * kChunk, a.grid_cols,
+        const int col_lo = (h ? k1 : k0) * kChunk;
+        if constexpr (kPm) {
+          // the taps of the double-precision coordinate, on the list's row and chunk
+          int dr = (r0 + j >= a.grid_rows ? r0 + j - a.grid_rows : r0 + j) - pm.r0;
+          if (dr < 0) dr += a.grid_rows;
+          PmEntry<W> e;
+          e.wr = 0.0;
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            if (k == dr) e.wr = pm.wr[k];
+            e.wc[k] = pm.wc[k];
+          }
+          e.t0 = pm.c0 - col_lo >= kChunk ? pm.c0 - col_lo - a.grid_cols : pm.c0 - col_lo;
+          e.sample = static_cast<uint32_t>(sample);
+          reinterpret_cast<PmEntry<W>*>(a.expanded)[slot] = e;
+        } else {
+          put_entry<W>(static_cast<uint32_t>(sample), c0, w[4 + j], w + 4 + W, col_lo, a.grid_cols,
                        a.expanded + slot * entry_bytes(W));
-        else
-          a.entries[slot] = static_cast<uint32_t>(sample);
+        }
       }
     }
   }
@@ -1837,18 +1871,19 @@ struct ColsPass {
 };
 
 // The binning lists of one call: per-sample records, list offsets, and the lists'
-// entries in sample order, as the row pass reads them (`expanded`) or as sample
-// indices alone (`entries`); and the call's tables where `tables` names them.  The
-// flags must already be cleared.
+// entries in sample order, as the row pass reads them or, where `pm` holds the
+// density weights' records, as their grid step does; and the call's tables where
+// `tables` names them.  The flags must already be cleared.
 template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* totals,
-                           uint32_t* offsets, uint32_t* entries, unsigned char* expanded, cudaStream_t stream,
+                           uint32_t* offsets, unsigned char* expanded, const void* pm, cudaStream_t stream,
                            uint32_t* frame_flags = nullptr, const TablesArgs* tables = nullptr) {
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
+  const auto place = pm ? k_place<W, true> : k_place<W, false>;
   if (cudaFuncSetAttribute(k_prepare<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, count_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_place<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
+      cudaFuncSetAttribute(place, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
     return KSJ_GPU_ERROR_CUDA;
   const dim3 blocks(s.bin_blocks, s.frames);
   {
@@ -1892,7 +1927,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.offsets = offsets;
     p.starts = counts;
     p.expanded = expanded;
-    p.entries = entries;
+    p.pm = pm;
     p.samples = s.samples;
     p.grid_rows = s.grid_rows;
     p.grid_cols = s.grid_cols;
@@ -1901,7 +1936,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.bin_span = s.bin_span;
     p.entries_per_frame = s.entries_per_frame;
     LaunchScope scope("k_place", stream);
-    launch_chained(k_place<W>, blocks, kBinThreads, place_smem, stream, p);
+    launch_chained(place, blocks, kBinThreads, place_smem, stream, p);
   }
   return KSJ_GPU_OK;
 }
@@ -1945,7 +1980,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   {
     const ksj_gpu_status st =
         build_lists<W>(s, d, d_traj, d_dcf, flags, records, reinterpret_cast<uint32_t*>(ws + l.counts),
-                       reinterpret_cast<uint32_t*>(ws + l.totals), offsets, nullptr, ws + l.expanded, stream,
+                       reinterpret_cast<uint32_t*>(ws + l.totals), offsets, ws + l.expanded, nullptr, stream,
                        reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables);
     if (st != KSJ_GPU_OK) return st;
   }
@@ -2068,17 +2103,124 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
 // give, per (row, 16-column chunk), the samples touching it in increasing
 // order, so each grid cell sums its samples in that order: deterministic.
 
-template <int W>
-struct PmRecord {
-  int r0, c0;  // first tap row and column (wrapped)
-  double wr[W];
-  double wc[W];
-};
-
 __device__ __forceinline__ double kb_weight64(double d, int width, double beta, double inv_i0_beta) {
   const double t = 2.0 * d / static_cast<double>(width);
   if (t * t > 1.0) return 0.0;
   return cyl_bessel_i0(beta * sqrt(1.0 - t * t)) * inv_i0_beta;
+}
+
+// The Kaiser-Bessel weight of tap j, at distance d = j - W/2 + 1 - f of a coordinate
+// with the fraction f in [0, 1), as a polynomial in z = 2 f - 1: I0(beta sqrt(1 - (2 d /
+// W)^2)) / I0(beta) is an entire function of d, so its Chebyshev coefficients fall
+// off factorially.  The host interpolates each tap at kKbNodes Chebyshev points (values
+// from the Maclaurin series sum (beta^2 s / 4)^k / (k!)^2, all terms positive) and
+// drops the terms below 2^-52 of the peak.  Tap W - 1 - j is tap j mirrored in z, so
+// its even and odd parts give both: 16 to 20 multiply-adds for two weights, where the
+// square root, the division by W and the Bessel function's two ranges took about
+// 70 FP64 instructions for one.  The largest error over the widths and oversamplings
+// of 1 to 4 is 7e-16 of the peak.  A beta that kKbNodes points do not resolve (above 28 to
+// 40, where the default for width 8 ends at 23) leaves `half` 0 and the weights to
+// kb_weight64.
+constexpr int kKbNodes = 32;
+struct KbTaps {
+  int half;               // even and odd coefficients kept of every tap, or 0
+  double c[4][kKbNodes];  // monomial coefficients in z of tap j < W / 2
+};
+
+KbTaps kb_taps(int width, double beta) {
+  constexpr double kPi = 3.14159265358979323846;
+  double series[64];  // (beta^2 / 4)^k / (k!)^2 over I0(beta)
+  int terms = 0;
+  {
+    long double term[64] = {1.0L}, top = 1.0L;
+    while (++terms < 63 && term[terms - 1] > 1e-19L * top) {
+      term[terms] = term[terms - 1] * (0.25L * beta * beta) / (static_cast<long double>(terms) * terms);
+      top += term[terms];
+    }
+    if (terms == 63) return KbTaps{};
+    for (int k = 0; k < terms; ++k) series[k] = static_cast<double>(term[k] / top);
+  }
+  // Horner's rule with the rounding errors carried along (Graillat, Langlois, Louvet 2005)
+  auto i0 = [&](double s) {
+    double sum = series[terms - 1], carry = 0.0;
+    for (int k = terms - 2; k >= 0; --k) {
+      const double product = sum * s, next = product + series[k], part = next - product;
+      carry = std::fma(carry, s, std::fma(sum, s, -product) + ((product - (next - part)) + (series[k] - part)));
+      sum = next;
+    }
+    return sum + carry;
+  };
+  double cosine[4 * kKbNodes];
+  for (int i = 0; i <= kKbNodes / 2; ++i) {  // angles up to pi / 4, then by symmetry
+    cosine[i] = std::cos(kPi * i / (2 * kKbNodes));
+    cosine[kKbNodes - i] = std::sin(kPi * i / (2 * kKbNodes));
+  }
+  for (int i = 1; i <= kKbNodes; ++i) cosine[kKbNodes + i] = -cosine[kKbNodes - i];
+  for (int i = 1; i < 2 * kKbNodes; ++i) cosine[2 * kKbNodes + i] = cosine[2 * kKbNodes - i];
+  KbTaps p{};
+  for (int tap = 0; tap < width / 2; ++tap) {
+    double value[kKbNodes], cheb[kKbNodes];
+    for (int j = 0; j < kKbNodes; ++j) {
+      const double t = (2.0 * (tap - width / 2 + 1) - 1.0 - cosine[2 * j + 1]) / width;  // 2 d / W
+      value[j] = i0(std::max(std::fma(-t, t, 1.0), 0.0));
+    }
+    int degree = 0;
+    for (int k = 0; k < kKbNodes; ++k) {
+      double sum = 0.0, carry = 0.0;
+      for (int j = 0; j < kKbNodes; ++j) {
+        const double product = value[j] * cosine[(k * (2 * j + 1)) % (4 * kKbNodes)], next = sum + product,
+                     part = next - sum;
+        carry += (sum - (next - part)) + (product - part);
+        sum = next;
+      }
+      cheb[k] = (k == 0 ? 1.0 : 2.0) / kKbNodes * (sum + carry);
+      if (std::fabs(cheb[k]) > 0x1p-52) degree = k;
+    }
+    if (degree > kKbNodes - 3) return KbTaps{};
+    p.half = std::max(p.half, degree / 2 + 1);
+    // T_k in monomials, by its recurrence
+    double t0[kKbNodes] = {1.0}, t1[kKbNodes] = {0.0, 1.0};
+    p.c[tap][0] = cheb[0];
+    for (int k = 1; k <= degree; ++k) {
+      for (int i = 0; i <= k; ++i) p.c[tap][i] += cheb[k] * t1[i];
+      double t2[kKbNodes] = {};
+      for (int i = 0; i < kKbNodes; ++i) t2[i] = (i > 0 ? 2.0 * t1[i - 1] : 0.0) - t0[i];
+      std::copy(t1, t1 + kKbNodes, t0);
+      std::copy(t2, t2 + kKbNodes, t1);
+    }
+  }
+  return p;
+}
+
+// The W weights of each of two coordinates with fractions f.
+template <int W>
+__device__ __forceinline__ void kb_weights64(const KbTaps& p, const double (&f)[2], double (&out)[2][W]) {
+  double x[2], z[2], even[2][W / 2], odd[2][W / 2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    z[i] = fma(2.0, f[i], -1.0);
+    x[i] = z[i] * z[i];
+#pragma unroll
+    for (int j = 0; j < W / 2; ++j) even[i][j] = odd[i][j] = 0.0;
+  }
+  for (int k = p.half - 1; k >= 0; --k) {
+#pragma unroll
+    for (int j = 0; j < W / 2; ++j) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        even[i][j] = fma(even[i][j], x[i], p.c[j][2 * k]);
+        odd[i][j] = fma(odd[i][j], x[i], p.c[j][2 * k + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+#pragma unroll
+    for (int j = 0; j < W / 2; ++j) {
+      out[i][j] = fma(z[i], odd[i][j], even[i][j]);
+      out[i][W - 1 - j] = fma(-z[i], odd[i][j], even[i][j]);
+    }
+  }
 }
 
 // Per sample: the double-precision tap weights and w = 1.  The coordinate
@@ -2086,7 +2228,8 @@ __device__ __forceinline__ double kb_weight64(double d, int width, double beta, 
 // division); a sample the gridding checks rejected gets w = 0.
 template <int W>
 __global__ void __launch_bounds__(256) k_pm_prepare(const float* traj, PmRecord<W>* pm, double* w, size_t total,
-                                                    int grid_rows, int grid_cols, double beta, double inv_i0_beta,
+                                                    int grid_rows, int grid_cols, const __grid_constant__ KbTaps taps,
+                                                    double beta, double inv_i0_beta,
                                                     int require_nyquist) {
   const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
@@ -2103,10 +2246,20 @@ __global__ void __launch_bounds__(256) k_pm_prepare(const float* traj, PmRecord<
     const int tc = static_cast<int>(floor(uc)) - W / 2 + 1;
     r.r0 = wrap_index(tr, grid_rows);
     r.c0 = wrap_index(tc, grid_cols);
+    if (taps.half > 0) {
+      const double f[2] = {ur - floor(ur), uc - floor(uc)};
+      double v[2][W];
+      kb_weights64<W>(taps, f, v);
 #pragma unroll
-    for (int j = 0; j < W; ++j) {
-      r.wr[j] = kb_weight64(static_cast<double>(tr + j) - ur, W, beta, inv_i0_beta);
-      r.wc[j] = kb_weight64(static_cast<double>(tc + j) - uc, W, beta, inv_i0_beta);
+      for (int j = 0; j < W; ++j) {
+        r.wr[j] = v[0][j];
+        r.wc[j] = v[1][j];
+      }
+    } else {
+      for (int j = 0; j < W; ++j) {
+        r.wr[j] = kb_weight64(static_cast<double>(tr + j) - ur, W, beta, inv_i0_beta);
+        r.wc[j] = kb_weight64(static_cast<double>(tc + j) - uc, W, beta, inv_i0_beta);
+      }
     }
   } else {
     r.r0 = 0;
@@ -2121,42 +2274,19 @@ __global__ void __launch_bounds__(256) k_pm_prepare(const float* traj, PmRecord<
   w[idx] = ok ? 1.0 : 0.0;
 }
 
-// The grid step, kPmLanes lanes per list: lane q takes the list's entries q,
-// q + kPmLanes, ... in order and, for every column tap of an entry that lands
-// in the list's 16-column chunk, adds u * wc[k] (u = w times the entry's row,
-// and plane, weights) to its own 16 cells in shared memory (cell t of thread
-// i at cells[t * kPmThreads + i]: the lanes of a warp always touch distinct
-// banks).  Then lane q sums cells 4q .. 4q+3 over the list's lanes, each cell
-// in a fixed order (starting at lane q), and writes them.  Every FP64
-// operation a lane issues is one a cell needs; with a lane per column
-// instead, 12 of every 16 lanes multiplied by taps outside their column, and
-// this step is bound by the FP64 pipe.  Lists are kPmLanes consecutive lanes
-// of one warp, so a warp barrier orders the two phases.
+// The grid step with kPmLanes lanes per list (3-D, and the longer lists in 2-D): lane q
+// takes the list's entries q, q + kPmLanes, ... in order and, for every column tap of
+// an entry that lands in the list's 16-column chunk, adds u * wc[k] (u = w times
+// the entry's row, and plane, weights) to its own 16 cells in shared memory; then lane q
+// sums cells 4q .. 4q+3 over the list's lanes, each cell in a fixed order
+// (starting at lane q).  Every FP64 operation a lane issues is one a cell
+// needs; with a lane per column instead, 12 of every 16 lanes multiplied by taps
+// outside their column.  Lists are kPmLanes consecutive lanes of one warp, so a
+// warp barrier orders the two phases.
 constexpr int kPmLanes = 4;
 constexpr int kPmThreads = 256;
 constexpr int kPmCellsPerLane = kChunk / kPmLanes;
 static_assert(kChunk == 16 && (kPmLanes & (kPmLanes - 1)) == 0 && 32 % kPmLanes == 0, "lanes of a list");
-
-// One lane's share of the list's entries [e0, e1) (every `step`-th), added to
-// its cells (cell[t * kPmThreads], t = column - lo).  `weight(r, sidx, &u)`
-// gives the entry's u, or false when its row (and plane) taps miss the list.
-template <int W, class Rec, class Weight>
-__device__ __forceinline__ void pm_accumulate(const uint32_t* entries, uint32_t e0, uint32_t e1, uint32_t step,
-                                              const Rec* rec, int lo, int grid_cols, double* cell, Weight weight) {
-  for (uint32_t e = e0; e < e1; e += step) {
-    const uint32_t sidx = __ldg(entries + e);
-    const Rec& r = rec[sidx];
-    double u;
-    if (!weight(r, sidx, &u)) continue;
-    int col = r.c0;
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
-      const int t = col - lo;
-      if (t >= 0 && t < kChunk) cell[t * kPmThreads] = fma(u, r.wc[k], cell[t * kPmThreads]);
-      if (++col == grid_cols) col = 0;
-    }
-  }
-}
 
 // Lane q of a list (its lane 0 is thread `lane0`): cells 4q .. 4q+3 summed
 // over the list's lanes, starting at lane q, written to row[lo + t] inside
@@ -2174,40 +2304,156 @@ __device__ __forceinline__ void pm_reduce_store(const double* cells, int lane0, 
   }
 }
 
+// The lists of a call ordered by length, longest first (bins of up to
+// kPmBins - 1 entries, longer ones in the last; any order within a bin): a warp of the
+// grid step issues every FP64 instruction for all its lanes, so lists of one
+// warp should end together.  bins: kPmBins counts, then kPmBins cursors, cleared before.
+constexpr int kPmBins = 256;
+constexpr int kPmOrderThreads = 1024;
+
+__device__ __forceinline__ uint32_t list_length(const uint32_t* offsets, size_t list, int lists_per_frame) {
+  const uint32_t* off = offsets + list + list / lists_per_frame;  // lists + 1 offsets per frame
+  return off[1] - off[0];
+}
+
+__global__ void __launch_bounds__(kPmOrderThreads) k_pm_bins(const uint32_t* offsets, size_t lists, int lists_per_frame,
+                                                             uint32_t* bins) {
+  __shared__ uint32_t count[kPmBins];
+  for (int i = threadIdx.x; i < kPmBins; i += kPmOrderThreads) count[i] = 0;
+  __syncthreads();
+  const size_t list = static_cast<size_t>(blockIdx.x) * kPmOrderThreads + threadIdx.x;
+  if (list < lists) atomicAdd(count + min(list_length(offsets, list, lists_per_frame), kPmBins - 1u), 1u);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kPmBins; i += kPmOrderThreads)
+    if (count[i] != 0) atomicAdd(bins + i, count[i]);
+}
+
+__global__ void __launch_bounds__(kPmOrderThreads) k_pm_order(const uint32_t* offsets, size_t lists,
+                                                              int lists_per_frame, uint32_t* bins, uint32_t* order) {
+  __shared__ uint32_t count[kPmBins], start[kPmBins];
+  for (int i = threadIdx.x; i < kPmBins; i += kPmOrderThreads) {
+    count[i] = 0;
+    uint32_t before = 0;  // lists of longer bins
+    for (int j = i + 1; j < kPmBins; ++j) before += __ldg(bins + j);
+    start[i] = before;
+  }
+  __syncthreads();
+  const size_t list = static_cast<size_t>(blockIdx.x) * kPmOrderThreads + threadIdx.x;
+  uint32_t bin = 0, rank = 0;
+  if (list < lists) {
+    bin = min(list_length(offsets, list, lists_per_frame), kPmBins - 1u);
+    rank = atomicAdd(count + bin, 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kPmBins; i += kPmOrderThreads)
+    if (count[i] != 0) start[i] += atomicAdd(bins + kPmBins + i, count[i]);
+  __syncthreads();
+  if (list < lists) order[start[bin] + rank] = static_cast<uint32_t>(list);
+}
+
+// The 2-D grid step: one lane per list of up to kPmAlone entries, kPmLanes lanes for a
+// longer one (which come first in `order`), each adding u * wc[k] (u = w times
+// the entry's row weight) for the column taps that land in the list's chunk to its
+// own 16 cells in shared memory; four lanes' cells are then added in a fixed
+// order.  A half-warp writes a list's cells.  The entries are streamed (16 + 8 W
+// bytes, written in list order once a call), the next one requested while one is added.
+//
+// Bound by the FP64 pipe (two lanes per clock and SM): 5 operations an entry and,
+// for the few lists of four lanes, 48 to add them.  Four lanes for every list, in grid
+// order, spent 4 of 5 issues on idle lanes and as many again on adding the lanes:
+// 275 us an iteration on 96 frames x 13056 samples, now 144.
+constexpr uint32_t kPmAlone = 32;
+constexpr int kPmPitch = kChunk + 1;  // cells of one thread, an odd number of doubles apart
+
 template <int W>
-__global__ void __launch_bounds__(kPmThreads) k_pm_grid(const uint32_t* offsets, const uint32_t* entries,
-                                                        const PmRecord<W>* pm, const double* w, double* grid,
-                                                        int frames, int samples, int grid_rows, int grid_cols,
-                                                        int nchunks, int lists_per_frame, size_t entries_per_frame) {
-  __shared__ double cells[kChunk * kPmThreads];
-  const size_t list = (static_cast<size_t>(blockIdx.x) * kPmThreads + threadIdx.x) / kPmLanes;
-  const int q = threadIdx.x & (kPmLanes - 1);
-  double* cell = cells + threadIdx.x;
+__global__ void __launch_bounds__(kPmThreads) k_pm_grid(const uint32_t* offsets, const PmEntry<W>* entries,
+                                                        const uint32_t* order, const uint32_t* bins, const double* w,
+                                                        double* grid, size_t lists, int samples, int grid_rows,
+                                                        int grid_cols, int nchunks, int lists_per_frame,
+                                                        size_t entries_per_frame) {
+  __shared__ double cells[kPmThreads * kPmPitch];
+  __shared__ uint32_t many_shared;
+  // lists of more than kPmAlone entries
+  if (threadIdx.x < 32) {
+    uint32_t n = 0;
+    for (int i = kPmAlone + 1 + threadIdx.x; i < kPmBins; i += 32) n += __ldg(bins + i);
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (threadIdx.x == 0) many_shared = n;
+  }
+  __syncthreads();
+  const size_t many = many_shared;
+  const size_t many_threads = (many * kPmLanes + kPmThreads - 1) / kPmThreads * kPmThreads;
+  const size_t thread = static_cast<size_t>(blockIdx.x) * kPmThreads + threadIdx.x;
+  const bool split = thread < many_threads;  // the same for a whole block
+  const size_t rank = split ? thread / kPmLanes : many + thread - many_threads;
+  const int q = split ? threadIdx.x & (kPmLanes - 1) : 0;
+  const bool active = rank < (split ? many : lists);
+  if (!__syncthreads_or(active)) return;
+  double* cell = cells + threadIdx.x * kPmPitch;
 #pragma unroll
-  for (int t = 0; t < kChunk; ++t) cell[t * kPmThreads] = 0.0;
-  const bool active = list < static_cast<size_t>(frames) * lists_per_frame;
-  int f = 0, row = 0, lo = 0;
+  for (int t = 0; t < kChunk; ++t) cell[t] = 0.0;
+  double* out = nullptr;  // the list's first cell in the grid
+  int width = 0;
   if (active) {
-    f = static_cast<int>(list / lists_per_frame);
-    const int l = static_cast<int>(list - static_cast<size_t>(f) * lists_per_frame);
-    row = l / nchunks;
-    lo = (l - row * nchunks) * kChunk;
+    const uint32_t list = __ldg(order + rank);
+    const int f = static_cast<int>(list / static_cast<uint32_t>(lists_per_frame));
+    const int l = static_cast<int>(list - static_cast<uint32_t>(f) * lists_per_frame);
+    const int row = l / nchunks, lo = (l - row * nchunks) * kChunk;
+    out = grid + (static_cast<size_t>(f) * grid_rows + row) * grid_cols + lo;
+    width = min(kChunk, grid_cols - lo);
     const uint32_t* off = offsets + static_cast<size_t>(f) * (lists_per_frame + 1);
-    const PmRecord<W>* rec = pm + static_cast<size_t>(f) * samples;
+    const PmEntry<W>* ent = entries + static_cast<size_t>(f) * entries_per_frame;
     const double* wf = w + static_cast<size_t>(f) * samples;
-    pm_accumulate<W>(entries + static_cast<size_t>(f) * entries_per_frame, off[l] + q, off[l + 1], kPmLanes, rec, lo,
-                     grid_cols, cell, [&](const PmRecord<W>& r, uint32_t sidx, double* u) {
-                       int dr = row - r.r0;
-                       if (dr < 0) dr += grid_rows;
-                       if (dr >= W) return false;
-                       *u = wf[sidx] * r.wr[dr];
-                       return true;
-                     });
+    const int wrap = nchunks == 1 ? grid_cols : 0;  // one chunk sees both ends of a wrapped stencil
+    const uint32_t end = off[l + 1], step = split ? kPmLanes : 1;
+    auto load = [&](uint32_t e) {
+      PmEntry<W> r;
+      const float4* src = reinterpret_cast<const float4*>(ent + e);
+      float4* dst = reinterpret_cast<float4*>(&r);
+#pragma unroll
+      for (int v = 0; v < static_cast<int>(sizeof(PmEntry<W>) / 16); ++v) dst[v] = __ldg(src + v);
+      return r;
+    };
+    uint32_t e = off[l] + q;
+    if (e < end) {
+      PmEntry<W> next = load(e);
+      for (; e < end; e += step) {
+        const PmEntry<W> r = next;
+        const double weight = wf[r.sample];
+        if (e + step < end) next = load(e + step);
+        const double u = weight * r.wr;
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+          int t = r.t0 + k;
+          if (wrap != 0 && t >= wrap) t -= wrap;
+          if (static_cast<uint32_t>(t) < kChunk) cell[t] = fma(u, r.wc[k], cell[t]);
+        }
+      }
+    }
   }
   __syncwarp();
-  if (active)
-    pm_reduce_store(cells, threadIdx.x - q, q, grid + (static_cast<size_t>(f) * grid_rows + row) * grid_cols, lo,
-                    grid_cols);
+  const int lane = threadIdx.x & 31;
+  if (split) {
+    // lane q of a list: cells 4q .. 4q + 3 over its lanes, starting at lane q, left in lane 0's
+    double sum[kPmCellsPerLane];
+#pragma unroll
+    for (int i = 0; i < kPmCellsPerLane; ++i) {
+      const double* c = cells + (threadIdx.x - q) * kPmPitch + q * kPmCellsPerLane + i;
+      sum[i] = c[q * kPmPitch];
+#pragma unroll
+      for (int j = 1; j < kPmLanes; ++j) sum[i] += c[((q + j) & (kPmLanes - 1)) * kPmPitch];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kPmCellsPerLane; ++i) cells[(threadIdx.x - q) * kPmPitch + q * kPmCellsPerLane + i] = sum[i];
+    __syncwarp();
+  }
+  // two lists at a time, a half-warp each
+  for (int i = (lane >> 4) * (split ? kPmLanes : 1); i < 32; i += 2 * (split ? kPmLanes : 1)) {
+    double* to = reinterpret_cast<double*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(out), i));
+    const int n = __shfl_sync(0xffffffffu, width, i);
+    if ((lane & 15) < n) to[lane & 15] = cells[(threadIdx.x - lane + i) * kPmPitch + (lane & 15)];
+  }
 }
 
 // Per sample: d = the grid read back through the sample's taps (row-major),
@@ -2246,7 +2492,7 @@ __global__ void __launch_bounds__(256) k_pm_update(const PmRecord<W>* pm, const 
 }
 
 struct PmLayout {
-  size_t flags, records, counts, totals, offsets, entries, pm, w, grid, total;
+  size_t flags, records, counts, totals, offsets, entries, bins, order, pm, w, grid, total;
 };
 
 PmLayout make_pm_layout(const Shape& s) {
@@ -2264,7 +2510,9 @@ PmLayout make_pm_layout(const Shape& s) {
   l.counts = take(nl * s.bin_blocks * 4);
   l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
-  l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * 4);
+  l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * (16 + 8 * static_cast<size_t>(s.width)));
+  l.bins = take(2 * kPmBins * 4);
+  l.order = take(nl * 4);
   l.pm = take(fm * (8 + 16 * static_cast<size_t>(s.width)));
   l.w = take(fm * sizeof(double));
   l.grid = take(static_cast<size_t>(s.frames) * s.grid_rows * s.grid_cols * sizeof(double));
@@ -2281,29 +2529,42 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
   if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   ksj_gpu_gridding_desc dd = *d;
   dd.dcf_mode = KSJ_GPU_DCF_NONE;
-  const ksj_gpu_status st =
-      build_lists<W>(s, &dd, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
-                     reinterpret_cast<uint32_t*>(ws + l.totals), reinterpret_cast<uint32_t*>(ws + l.offsets),
-                     reinterpret_cast<uint32_t*>(ws + l.entries), nullptr, stream);
-  if (st != KSJ_GPU_OK) return st;
+  static_assert(sizeof(PmEntry<W>) == 16 + 8 * W, "PmEntry layout");
   const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   PmRecord<W>* pm = reinterpret_cast<PmRecord<W>*>(ws + l.pm);
   double* w = reinterpret_cast<double*>(ws + l.w);
   double* grid = reinterpret_cast<double*>(ws + l.grid);
-  const double beta = s.beta;
   {
     LaunchScope scope("k_pm_prepare", stream);
     k_pm_prepare<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
-        d_traj, pm, w, fm, s.grid_rows, s.grid_cols, beta, 1.0 / std::cyl_bessel_i(0.0, beta), d->require_nyquist);
+        d_traj, pm, w, fm, s.grid_rows, s.grid_cols, kb_taps(W, s.beta), s.beta,
+        1.0 / std::cyl_bessel_i(0.0, static_cast<double>(s.beta)), d->require_nyquist);
   }
+  const ksj_gpu_status st =
+      build_lists<W>(s, &dd, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
+                     reinterpret_cast<uint32_t*>(ws + l.totals), reinterpret_cast<uint32_t*>(ws + l.offsets),
+                     ws + l.entries, pm, stream);
+  if (st != KSJ_GPU_OK) return st;
   const size_t lists = static_cast<size_t>(s.frames) * s.lists_per_frame;
+  const uint32_t* offsets = reinterpret_cast<const uint32_t*>(ws + l.offsets);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(ws + l.bins);
+  uint32_t* order = reinterpret_cast<uint32_t*>(ws + l.order);
+  if (cudaMemsetAsync(bins, 0, 2 * kPmBins * 4, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  const unsigned order_blocks = static_cast<unsigned>((lists + kPmOrderThreads - 1) / kPmOrderThreads);
+  {
+    LaunchScope scope("k_pm_bins", stream);
+    k_pm_bins<<<order_blocks, kPmOrderThreads, 0, stream>>>(offsets, lists, s.lists_per_frame, bins);
+  }
+  {
+    LaunchScope scope("k_pm_order", stream);
+    k_pm_order<<<order_blocks, kPmOrderThreads, 0, stream>>>(offsets, lists, s.lists_per_frame, bins, order);
+  }
   for (uint32_t it = 0; it < iterations; ++it) {
     {
       LaunchScope scope("k_pm_grid", stream);
-      k_pm_grid<W><<<static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads), kPmThreads, 0, stream>>>(
-          reinterpret_cast<const uint32_t*>(ws + l.offsets), reinterpret_cast<const uint32_t*>(ws + l.entries), pm,
-          w, grid, s.frames, s.samples, s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame,
-          s.entries_per_frame);
+      k_pm_grid<W><<<static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads + 1), kPmThreads, 0, stream>>>(
+          offsets, reinterpret_cast<const PmEntry<W>*>(ws + l.entries), order, bins, w, grid, lists, s.samples,
+          s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame);
     }
     LaunchScope scope("k_pm_update", stream);
     k_pm_update<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
@@ -2933,7 +3194,8 @@ __device__ __forceinline__ void pm3_accumulate(const uint32_t* entries, uint32_t
 }
 
 // The 3-D grid step for lists of at most `capacity` entries: the
-// lanes-per-list form of k_pm_grid, with the entry's plane weight in u.
+// kPmLanes lanes per list, with the entry's plane weight in u; cell t of thread i at
+// cells[t * kPmThreads + i], so that the lanes of a warp always touch distinct banks.
 // Longer lists (queued by k_pm_queue) are left to k_pm_long3.
 template <int W, bool kFirst>
 __global__ void __launch_bounds__(kPmThreads) k_pm_grid3(const uint32_t* offsets, const uint32_t* entries,
