@@ -2356,23 +2356,25 @@ __global__ void __launch_bounds__(kPmOrderThreads) k_pm_order(const uint32_t* of
 // the entry's row weight) for the column taps that land in the list's chunk to its
 // own 16 cells in shared memory; four lanes' cells are then added in a fixed
 // order.  A half-warp writes a list's cells.  The entries are streamed (16 + 8 W
-// bytes, written in list order once a call), the next one requested while one is added.
+// bytes, written in list order once a call), two requested ahead and the next
+// one's sample weight with them (one ahead, its weight fetched when it is used, 144 us an iteration, now 128).
 //
 // Bound by the FP64 pipe (two lanes per clock and SM): 5 operations an entry and,
 // for the few lists of four lanes, 48 to add them.  Four lanes for every list, in grid
 // order, spent 4 of 5 issues on idle lanes and as many again on adding the lanes:
-// 275 us an iteration on 96 frames x 13056 samples, now 144.
+// 275 us an iteration on 96 frames x 13056 samples, now 128.
 constexpr uint32_t kPmAlone = 32;
 constexpr int kPmPitch = kChunk + 1;  // cells of one thread, an odd number of doubles apart
 
 template <int W>
-__global__ void __launch_bounds__(kPmThreads) k_pm_grid(const uint32_t* offsets, const PmEntry<W>* entries,
+__global__ void __launch_bounds__(kPmThreads, W <= 4 ? 4 : 2) k_pm_grid(const uint32_t* offsets, const PmEntry<W>* entries,
                                                         const uint32_t* order, const uint32_t* bins, const double* w,
                                                         double* grid, size_t lists, int samples, int grid_rows,
                                                         int grid_cols, int nchunks, int lists_per_frame,
                                                         size_t entries_per_frame) {
   __shared__ double cells[kPmThreads * kPmPitch];
   __shared__ uint32_t many_shared;
+  chain_begin();
   // lists of more than kPmAlone entries
   if (threadIdx.x < 32) {
     uint32_t n = 0;
@@ -2416,12 +2418,15 @@ __global__ void __launch_bounds__(kPmThreads) k_pm_grid(const uint32_t* offsets,
     };
     uint32_t e = off[l] + q;
     if (e < end) {
-      PmEntry<W> next = load(e);
+      PmEntry<W> next = load(e), after = next;
+      double weight = wf[next.sample];
+      if (e + step < end) after = load(e + step);
       for (; e < end; e += step) {
         const PmEntry<W> r = next;
-        const double weight = wf[r.sample];
-        if (e + step < end) next = load(e + step);
         const double u = weight * r.wr;
+        next = after;
+        if (e + step < end) weight = wf[next.sample];
+        if (e + 2 * step < end) after = load(e + 2 * step);
 #pragma unroll
         for (int k = 0; k < W; ++k) {
           int t = r.t0 + k;
@@ -2462,6 +2467,7 @@ __global__ void __launch_bounds__(kPmThreads) k_pm_grid(const uint32_t* offsets,
 template <int W>
 __global__ void __launch_bounds__(256) k_pm_update(const PmRecord<W>* pm, const double* grid, double* w, float* out,
                                                    size_t total, int samples, int grid_rows, int grid_cols) {
+  chain_begin();
   const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const size_t f = idx / samples;
@@ -2562,13 +2568,16 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
   for (uint32_t it = 0; it < iterations; ++it) {
     {
       LaunchScope scope("k_pm_grid", stream);
-      k_pm_grid<W><<<static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads + 1), kPmThreads, 0, stream>>>(
-          offsets, reinterpret_cast<const PmEntry<W>*>(ws + l.entries), order, bins, w, grid, lists, s.samples,
+      launch_chained(k_pm_grid<W>, dim3(static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads + 1)),
+                     dim3(kPmThreads), 0, stream,
+          offsets, reinterpret_cast<const PmEntry<W>*>(ws + l.entries), static_cast<const uint32_t*>(order),
+                     static_cast<const uint32_t*>(bins), static_cast<const double*>(w), grid, lists, s.samples,
           s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame);
     }
     LaunchScope scope("k_pm_update", stream);
-    k_pm_update<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
-        pm, grid, w, it + 1 == iterations ? d_dcf : nullptr, fm, s.samples, s.grid_rows, s.grid_cols);
+    launch_chained(k_pm_update<W>, dim3(static_cast<unsigned>((fm + 255) / 256)), dim3(256), 0, stream,
+                   static_cast<const PmRecord<W>*>(pm), static_cast<const double*>(grid), w,
+                   it + 1 == iterations ? d_dcf : nullptr, fm, s.samples, s.grid_rows, s.grid_cols);
   }
   return check_launch();
 }
