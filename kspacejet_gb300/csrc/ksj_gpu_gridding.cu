@@ -1032,16 +1032,27 @@ __device__ __forceinline__ uint32_t stage_entries(int w, float* slots, const uns
   return halves;
 }
 
+// A chunk's cells of one coil in registers: real and imaginary parts of columns 2 t
+// and 2 t + 1 as packed pairs, so that the staged weights are operands as they lie
+// (parts of one column as a pair would need every weight twice).
+struct ChunkCells {
+  float2 re[kChunk / 2], im[kChunk / 2];
+  __device__ __forceinline__ float2 cell(int t) const {
+    return t & 1 ? make_float2(re[t / 2].y, im[t / 2].y) : make_float2(re[t / 2].x, im[t / 2].x);
+  }
+};
+
 // Eight columns of the chunk: the staged weights of one entry on its sample.
 template <int kFirst>
-__device__ __forceinline__ void half_taps(float2 (&r)[kChunk], const float* slot, float2 y) {
+__device__ __forceinline__ void half_taps(ChunkCells& r, const float* slot, float2 y) {
   const float4 a = reinterpret_cast<const float4*>(slot)[kFirst / 4];
   const float4 b = reinterpret_cast<const float4*>(slot)[kFirst / 4 + 1];
-  const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const float2 w[4] = {{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}};
+  const float2 re = make_float2(y.x, y.x), im = make_float2(y.y, y.y);
 #pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    r[kFirst + t].x = fmaf(y.x, w[t], r[kFirst + t].x);
-    r[kFirst + t].y = fmaf(y.y, w[t], r[kFirst + t].y);
+  for (int t = 0; t < 4; ++t) {
+    r.re[kFirst / 2 + t] = __ffma2_rn(re, w[t], r.re[kFirst / 2 + t]);
+    r.im[kFirst / 2 + t] = __ffma2_rn(im, w[t], r.im[kFirst / 2 + t]);
   }
 }
 
@@ -1055,17 +1066,17 @@ __device__ __forceinline__ void half_taps(float2 (&r)[kChunk], const float* slot
 // bounded: on a timeout the lane's partial sums are dropped, it still counts
 // itself in (the later segments do not wait out the limit as well) and
 // KSJ_GPU_FLAG_WAIT_TIMEOUT is raised.
-__device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst, int stride, int width, int seg,
+__device__ __forceinline__ void put_chunk(const ChunkCells& r, float2* dst, int stride, int width, int seg,
                                           int lanes, int* counter, uint32_t* flags, uint32_t wait_limit,
                                           int wait_beyond) {
   if (counter == nullptr) {
     if (width == kChunk) {  // every chunk of the row but a partial last one
 #pragma unroll
-      for (int t = 0; t < kChunk; ++t) dst[t * stride] = r[t];
+      for (int t = 0; t < kChunk; ++t) dst[t * stride] = r.cell(t);
     } else {
 #pragma unroll
       for (int t = 0; t < kChunk; ++t)
-        if (t < width) dst[t * stride] = r[t];
+        if (t < width) dst[t * stride] = r.cell(t);
     }
     return;
   }
@@ -1087,7 +1098,7 @@ __device__ __forceinline__ void put_chunk(const float2 (&r)[kChunk], float2* dst
 #pragma unroll
     for (int t = 0; t < kChunk; ++t) {
       if (t < width) {
-        float2 v = r[t];
+        float2 v = r.cell(t);
         if (seg > 0) {
           const float2 c = dst[t * stride];
           v = make_float2(c.x + v.x, c.y + v.y);
@@ -1239,9 +1250,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
       // (lanes past the channels read the first coil: their lines are not kept)
       const SampleRows<KSJ_GPU_SAMPLES_CF32> sample_row(
           samples, cgi * cg + coil < a.channels ? cgi * cg + coil : 0, a.channels);
-      float2 r[kChunk];
+      ChunkCells r;
 #pragma unroll
-      for (int t = 0; t < kChunk; ++t) r[t] = make_float2(0.0f, 0.0f);
+      for (int t = 0; t < kChunk / 2; ++t) r.re[t] = r.im[t] = make_float2(0.0f, 0.0f);
       const int most = __reduce_max_sync(0xffffffffu, cnt);
       for (int base = 0; base < most; base += kRowsBatch) {
         __syncwarp();  // the previous batch is read by every lane before it is replaced
@@ -1252,8 +1263,9 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
         float2 y[kRowsBatch];
 #pragma unroll
         for (int i = 0; i < kRowsBatch; ++i) {
+          // (32 lanes: a slot past the list has no weights and is skipped as a whole)
           y[i] = make_float2(0.0f, 0.0f);
-          if (base + i < cnt)
+          if (kLgL == 5 || base + i < cnt)
             y[i] = sample_row(reinterpret_cast<const uint32_t*>(slots + i * kSlotFloats)[kChunk]);
         }
 #pragma unroll
