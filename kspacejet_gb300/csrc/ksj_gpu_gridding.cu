@@ -666,6 +666,94 @@ __global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* 
   totals[static_cast<size_t>(blockIdx.y) * lists + l] = run;
 }
 
+// [frame][channel][sample] -> [frame][sample][channel] complex64, each sample
+// times its weight and phase (dcf * exp(i * origin phase), in its record), in tiles of 32 samples x 32
+// channels, checking every sample on the way: a
+// non-finite value (either component; bf16 exponent all ones) raises
+// KSJ_GPU_FLAG_NONFINITE_SAMPLE.  The product is formed here, once, and not by
+// each of the W rows (W^2 in 3-D) that read the sample.
+//
+// Ragged batches (frame_channels / frame_samples / frame_src non-null):
+// frame f holds frame_channels[f] coils of frame_samples[f] samples, packed
+// [channel][sample] at address frame_src[f] (device memory, or host memory
+// the device reads in place); the padding up to the call's channels and
+// samples is written as zeros.
+struct CoilLastArgs {
+  const void* in;
+  float2* out;
+  const unsigned char* scales;  // the records' scale fields, `scale_stride` bytes apart
+  int scale_stride;
+  int channels, samples;
+  uint32_t* flags;
+  const uint32_t* frame_channels;
+  const uint32_t* frame_samples;
+  const uint64_t* frame_src;
+  int frame0;
+  uint32_t* frame_flags;
+};
+using CoilLastTile = float2[32][33];
+
+// One tile by 256 consecutive threads (tx, ty) of a block, (tx, 0 .. 7); every thread
+// of the block takes part, with tiles of the same frame.
+template <uint32_t kFormat>
+__device__ __forceinline__ void coil_last_tile(const CoilLastArgs& a, int f, int s0, int c0, CoilLastTile& t, int tx,
+                                               int ty) {
+  using T = typename std::conditional<kFormat == KSJ_GPU_SAMPLES_BF16, uint32_t, unsigned long long>::type;
+  const int channels = a.channels, samples = a.samples;
+  float2* dst = a.out + static_cast<size_t>(f) * channels * samples;
+  const int live_c = a.frame_channels ? min(channels, static_cast<int>(__ldg(a.frame_channels + f))) : channels;
+  const int live_s = a.frame_samples ? min(samples, static_cast<int>(__ldg(a.frame_samples + f))) : samples;
+  // ragged frames are packed at their own sample count
+  const T* src = a.frame_src ? reinterpret_cast<const T*>(__ldg(a.frame_src + f))
+                             : static_cast<const T*>(a.in) + static_cast<size_t>(f) * channels * samples;
+  const int pitch = a.frame_src ? live_s : samples;
+  const int sm = s0 + tx;
+  float2 scale = make_float2(0.0f, 0.0f);
+  if (sm < live_s)
+    scale = __ldg(reinterpret_cast<const float2*>(
+        a.scales + (static_cast<size_t>(f) * samples + sm) * static_cast<size_t>(a.scale_stride)));
+  bool bad = false;
+#pragma unroll
+  for (int y = ty; y < 32; y += 8) {
+    const int c = c0 + y;
+    if (c < channels && sm < samples) {
+      if (c >= live_c || sm >= live_s) {
+        t[y][tx] = make_float2(0.0f, 0.0f);
+        continue;
+      }
+      const T v = __ldg(src + static_cast<size_t>(c) * pitch + sm);
+      float2 x;
+      if constexpr (kFormat == KSJ_GPU_SAMPLES_BF16) {
+        bad |= (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u;
+        x = make_float2(bf16_to_float(static_cast<uint16_t>(v & 0xffffu)), bf16_to_float(static_cast<uint16_t>(v >> 16)));
+      } else {
+        bad |= (v & 0x7f800000ull) == 0x7f800000ull || (v & 0x7f80000000000000ull) == 0x7f80000000000000ull;
+        x = make_float2(__uint_as_float(static_cast<uint32_t>(v)), __uint_as_float(static_cast<uint32_t>(v >> 32)));
+      }
+      t[y][tx] = cmul(x, scale);
+    }
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0 && threadIdx.y == 0) {
+    atomicOr(a.flags, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
+    if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
+  }
+#pragma unroll
+  for (int y = ty; y < 32; y += 8) {
+    const int so = s0 + y, c = c0 + tx;
+    if (c < channels && so < samples) dst[static_cast<size_t>(so) * channels + c] = t[tx][y];
+  }
+}
+
+// The tiles as a launch of their own ((32, 8) threads, grid (ceil(samples/32),
+// ceil(channels/32), frames)): calls of more samples than the scan's launch takes, 3-D, and
+// passes whose samples arrive one by one.
+template <uint32_t kFormat>
+__global__ void __launch_bounds__(256) k_samples_coil_last(CoilLastArgs a) {
+  __shared__ CoilLastTile t;
+  chain_wait();  // (row-pass blocks waiting beside these would hold shared memory their cache uses)
+  coil_last_tile<kFormat>(a, a.frame0 + blockIdx.z, blockIdx.x * 32, blockIdx.y * 32, t, threadIdx.x, threadIdx.y);
+}
+
 // Exclusive scan of one frame's list lengths, one block per frame.  Bound by latency (one block
 // for a single frame), so a warp holds its whole stretch of counts in registers,
 // 32 consecutive ones per load, all loads in flight at once (per-thread
@@ -674,13 +762,42 @@ __global__ void __launch_bounds__(128) k_bin_prefix(uint32_t* counts, uint32_t* 
 // Blocks from `frames` on fill the call's tables meanwhile, 64 entries each: their FP64
 // functions run at a few lanes per clock and SM, so they are spread over many
 // (a kernel of their own on one or two SMs took 7 to 20 us).
+// The blocks after those bring the samples themselves into the row pass's order
+// (coil_last_tile), which needs the records alone, where the launch fits the SMs in
+// one round (kScanSampleBlocks): a frame's scan leaves the others idle.  One frame of 13056
+// samples x 32 coils 64.1 -> 60.1 us a call.  Beyond that they are a launch of their
+// own with small blocks (512 blocks here: 30 us against 9 + 16; 96 frames 317 against 10 + 153).
 constexpr int kScanPer = kMaxGrid * (kMaxGrid / kChunk) / 1024;  // counts per thread, at most
 constexpr int kTablesPerBlock = 64;
+constexpr int kCoilLastTiles = 1024 / 256;  // tiles of a block, of consecutive samples
+constexpr int kScanSampleBlocks = 144;      // with a few for the tables, one round of the SMs
+struct ScanSamples {
+  CoilLastArgs a;
+  int first_block;  // of the launch
+  int bf16, none;
+};
 
 __global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t* offsets, int lists,
                                                int frames,
-                                               const __grid_constant__ TablesArgs tables) {
-  chain_begin();
+                                               const __grid_constant__ TablesArgs tables,
+                                               const __grid_constant__ ScanSamples samples) {
+  __shared__ CoilLastTile tiles[kCoilLastTiles];
+  chain_wait();
+  // (blocks of the next launch would take the places of those that move samples)
+  if (samples.none) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (static_cast<int>(blockIdx.x) >= samples.first_block) {
+    const int per_block = 32 * kCoilLastTiles;
+    const int blocks = (samples.a.samples + per_block - 1) / per_block, groups = (samples.a.channels + 31) / 32;
+    const int i = blockIdx.x - samples.first_block, frame = i / (blocks * groups);
+    const int j = i - frame * blocks * groups, group = j / blocks, tile = threadIdx.x / 256;
+    const int s0 = (j - group * blocks) * per_block + tile * 32;
+    const int tx = threadIdx.x & 31, ty = (threadIdx.x >> 5) & 7;
+    if (samples.bf16)
+      coil_last_tile<KSJ_GPU_SAMPLES_BF16>(samples.a, frame, s0, group * 32, tiles[tile], tx, ty);
+    else
+      coil_last_tile<KSJ_GPU_SAMPLES_CF32>(samples.a, frame, s0, group * 32, tiles[tile], tx, ty);
+    return;
+  }
   if (static_cast<int>(blockIdx.x) >= frames) {
     const int i = (blockIdx.x - frames) * kTablesPerBlock + threadIdx.x;
     if (threadIdx.x < kTablesPerBlock && i < table_entries(tables)) table_entry(tables, i);
@@ -728,12 +845,30 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t* counts, uint32_t*
   if (threadIdx.x == 0) o[lists] = warp_sums[31];
 }
 
-// The scan of `frames` frames, with the tables where they are wanted.
+// Blocks that move the samples of `frames` frames in the scan's launch.
+inline size_t scan_sample_blocks(int samples, int channels, int frames) {
+  return static_cast<size_t>((samples + 32 * kCoilLastTiles - 1) / (32 * kCoilLastTiles)) * ((channels + 31) / 32) *
+         frames;
+}
+
+// The scan of `frames` frames, with the tables and the move of the samples where they are
+// wanted.
 ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, int lists, int frames,
-                           const TablesArgs* tables, cudaStream_t stream) {
+                           const TablesArgs* tables, cudaStream_t stream, const CoilLastArgs* coil_last = nullptr,
+                           bool bf16 = false) {
   const int extra = tables ? (table_entries(*tables) + kTablesPerBlock - 1) / kTablesPerBlock : 0;
   LaunchScope scope("k_scan", stream);
-  launch_chained(k_scan, frames + extra, 1024, 0, stream, counts, offsets, lists, frames, tables ? *tables : TablesArgs{});
+  ScanSamples samples{};
+  samples.first_block = frames + extra;
+  samples.none = coil_last == nullptr;
+  size_t total = samples.first_block;
+  if (coil_last != nullptr) {
+    samples.a = *coil_last;
+    samples.bf16 = bf16;
+    total += scan_sample_blocks(coil_last->samples, coil_last->channels, frames);
+  }
+  launch_chained(k_scan, dim3(static_cast<unsigned>(total)), 1024, 0, stream, counts, offsets, lists, frames,
+                 tables ? *tables : TablesArgs{}, samples);
   return KSJ_GPU_OK;
 }
 
@@ -852,86 +987,6 @@ __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
         }
       }
     }
-  }
-}
-
-// [frame][channel][sample] -> [frame][sample][channel] complex64, each sample
-// times its weight and phase (dcf * exp(i * origin phase), in its record), through
-// a 32x33 shared tile (launch (32, 8) threads, grid (ceil(samples/32),
-// ceil(channels/32), frames)), checking every sample on the way: a
-// non-finite value (either component; bf16 exponent all ones) raises
-// KSJ_GPU_FLAG_NONFINITE_SAMPLE.  The product is formed here, once, and not by
-// each of the W rows (W^2 in 3-D) that read the sample.
-//
-// Ragged batches (frame_channels / frame_samples / frame_src non-null):
-// frame f holds frame_channels[f] coils of frame_samples[f] samples, packed
-// [channel][sample] at address frame_src[f] (device memory, or host memory
-// the device reads in place); the padding up to the call's channels and
-// samples is written as zeros.
-struct CoilLastArgs {
-  const void* in;
-  float2* out;
-  const unsigned char* scales;  // the records' scale fields, `scale_stride` bytes apart
-  int scale_stride;
-  int channels, samples;
-  uint32_t* flags;
-  const uint32_t* frame_channels;
-  const uint32_t* frame_samples;
-  const uint64_t* frame_src;
-  int frame0;
-  uint32_t* frame_flags;
-};
-
-template <uint32_t kFormat>
-__global__ void __launch_bounds__(256) k_samples_coil_last(CoilLastArgs a) {
-  using T = typename std::conditional<kFormat == KSJ_GPU_SAMPLES_BF16, uint32_t, unsigned long long>::type;
-  __shared__ float2 t[32][33];
-  chain_wait();  // (row-pass blocks waiting beside these would hold shared memory their cache uses)
-  const int channels = a.channels, samples = a.samples;
-  const int f = a.frame0 + blockIdx.z;
-  const int s0 = blockIdx.x * 32;
-  const int c0 = blockIdx.y * 32;
-  float2* dst = a.out + static_cast<size_t>(f) * channels * samples;
-  const int live_c = a.frame_channels ? min(channels, static_cast<int>(__ldg(a.frame_channels + f))) : channels;
-  const int live_s = a.frame_samples ? min(samples, static_cast<int>(__ldg(a.frame_samples + f))) : samples;
-  // ragged frames are packed at their own sample count
-  const T* src = a.frame_src ? reinterpret_cast<const T*>(__ldg(a.frame_src + f))
-                             : static_cast<const T*>(a.in) + static_cast<size_t>(f) * channels * samples;
-  const int pitch = a.frame_src ? live_s : samples;
-  const int sm = s0 + threadIdx.x;
-  float2 scale = make_float2(0.0f, 0.0f);
-  if (sm < live_s)
-    scale = __ldg(reinterpret_cast<const float2*>(
-        a.scales + (static_cast<size_t>(f) * samples + sm) * static_cast<size_t>(a.scale_stride)));
-  bool bad = false;
-#pragma unroll
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int c = c0 + y;
-    if (c < channels && sm < samples) {
-      if (c >= live_c || sm >= live_s) {
-        t[y][threadIdx.x] = make_float2(0.0f, 0.0f);
-        continue;
-      }
-      const T v = __ldg(src + static_cast<size_t>(c) * pitch + sm);
-      float2 x;
-      if constexpr (kFormat == KSJ_GPU_SAMPLES_BF16) {
-        bad |= (v & 0x7f80u) == 0x7f80u || (v & 0x7f800000u) == 0x7f800000u;
-        x = make_float2(bf16_to_float(static_cast<uint16_t>(v & 0xffffu)), bf16_to_float(static_cast<uint16_t>(v >> 16)));
-      } else {
-        bad |= (v & 0x7f800000ull) == 0x7f800000ull || (v & 0x7f80000000000000ull) == 0x7f80000000000000ull;
-        x = make_float2(__uint_as_float(static_cast<uint32_t>(v)), __uint_as_float(static_cast<uint32_t>(v >> 32)));
-      }
-      t[y][threadIdx.x] = cmul(x, scale);
-    }
-  }
-  if (__syncthreads_or(bad) && threadIdx.x == 0 && threadIdx.y == 0) {
-    atomicOr(a.flags, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
-    if (a.frame_flags) atomicOr(a.frame_flags + f, KSJ_GPU_FLAG_NONFINITE_SAMPLE);
-  }
-#pragma unroll
-  for (int y = threadIdx.y; y < 32; y += 8) {
-    const int so = s0 + y, c = c0 + threadIdx.x;
-    if (c < channels && so < samples) dst[static_cast<size_t>(so) * channels + c] = t[threadIdx.x][y];
   }
 }
 
@@ -1885,12 +1940,14 @@ struct ColsPass {
 // The binning lists of one call: per-sample records, list offsets, and the lists'
 // entries in sample order, as the row pass reads them or, where `pm` holds the
 // density weights' records, as their grid step does; and the call's tables where
-// `tables` names them.  The flags must already be cleared.
+// `tables` names them, and the samples in the row pass's order where `coil_last` does.  The
+// flags must already be cleared.
 template <int W>
 ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const float* d_traj, const float* d_dcf,
                            uint32_t* flags, unsigned char* records, uint32_t* counts, uint32_t* totals,
                            uint32_t* offsets, unsigned char* expanded, const void* pm, cudaStream_t stream,
-                           uint32_t* frame_flags = nullptr, const TablesArgs* tables = nullptr) {
+                           uint32_t* frame_flags = nullptr, const TablesArgs* tables = nullptr,
+                           const CoilLastArgs* coil_last = nullptr) {
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
   const auto place = pm ? k_place<W, true> : k_place<W, false>;
@@ -1932,7 +1989,8 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream, counts, totals,
                    s.bin_blocks, s.lists_per_frame);
   }
-  launch_scan(totals, offsets, s.lists_per_frame, s.frames, tables, stream);
+  launch_scan(totals, offsets, s.lists_per_frame, s.frames, tables, stream, coil_last,
+              d->sample_format == KSJ_GPU_SAMPLES_BF16);
   {
     PlaceArgs p{};
     p.records = records;
@@ -1989,22 +2047,26 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   const TablesArgs tables{tw_rows, tw_cols, inv_dr, inv_dc, pos_rows, pos_cols, s.grid_rows, s.grid_cols, s.out_rows,
                           s.out_cols, s.plan_rows, s.plan_cols, s.kb ? 1 : 0, s.width, beta,
                           s.kb ? std::cyl_bessel_i(0.0, beta) : 1.0};
+  CoilLastArgs coil_last{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t), records + offsetof(SampleRecord<W>, scale),
+                         static_cast<int>(sizeof(SampleRecord<W>)), s.channels, s.samples, flags, s.frame_channels,
+                         s.frame_samples, s.frame_kspace, 0, reinterpret_cast<uint32_t*>(ws + l.frame_flags)};
+  const bool samples_here = io == nullptr || io->copy == nullptr;  // (else pass by pass)
+  const bool with_scan =
+      samples_here && s.frames + scan_sample_blocks(s.samples, s.channels, s.frames) <= kScanSampleBlocks;
   {
     const ksj_gpu_status st =
         build_lists<W>(s, d, d_traj, d_dcf, flags, records, reinterpret_cast<uint32_t*>(ws + l.counts),
                        reinterpret_cast<uint32_t*>(ws + l.totals), offsets, ws + l.expanded, nullptr, stream,
-                       reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables);
+                       reinterpret_cast<uint32_t*>(ws + l.frame_flags), &tables, with_scan ? &coil_last : nullptr);
     if (st != KSJ_GPU_OK) return st;
   }
   auto to_coil_last = [&](int f0, int nf, cudaStream_t st) {
     const dim3 tg((s.samples + 31) / 32, (s.channels + 31) / 32, nf);
     LaunchScope scope("k_samples_coil_last", st);
-    const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t), records + offsetof(SampleRecord<W>, scale),
-                         static_cast<int>(sizeof(SampleRecord<W>)), s.channels, s.samples, flags, s.frame_channels,
-                         s.frame_samples, s.frame_kspace, f0, reinterpret_cast<uint32_t*>(ws + l.frame_flags)};
-    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, st, a);
+    coil_last.frame0 = f0;
+    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, st, coil_last);
   };
-  if (io == nullptr || io->copy == nullptr) to_coil_last(0, s.frames, stream);
+  if (samples_here && !with_scan) to_coil_last(0, s.frames, stream);
   RowsArgs r{};
   r.samples_t = reinterpret_cast<const float2*>(ws + l.samples_t);
   r.sample_frame_stride = static_cast<size_t>(s.samples) * s.channels;
