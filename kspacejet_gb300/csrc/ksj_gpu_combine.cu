@@ -120,6 +120,7 @@ __device__ __forceinline__ void normalise(float2* v) {
 template <int C>
 __global__ void __launch_bounds__(kWalshThreads) k_walsh(const float2* __restrict__ in, float2* out, int rows, int cols,
                                                          int half, int iterations) {
+  chain_begin();
   extern __shared__ float2 walsh_smem[];
   const int span = kWalshCols + 2 * half, tall = kWalshRows + 2 * half;
   float2* tile = walsh_smem;                                        // [coil][tall][span]
@@ -275,10 +276,9 @@ ksj_gpu_status launch_walsh(uint32_t rows, uint32_t cols, int half, uint32_t ite
     return KSJ_GPU_ERROR_CUDA;
   const unsigned grid = ((cols + kWalshCols - 1) / kWalshCols) * ((rows + kWalshRows - 1) / kWalshRows);
   LaunchScope scope("k_walsh", stream);
-  k_walsh<C><<<grid, kWalshThreads, smem, stream>>>(static_cast<const float2*>(in),
-                                                              static_cast<float2*>(out), static_cast<int>(rows),
-                                                              static_cast<int>(cols), half,
-                                                              static_cast<int>(iterations));
+  launch_chained(k_walsh<C>, dim3(grid), dim3(kWalshThreads), smem, stream, static_cast<const float2*>(in),
+                 static_cast<float2*>(out), static_cast<int>(rows), static_cast<int>(cols), half,
+                 static_cast<int>(iterations));
   return check_launch();
 }
 
@@ -441,6 +441,7 @@ __device__ __forceinline__ void cov_store(unsigned char* stage, const float2 (&v
 // Bound by reading X once: 412160 samples x 32 coils (105 MB) in 27 us; splitting into a
 // bf16 operand in memory first (another 105 MB written and read) took 58.
 __global__ void __launch_bounds__(kCovThreads, 2) k_cov_mma(CovArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char cov_smem[];
   // stage buffers on a 1024-byte boundary (128-byte swizzle atoms)
   unsigned char* base = cov_smem + ((1024u - (smem_addr(cov_smem) & 1023u)) & 1023u);
@@ -548,6 +549,7 @@ __global__ void __launch_bounds__(kCovSumElems * kCovSumSlices) k_cov_form(const
                                                                            float inv_m,
                                                                            const float2* __restrict__ means,
                                                                            float2* cov) {
+  chain_begin();
   __shared__ float part[kCovSumSlices][kCovSumElems];
   __shared__ bool last;
   const int el = threadIdx.x % kCovSumElems, slice = threadIdx.x / kCovSumElems;
@@ -673,7 +675,7 @@ ksj_gpu_status covariance_run(uint32_t channels, uint32_t samples, const void* d
     const CovArgs args{static_cast<const float2*>(d_kspace), partials, flags, static_cast<int>(channels),
                        static_cast<int>(samples), l.ktiles};
     LaunchScope scope("k_cov_mma", cs);
-    k_cov_mma<<<l.blocks, kCovThreads, smem, cs>>>(args);
+    launch_chained(k_cov_mma, dim3(l.blocks), dim3(kCovThreads), smem, cs, args);
   }
   float2* means = nullptr;
   if (noise) {
@@ -682,9 +684,9 @@ ksj_gpu_status covariance_run(uint32_t channels, uint32_t samples, const void* d
     k_channel_means<<<channels, 256, 0, cs>>>(static_cast<const float2*>(d_kspace), static_cast<int>(samples), means);
   }
   LaunchScope scope("k_cov_form", cs);
-  k_cov_form<<<kCovRows * 64 / kCovSumElems, kCovSumElems * kCovSumSlices, 0, cs>>>(
-      partials, l.blocks, reinterpret_cast<float*>(ws + l.sum), flags + 1, static_cast<int>(channels),
-      1.0f / static_cast<float>(samples), means, static_cast<float2*>(d_cov));
+  launch_chained(k_cov_form, dim3(kCovRows * 64 / kCovSumElems), dim3(kCovSumElems * kCovSumSlices), 0, cs, partials,
+                 l.blocks, reinterpret_cast<float*>(ws + l.sum), flags + 1, static_cast<int>(channels),
+                 1.0f / static_cast<float>(samples), means, static_cast<float2*>(d_cov));
   return check_launch();
 }
 
@@ -725,6 +727,7 @@ template <int kV, int kS>
 __global__ void __launch_bounds__(compress_threads(kV)) k_coil_compress(const float2* __restrict__ basis,
                                                                         const float2* __restrict__ x, float2* y,
                                                                         int channels, int samples) {
+  chain_begin();
   constexpr int kP = (kV + 1) / 2;  // pairs of outputs
   __shared__ float4 b[32 * kP];
   for (int i = threadIdx.x; i < 32 * kP * 2; i += blockDim.x) {
@@ -792,7 +795,7 @@ ksj_gpu_status launch_compress(uint32_t channels, uint32_t samples, const void* 
   const auto kernel = pairs ? k_coil_compress<kV, 2> : k_coil_compress<kV, 1>;
   const uint32_t per_block = compress_threads(kV) * (pairs ? 2 : 1);
   LaunchScope scope("k_coil_compress", stream);
-  kernel<<<(samples + per_block - 1) / per_block, compress_threads(kV), 0, stream>>>(
+  launch_chained(kernel, dim3((samples + per_block - 1) / per_block), dim3(compress_threads(kV)), 0, stream,
       static_cast<const float2*>(basis), static_cast<const float2*>(x), static_cast<float2*>(y),
       static_cast<int>(channels), static_cast<int>(samples));
   return check_launch();

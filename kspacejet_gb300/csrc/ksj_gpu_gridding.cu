@@ -3673,6 +3673,7 @@ __device__ __forceinline__ void dft_direct_lines(const float2* x, int lg, int n,
 // axis's transform (two-step slot or digit-reversed position).
 __global__ void k_cart_tables(float2* tw_rows, int rows, float2* tw_cols, int cols, float* inv_dr, float* inv_dc,
                               int* pos_rows, int* pos_cols, DifPlan plan_rows, DifPlan plan_cols) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < rows) {
     tw_rows[i] = twiddle(i, rows);
@@ -3700,6 +3701,7 @@ __global__ void __launch_bounds__(kCartThreads) k_cart_rows(const float2* __rest
                                                             const float2* __restrict__ tw_cols,
                                                             const int* __restrict__ pos_cols, DifPlan plan, int rows,
                                                             int cols, int channels, int cg, int cpitch) {
+  chain_begin();
   extern __shared__ __align__(16) float2 cart_smem[];
   float2* acc = cart_smem;
   float2* tw = cart_smem + static_cast<size_t>(cols) * (kN > 0 ? cg + 1 : cg);
@@ -4312,9 +4314,8 @@ extern "C" ksj_gpu_status ksj_gpu_cartesian_ifft2(uint32_t rows, uint32_t cols, 
   {
     const int n = static_cast<int>(std::max(rows, cols));
     LaunchScope scope("k_cart_tables", cstream);
-    k_cart_tables<<<(n + 255) / 256, 256, 0, cstream>>>(tw_rows, static_cast<int>(rows), tw_cols,
-                                                       static_cast<int>(cols), inv_dr, inv_dc, pos_rows, pos_cols,
-                                                       s.plan_rows, s.plan_cols);
+    launch_chained(k_cart_tables, dim3((n + 255) / 256), dim3(256), 0, cstream, tw_rows, static_cast<int>(rows), tw_cols,
+                   static_cast<int>(cols), inv_dr, inv_dc, pos_rows, pos_cols, s.plan_rows, s.plan_cols);
   }
   {
     const CartRowsKernel rk = cart_rows_for(static_cast<int>(cols));
@@ -4323,8 +4324,9 @@ extern "C" ksj_gpu_status ksj_gpu_cartesian_ifft2(uint32_t rows, uint32_t cols, 
       return KSJ_GPU_ERROR_CUDA;
     const dim3 grid(rows, (channels + cs.cg - 1) / cs.cg, frames);
     LaunchScope scope("k_cart_rows", cstream);
-    rk<<<grid, kCartThreads, smem, cstream>>>(static_cast<const float2*>(d_kspace), inter, tw_cols, pos_cols, s.plan_cols, static_cast<int>(rows),
-                                             static_cast<int>(cols), static_cast<int>(channels), cs.cg, s.cpitch);
+    launch_chained(rk, grid, dim3(kCartThreads), smem, cstream, static_cast<const float2*>(d_kspace), inter, tw_cols,
+                   pos_cols, s.plan_cols, static_cast<int>(rows), static_cast<int>(cols), static_cast<int>(channels),
+                   cs.cg, s.cpitch);
   }
   if (!is_fft_size(rows)) {
     // direct DFT along the columns, coil-last into the output (or into the
