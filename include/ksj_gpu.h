@@ -111,7 +111,7 @@ typedef struct ksj_gpu_gridding_tuning {
   uint32_t list_capacity;   /* accepted (a power of two, 64..2048) and not used: the lists are built in order */
   uint32_t frames_per_pass; /* frames per row/column pass; passes alternate between two streams (0: two passes
                                 once there are 4 or more frames) */
-  uint32_t rows_blocks_per_sm; /* 1 or 2 resident row CTAs per SM (2 caps registers at 80 per thread) */
+  uint32_t rows_blocks_per_sm; /* accepted (0 to 2) and not used: two row CTAs are resident per SM */
   uint32_t coil_parts;      /* 1 or 2: a row CTA's coil group is split into this many independent list tasks */
   uint32_t column_pass;     /* 0 heuristic, 1 one CTA per (frame, column block), 2 persistent CTAs with a
                                 two-stage TMA ring of 16-line tiles (two-step column lengths only) */

@@ -4147,7 +4147,6 @@ extern "C" ksj_gpu_status ksj_gpu_gridding_tune(const ksj_gpu_gridding_desc* des
     if (cg * 4 < desc->channels && cg < 8) continue;
     for (uint32_t cbm : {1u, 2u})
     for (uint32_t fpp : {0u, 12u, 48u})
-    for (uint32_t rb : {1u, 2u})
     for (uint32_t colp : {1u, 2u})
     for (uint32_t parts : {1u, 2u}) {
       if (fpp >= desc->frames) continue;
@@ -4159,7 +4158,7 @@ extern "C" ksj_gpu_status ksj_gpu_gridding_tune(const ksj_gpu_gridding_desc* des
       t.coil_group = cg;
       t.column_block = cbm * std::max(1u, 32u / gcols);
       t.frames_per_pass = fpp;
-      t.rows_blocks_per_sm = rb;
+      t.rows_blocks_per_sm = 2;
       t.coil_parts = parts;
       t.column_pass = colp;
       Shape s{};
