@@ -370,12 +370,12 @@ def kernel_bytes(g, entries: int) -> dict:
     F, C, M = g.frames, g.channels, g.samples
     N, G = IMAGE, GRID
     rec = 16 + 8 * WIDTH                      # per-sample record written by k_prepare
-    expanded = 16 * (1 + (WIDTH + 3) // 4)    # per list entry as the row pass reads it
+    entry = 8 + 4 * WIDTH                     # per list entry as the row pass reads it
     inter = F * C * G * N * 8                 # row-transformed grid, kept columns only
     return {
-        "k_rows": F * M * C * 8 + entries * expanded + inter,
+        "k_rows": F * M * C * 8 + entries * entry + inter,
         "k_cols": inter + F * N * N * 4,
-        "k_sort": entries * (4 + 4 + expanded) + F * M * rec,
+        "k_place": entries * entry + F * M * rec,
         "k_samples_coil_last": 2 * F * C * M * 8,
         "k_prepare": F * M * 8 + F * M * rec,
     }
