@@ -2610,13 +2610,22 @@ PmLayout make_pm_layout(const Shape& s) {
   return l;
 }
 
+// Frames of one pass: as many as keep the entries (48 bytes for a width of 4, up to
+// 2 W of them a sample) within 4 GB, and at least one.  Frames are independent, so a
+// call of more takes them in passes through one workspace.
+uint32_t pm_pass_frames(const Shape& s) {
+  const size_t frame = s.entries_per_frame * (16 + 8 * static_cast<size_t>(s.width));
+  return static_cast<uint32_t>(
+      std::min<size_t>(s.frames, std::max<size_t>(1, (size_t{4} << 30) / std::max<size_t>(frame, 1))));
+}
+
+// The flags must already be cleared.
 template <int W>
 ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gpu_gridding_desc* d,
                                  uint32_t iterations, const float* d_traj, float* d_dcf, unsigned char* ws,
                                  cudaStream_t stream) {
   static_assert(sizeof(PmRecord<W>) == 8 + 16 * W, "PmRecord layout");
   uint32_t* flags = reinterpret_cast<uint32_t*>(ws + l.flags);
-  if (cudaMemsetAsync(flags, 0, kFlagBytes, stream) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
   ksj_gpu_gridding_desc dd = *d;
   dd.dcf_mode = KSJ_GPU_DCF_NONE;
   static_assert(sizeof(PmEntry<W>) == 16 + 8 * W, "PmEntry layout");
@@ -4195,7 +4204,9 @@ extern "C" size_t ksj_gpu_pipe_menon_workspace_bytes(const ksj_gpu_gridding_desc
   Shape s{};
   if (desc == nullptr || desc->kernel != KSJ_GPU_KERNEL_KAISER_BESSEL || make_shape(desc, nullptr, &s) != KSJ_GPU_OK)
     return 0;
-  return make_pm_layout(s).total;
+  ksj_gpu_gridding_desc pass = *desc;
+  pass.frames = pm_pass_frames(s);
+  return make_shape(&pass, nullptr, &s) == KSJ_GPU_OK ? make_pm_layout(s).total : 0;
 }
 
 extern "C" ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* desc, uint32_t iterations,
@@ -4209,18 +4220,31 @@ extern "C" ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* de
   if (d_traj == nullptr || d_dcf == nullptr || (reinterpret_cast<uintptr_t>(d_traj) & 7u) != 0 ||
       (reinterpret_cast<uintptr_t>(d_dcf) & 3u) != 0)
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  const PmLayout l = make_pm_layout(s);
-  if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 || workspace_bytes < l.total)
+  const uint32_t per_pass = pm_pass_frames(s);
+  if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 ||
+      workspace_bytes < ksj_gpu_pipe_menon_workspace_bytes(desc))
     return KSJ_GPU_ERROR_WORKSPACE;
   unsigned char* ws = static_cast<unsigned char*>(d_workspace);
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  switch (s.width) {
-    case 2: return launch_pipe_menon<2>(s, l, desc, iterations, d_traj, d_dcf, ws, cs);
-    case 4: return launch_pipe_menon<4>(s, l, desc, iterations, d_traj, d_dcf, ws, cs);
-    case 6: return launch_pipe_menon<6>(s, l, desc, iterations, d_traj, d_dcf, ws, cs);
-    case 8: return launch_pipe_menon<8>(s, l, desc, iterations, d_traj, d_dcf, ws, cs);
-    default: return KSJ_GPU_ERROR_UNSUPPORTED;
+  if (cudaMemsetAsync(ws, 0, kFlagBytes, cs) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
+  for (uint32_t f0 = 0; f0 < desc->frames; f0 += per_pass) {
+    ksj_gpu_gridding_desc pass = *desc;
+    pass.frames = std::min(per_pass, desc->frames - f0);
+    const ksj_gpu_status ps = make_shape(&pass, nullptr, &s);
+    if (ps != KSJ_GPU_OK) return ps;
+    const PmLayout l = make_pm_layout(s);
+    const float* traj = d_traj + static_cast<size_t>(f0) * s.samples * 2;
+    float* dcf = d_dcf + static_cast<size_t>(f0) * s.samples;
+    ksj_gpu_status run = KSJ_GPU_ERROR_UNSUPPORTED;
+    switch (s.width) {
+      case 2: run = launch_pipe_menon<2>(s, l, &pass, iterations, traj, dcf, ws, cs); break;
+      case 4: run = launch_pipe_menon<4>(s, l, &pass, iterations, traj, dcf, ws, cs); break;
+      case 6: run = launch_pipe_menon<6>(s, l, &pass, iterations, traj, dcf, ws, cs); break;
+      case 8: run = launch_pipe_menon<8>(s, l, &pass, iterations, traj, dcf, ws, cs); break;
+    }
+    if (run != KSJ_GPU_OK) return run;
   }
+  return KSJ_GPU_OK;
 }
 
 extern "C" size_t ksj_gpu_gridding3_workspace_bytes(const ksj_gpu_gridding3_desc* desc) {

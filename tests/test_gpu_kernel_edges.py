@@ -180,6 +180,18 @@ def test_density_weights_of_every_width(native, cuda, orc, image, grid, width, s
         assert oracle.rel_l2(got[f].astype(np.float64), want) <= 1e-7
 
 
+def test_density_weights_in_passes_of_frames(native, cuda):
+    """Two frames whose entries (2 M samples x 16 x 80 bytes each) exceed one pass together."""
+    from kspacejet_gb300 import gpu
+
+    torch = _torch()
+    rng = np.random.default_rng(5)
+    tr = torch.from_numpy(rng.uniform(-np.pi, np.pi, size=(2, 2_000_000, 2)).astype(np.float32)).to(cuda)
+    both = gpu.pipe_menon_dcf(tr, 128, 256, width=8, iterations=2)
+    for f in range(2):
+        assert torch.equal(both[f], gpu.pipe_menon_dcf(tr[f].contiguous(), 128, 256, width=8, iterations=2))
+
+
 @pytest.mark.parametrize("width,beta", [(2, 27.0), (2, 31.0), (4, 12.5), (4, 60.0), (8, 39.0), (8, 120.0)])
 def test_density_weights_of_a_given_beta(native, cuda, orc, width, beta):
     """Both sides of what the tap polynomials resolve (the rest takes the Bessel function)."""
