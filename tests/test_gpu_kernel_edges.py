@@ -164,6 +164,30 @@ def test_samples_moved_beside_the_scan_and_alone(native, cuda, samples, channels
     assert outs[0].tobytes() == outs[1].tobytes()
 
 
+@pytest.mark.parametrize("image,grid,coils", [(12, 24, 20), (2, 12, 11), (16, 24, 24), (10, 20, 40), (10, 20, 17)])
+def test_3d_coils_in_parts(native, cuda, orc, image, grid, coils):
+    """Coil counts whose columns are transformed in parts of 4 or 8 coils, and one that is not."""
+    from kspacejet_gb300 import gpu
+
+    torch = _torch()
+    samples = 600
+    tr = _scattered(samples, 1, 3, seed=coils)[0]
+    k = _complex(np.random.default_rng(coils), coils, samples)
+    outs = {}
+    for output in (gpu.OUTPUT_COIL_LAST, gpu.OUTPUT_RSS):
+        g = gpu.Gridding3(image=image, grid=grid, channels=coils, samples=samples, width=4, output=output,
+                          dcf=gpu.DCF_NONE)
+        ws = g.new_workspace(cuda).fill_(255)  # coils past the last one start as NaN
+        outs[output] = g.new_output(cuda)
+        g.run(torch.from_numpy(k).to(cuda), torch.from_numpy(tr).to(cuda), outs[output], ws)
+    images = outs[gpu.OUTPUT_COIL_LAST].cpu().numpy().reshape(image, image, image, coils)
+    for c in range(0, coils, 3):
+        ref = orc.kb_gridding3(grid, image, k[c].astype(np.complex128), tr.astype(np.float64), np.ones(samples), width=4)
+        assert oracle.rel_l2(images[..., c], ref) <= TOL
+    rss = np.sqrt((np.abs(images.astype(np.complex128)) ** 2).sum(-1))
+    assert oracle.rel_l2(outs[gpu.OUTPUT_RSS].cpu().numpy().reshape(rss.shape), rss) <= 4 * coils * EPS
+
+
 # -------------------------------------------------------- density weights
 
 
