@@ -127,6 +127,12 @@ constexpr uint32_t kWaitLimit = 1u << 22;  // polls before a bounded wait gives 
 constexpr int kBinThreads = 512;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr size_t kPlaceListBytes = 4;  // of k_place: the list's running position
+constexpr int kSms = 152;              // of a GB300
+// A call keeps one count per list for each of its blocks: at most this many (64 MB), or one
+// block a frame where that is more.
+constexpr size_t kBinCounts = size_t{1} << 24;
+// 3-D: most blocks of the plane stage of the binning (four per SM)
+constexpr int kPlaneStageBlocks = 4 * kSms;
 
 struct Shape {
   int frames, channels, samples;
@@ -148,6 +154,9 @@ struct Shape {
   float row_origin, col_origin;
   float phase_row, phase_col, phase_sign;  // origin-phase coefficients
   int bin_blocks, bin_span;  // 2-D binning: blocks per frame and samples per block
+  // blocks of all frames that the counts have room for: never fewer for more samples or
+  // frames, where bin_blocks rises and falls, so that a workspace serves every smaller call
+  size_t bin_capacity;
   int coil_group, column_block, frames_per_pass, coil_parts;
   uint32_t wait_fault;  // tests only: segment waits that cannot succeed, given up after this many polls
   int column_pass;      // 1 one CTA per tile (k_cols), 2 persistent ring (k_cols_ring)
@@ -225,17 +234,22 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
     // 26 turns: 3, 4, 6 blocks a frame take 108, 161, 132 us of k_place).
     const int turns = (s->samples + kBinThreads - 1) / kBinThreads;
     const double load = s->lists_per_frame / 4608.0;
-    double best = 0.0;
+    const size_t most = std::max<size_t>(s->frames, kBinCounts / s->lists_per_frame);
+    double best = HUGE_VAL;
+    s->bin_span = turns * kBinThreads;
+    s->bin_blocks = 1;
     for (int t = 1; t <= turns; t += 1 + t / 16) {
       const int blocks = (turns + t - 1) / t;
-      const double rounds = std::ceil(static_cast<double>(blocks) * s->frames / 152.0);
+      if (static_cast<size_t>(blocks) * s->frames > most) continue;
+      const double rounds = std::ceil(static_cast<double>(blocks) * s->frames / kSms);
       const double cost = (t + load) * std::max(rounds, 1.5);
-      if (t == 1 || cost <= best) {
+      if (cost <= best) {
         best = cost;
         s->bin_span = t * kBinThreads;
         s->bin_blocks = blocks;
       }
     }
+    s->bin_capacity = std::min(static_cast<size_t>(s->frames) * turns, most);
   }
   s->out_rows = s->rows;
   s->out_cols = s->cols;
@@ -355,7 +369,7 @@ Layout make_layout(const Shape& s, const ksj_gpu_gridding_desc* d) {
   l.frame_flags = take(static_cast<size_t>(s.frames) * 4);
   l.cleared = off;
   l.records = take(fm * record_bytes(s.width));
-  l.counts = take(nl * s.bin_blocks * 4);
+  l.counts = take(s.bin_capacity * s.lists_per_frame * 4);
   l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.expanded = take(static_cast<size_t>(s.frames) * s.entries_per_frame * entry_bytes(s.width));
@@ -2597,7 +2611,7 @@ PmLayout make_pm_layout(const Shape& s) {
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
   l.flags = take(kFlagBytes);
   l.records = take(fm * record_bytes(s.width));
-  l.counts = take(nl * s.bin_blocks * 4);
+  l.counts = take(s.bin_capacity * s.lists_per_frame * 4);
   l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
   l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * (16 + 8 * static_cast<size_t>(s.width)));
@@ -2926,7 +2940,7 @@ template <class Take>
 Lists3 take_lists3(const Shape& s, Take&& take) {
   const size_t g = static_cast<size_t>(s.grid_rows), nl = g * s.lists_per_frame;
   Lists3 l{};
-  l.plane_counts = take(static_cast<size_t>(s.bin_blocks) * g * 4);
+  l.plane_counts = take(s.bin_capacity * g * 4);
   l.plane_totals = take(g * 4);
   l.plane_offsets = take((g + 1) * 4);
   l.plane_samples = take(static_cast<size_t>(s.samples) * s.width * 4);
@@ -3011,9 +3025,10 @@ ksj_gpu_status make_shape3(const ksj_gpu_gridding3_desc* d, const ksj_gpu_griddi
   const ksj_gpu_status st = make_shape(&d2, t, s);
   if (st != KSJ_GPU_OK) return st;
   s->entries_per_frame = 0;  // absolute offsets into one entry array
-  // the plane stage of the binning: one frame, planes for lists (four blocks per SM)
+  // the plane stage of the binning: one frame, planes for lists
   const int turns = (s->samples + kBinThreads - 1) / kBinThreads;
-  const int blocks = std::min(turns, 152 * 4);
+  const int blocks = std::min(turns, kPlaneStageBlocks);
+  s->bin_capacity = blocks;
   s->bin_span = (turns + blocks - 1) / blocks * kBinThreads;
   s->bin_blocks = (s->samples + s->bin_span - 1) / s->bin_span;
   return KSJ_GPU_OK;
