@@ -2599,38 +2599,49 @@ struct PmLayout {
   size_t flags, records, counts, totals, offsets, entries, bins, order, pm, w, grid, total;
 };
 
-PmLayout make_pm_layout(const Shape& s) {
-  PmLayout l{};
+// Frames are independent, so a call takes them in passes through one workspace: as many at
+// once as keep their entries (48 bytes for a width of 4, up to 2 W of them a sample) and
+// their grids within kPmPassBytes each, and at least one.
+constexpr size_t kPmPassBytes = size_t{4} << 30;
+
+// The workspace of a call, which every pass of it uses as it is: the regions hold the most
+// samples and frames of any pass, of this call and of every smaller one.
+ksj_gpu_status make_pm_layout(const ksj_gpu_gridding_desc* desc, PmLayout* layout, uint32_t* pass_frames) {
+  Shape s{};
+  ksj_gpu_gridding_desc d = *desc;
+  ksj_gpu_status st = make_shape(&d, nullptr, &s);
+  if (st != KSJ_GPU_OK) return st;
+  const size_t grid_bytes = static_cast<size_t>(s.grid_rows) * s.grid_cols * sizeof(double);
+  d.frames = static_cast<uint32_t>(std::min<size_t>(d.frames, kPmPassBytes / grid_bytes));
+  st = make_shape(&d, nullptr, &s);
+  if (st != KSJ_GPU_OK) return st;
+  const size_t entry = 16 + 8 * static_cast<size_t>(s.width), m = static_cast<size_t>(s.samples);
+  const size_t per_sample = s.entries_per_frame / m;
+  const size_t held = std::max(kPmPassBytes / (per_sample * entry), m);  // samples of one pass, at most
+  const size_t fm = std::min(s.frames * m, held);
+  *pass_frames = static_cast<uint32_t>(fm / m);
+  PmLayout& l = *layout;
+  l = PmLayout{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
     off = align_up(off + bytes, 256);
     return at;
   };
-  const size_t fm = static_cast<size_t>(s.frames) * s.samples;
   const size_t nl = static_cast<size_t>(s.frames) * s.lists_per_frame;
   l.flags = take(kFlagBytes);
   l.records = take(fm * record_bytes(s.width));
   l.counts = take(s.bin_capacity * s.lists_per_frame * 4);
   l.totals = take(nl * 4);
   l.offsets = take((nl + s.frames) * 4);
-  l.entries = take(static_cast<size_t>(s.frames) * s.entries_per_frame * (16 + 8 * static_cast<size_t>(s.width)));
+  l.entries = take(fm * per_sample * entry);
   l.bins = take(2 * kPmBins * 4);
   l.order = take(nl * 4);
   l.pm = take(fm * (8 + 16 * static_cast<size_t>(s.width)));
   l.w = take(fm * sizeof(double));
-  l.grid = take(static_cast<size_t>(s.frames) * s.grid_rows * s.grid_cols * sizeof(double));
+  l.grid = take(s.frames * grid_bytes);
   l.total = off;
-  return l;
-}
-
-// Frames of one pass: as many as keep the entries (48 bytes for a width of 4, up to
-// 2 W of them a sample) within 4 GB, and at least one.  Frames are independent, so a
-// call of more takes them in passes through one workspace.
-uint32_t pm_pass_frames(const Shape& s) {
-  const size_t frame = s.entries_per_frame * (16 + 8 * static_cast<size_t>(s.width));
-  return static_cast<uint32_t>(
-      std::min<size_t>(s.frames, std::max<size_t>(1, (size_t{4} << 30) / std::max<size_t>(frame, 1))));
+  return KSJ_GPU_OK;
 }
 
 // The flags must already be cleared.
@@ -4255,28 +4266,28 @@ extern "C" ksj_gpu_status ksj_gpu_gridding_tune(const ksj_gpu_gridding_desc* des
 }
 
 extern "C" size_t ksj_gpu_pipe_menon_workspace_bytes(const ksj_gpu_gridding_desc* desc) {
-  Shape s{};
-  if (desc == nullptr || desc->kernel != KSJ_GPU_KERNEL_KAISER_BESSEL || make_shape(desc, nullptr, &s) != KSJ_GPU_OK)
+  PmLayout l{};
+  uint32_t per_pass = 0;
+  if (desc == nullptr || desc->struct_size < sizeof(ksj_gpu_gridding_desc) ||
+      desc->kernel != KSJ_GPU_KERNEL_KAISER_BESSEL)
     return 0;
-  ksj_gpu_gridding_desc pass = *desc;
-  pass.frames = pm_pass_frames(s);
-  return make_shape(&pass, nullptr, &s) == KSJ_GPU_OK ? make_pm_layout(s).total : 0;
+  return make_pm_layout(desc, &l, &per_pass) == KSJ_GPU_OK ? l.total : 0;
 }
 
 extern "C" ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* desc, uint32_t iterations,
                                                  const float* d_traj, float* d_dcf, void* d_workspace,
                                                  size_t workspace_bytes, void* stream) {
-  if (desc == nullptr || desc->kernel != KSJ_GPU_KERNEL_KAISER_BESSEL || iterations == 0 || iterations > 1000)
+  if (desc == nullptr || desc->struct_size < sizeof(ksj_gpu_gridding_desc) ||
+      desc->kernel != KSJ_GPU_KERNEL_KAISER_BESSEL || iterations == 0 || iterations > 1000)
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  Shape s{};
-  const ksj_gpu_status st = make_shape(desc, nullptr, &s);
+  PmLayout l{};
+  uint32_t per_pass = 0;
+  const ksj_gpu_status st = make_pm_layout(desc, &l, &per_pass);
   if (st != KSJ_GPU_OK) return st;
   if (d_traj == nullptr || d_dcf == nullptr || (reinterpret_cast<uintptr_t>(d_traj) & 7u) != 0 ||
       (reinterpret_cast<uintptr_t>(d_dcf) & 3u) != 0)
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  const uint32_t per_pass = pm_pass_frames(s);
-  if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 ||
-      workspace_bytes < ksj_gpu_pipe_menon_workspace_bytes(desc))
+  if (d_workspace == nullptr || (reinterpret_cast<uintptr_t>(d_workspace) & 255u) != 0 || workspace_bytes < l.total)
     return KSJ_GPU_ERROR_WORKSPACE;
   unsigned char* ws = static_cast<unsigned char*>(d_workspace);
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
@@ -4284,9 +4295,9 @@ extern "C" ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* de
   for (uint32_t f0 = 0; f0 < desc->frames; f0 += per_pass) {
     ksj_gpu_gridding_desc pass = *desc;
     pass.frames = std::min(per_pass, desc->frames - f0);
+    Shape s{};
     const ksj_gpu_status ps = make_shape(&pass, nullptr, &s);
     if (ps != KSJ_GPU_OK) return ps;
-    const PmLayout l = make_pm_layout(s);
     const float* traj = d_traj + static_cast<size_t>(f0) * s.samples * 2;
     float* dcf = d_dcf + static_cast<size_t>(f0) * s.samples;
     ksj_gpu_status run = KSJ_GPU_ERROR_UNSUPPORTED;

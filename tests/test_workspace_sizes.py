@@ -64,3 +64,14 @@ def test_3d_size_grows_with_samples(gpu, grid):
             sizes3w.append(int(gpu.lib().ksj_gpu_pipe_menon3_workspace_bytes(ctypes.byref(d))))
     _grows(sizes3)
     _grows(sizes3w)
+
+
+@pytest.mark.parametrize("grid,width", [(64, 4), (512, 8)])
+def test_weights_size_grows_across_the_passes(gpu, grid, width):
+    """Frames of one to several passes of 4 GB of entries; frames of a few samples by the thousand."""
+    for frames in (1, 2, 3, 7, 5000, 65535):
+        _grows(_weights(gpu, grid, width, 1, m, frames) for m in
+               [1, 700, 40_000, 800_000, 1_100_000, 1_118_481, 1_118_482, 1_677_721, 1_677_722, 3_355_443, 3_355_444,
+                5_592_405, 5_592_406, 11_184_810, 11_184_811, 1 << 26])
+    for m in (1, 40_000, 1_118_482, 5_592_406):
+        _grows(_weights(gpu, grid, width, 1, m, f) for f in [1, 2, 3, 4, 5, 10, 83, 84, 2047, 2048, 2049, 65535])
