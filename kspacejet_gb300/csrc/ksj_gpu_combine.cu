@@ -278,14 +278,12 @@ ksj_gpu_status launch_walsh(uint32_t rows, uint32_t cols, int half, uint32_t ite
                             cudaStream_t stream) {
   const int span = kWalshCols + 2 * half, tall = kWalshRows + 2 * half;
   const size_t smem = static_cast<size_t>(span) * C * (tall * sizeof(float2) + kWalshRows * C * sizeof(float));
-  if (cudaFuncSetAttribute(k_walsh<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-      cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
+  KSJ_TRY(allow_smem(k_walsh<C>, smem));
   const unsigned grid = ((cols + kWalshCols - 1) / kWalshCols) * ((rows + kWalshRows - 1) / kWalshRows);
   LaunchScope scope("k_walsh", stream);
-  launch_chained(k_walsh<C>, dim3(grid), dim3(kWalshThreads), smem, stream, static_cast<const float2*>(in),
+  KSJ_TRY(launch_chained(k_walsh<C>, dim3(grid), dim3(kWalshThreads), smem, stream, static_cast<const float2*>(in),
                  static_cast<float2*>(out), static_cast<int>(rows), static_cast<int>(cols), half,
-                 static_cast<int>(iterations));
+                 static_cast<int>(iterations)));
   return check_launch();
 }
 
@@ -682,18 +680,19 @@ ksj_gpu_status covariance_run(uint32_t channels, uint32_t samples, const void* d
     const CovArgs args{static_cast<const float2*>(d_kspace), partials, flags, static_cast<int>(channels),
                        static_cast<int>(samples), l.ktiles};
     LaunchScope scope("k_cov_mma", cs);
-    launch_chained(k_cov_mma, dim3(l.blocks), dim3(kCovThreads), smem, cs, args);
+    KSJ_TRY(launch_chained(k_cov_mma, dim3(l.blocks), dim3(kCovThreads), smem, cs, args));
   }
   float2* means = nullptr;
   if (noise) {
     means = reinterpret_cast<float2*>(ws + l.means);
     LaunchScope scope("k_channel_means", cs);
     k_channel_means<<<channels, 256, 0, cs>>>(static_cast<const float2*>(d_kspace), static_cast<int>(samples), means);
+    KSJ_TRY(check_launch());
   }
   LaunchScope scope("k_cov_form", cs);
-  launch_chained(k_cov_form, dim3(kCovRows * 64 / kCovSumElems), dim3(kCovSumElems * kCovSumSlices), 0, cs, partials,
+  KSJ_TRY(launch_chained(k_cov_form, dim3(kCovRows * 64 / kCovSumElems), dim3(kCovSumElems * kCovSumSlices), 0, cs, partials,
                  l.blocks, reinterpret_cast<float*>(ws + l.sum), flags + 1, static_cast<int>(channels),
-                 1.0f / static_cast<float>(samples), means, static_cast<float2*>(d_cov));
+                 1.0f / static_cast<float>(samples), means, static_cast<float2*>(d_cov)));
   return check_launch();
 }
 
@@ -802,9 +801,9 @@ ksj_gpu_status launch_compress(uint32_t channels, uint32_t samples, const void* 
   const auto kernel = pairs ? k_coil_compress<kV, 2> : k_coil_compress<kV, 1>;
   const uint32_t per_block = compress_threads(kV) * (pairs ? 2 : 1);
   LaunchScope scope("k_coil_compress", stream);
-  launch_chained(kernel, dim3((samples + per_block - 1) / per_block), dim3(compress_threads(kV)), 0, stream,
+  KSJ_TRY(launch_chained(kernel, dim3((samples + per_block - 1) / per_block), dim3(compress_threads(kV)), 0, stream,
       static_cast<const float2*>(basis), static_cast<const float2*>(x), static_cast<float2*>(y),
-      static_cast<int>(channels), static_cast<int>(samples));
+      static_cast<int>(channels), static_cast<int>(samples)));
   return check_launch();
 }
 

@@ -347,22 +347,24 @@ extern "C" ksj_gpu_status ksj_gpu_kb_forward(const ksj_gpu_gridding_desc* desc, 
     const double beta_t = static_cast<double>(static_cast<float>(s.beta));
     k_fwd_tables<<<(s.g + 255) / 256, 256, 0, cs>>>(tw, inv_d, pos, s.n, s.g, s.width, beta_t,
                                                     std::cyl_bessel_i(0.0, beta_t), s.plan);
+    KSJ_TRY(check_launch());
   }
   FwdArgs a{tw, inv_d, pos, s.plan, s.frames, s.channels, s.samples, s.n, s.g, s.cg, s.cpitch};
   FwdKernel cols_k = nullptr, rows_k = nullptr;
   fwd_kernels_for(s.g, s.n, &cols_k, &rows_k);
   const size_t smem = (static_cast<size_t>(s.g) * s.cg + s.g) * sizeof(float2) + static_cast<size_t>(s.n) * sizeof(float);
-  if (cudaFuncSetAttribute(cols_k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
-      cudaFuncSetAttribute(rows_k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
+  KSJ_TRY(allow_smem(cols_k, smem));
+  KSJ_TRY(allow_smem(rows_k, smem));
   const int groups = (s.channels + s.cg - 1) / s.cg;
   {
     LaunchScope scope("k_fwd_cols", cs);
     cols_k<<<dim3(s.n, groups, s.frames), kFwdLineThreads, smem, cs>>>(static_cast<const float2*>(d_image), t1, a);
+    KSJ_TRY(check_launch());
   }
   {
     LaunchScope scope("k_fwd_rows", cs);
     rows_k<<<dim3(s.g, groups, s.frames), kFwdLineThreads, smem, cs>>>(t1, grid, a);
+    KSJ_TRY(check_launch());
   }
   InterpArgs ia{grid, d_traj, static_cast<float2*>(d_samples), flags, s.frames, s.channels, s.samples, s.g, s.cpitch,
                 static_cast<float>(s.beta), 2.0f / static_cast<float>(s.width),

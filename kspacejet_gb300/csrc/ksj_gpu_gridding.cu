@@ -127,6 +127,8 @@ constexpr uint32_t kWaitLimit = 1u << 22;  // polls before a bounded wait gives 
 constexpr int kBinThreads = 512;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr size_t kPlaceListBytes = 4;  // of k_place: the list's running position
+constexpr size_t kListSmem = kMaxGrid * (kMaxGrid / kChunk) * 4;  // a word of every list of the largest grid
+constexpr size_t kRowsSmem = 200 * 1024;                          // of a k_rows block, at most
 constexpr int kSms = 152;              // of a GB300
 // A call keeps one count per list for each of its blocks: at most this many (64 MB), or one
 // block a frame where that is more.
@@ -296,7 +298,7 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   int cap = t && t->list_capacity ? static_cast<int>(t->list_capacity) : 0;
   if (cap == 0) cap = 512;
   if (cap < 64 || cap > 2048 || (cap & (cap - 1)) != 0) return KSJ_GPU_ERROR_INVALID_ARGUMENT;
-  const size_t smem_limit = 200 * 1024;
+  const size_t smem_limit = kRowsSmem;
   const int parts = t && t->struct_size >= offsetof(ksj_gpu_gridding_tuning, coil_parts) + 4 && t->coil_parts
                         ? static_cast<int>(t->coil_parts)
                         : 1;
@@ -891,9 +893,8 @@ ksj_gpu_status launch_scan(const uint32_t* counts, uint32_t* offsets, int lists,
     samples.bf16 = bf16;
     total += scan_sample_blocks(coil_last->samples, coil_last->channels, frames);
   }
-  launch_chained(k_scan, dim3(static_cast<unsigned>(total)), 1024, 0, stream, counts, offsets, lists, frames,
-                 tables ? *tables : TablesArgs{}, samples);
-  return KSJ_GPU_OK;
+  return launch_chained(k_scan, dim3(static_cast<unsigned>(total)), 1024, 0, stream, counts, offsets, lists, frames,
+                        tables ? *tables : TablesArgs{}, samples);
 }
 
 // One list entry (entry_bytes(W)) from its sample's record.
@@ -1800,8 +1801,7 @@ struct RowsLauncher {
     threads = rows_threads_for(s.grid_cols, lanes, s.coil_group);
     smem = rows_smem_for(s.grid_cols, s.coil_group, lanes, threads);
     kernel = rows_kernel_for(s.grid_cols, s.coil_parts == 1 ? s.coil_group : 0, s.kb && s.out_cols * 2 == s.grid_cols);
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
-               cudaSuccess &&
+    return allow_smem(kernel, smem, kRowsSmem) == KSJ_GPU_OK &&
            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
   }
 
@@ -1809,10 +1809,10 @@ struct RowsLauncher {
   // A launch of few waves takes the rows in from both ends: frequency 0, where radial
   // scans crowd, is at row 0, and the rows before it, at the end, should not be the
   // last to start (a 32-coil frame 72 -> 65 us; 48 frames, 61 waves, 1 % slower).
-  void launch(RowsArgs r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
+  ksj_gpu_status launch(RowsArgs r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
     r.both_ends = static_cast<long long>(grid_rows) * groups * nf <= 16 * 304;
     LaunchScope scope("k_rows", stream);
-    launch_chained(kernel, dim3(grid_rows, groups, nf), threads, smem, stream, r);
+    return launch_chained(kernel, dim3(grid_rows, groups, nf), threads, smem, stream, r);
   }
 };
 
@@ -1849,7 +1849,7 @@ ColsKernel cols_kernel_for(int n, bool half = false, bool lines32 = false) {
 
 // Opt a k_cols instance into its dynamic shared memory.
 bool cols_kernel_setup(ColsKernel k, size_t smem) {
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+  return allow_smem(k, smem) == KSJ_GPU_OK &&
          cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
 }
 
@@ -1950,14 +1950,13 @@ struct ColsPass {
   }
 
   // The column pass over nf frames starting at c.frame0.
-  void launch(ColsArgs c, int nf, cudaStream_t stream, const char* name) const {
+  ksj_gpu_status launch(ColsArgs c, int nf, cudaStream_t stream, const char* name) const {
     LaunchScope scope(name, stream);
-    if (ring) {
-      c.units = nf * c.col_blocks;
-      launch_chained(kernel, std::min(ctas, c.units), threads, smem, stream, map, c);
-    } else {
-      launch_chained(kernel, dim3((out_cols + column_block - 1) / column_block, nf), kColsThreads, smem, stream, map, c);
-    }
+    if (!ring)
+      return launch_chained(kernel, dim3((out_cols + column_block - 1) / column_block, nf), kColsThreads, smem, stream,
+                            map, c);
+    c.units = nf * c.col_blocks;
+    return launch_chained(kernel, std::min(ctas, c.units), threads, smem, stream, map, c);
   }
 };
 
@@ -1975,9 +1974,8 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
   const auto place = pm ? k_place<W, true> : k_place<W, false>;
-  if (cudaFuncSetAttribute(k_prepare<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, count_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(place, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
+  KSJ_TRY(allow_smem(k_prepare<W>, count_smem, kListSmem));
+  KSJ_TRY(allow_smem(place, place_smem, kListSmem));
   const dim3 blocks(s.bin_blocks, s.frames);
   {
     PrepareArgs p{};
@@ -2006,15 +2004,15 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.phase_col = s.phase_col;
     p.phase_sign = s.phase_sign;
     LaunchScope scope("k_prepare", stream);
-    launch_chained(k_prepare<W>, blocks, kBinThreads, count_smem, stream, p);
+    KSJ_TRY(launch_chained(k_prepare<W>, blocks, kBinThreads, count_smem, stream, p));
   }
   {
     LaunchScope scope("k_bin_prefix", stream);
-    launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream, counts, totals,
-                   s.bin_blocks, s.lists_per_frame);
+    KSJ_TRY(launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, s.frames), 128, 0, stream, counts, totals,
+                   s.bin_blocks, s.lists_per_frame));
   }
-  launch_scan(totals, offsets, s.lists_per_frame, s.frames, tables, stream, coil_last,
-              d->sample_format == KSJ_GPU_SAMPLES_BF16);
+  KSJ_TRY(launch_scan(totals, offsets, s.lists_per_frame, s.frames, tables, stream, coil_last,
+                      d->sample_format == KSJ_GPU_SAMPLES_BF16));
   {
     PlaceArgs p{};
     p.records = records;
@@ -2030,7 +2028,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.bin_span = s.bin_span;
     p.entries_per_frame = s.entries_per_frame;
     LaunchScope scope("k_place", stream);
-    launch_chained(place, blocks, kBinThreads, place_smem, stream, p);
+    KSJ_TRY(launch_chained(place, blocks, kBinThreads, place_smem, stream, p));
   }
   return KSJ_GPU_OK;
 }
@@ -2088,9 +2086,9 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
     const dim3 tg((s.samples + 31) / 32, (s.channels + 31) / 32, nf);
     LaunchScope scope("k_samples_coil_last", st);
     coil_last.frame0 = f0;
-    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, st, coil_last);
+    return launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, st, coil_last);
   };
-  if (samples_here && !with_scan) to_coil_last(0, s.frames, stream);
+  if (samples_here && !with_scan) KSJ_TRY(to_coil_last(0, s.frames, stream));
   RowsArgs r{};
   r.samples_t = reinterpret_cast<const float2*>(ws + l.samples_t);
   r.sample_frame_stride = static_cast<size_t>(s.samples) * s.channels;
@@ -2150,7 +2148,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   if (io != nullptr && s.frames > s.frames_per_pass &&
       (cudaEventRecord(io->ready, stream) != cudaSuccess || cudaStreamWaitEvent(io->alt, io->ready, 0) != cudaSuccess))
     return KSJ_GPU_ERROR_CUDA;
-  for (int f0 = 0, pass = 0; f0 < s.frames; f0 += s.frames_per_pass, ++pass) {
+  auto run_pass = [&](int f0, int pass) {
     const int nf = std::min(s.frames_per_pass, s.frames - f0);
     cudaStream_t ps = stream;
     if (io != nullptr) {
@@ -2160,13 +2158,13 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
       }
       if (io->copy != nullptr) {
         if (cudaStreamWaitEvent(ps, io->in[pass], 0) != cudaSuccess) return KSJ_GPU_ERROR_CUDA;
-        to_coil_last(f0, nf, ps);
+        KSJ_TRY(to_coil_last(f0, nf, ps));
       }
     }
     r.frame0 = f0;
     c.frame0 = f0;
-    rows_launch.launch(r, s.grid_rows, (s.channels + s.coil_group - 1) / s.coil_group, nf, ps);
-    cols_pass.launch(c, nf, ps, "k_cols");
+    KSJ_TRY(rows_launch.launch(r, s.grid_rows, (s.channels + s.coil_group - 1) / s.coil_group, nf, ps));
+    KSJ_TRY(cols_pass.launch(c, nf, ps, "k_cols"));
     if (coil_major) {
       // [frame][pixel][channel] -> [frame][channel][pixel], this pass's frames
       const size_t fe = static_cast<size_t>(pixels) * s.channels;
@@ -2175,6 +2173,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
       k_transpose<unsigned long long><<<tg, dim3(32, 8), 0, ps>>>(
           reinterpret_cast<const unsigned long long*>(ws + l.coil_last) + f0 * fe,
           static_cast<unsigned long long*>(d_out) + f0 * fe, pixels, s.channels);
+      KSJ_TRY(check_launch());
     }
     if (io != nullptr && io->copy != nullptr) {
       const size_t off = static_cast<size_t>(f0) * io->out_frame_bytes;
@@ -2185,12 +2184,16 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
               cudaSuccess)
         return KSJ_GPU_ERROR_CUDA;
     }
-  }
-  // the second compute stream joins back before the call's stream goes on
+    return check_launch();
+  };
+  ksj_gpu_status result = KSJ_GPU_OK;
+  for (int f0 = 0, pass = 0; f0 < s.frames && result == KSJ_GPU_OK; f0 += s.frames_per_pass, ++pass)
+    result = run_pass(f0, pass);
+  // the second compute stream joins back before the call's stream goes on, after a failure too
   if (alt_used &&
       (cudaEventRecord(io->alt_done, io->alt) != cudaSuccess || cudaStreamWaitEvent(stream, io->alt_done, 0) != cudaSuccess))
     return KSJ_GPU_ERROR_CUDA;
-  return check_launch();
+  return result;
 }
 
 // ------------------------------------------------- Pipe-Menon density weights
@@ -2663,6 +2666,7 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
     k_pm_prepare<W><<<static_cast<unsigned>((fm + 255) / 256), 256, 0, stream>>>(
         d_traj, pm, w, fm, s.grid_rows, s.grid_cols, kb_taps(W, s.beta), s.beta,
         1.0 / std::cyl_bessel_i(0.0, static_cast<double>(s.beta)), d->require_nyquist);
+    KSJ_TRY(check_launch());
   }
   const ksj_gpu_status st =
       build_lists<W>(s, &dd, d_traj, nullptr, flags, ws + l.records, reinterpret_cast<uint32_t*>(ws + l.counts),
@@ -2678,24 +2682,26 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
   {
     LaunchScope scope("k_pm_bins", stream);
     k_pm_bins<<<order_blocks, kPmOrderThreads, 0, stream>>>(offsets, lists, s.lists_per_frame, bins);
+    KSJ_TRY(check_launch());
   }
   {
     LaunchScope scope("k_pm_order", stream);
     k_pm_order<<<order_blocks, kPmOrderThreads, 0, stream>>>(offsets, lists, s.lists_per_frame, bins, order);
+    KSJ_TRY(check_launch());
   }
   for (uint32_t it = 0; it < iterations; ++it) {
     {
       LaunchScope scope("k_pm_grid", stream);
-      launch_chained(k_pm_grid<W>, dim3(static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads + 1)),
+      KSJ_TRY(launch_chained(k_pm_grid<W>, dim3(static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads + 1)),
                      dim3(kPmThreads), 0, stream,
           offsets, reinterpret_cast<const PmEntry<W>*>(ws + l.entries), static_cast<const uint32_t*>(order),
                      static_cast<const uint32_t*>(bins), static_cast<const double*>(w), grid, lists, s.samples,
-          s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame);
+          s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame));
     }
     LaunchScope scope("k_pm_update", stream);
-    launch_chained(k_pm_update<W>, dim3(static_cast<unsigned>((fm + 255) / 256)), dim3(256), 0, stream,
+    KSJ_TRY(launch_chained(k_pm_update<W>, dim3(static_cast<unsigned>((fm + 255) / 256)), dim3(256), 0, stream,
                    static_cast<const PmRecord<W>*>(pm), static_cast<const double*>(grid), w,
-                   it + 1 == iterations ? d_dcf : nullptr, fm, s.samples, s.grid_rows, s.grid_cols);
+                   it + 1 == iterations ? d_dcf : nullptr, fm, s.samples, s.grid_rows, s.grid_cols));
   }
   return check_launch();
 }
@@ -3058,9 +3064,8 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
   auto at = [&](size_t offset) { return reinterpret_cast<uint32_t*>(ws + offset); };
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
-  if (cudaFuncSetAttribute(k_count3<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, count_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_place3<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, place_smem) != cudaSuccess)
-    return KSJ_GPU_ERROR_CUDA;
+  KSJ_TRY(allow_smem(k_count3<W>, count_smem, kListSmem));
+  KSJ_TRY(allow_smem(k_place3<W>, place_smem, kListSmem));
   {
     Prepare3Args p{};
     p.traj = d_traj;
@@ -3078,41 +3083,47 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     p.phase = s.phase_row;
     LaunchScope scope("k_prepare3", stream);
     k_prepare3<W><<<s.bin_blocks, kBinThreads, 0, stream>>>(p);
+    KSJ_TRY(check_launch());
   }
   {
     LaunchScope scope("k_bin_prefix", stream);
-    launch_chained(k_bin_prefix, (g + 127) / 128, 128, 0, stream, at(l.plane_counts), at(l.plane_totals), s.bin_blocks, g);
+    KSJ_TRY(launch_chained(k_bin_prefix, (g + 127) / 128, 128, 0, stream, at(l.plane_counts), at(l.plane_totals), s.bin_blocks, g));
   }
-  launch_scan(at(l.plane_totals), at(l.plane_offsets), g, 1, tables, stream);
+  KSJ_TRY(launch_scan(at(l.plane_totals), at(l.plane_offsets), g, 1, tables, stream));
   {
     LaunchScope scope("k_plane_place", stream);
     k_plane_place<W><<<s.bin_blocks, kBinThreads, 0, stream>>>(records, at(l.plane_offsets), at(l.plane_counts),
                                                               at(l.plane_samples), s.samples, g, s.bin_span);
+    KSJ_TRY(check_launch());
   }
   const dim3 blocks(kPlaneBlocks, g);
   {
     LaunchScope scope("k_count3", stream);
     k_count3<W><<<blocks, kBinThreads, count_smem, stream>>>(records, at(l.plane_offsets), at(l.plane_samples),
                                                             at(l.counts), g, s.nchunks, s.lists_per_frame);
+    KSJ_TRY(check_launch());
   }
   {
     LaunchScope scope("k_bin_prefix", stream);
-    launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, g), 128, 0, stream, at(l.counts), at(l.totals),
-                   kPlaneBlocks, s.lists_per_frame);
+    KSJ_TRY(launch_chained(k_bin_prefix, dim3((s.lists_per_frame + 127) / 128, g), 128, 0, stream, at(l.counts), at(l.totals),
+                   kPlaneBlocks, s.lists_per_frame));
   }
-  launch_scan(at(l.totals), at(l.offsets), s.lists_per_frame, g, nullptr, stream);
+  KSJ_TRY(launch_scan(at(l.totals), at(l.offsets), s.lists_per_frame, g, nullptr, stream));
   {
     LaunchScope scope("k_plane_offsets", stream);
     k_plane_bases<<<1, 512, 0, stream>>>(at(l.offsets), g, s.lists_per_frame, at(l.bases));
+    KSJ_TRY(check_launch());
     const size_t total = static_cast<size_t>(g) * (s.lists_per_frame + 1);
     k_offsets_add<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(at(l.offsets), g, s.lists_per_frame,
                                                                                 at(l.bases));
+    KSJ_TRY(check_launch());
   }
   {
     const Place3Args p{records, at(l.plane_offsets), at(l.plane_samples), at(l.offsets), at(l.counts), expanded, entries,
                        g, s.nchunks, s.lists_per_frame};
     LaunchScope scope("k_place3", stream);
     k_place3<W><<<blocks, kBinThreads, place_smem, stream>>>(p);
+    KSJ_TRY(check_launch());
   }
   return KSJ_GPU_OK;
 }
@@ -3148,6 +3159,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   {
     LaunchScope scope("k_fill_ones", stream);
     k_fill<<<(n * n + 255) / 256, 256, 0, stream>>>(ones, n * n, 1.0f);
+    KSJ_TRY(check_launch());
   }
   {
     const ksj_gpu_status st = build_lists3<W>(s, d->dcf_mode, d_traj, d_dcf, flags, ws + l.records, ws, l.lists, nullptr,
@@ -3157,6 +3169,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   if (parts > 1) {
     LaunchScope scope("k_repeat", stream);
     k_repeat<<<(n * parts + 255) / 256, 256, 0, stream>>>(inv_dc, inv_dc_parts, parts, n * parts);
+    KSJ_TRY(check_launch());
   }
   {
     const dim3 tg((s.samples + 31) / 32, (s.channels + 31) / 32, 1);
@@ -3164,7 +3177,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
     const CoilLastArgs a{d_kspace, reinterpret_cast<float2*>(ws + l.samples_t),
                          ws + l.records + offsetof(SampleRecord3<W>, scale), static_cast<int>(sizeof(SampleRecord3<W>)),
                          s.channels, s.samples, flags, nullptr, nullptr, nullptr, 0, nullptr};
-    launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, stream, a);
+    KSJ_TRY(launch_chained(k_samples_coil_last<kFormat>, tg, dim3(32, 8), 0, stream, a));
   }
   // rows of every plane (x transformed, kept columns, coil-last)
   RowsArgs r{};
@@ -3236,8 +3249,8 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
     const int nf = std::min(s.frames_per_pass, g - f0);
     r.frame0 = f0;
     cy.frame0 = f0;
-    rows_launch.launch(r, g, (s.channels + s.coil_group - 1) / s.coil_group, nf, stream);
-    cols_pass.launch(cy, nf, stream, "k_cols");
+    KSJ_TRY(rows_launch.launch(r, g, (s.channels + s.coil_group - 1) / s.coil_group, nf, stream));
+    KSJ_TRY(cols_pass.launch(cy, nf, stream, "k_cols"));
   }
   // z: the column pass over [plane][pixel][cpitch] with planes as rows and pixels as columns
   Shape z = s;
@@ -3253,7 +3266,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   cz.out_pitch = s.channels;
   ColsPass z_pass;
   if (!z_pass.setup(z, inter2, &cz)) return KSJ_GPU_ERROR_CUDA;
-  z_pass.launch(cz, 1, stream, "k_cols_z");
+  KSJ_TRY(z_pass.launch(cz, 1, stream, "k_cols_z"));
   return check_launch();
 }
 
@@ -3626,6 +3639,7 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
     LaunchScope scope("k_pm_prepare3", stream);
     k_pm_prepare3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(d_traj, pm, pmc, w, s.samples, g, s.beta,
                                                                  1.0 / std::cyl_bessel_i(0.0, static_cast<double>(s.beta)));
+    KSJ_TRY(check_launch());
   }
   const uint32_t* offsets = reinterpret_cast<const uint32_t*>(ws + l.lists.offsets);
   const uint32_t* entries = reinterpret_cast<const uint32_t*>(ws + l.entries);
@@ -3639,10 +3653,12 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
     const size_t lists = static_cast<size_t>(g) * s.lists_per_frame;
     k_pm_queue<<<static_cast<unsigned>((lists + 255) / 256), 256, 0, stream>>>(
         offsets, g, s.lists_per_frame, reinterpret_cast<uint32_t*>(ws + l.long_lists));
+    KSJ_TRY(check_launch());
   }
   {
     LaunchScope scope("k_pm_long_parts", stream);
     k_pm_long_parts<<<1, 1024, 0, stream>>>(long_lists, offsets, s.lists_per_frame, part_base);
+    KSJ_TRY(check_launch());
   }
   const size_t lists = static_cast<size_t>(g) * s.lists_per_frame;
   const unsigned grid_blocks = static_cast<unsigned>((lists * kPmLanes + kPmThreads - 1) / kPmThreads);
@@ -3659,16 +3675,19 @@ ksj_gpu_status launch_pipe_menon3(const Shape& s, const PmLayout3& l, uint32_t i
       auto kernel = it == 0 ? k_pm_grid3<W, true> : k_pm_grid3<W, false>;
       kernel<<<grid_blocks, kPmThreads, 0, stream>>>(offsets, entries, pm, pmc, w, wzr, grid, g, s.nchunks,
                                                      s.lists_per_frame, kPmLong);
+      KSJ_TRY(check_launch());
     }
     {
       LaunchScope scope("k_pm_long3", stream);
       auto kernel = it == 0 ? k_pm_long3<W, true> : k_pm_long3<W, false>;
       kernel<<<long_blocks, kPmThreads, 0, stream>>>(long_lists, part_base, offsets, entries, pm, pmc, w, wzr, grid, g,
                                                  s.nchunks, s.lists_per_frame, partial, counters);
+      KSJ_TRY(check_launch());
     }
     LaunchScope scope("k_pm_update3", stream);
     k_pm_update3<W><<<(s.samples + 255) / 256, 256, 0, stream>>>(pm, grid, w, it + 1 == iterations ? d_dcf : nullptr,
                                                                 s.samples, g);
+    KSJ_TRY(check_launch());
   }
   return check_launch();
 }
@@ -4412,38 +4431,34 @@ extern "C" ksj_gpu_status ksj_gpu_cartesian_ifft2(uint32_t rows, uint32_t cols, 
   {
     const int n = static_cast<int>(std::max(rows, cols));
     LaunchScope scope("k_cart_tables", cstream);
-    launch_chained(k_cart_tables, dim3((n + 255) / 256), dim3(256), 0, cstream, tw_rows, static_cast<int>(rows), tw_cols,
-                   static_cast<int>(cols), inv_dr, inv_dc, pos_rows, pos_cols, s.plan_rows, s.plan_cols);
+    KSJ_TRY(launch_chained(k_cart_tables, dim3((n + 255) / 256), dim3(256), 0, cstream, tw_rows, static_cast<int>(rows), tw_cols,
+                   static_cast<int>(cols), inv_dr, inv_dc, pos_rows, pos_cols, s.plan_rows, s.plan_cols));
   }
   {
     const CartRowsKernel rk = cart_rows_for(static_cast<int>(cols));
     const size_t smem = (static_cast<size_t>(cols) * (cs.cg + 1) + cols) * sizeof(float2);
-    if (cudaFuncSetAttribute(rk, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-      return KSJ_GPU_ERROR_CUDA;
+    KSJ_TRY(allow_smem(rk, smem));
     const dim3 grid(rows, (channels + cs.cg - 1) / cs.cg, frames);
     LaunchScope scope("k_cart_rows", cstream);
-    launch_chained(rk, grid, dim3(kCartThreads), smem, cstream, static_cast<const float2*>(d_kspace), inter, tw_cols,
+    KSJ_TRY(launch_chained(rk, grid, dim3(kCartThreads), smem, cstream, static_cast<const float2*>(d_kspace), inter, tw_cols,
                    pos_cols, s.plan_cols, static_cast<int>(rows), static_cast<int>(cols), static_cast<int>(channels),
-                   cs.cg, s.cpitch);
+                   cs.cg, s.cpitch));
   }
   if (!is_fft_size(rows)) {
     // direct DFT along the columns, coil-last into the output (or into the
     // workspace, then its RSS)
     float2* dst = output == KSJ_GPU_OUTPUT_COIL_LAST ? static_cast<float2*>(d_out) : coil_last;
     const size_t smem = (static_cast<size_t>(rows) * cs.cg + rows) * sizeof(float2);
-    if (cudaFuncSetAttribute(k_cart_cols_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return KSJ_GPU_ERROR_CUDA;
+    KSJ_TRY(allow_smem(k_cart_cols_direct, smem));
     {
       const dim3 grid(cols, (channels + cs.cg - 1) / cs.cg, frames);
       LaunchScope scope("k_cart_cols_direct", cstream);
       k_cart_cols_direct<<<grid, kCartThreads, smem, cstream>>>(inter, dst, tw_rows, static_cast<int>(rows),
                                                                static_cast<int>(cols), static_cast<int>(channels),
                                                                cs.cg, s.cpitch);
+      KSJ_TRY(check_launch());
     }
     if (output == KSJ_GPU_OUTPUT_RSS) {
-      const ksj_gpu_status rs = check_launch();
-      if (rs != KSJ_GPU_OK) return rs;
       return ksj_gpu_rss_coil_last(static_cast<uint64_t>(frames) * rows * cols, channels, coil_last,
                                    static_cast<float*>(d_out), stream);
     }
@@ -4472,6 +4487,6 @@ extern "C" ksj_gpu_status ksj_gpu_cartesian_ifft2(uint32_t rows, uint32_t cols, 
   c.frame0 = 0;
   ColsPass cols_pass;
   if (!cols_pass.setup(s, inter, &c)) return KSJ_GPU_ERROR_CUDA;
-  cols_pass.launch(c, s.frames, cstream, "k_cols");
+  KSJ_TRY(cols_pass.launch(c, s.frames, cstream, "k_cols"));
   return check_launch();
 }

@@ -34,14 +34,36 @@ class LaunchScope {
   cudaEvent_t start_ = nullptr;
 };
 
+// Returns from the function at the first step that fails, so that no later kernel runs on what
+// a missing one should have written.
+#define KSJ_TRY(expr)                                      \
+  do {                                                     \
+    const ksj_gpu_status ksj_try_status = (expr);          \
+    if (ksj_try_status != KSJ_GPU_OK) return ksj_try_status; \
+  } while (0)
+
+// The most dynamic shared memory that a kernel's launches may ask for.  It is a property of the
+// kernel in the whole process, so every call sets it to the same value, the kernel's
+// largest: set to what one call needs, it could be lowered by another thread's
+// smaller call before this one's launch, which is then refused.
+constexpr size_t kMostSmem = 227 * 1024;  // of a block without static shared memory
+
+template <typename... Params>
+inline ksj_gpu_status allow_smem(void (*kernel)(Params...), size_t needed, size_t most = kMostSmem) {
+  return needed <= most && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(most)) == cudaSuccess
+             ? KSJ_GPU_OK
+             : KSJ_GPU_ERROR_CUDA;
+}
+
 // A launch that may begin while the stream's previous kernel ends (programmatic
 // dependent launch): its blocks take the places that kernel's last blocks leave
 // and wait there, so that the launch itself costs nothing between the two.  The
 // kernel must begin with chain_wait() or chain_begin(), before it touches memory that earlier
 // kernels write or read.
 template <typename... Params, typename... Args>
-inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                           Args&&... args) {
+[[nodiscard]] inline ksj_gpu_status launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                                   cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
@@ -52,7 +74,9 @@ inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
   config.numAttrs = 1;
-  cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  if (cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...) == cudaSuccess) return KSJ_GPU_OK;
+  cudaGetLastError();
+  return KSJ_GPU_ERROR_CUDA;
 }
 
 // The wait for all earlier kernels of the stream (and their memory).
