@@ -31,7 +31,12 @@ namespace {
 constexpr int kWalshCols = 32, kWalshRows = 8;  // pixels of a block's tile, a warp per row
 constexpr int kWalshThreads = kWalshCols * kWalshRows;
 constexpr int kWalshMaxHalf = 4;  // windows 1, 3, ..., 9
-constexpr int kWalshSquare = 12;  // power iterations from which R^4 is formed first
+constexpr int kWalshSquare = 12;  // power iterations left from which R^4 is formed first
+// ... where R v (v of unit length, R of trace 1/2 to 1) is at least 2^-6 long: then R^4 v is
+// at least 2^-24. A vector in the space of a small eigenvalue (coils that share no pixel of the window)
+// is taken to its fourth power, whose square is below FP32's range from 2e-6 of the trace
+// on; there R itself goes on.
+constexpr float kWalshSquareNorm = 0x1p-12f;  // its square
 
 // Hermitian C x C matrix: real diagonal, upper triangle row by row.
 template <int C>
@@ -119,7 +124,7 @@ __device__ __forceinline__ void normalise(float2* v) {
 // stays within range.  The sums across run over the window's columns with all 64 sums of a pixel
 // inside (a loop for each sum was 64 loops of code, and the kernel waited for the
 // instruction cache more than for anything else).  256 x 256 pixels, 8 coils: 57 us -> 34, with
-// the sums across so 24.
+// the sums across so 24.1, and 24.6 with the look at each product's length.
 template <int C>
 __global__ void __launch_bounds__(kWalshThreads, 2) k_walsh(const float2* __restrict__ in, float2* out, int rows, int cols,
                                                          int half, int iterations) {
@@ -223,39 +228,46 @@ __global__ void __launch_bounds__(kWalshThreads, 2) k_walsh(const float2* __rest
       for (int c = 0; c < C; ++c) big = fmaxf(big, fmaxf(fabsf(v[c].x), fabsf(v[c].y)));
       const float inv = 1.0f / big;
 #pragma unroll
-      for (int c = 0; c < C; ++c) u[c] = cscale(v[c], inv);
-      normalise<C>(u);
+      for (int c = 0; c < C; ++c) v[c] = cscale(v[c], inv);
+      normalise<C>(v);
     }
-    hermitian_apply<C>(R, u, v);
-    if (!(norm2<C>(v) > 0.0f)) {  // R takes it to nothing: the start vector stays
+    int left = iterations;
+    bool fourth = false;
+#pragma unroll 1
+    while (left > 0 && !fourth) {
+      hermitian_apply<C>(R, v, u);
+      float n = norm2<C>(u);
+      const bool fits = n >= kWalshSquareNorm;
+      if (n < 0x1p-100f) {  // squares may have underflowed
+#pragma unroll
+        for (int c = 0; c < C; ++c) u[c] = cscale(u[c], 0x1p100f);
+        n = norm2<C>(u);
+      }
+      if (!(n > 0.0f)) break;  // R takes it to nothing: it stays
+      const float inv = rsqrtf(n);
+#pragma unroll
+      for (int c = 0; c < C; ++c) v[c] = cscale(u[c], inv);
+      --left;
+      fourth = left >= kWalshSquare && (left & 3) == 0 && fits;
+    }
+    if (left == iterations) {  // (its first product: the start vector as it came)
       const bool some = norm2<C>(own) > 0.0f;
 #pragma unroll
       for (int c = 0; c < C; ++c) v[c] = some ? own[c] : make_float2(c == 0 ? 1.0f : 0.0f, 0.0f);
-    } else {
-      normalise<C>(v);
-      int left = iterations - 1;
-      const bool fourth = left >= kWalshSquare;
-      while (fourth ? (left & 3) != 0 : left > 0) {
+    }
+    if (fourth) {
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        Hermitian<C> s;
+        hermitian_square<C>(R, s);
+        R = s;
+      }
+#pragma unroll 1
+      for (; left > 0; left -= 4) {
         hermitian_apply<C>(R, v, u);
 #pragma unroll
         for (int c = 0; c < C; ++c) v[c] = u[c];
         normalise<C>(v);
-        --left;
-      }
-      if (fourth) {
-#pragma unroll 1
-        for (int k = 0; k < 2; ++k) {
-          Hermitian<C> s;
-          hermitian_square<C>(R, s);
-          R = s;
-        }
-#pragma unroll 1
-        for (; left > 0; left -= 4) {
-          hermitian_apply<C>(R, v, u);
-#pragma unroll
-          for (int c = 0; c < C; ++c) v[c] = u[c];
-          normalise<C>(v);
-        }
       }
     }
   }
