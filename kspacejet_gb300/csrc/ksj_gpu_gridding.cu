@@ -1267,23 +1267,21 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
         key = (lower == desc) ? max(key, other) : min(key, other);
       }
     }
-    // segments per rank and their exclusive prefix (from the key's length,
-    // capped at 2^22 entries: the same count, since kSegMin * kSegMax entries
-    // already take the most segments)
-    const int len = lane < a.nchunks ? (key >> 8) : 0;
-    const int unit = max(kSegMin, (__reduce_add_sync(0xffffffffu, len) + 32 - 1) / 32);
-    const int nseg = lane < a.nchunks ? list_segments(len, unit) : 0;
+    const int chunk = key & 31;
+    start = __shfl_sync(0xffffffffu, start, chunk);
+    length = __shfl_sync(0xffffffffu, length, chunk);
+    // segments per rank and their exclusive prefix (the key's length is capped for the
+    // order alone)
+    const int n = lane < a.nchunks ? static_cast<int>(length) : 0;
+    const int unit = max(kSegMin, (__reduce_add_sync(0xffffffffu, n) + 32 - 1) / 32);
+    const int nseg = lane < a.nchunks ? list_segments(n, unit) : 0;
     int incl = nseg;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += v;
     }
-    const int chunk = key & 31;
-    start = __shfl_sync(0xffffffffu, start, chunk);
-    length = __shfl_sync(0xffffffffu, length, chunk);
     if (lane < a.nchunks) {
-      const int n = static_cast<int>(length);
       task_list[lane] = make_int4(static_cast<int>(start), n, segment_length(n, unit), chunk);
       task_base[lane] = incl - nseg;
     }
