@@ -263,9 +263,9 @@ KSJ_GPU_API ksj_gpu_status ksj_gpu_gridding3_adjoint(const ksj_gpu_gridding3_des
  *   d_dcf  [frame][sample] float32 out: the final weights, usable as
  *          KSJ_GPU_DCF_EXTERNAL for the same gridding
  * Workspace: ksj_gpu_pipe_menon_workspace_bytes (0 on a bad desc).  Most of it
- * are the lists' entries, 2 W (16 + 8 W) bytes a sample; frames are taken in
- * passes of at most 4 GB of them (and of grids), one frame as a whole (10 M
- * samples of width 4: 3.8 GB). */
+ * are the lists' entries, 2 W (16 + 8 W) bytes a sample (3 W where g mod 16 is 1
+ * to W - 2: a stencil may then reach three 16-column chunks); frames are taken in passes of at
+ * most 4 GB of them (and of grids), one frame as a whole (10 M samples of width 4: 3.8 GB). */
 KSJ_GPU_API size_t ksj_gpu_pipe_menon_workspace_bytes(const ksj_gpu_gridding_desc* desc);
 KSJ_GPU_API ksj_gpu_status ksj_gpu_pipe_menon_dcf(const ksj_gpu_gridding_desc* desc, uint32_t iterations,
                                                   const float* d_traj, float* d_dcf, void* d_workspace,

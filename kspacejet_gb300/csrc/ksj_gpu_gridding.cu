@@ -36,7 +36,8 @@
 //
 // Binning lists are (frame, grid row, 16-column chunk); a sample is listed
 // once per row its stencil covers and per chunk its W columns fall into
-// (one or two).  The "reference permutation" a list must equal is the
+// (one or two; three where the last chunk of a row is narrower than a stencil's inner
+// columns, which then reach over it into the first).  The "reference permutation" a list must equal is the
 // increasing sequence of sample indices whose stencil touches that row and
 // chunk, with the lower tap index floor(k N / 2 pi) of the exact coordinate
 // (the value the reference's double-precision grid_coordinate computes,
@@ -141,8 +142,10 @@ struct Shape {
   int rows, cols;          // image
   int grid_rows, grid_cols;
   int width;
-  int nchunks;             // ceil(grid_cols / 32)
+  int nchunks;             // ceil(grid_cols / kChunk)
   int lists_per_frame;     // grid_rows * nchunks
+  int lists_per_row;       // most chunks a stencil's columns fall into: 2, or 3 (see list_chunks)
+  int first_of_two;        // 1: two chunks, and the first may see both ends of a stencil that wraps
   size_t entries_per_frame;
   int out_rows, out_cols;  // kept image region
   int col_group;           // coils per column-pass tile: a power of two >= 2, <= 32
@@ -227,7 +230,13 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
   s->width = static_cast<int>(d->kernel_width);
   s->nchunks = (s->grid_cols + kChunk - 1) / kChunk;
   s->lists_per_frame = s->grid_rows * s->nchunks;
-  s->entries_per_frame = static_cast<size_t>(s->samples) * s->width * 2;
+  {
+    const int tail = s->grid_cols % kChunk;  // columns of a narrower last chunk
+    const bool over = s->nchunks > 1 && tail != 0 && tail < s->width - 1;
+    s->lists_per_row = over ? 3 : 2;
+    s->first_of_two = over && s->nchunks == 2 ? 1 : 0;
+  }
+  s->entries_per_frame = static_cast<size_t>(s->samples) * s->width * s->lists_per_row;
   {
     // Samples per block of the binning, in turns of kBinThreads: the time is about
     // the turns an SM gets, with the loading of the list positions (one turn per
@@ -463,52 +472,71 @@ struct PrepareArgs {
   float phase_row, phase_col, phase_sign;
 };
 
-template <int W>
-__device__ __forceinline__ void list_chunks(int c0, int grid_cols, int* k0, int* k1) {
-  const int last = c0 + W - 1 >= grid_cols ? c0 + W - 1 - grid_cols : c0 + W - 1;
-  *k0 = c0 / kChunk;
-  *k1 = last / kChunk;
+// The chunks that the columns c0 .. c0 + W - 1 (wrapped) fall into: those of the first and the
+// last (k[1] = k[0] where it is the same) and, for kLists 3, the row's last chunk where the columns
+// begin before it, cover it and go on at column 0 (else k[2] = -1).
+template <int W, int kLists>
+__device__ __forceinline__ void list_chunks(int c0, int grid_cols, int (&k)[kLists]) {
+  const bool wraps = c0 + W - 1 >= grid_cols;
+  const int last = wraps ? c0 + W - 1 - grid_cols : c0 + W - 1;
+  k[0] = c0 / kChunk;
+  k[1] = last / kChunk;
+  if constexpr (kLists == 3) {
+    const int tail = (grid_cols - 1) / kChunk;
+    k[2] = wraps && k[0] != tail ? tail : -1;
+  }
+}
+
+// Whether k[h] names a list that no earlier one of k does.
+template <int kLists>
+__device__ __forceinline__ bool own_list(const int (&k)[kLists], int h) {
+  return h == 0 || (h == 1 ? k[1] != k[0] : k[h] >= 0);
 }
 
 // A warp's samples, one per lane: how many lanes below this one join each of this
-// lane's lists (rows r0 + j wrapped, chunks k0 and k1), and whether one above does.
-// Byte j of below[h] is the count for (row r0 + j, chunk k0 or k1); bit j of
+// lane's lists (rows r0 + j wrapped, chunks k), and whether one above does.
+// Byte j of below[h] is the count for (row r0 + j, chunk k[h]); bit j of
 // above[h].  r0 < 0: no sample.  Every lane's rows and chunks go round the warp once.
-template <int W>
+template <int W, int kLists>
 struct WarpRanks {
   static constexpr int kWords = (W + 3) / 4;
-  uint32_t below[2][kWords], above[2];
+  uint32_t below[kLists][kWords], above[kLists];
 };
 
-template <int W>
-__device__ __forceinline__ WarpRanks<W> warp_ranks(int r0, int k0, int k1, int grid_rows) {
+template <int W, int kLists>
+__device__ __forceinline__ WarpRanks<W, kLists> warp_ranks(int r0, const int (&k)[kLists], int grid_rows) {
   constexpr uint32_t kRows = (1u << W) - 1u;
-  WarpRanks<W> out;
+  constexpr int kWords = WarpRanks<W, kLists>::kWords;
+  WarpRanks<W, kLists> out;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < kLists; ++h) {
     out.above[h] = 0;
 #pragma unroll
-    for (int q = 0; q < WarpRanks<W>::kWords; ++q) out.below[h][q] = 0;
+    for (int q = 0; q < kWords; ++q) out.below[h][q] = 0;
   }
   const int lane = threadIdx.x & 31;
-  // row, chunk, chunk (63, 63: no sample)
-  const uint32_t mine = r0 < 0 ? 0xfffu : static_cast<uint32_t>(r0) << 12 | static_cast<uint32_t>(k0) << 6 | static_cast<uint32_t>(k1);
+  // row, then the chunks (63: none)
+  uint32_t mine = r0 < 0 ? 0u : static_cast<uint32_t>(r0);
+#pragma unroll
+  for (int h = 0; h < kLists; ++h) mine = mine << 6 | (r0 < 0 ? 63u : static_cast<uint32_t>(k[h]) & 63u);
 #pragma unroll 4
   for (int i = 0; i < 32; ++i) {
     const uint32_t other = __shfl_sync(0xffffffffu, mine, i);
     // this lane's rows that the other sample's stencil covers: its rows start
     // d before ours, or (across the wrap) grid_rows - d after
-    int d = r0 - static_cast<int>(other >> 12);
+    int d = r0 - static_cast<int>(other >> (6 * kLists));
     if (d < 0) d += grid_rows;
     const uint32_t rows = (kRows >> min(d, 31)) | ((kRows << min(grid_rows - d, 31)) & kRows);
-    const uint32_t o0 = (other >> 6) & 63u, o1 = other & 63u;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t k = static_cast<uint32_t>(h ? k1 : k0);
-      const uint32_t m = k == o0 || k == o1 ? rows : 0u;
+    for (int h = 0; h < kLists; ++h) {
+      const uint32_t own = static_cast<uint32_t>(k[h]);
+      bool same = false;
+#pragma unroll
+      for (int o = 0; o < kLists; ++o) same = same || own == ((other >> (6 * o)) & 63u);
+      const uint32_t m = same ? rows : 0u;
       if (i < lane) {
 #pragma unroll
-        for (int q = 0; q < WarpRanks<W>::kWords; ++q)  // bit j of a nibble to byte j
+        for (int q = 0; q < kWords; ++q)  // bit j of a nibble to byte j
           out.below[h][q] += (((m >> (4 * q)) & 15u) * 0x00204081u) & 0x01010101u;
       } else if (i > lane) {
         out.above[h] |= m;
@@ -519,20 +547,20 @@ __device__ __forceinline__ WarpRanks<W> warp_ranks(int r0, int k0, int k1, int g
 }
 
 // Places of one sample per thread in the lists of rows r0 .. r0 + W - 1
-// (wrapped) and chunks k0 and k1 (r0 < 0: no sample), in thread order: a list's
+// (wrapped) and chunks k (r0 < 0: no sample), in thread order: a list's
 // entries have to stand in sample order.  at: running position of each list.  The
 // ranks within the warps are found first, by all warps at once; then the warps take
 // turns, passed on by named barriers: each reads its lists' positions, adds the ranks,
 // and the last lane of a list moves its position on.  Called by the whole block;
 // synchronises it first.
-template <int W>
-__device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1, int nchunks, int grid_rows,
-                                           uint32_t (&pos)[W][2]) {
+template <int W, int kLists>
+__device__ __forceinline__ void place_turn(uint32_t* at, int r0, const int (&k)[kLists], int nchunks, int grid_rows,
+                                           uint32_t (&pos)[W][kLists]) {
   const int warp = threadIdx.x >> 5;
-  const WarpRanks<W> ranks = warp_ranks<W>(r0, k0, k1, grid_rows);
-  int first[2];  // list of row r0 and each chunk, -1: none
-  first[0] = r0 >= 0 ? r0 * nchunks + k0 : -1;
-  first[1] = r0 >= 0 && k1 != k0 ? r0 * nchunks + k1 : -1;
+  const WarpRanks<W, kLists> ranks = warp_ranks<W>(r0, k, grid_rows);
+  int first[kLists];  // list of row r0 and each chunk, -1: none
+#pragma unroll
+  for (int h = 0; h < kLists; ++h) first[h] = r0 >= 0 && own_list(k, h) ? r0 * nchunks + k[h] : -1;
   const int wrap = grid_rows - r0;  // rows from here on wrap
   auto list_of = [&](int j, int h) { return first[h] + (j >= wrap ? j - grid_rows : j) * nchunks; };
   __syncthreads();  // the positions are loaded, and every warp's last turn is over
@@ -540,13 +568,13 @@ __device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1,
 #pragma unroll
   for (int j = 0; j < W; ++j)
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < kLists; ++h)
       if (first[h] >= 0) pos[j][h] = at[list_of(j, h)];
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < W; ++j) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    for (int h = 0; h < kLists; ++h) {
       if (first[h] >= 0) {
         pos[j][h] += (ranks.below[h][j / 4] >> (8 * (j & 3))) & 255u;
         if (!((ranks.above[h] >> j) & 1u)) at[list_of(j, h)] = pos[j][h] + 1;
@@ -558,19 +586,21 @@ __device__ __forceinline__ void place_turn(uint32_t* at, int r0, int k0, int k1,
 }
 
 // One sample counted in its lists (shared memory).
-template <int W>
-__device__ __forceinline__ void count_lists(uint32_t* counts, int r0, int k0, int k1, int nchunks, int grid_rows) {
+template <int W, int kLists>
+__device__ __forceinline__ void count_lists(uint32_t* counts, int r0, const int (&k)[kLists], int nchunks,
+                                            int grid_rows) {
 #pragma unroll
   for (int j = 0; j < W; ++j) {
     int row = r0 + j;
     if (row >= grid_rows) row -= grid_rows;
-    atomicAdd(counts + row * nchunks + k0, 1u);
-    if (k1 != k0) atomicAdd(counts + row * nchunks + k1, 1u);
+#pragma unroll
+    for (int h = 0; h < kLists; ++h)
+      if (own_list(k, h)) atomicAdd(counts + row * nchunks + k[h], 1u);
   }
 }
 
 // One sample's record, and its entries counted in `counts` (shared memory, per list).
-template <int W>
+template <int W, int kLists>
 __device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int sample, uint32_t* counts) {
   const size_t idx = static_cast<size_t>(f) * a.samples + sample;
   if (a.frame_samples != nullptr && static_cast<uint32_t>(sample) >= __ldg(a.frame_samples + f)) {
@@ -646,15 +676,15 @@ __device__ __forceinline__ void prepare_sample(const PrepareArgs& a, int f, int 
     rec.scale = cscale(e, w);
   }
   reinterpret_cast<SampleRecord<W>*>(a.records)[idx] = rec;
-  int k0, k1;
-  list_chunks<W>(rec.c0, a.grid_cols, &k0, &k1);
-  count_lists<W>(counts, rec.r0, k0, k1, a.nchunks, a.grid_rows);
+  int chunks[kLists];
+  list_chunks<W>(rec.c0, a.grid_cols, chunks);
+  count_lists<W>(counts, rec.r0, chunks, a.nchunks, a.grid_rows);
 }
 
 // One block per (block of samples, frame).  The counts go to shared memory: as atomics on
 // global memory the samples of a radial scan's centre, all in the same few
 // lists, were serialised (25 us for 205824 samples on a 512 grid, this 17).
-template <int W>
+template <int W, int kLists>
 __global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
   extern __shared__ uint32_t prepare_counts[];
   chain_begin();
@@ -663,7 +693,7 @@ __global__ void __launch_bounds__(kBinThreads) k_prepare(PrepareArgs a) {
   __syncthreads();
   const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
   for (int sample = s0 + threadIdx.x; sample < s1; sample += kBinThreads)
-    prepare_sample<W>(a, f, sample, prepare_counts);
+    prepare_sample<W, kLists>(a, f, sample, prepare_counts);
   __syncthreads();
   uint32_t* out = a.counts + (static_cast<size_t>(f) * gridDim.x + blockIdx.x) * a.lists_per_frame;
   for (int l = threadIdx.x; l < a.lists_per_frame; l += kBinThreads) out[l] = prepare_counts[l];
@@ -955,7 +985,7 @@ struct PlaceArgs {
 // slice, 92 us of 205824 samples on a 512 grid, 219 us of 96 frames of 13056
 // samples) where this and k_bin_prefix take 21, 60 and 144.  (Finding the ranks inside the
 // turns, by lane masks per list in shared memory, took 203 of the 144.)
-template <int W, bool kPm>
+template <int W, bool kPm, int kLists>
 __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
   extern __shared__ uint32_t place_smem[];
   chain_begin();
@@ -980,20 +1010,20 @@ __global__ void __launch_bounds__(kBinThreads) k_place(PlaceArgs a) {
     const float* w = reinterpret_cast<const float*>(q);
     const int r0 = sample < s1 ? __float_as_int(w[0]) : -1;  // -1: also a padding sample of a ragged batch
     const int c0 = r0 >= 0 ? __float_as_int(w[1]) : 0;
-    int k0, k1;
-    list_chunks<W>(c0, a.grid_cols, &k0, &k1);
-    uint32_t pos[W][2];
-    place_turn<W>(at, r0, k0, k1, a.nchunks, a.grid_rows, pos);
+    int chunks[kLists];
+    list_chunks<W>(c0, a.grid_cols, chunks);
+    uint32_t pos[W][kLists];
+    place_turn<W>(at, r0, chunks, a.nchunks, a.grid_rows, pos);
     if (r0 < 0) continue;
     PmRecord<W> pm;
     if constexpr (kPm) pm = static_cast<const PmRecord<W>*>(a.pm)[static_cast<size_t>(f) * a.samples + sample];
 #pragma unroll
     for (int j = 0; j < W; ++j) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h && k1 == k0) continue;
+      for (int h = 0; h < kLists; ++h) {
+        if (!own_list(chunks, h)) continue;
         const size_t slot = static_cast<size_t>(f) * a.entries_per_frame + pos[j][h];
-        const int col_lo = (h ? k1 : k0) * kChunk;
+        const int col_lo = chunks[h] * kChunk;
         if constexpr (kPm) {
           // the taps of the double-precision coordinate, on the list's row and chunk
           int dr = (r0 + j >= a.grid_rows ? r0 + j - a.grid_rows : r0 + j) - pm.r0;
@@ -1033,6 +1063,7 @@ struct RowsArgs {
   int both_ends;  // block x takes rows in from both ends
   int out_cols, cpitch;
   int col_shift;  // kept column of frequency k: (k + col_shift) mod grid_cols, when below out_cols
+  int first_of_two;  // as in Shape
   uint32_t wait_limit;   // polls before a segment wait gives up
   int wait_beyond;       // added to every segment wait's target: 0, or unreachable in the wait-fault test mode
   DifPlan plan;
@@ -1066,8 +1097,8 @@ __device__ __forceinline__ int segment_length(int n, int unit) {
 // lanes, this one is `gl`): slot i gets entry i's weights spread over the
 // chunk's 16 columns, so that the lanes that apply them need no column
 // arithmetic and no branch per tap, and lane groups on different lists run in
-// step.  Slots from cnt on get no weights.  wrap: the grid's one chunk sees both
-// ends of a wrapped stencil (its length, else 0).  Returns this lane's share of the
+// step.  Slots from cnt on get no weights.  wrap: the row's length where
+// its first chunk may see both ends of a wrapped stencil, else 0.  Returns this lane's share of the
 // halves its slots touch: bit 2 i the low, 2 i + 1 the high half of slot i.
 __device__ __forceinline__ uint32_t stage_entries(int w, float* slots, const unsigned char* ent, int cnt, int gl,
                                                   int lanes, int wrap) {
@@ -1300,7 +1331,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
                    static_cast<size_t>(warp * groups + g) * kRowsBatch * kSlotFloats;
     const int ntasks = task_base[a.nchunks] << lg_parts;
     const bool segmented_row = task_base[a.nchunks] != a.nchunks;
-    const int wrap = a.nchunks == 1 ? a.grid_cols : 0;
+    const int wrap = a.nchunks == 1 || a.first_of_two ? a.grid_cols : 0;
     const float2* samples = a.samples_t + static_cast<size_t>(f) * a.sample_frame_stride;
     const unsigned char* ents = a.expanded + static_cast<size_t>(f) * a.entries_per_frame * entry_bytes(a.width);
     for (;;) {
@@ -1973,8 +2004,15 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
                            const CoilLastArgs* coil_last = nullptr) {
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
-  const auto place = pm ? k_place<W, true> : k_place<W, false>;
-  KSJ_TRY(allow_smem(k_prepare<W>, count_smem, kListSmem));
+  auto prepare = k_prepare<W, 2>;
+  auto place = pm ? k_place<W, true, 2> : k_place<W, false, 2>;
+  if constexpr (W > 2) {
+    if (s.lists_per_row == 3) {
+      prepare = k_prepare<W, 3>;
+      place = pm ? k_place<W, true, 3> : k_place<W, false, 3>;
+    }
+  }
+  KSJ_TRY(allow_smem(prepare, count_smem, kListSmem));
   KSJ_TRY(allow_smem(place, place_smem, kListSmem));
   const dim3 blocks(s.bin_blocks, s.frames);
   {
@@ -2004,7 +2042,7 @@ ksj_gpu_status build_lists(const Shape& s, const ksj_gpu_gridding_desc* d, const
     p.phase_col = s.phase_col;
     p.phase_sign = s.phase_sign;
     LaunchScope scope("k_prepare", stream);
-    KSJ_TRY(launch_chained(k_prepare<W>, blocks, kBinThreads, count_smem, stream, p));
+    KSJ_TRY(launch_chained(prepare, blocks, kBinThreads, count_smem, stream, p));
   }
   {
     LaunchScope scope("k_bin_prefix", stream);
@@ -2115,6 +2153,7 @@ ksj_gpu_status launch_all(const Shape& s, const Layout& l, const ksj_gpu_griddin
   r.cpitch = s.cpitch;
   r.plan = s.plan_cols;
   r.col_shift = s.kb ? s.out_cols / 2 : 0;
+  r.first_of_two = s.first_of_two;
   RowsLauncher rows_launch;
   if (!rows_launch.setup(s)) return KSJ_GPU_ERROR_CUDA;
 
@@ -2472,7 +2511,7 @@ __global__ void __launch_bounds__(kPmThreads, W <= 4 ? 4 : 2) k_pm_grid(const ui
                                                         const uint32_t* order, const uint32_t* bins, const double* w,
                                                         double* grid, size_t lists, int samples, int grid_rows,
                                                         int grid_cols, int nchunks, int lists_per_frame,
-                                                        size_t entries_per_frame) {
+                                                        size_t entries_per_frame, int first_of_two) {
   __shared__ double cells[kPmThreads * kPmPitch];
   __shared__ uint32_t many_shared;
   chain_begin();
@@ -2507,7 +2546,8 @@ __global__ void __launch_bounds__(kPmThreads, W <= 4 ? 4 : 2) k_pm_grid(const ui
     const uint32_t* off = offsets + static_cast<size_t>(f) * (lists_per_frame + 1);
     const PmEntry<W>* ent = entries + static_cast<size_t>(f) * entries_per_frame;
     const double* wf = w + static_cast<size_t>(f) * samples;
-    const int wrap = nchunks == 1 ? grid_cols : 0;  // one chunk sees both ends of a wrapped stencil
+    // one chunk, or the first of two, may see both ends of a wrapped stencil
+    const int wrap = nchunks == 1 || first_of_two ? grid_cols : 0;
     const uint32_t end = off[l + 1], step = split ? kPmLanes : 1;
     auto load = [&](uint32_t e) {
       PmEntry<W> r;
@@ -2603,7 +2643,7 @@ struct PmLayout {
 };
 
 // Frames are independent, so a call takes them in passes through one workspace: as many at
-// once as keep their entries (48 bytes for a width of 4, up to 2 W of them a sample) and
+// once as keep their entries (48 bytes for a width of 4, up to 2 or 3 W of them a sample) and
 // their grids within kPmPassBytes each, and at least one.
 constexpr size_t kPmPassBytes = size_t{4} << 30;
 
@@ -2696,7 +2736,8 @@ ksj_gpu_status launch_pipe_menon(const Shape& s, const PmLayout& l, const ksj_gp
                      dim3(kPmThreads), 0, stream,
           offsets, reinterpret_cast<const PmEntry<W>*>(ws + l.entries), static_cast<const uint32_t*>(order),
                      static_cast<const uint32_t*>(bins), static_cast<const double*>(w), grid, lists, s.samples,
-          s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame));
+          s.grid_rows, s.grid_cols, s.nchunks, s.lists_per_frame, s.entries_per_frame,
+                     s.first_of_two));
     }
     LaunchScope scope("k_pm_update", stream);
     KSJ_TRY(launch_chained(k_pm_update<W>, dim3(static_cast<unsigned>((fm + 255) / 256)), dim3(256), 0, stream,
@@ -2794,7 +2835,8 @@ __global__ void __launch_bounds__(kBinThreads) k_prepare3(Prepare3Args a) {
   const int s0 = blockIdx.x * a.bin_span, s1 = min(s0 + a.bin_span, a.samples);
   for (int base = s0; base < s1; base += kBinThreads) {
     const int sample = base + threadIdx.x;
-    if (sample < s1) count_lists<W>(counts, prepare_sample3<W>(a, sample), 0, 0, 1, a.grid);
+    const int one[2] = {0, 0};  // a plane is a row of one list
+    if (sample < s1) count_lists<W>(counts, prepare_sample3<W>(a, sample), one, 1, a.grid);
   }
   __syncthreads();
   for (int p = threadIdx.x; p < a.grid; p += kBinThreads) a.counts[blockIdx.x * a.grid + p] = counts[p];
@@ -2812,8 +2854,9 @@ __global__ void __launch_bounds__(kBinThreads) k_plane_place(const unsigned char
   for (int base = s0; base < s1; base += kBinThreads) {
     const int sample = base + threadIdx.x;
     const int z0 = sample < s1 ? reinterpret_cast<const SampleRecord3<W>*>(records)[sample].z0 : -1;
+    const int one[2] = {0, 0};
     uint32_t pos[W][2];
-    place_turn<W>(at, z0, 0, 0, 1, grid, pos);
+    place_turn<W>(at, z0, one, 1, grid, pos);
     if (z0 < 0) continue;
 #pragma unroll
     for (int j = 0; j < W; ++j) plane_samples[pos[j][0]] = static_cast<uint32_t>(sample);
@@ -2831,7 +2874,7 @@ __device__ __forceinline__ void plane_span(const uint32_t* plane_offsets, int p,
 }
 
 // One block per (block of a plane's samples, plane): their counts per list.
-template <int W>
+template <int W, int kLists>
 __global__ void __launch_bounds__(kBinThreads) k_count3(const unsigned char* records, const uint32_t* plane_offsets,
                                                         const uint32_t* plane_samples, uint32_t* counts, int grid,
                                                         int nchunks, int lists_per_plane) {
@@ -2849,9 +2892,9 @@ __global__ void __launch_bounds__(kBinThreads) k_count3(const unsigned char* rec
       r0 = first.y;
       c0 = first.z;
     }
-    int k0, k1;
-    list_chunks<W>(c0, grid, &k0, &k1);
-    if (r0 >= 0) count_lists<W>(list_counts, r0, k0, k1, nchunks, grid);
+    int chunks[kLists];
+    list_chunks<W>(c0, grid, chunks);
+    if (r0 >= 0) count_lists<W>(list_counts, r0, chunks, nchunks, grid);
   }
   __syncthreads();
   uint32_t* out = counts + (static_cast<size_t>(blockIdx.y) * kPlaneBlocks + blockIdx.x) * lists_per_plane;
@@ -2870,7 +2913,7 @@ struct Place3Args {
 };
 
 // One block per (block of a plane's samples, plane): the entries of its lists.
-template <int W>
+template <int W, int kLists>
 __global__ void __launch_bounds__(kBinThreads) k_place3(Place3Args a) {
   extern __shared__ uint32_t place_smem[];
   uint32_t* at = place_smem;
@@ -2897,10 +2940,10 @@ __global__ void __launch_bounds__(kBinThreads) k_place3(Place3Args a) {
     }
     const float* w = reinterpret_cast<const float*>(q);
     const int r0 = i < i1 ? __float_as_int(w[1]) : -1, c0 = i < i1 ? __float_as_int(w[2]) : 0;
-    int k0, k1;
-    list_chunks<W>(c0, a.grid, &k0, &k1);
-    uint32_t pos[W][2];
-    place_turn<W>(at, r0, k0, k1, a.nchunks, a.grid, pos);
+    int chunks[kLists];
+    list_chunks<W>(c0, a.grid, chunks);
+    uint32_t pos[W][kLists];
+    place_turn<W>(at, r0, chunks, a.nchunks, a.grid, pos);
     if (r0 < 0) continue;
     int tz = plane - __float_as_int(w[0]);
     if (tz < 0) tz += a.grid;
@@ -2911,10 +2954,10 @@ __global__ void __launch_bounds__(kBinThreads) k_place3(Place3Args a) {
 #pragma unroll
     for (int j = 0; j < W; ++j) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h && k1 == k0) continue;
+      for (int h = 0; h < kLists; ++h) {
+        if (!own_list(chunks, h)) continue;
         if (a.expanded != nullptr)
-          put_entry<W>(sample, c0, w[6 + W + j] * wz, w + 6 + 2 * W, (h ? k1 : k0) * kChunk, a.grid,
+          put_entry<W>(sample, c0, w[6 + W + j] * wz, w + 6 + 2 * W, chunks[h] * kChunk, a.grid,
                        a.expanded + static_cast<size_t>(pos[j][h]) * entry_bytes(W));
         else
           a.entries[pos[j][h]] = sample;
@@ -3004,7 +3047,7 @@ Layout3 make_layout3(const Shape& s) {
     return at;
   };
   const size_t g = static_cast<size_t>(s.grid_rows), n = static_cast<size_t>(s.rows);
-  l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
+  l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * s.lists_per_row;
   l.flags = take(kFlagBytes);
   l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
   l.lists = take_lists3(s, take);
@@ -3064,8 +3107,16 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
   auto at = [&](size_t offset) { return reinterpret_cast<uint32_t*>(ws + offset); };
   const int count_smem = s.lists_per_frame * 4;
   const int place_smem = s.lists_per_frame * static_cast<int>(kPlaceListBytes);
-  KSJ_TRY(allow_smem(k_count3<W>, count_smem, kListSmem));
-  KSJ_TRY(allow_smem(k_place3<W>, place_smem, kListSmem));
+  auto count = k_count3<W, 2>;
+  auto place = k_place3<W, 2>;
+  if constexpr (W > 2) {
+    if (s.lists_per_row == 3) {
+      count = k_count3<W, 3>;
+      place = k_place3<W, 3>;
+    }
+  }
+  KSJ_TRY(allow_smem(count, count_smem, kListSmem));
+  KSJ_TRY(allow_smem(place, place_smem, kListSmem));
   {
     Prepare3Args p{};
     p.traj = d_traj;
@@ -3099,7 +3150,7 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
   const dim3 blocks(kPlaneBlocks, g);
   {
     LaunchScope scope("k_count3", stream);
-    k_count3<W><<<blocks, kBinThreads, count_smem, stream>>>(records, at(l.plane_offsets), at(l.plane_samples),
+    count<<<blocks, kBinThreads, count_smem, stream>>>(records, at(l.plane_offsets), at(l.plane_samples),
                                                             at(l.counts), g, s.nchunks, s.lists_per_frame);
     KSJ_TRY(check_launch());
   }
@@ -3122,7 +3173,7 @@ ksj_gpu_status build_lists3(const Shape& s, uint32_t dcf_mode, const float* d_tr
     const Place3Args p{records, at(l.plane_offsets), at(l.plane_samples), at(l.offsets), at(l.counts), expanded, entries,
                        g, s.nchunks, s.lists_per_frame};
     LaunchScope scope("k_place3", stream);
-    k_place3<W><<<blocks, kBinThreads, place_smem, stream>>>(p);
+    place<<<blocks, kBinThreads, place_smem, stream>>>(p);
     KSJ_TRY(check_launch());
   }
   return KSJ_GPU_OK;
@@ -3206,6 +3257,7 @@ ksj_gpu_status launch_all3(const Shape& s, const Layout3& l, const ksj_gpu_gridd
   r.cpitch = s.cpitch;
   r.plan = s.plan_cols;
   r.col_shift = n / 2;
+  r.first_of_two = s.first_of_two;
   RowsLauncher rows_launch;
   if (!rows_launch.setup(s)) return KSJ_GPU_ERROR_CUDA;
   // columns of every plane (y transformed, cropped, y/x deapodised): [plane][pixel][cpitch]
@@ -3596,7 +3648,7 @@ PmLayout3 make_pm_layout3(const Shape& s) {
     return at;
   };
   const size_t g = static_cast<size_t>(s.grid_rows);
-  l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * 2;
+  l.entries_total = static_cast<size_t>(s.samples) * s.width * s.width * s.lists_per_row;
   l.max_long = l.entries_total / (kPmLong + 1) + 2;
   l.flags = take(kFlagBytes);
   l.records = take(static_cast<size_t>(s.samples) * record3_bytes(s.width));
