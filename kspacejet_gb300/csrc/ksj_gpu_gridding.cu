@@ -1069,24 +1069,36 @@ struct RowsArgs {
   DifPlan plan;
 };
 
-// Lists longer than a row's unit are gridded in segments (at most
-// kSegMax, all but the last of segment_length entries) that different lane
+// Lists longer than a row's unit are gridded in segments (all but the last of
+// segment_length entries) that different lane
 // groups take at once, so that a row's long lists do not hold its CTA at the
 // barrier after the gridding while one warp works through each; a cell is then
 // the sum, in segment order, of its segments' partial sums, each partial sum
 // in sample order from zero.  Shorter lists are one segment: the cell is its
 // samples' sum in sample order.  The unit is kSegMin entries, or a 32nd of the
 // row's where that is more (a row with that many has lists enough to share out,
-// and every segment pays for putting its 16 cells in turn): it depends on the
+// and every segment pays for putting its 16 cells in turn), up to kSegMost, beyond
+// which it is kSegFull: it depends on the
 // lists alone, so every coil grouping gives the same cells.  Units of 32, 64, 128 entries
 // and this rule measured, us of the row pass: 8 coils on a 128 grid 35, 29, 33,
 // 28, on a 512 grid 131, 107, 99, 95; a 32-coil frame 35, 31, 37, 32.
+// The upper bound keeps the sums short where rows are crowded (the centre of a
+// kooshball: rows of 3e5 entries, lists of half of them).  Without it (32 to 17 segments of up to
+// 9000 entries) the images of 2 M samples on a 48^3 grid were 2.9e-6 from double precision,
+// with it 1.0e-6 (units of a 32nd of the list 1.3e-6).  Many even segments also share out better: row
+// pass of 10.2 M samples x 20 coils on 384^3 19.3 ms without the bound, 19.0 with it (plain bounds
+// of 128, 256, 512, 1024: 19.5, 19.3, 19.2, 19.2).  Rows between the two (the 512 grid's centre has
+// units of 281) keep their 32nd: at 256 they would be a few tasks more than the block takes
+// at once (82 -> 90 us).
 constexpr int kSegMin = 64;
-constexpr int kSegMax = 32;
+constexpr int kSegMost = 512;
+constexpr int kSegFull = 256;
 
-__device__ __forceinline__ int list_segments(int n, int unit) {
-  return n <= unit ? 1 : min((n + unit - 1) / unit, kSegMax);
+__device__ __forceinline__ int segment_unit(int row_entries) {
+  const int unit = max(kSegMin, (row_entries + 32 - 1) / 32);
+  return unit <= kSegMost ? unit : kSegFull;
 }
+__device__ __forceinline__ int list_segments(int n, int unit) { return n <= unit ? 1 : (n + unit - 1) / unit; }
 __device__ __forceinline__ int segment_length(int n, int unit) {
   if (n <= unit) return n;  // one segment (most lists): no division
   const int sg = list_segments(n, unit);
@@ -1304,7 +1316,7 @@ __global__ void __launch_bounds__(kRowsThreads, 2) k_rows(RowsArgs a) {
     // segments per rank and their exclusive prefix (the key's length is capped for the
     // order alone)
     const int n = lane < a.nchunks ? static_cast<int>(length) : 0;
-    const int unit = max(kSegMin, (__reduce_add_sync(0xffffffffu, n) + 32 - 1) / 32);
+    const int unit = segment_unit(__reduce_add_sync(0xffffffffu, n));
     const int nseg = lane < a.nchunks ? list_segments(n, unit) : 0;
     int incl = nseg;
 #pragma unroll
