@@ -354,7 +354,7 @@ constexpr int kCovStages = 2;
 constexpr uint32_t kCovStageBytes = kCovRows * kCovKTile * 2;
 constexpr int kCovThreads = 256;
 constexpr uint32_t kCovWaitLimit = 1u << 22;
-constexpr int kCovMaxBlocks = 304;  // two per SM
+constexpr int kCovMaxBlocks = 2 * kSms;
 
 // Four consecutive samples of one coil per thread and turn, two turns per tile
 // (32 coils x 64 samples): eight 8-byte loads in flight, one 8-byte store per

@@ -130,7 +130,6 @@ constexpr int kBinWarps = kBinThreads / 32;
 constexpr size_t kPlaceListBytes = 4;  // of k_place: the list's running position
 constexpr size_t kListSmem = kMaxGrid * (kMaxGrid / kChunk) * 4;  // a word of every list of the largest grid
 constexpr size_t kRowsSmem = 200 * 1024;                          // of a k_rows block, at most
-constexpr int kSms = 152;              // of a GB300
 // A call keeps one count per list for each of its blocks: at most this many (64 MB), or one
 // block a frame where that is more.
 constexpr size_t kBinCounts = size_t{1} << 24;
@@ -828,7 +827,7 @@ __global__ void __launch_bounds__(256) k_samples_coil_last(CoilLastArgs a) {
 constexpr int kScanPer = kMaxGrid * (kMaxGrid / kChunk) / 1024;  // counts per thread, at most
 constexpr int kTablesPerBlock = 64;
 constexpr int kCoilLastTiles = 1024 / 256;  // tiles of a block, of consecutive samples
-constexpr int kScanSampleBlocks = 144;      // with a few for the tables, one round of the SMs
+constexpr int kScanSampleBlocks = kSms - 8;  // with a few for the tables, one round of the SMs
 struct ScanSamples {
   CoilLastArgs a;
   int first_block;  // of the launch
@@ -1853,7 +1852,7 @@ struct RowsLauncher {
   // scans crowd, is at row 0, and the rows before it, at the end, should not be the
   // last to start (a 32-coil frame 72 -> 65 us; 48 frames, 61 waves, 1 % slower).
   ksj_gpu_status launch(RowsArgs r, int grid_rows, int groups, int nf, cudaStream_t stream) const {
-    r.both_ends = static_cast<long long>(grid_rows) * groups * nf <= 16 * 304;
+    r.both_ends = static_cast<long long>(grid_rows) * groups * nf <= 16 * 2 * kSms;
     LaunchScope scope("k_rows", stream);
     return launch_chained(kernel, dim3(grid_rows, groups, nf), threads, smem, stream, r);
   }

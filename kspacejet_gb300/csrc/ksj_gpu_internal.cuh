@@ -14,6 +14,10 @@
 
 namespace ksj_gpu {
 
+// SMs of a GB300: what launches are shaped by (a constant, not asked of the device, so that
+// workspace sizes follow from the problem alone).
+constexpr int kSms = 152;
+
 // ------------------------------------------------------------------ launches
 
 ksj_gpu_status check_launch();       // cudaGetLastError -> status
