@@ -369,7 +369,7 @@ extern "C" ksj_gpu_status ksj_gpu_aggregate_acquisitions(uint32_t acquisitions, 
   const size_t total = static_cast<size_t>(acquisitions) * channels * samples_per_acquisition;
   if (total > (static_cast<size_t>(1) << 34)) return KSJ_GPU_ERROR_UNSUPPORTED;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  const unsigned blocks = static_cast<unsigned>(std::min<size_t>((total + 255) / 256, 152 * 16));
+  const unsigned blocks = static_cast<unsigned>(std::min<size_t>((total + 255) / 256, kSms * 16));
   LaunchScope scope("k_aggregate_acquisitions", cs);
   k_aggregate_acquisitions<<<blocks, 256, 0, cs>>>(static_cast<const float2*>(d_in), static_cast<float2*>(d_out),
                                                    static_cast<int>(acquisitions), static_cast<int>(channels),
