@@ -1076,26 +1076,22 @@ struct RowsArgs {
 // in sample order from zero.  Shorter lists are one segment: the cell is its
 // samples' sum in sample order.  The unit is kSegMin entries, or a 32nd of the
 // row's where that is more (a row with that many has lists enough to share out,
-// and every segment pays for putting its 16 cells in turn), up to kSegMost, beyond
-// which it is kSegFull: it depends on the
+// and every segment pays for putting its 16 cells in turn), but at most kSegMost: it depends on the
 // lists alone, so every coil grouping gives the same cells.  Units of 32, 64, 128 entries
 // and this rule measured, us of the row pass: 8 coils on a 128 grid 35, 29, 33,
 // 28, on a 512 grid 131, 107, 99, 95; a 32-coil frame 35, 31, 37, 32.
 // The upper bound keeps the sums short where rows are crowded (the centre of a
-// kooshball: rows of 3e5 entries, lists of half of them).  Without it (32 to 17 segments of up to
-// 9000 entries) the images of 2 M samples on a 48^3 grid were 2.9e-6 from double precision,
-// with it 1.0e-6 (units of a 32nd of the list 1.3e-6).  Many even segments also share out better: row
-// pass of 10.2 M samples x 20 coils on 384^3 19.3 ms without the bound, 19.0 with it (plain bounds
-// of 128, 256, 512, 1024: 19.5, 19.3, 19.2, 19.2).  Rows between the two (the 512 grid's centre has
-// units of 281) keep their 32nd: at 256 they would be a few tasks more than the block takes
-// at once (82 -> 90 us).
+// kooshball: rows of 3e5 entries, lists of half of them, which without it are 16 segments of 9000).
+// Mean and largest error against double precision of 24 images, 256 000 to 2 M kooshball samples on 24^3 to 96^3 grids,
+// 1e-7: no bound 9.9, 29; bounds of 128, 256, 512, 1024: 7.1, 12; 6.0, 10; 5.6, 6.8; 5.6, 7.0 (the
+// sum of the segments grows as they get shorter).  Row pass of 10.2 M samples x 20 coils on 384^3, ms:
+// 19.46 without, 19.53, 19.29, 19.18, 19.18; of the 512 grid above, whose centre has units of 281,
+// us: 82, 87, 90, 82, 82 (a few tasks more than a block takes at once are a round more).
 constexpr int kSegMin = 64;
 constexpr int kSegMost = 512;
-constexpr int kSegFull = 256;
 
 __device__ __forceinline__ int segment_unit(int row_entries) {
-  const int unit = max(kSegMin, (row_entries + 32 - 1) / 32);
-  return unit <= kSegMost ? unit : kSegFull;
+  return min(max(kSegMin, (row_entries + 32 - 1) / 32), kSegMost);
 }
 __device__ __forceinline__ int list_segments(int n, int unit) { return n <= unit ? 1 : (n + unit - 1) / unit; }
 __device__ __forceinline__ int segment_length(int n, int unit) {

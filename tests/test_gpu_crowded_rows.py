@@ -2,9 +2,8 @@
 
 All samples lie at one place and have one value a coil, so each cell is the sum
 of n equal terms, where the roundings of a running sum add up instead of
-cancelling.  A cell's sum is taken in partial sums of at most 512 entries (256
-in rows as full as these) that are then added up in turn: 256 + n / 256 additions
-deep, each off by at most 2^-24 of the sum.  The image is that of one sample of n times
+cancelling.  A cell's sum is taken in partial sums of at most 512 entries
+that are then added up in turn: 512 + n / 512 additions deep, each off by at most 2^-24 of the sum.  The image is that of one sample of n times
 the value; its relative error is that of the cells."""
 import numpy as np
 import pytest
@@ -15,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 SAMPLES = 1 << 17
 COILS = 32
-TOL = (256 + SAMPLES // 256) * 2.0 ** -24  # 4.6e-5
+TOL = (512 + SAMPLES // 512) * 2.0 ** -24  # 4.6e-5
 
 
 @pytest.mark.parametrize("dims", [2, 3])
