@@ -186,7 +186,7 @@ KSJ_GPU_API ksj_gpu_status ksj_gpu_gridding_adjoint_host(const ksj_gpu_gridding_
                                                          const float* h_traj, const float* h_dcf, void* h_out,
                                                          void* d_workspace, size_t workspace_bytes, void* stream);
 
-/* The sorted binning lists of the last call that used `d_workspace`, copied to
+/* The binning lists of the last call that used `d_workspace`, copied to
  * host memory: for every frame, list (grid_row, column_chunk) in row-major
  * order, the sample indices that touch it in increasing order (read from the
  * expanded entries the row pass consumes).  out_offsets

@@ -21,7 +21,7 @@
 //              the sample's weight and phase, so the row pass reads one
 //              sample's coils as one coalesced segment
 //   k_rows     per (frame, grid row, coil group): groups of lanes (lane =
-//              coil) take the row's sorted lists, one 16-column chunk each,
+//              coil) take the row's lists, one 16-column chunk each,
 //              and sum its cells in registers with no atomics (a cell is
 //              only ever touched by its owning group, in list order); the block
 //              then runs the row inverse FFT of every coil line in place and
@@ -90,7 +90,7 @@ struct alignas(16) SampleRecord3 {
   float wc[W];
 };
 
-// One sorted list entry as the row pass reads it: the first tap's column as
+// One list entry as the row pass reads it: the first tap's column as
 // seen from the list's chunk (-7 .. 15; a row length lower when the taps reaching
 // the chunk wrapped past the last column), the sample index, and the W column
 // weights times the list's row (and plane) weight.
@@ -947,7 +947,7 @@ __device__ __forceinline__ void put_entry(uint32_t sidx, int c0, float wrow, con
   }
 }
 
-// Density weights (2-D): a sample's double-precision taps, and one sorted list
+// Density weights (2-D): a sample's double-precision taps, and one list
 // entry as the grid step streams it.
 template <int W>
 struct PmRecord {
@@ -1051,7 +1051,7 @@ struct RowsArgs {
   const float2* samples_t;     // [frame][sample][channel], weighted
   size_t sample_frame_stride;  // elements between frames of samples_t (0: one sample set for all frames)
   const uint32_t* offsets;
-  const unsigned char* expanded;  // sorted list entries (entry_bytes(width) each)
+  const unsigned char* expanded;  // list entries (entry_bytes(width) each)
   const float2* tw_cols;
   const int* pos_cols;    // DIF output position of each kept column
   float2* inter;          // [frame][grid_row][out_col][cpitch]
