@@ -177,6 +177,25 @@ struct Shape {
 // Column tiles that take all the coils of a column.
 inline int column_groups(const Shape& s) { return (s.cpitch + s.col_group - 1) / s.col_group; }
 
+// TMA boxes of equal rows, at most 256 each, that take a tile of `rows` rows.
+inline int tile_boxes(int rows) {
+  int boxes = 1;
+  while (rows / boxes > 256 || rows % boxes != 0) ++boxes;
+  return boxes;
+}
+
+// Columns of a column tile, `cb` or more: each of a tile's boxes has to start on 128 bytes of
+// shared memory (a TMA copy to any other address faults).  Where there are several boxes and a
+// row is fewer than 16 lines (128 bytes), their size may not be a multiple of that (315 rows x 8
+// lines: three of 6720 bytes); the tile then takes more columns, of which those past
+// the image are filled with zeros and not written.
+inline int aligned_column_block(int rows, int col_group, int cb) {
+  const int boxes = tile_boxes(rows);
+  if (boxes > 1)
+    while (static_cast<size_t>(rows / boxes) * cb * col_group * sizeof(float2) % 128 != 0) cb <<= 1;
+  return cb;
+}
+
 struct Layout {
   size_t flags, frame_flags, cleared, records, counts, totals, offsets, expanded, samples_t, inter,
       coil_last, tables, total;
@@ -341,7 +360,7 @@ ksj_gpu_status make_shape(const ksj_gpu_gridding_desc* d, const ksj_gpu_gridding
       cols_tile(cb) > smem_limit)
     return KSJ_GPU_ERROR_INVALID_ARGUMENT;
   s->coil_group = cg;
-  s->column_block = cb;
+  s->column_block = aligned_column_block(s->grid_rows, s->col_group, cb);
   // frames per k_rows/k_cols pass: keep one pass's row-transformed grid
   // (channels x grid_rows x out_cols complex) within ~64 MB of L2
   // fields appended to the tuning struct are read only when the caller's
@@ -1912,10 +1931,8 @@ EncodeTiledFn encode_tiled() {
 bool make_inter_map(const Shape& s, void* inter, CUtensorMap* map, int* box_rows, int* boxes) {
   EncodeTiledFn enc = encode_tiled();
   if (enc == nullptr) return false;
-  int nb = 1;
-  while (s.grid_rows / nb > 256 || s.grid_rows % nb != 0) ++nb;
-  *boxes = nb;
-  *box_rows = s.grid_rows / nb;
+  *boxes = tile_boxes(s.grid_rows);
+  *box_rows = s.grid_rows / *boxes;
   const cuuint64_t dims[3] = {static_cast<cuuint64_t>(s.cpitch), static_cast<cuuint64_t>(s.out_cols),
                               static_cast<cuuint64_t>(s.frames) * s.grid_rows};
   const cuuint64_t strides[2] = {static_cast<cuuint64_t>(s.cpitch) * 8,
@@ -3972,6 +3989,7 @@ ksj_gpu_status make_cart_shape(uint32_t rows, uint32_t cols, uint32_t channels, 
   if (is_fft_size(rows)) {  // the column pass k_cols and its tile
     while (cb > 1 && (tile(cb) > 110 * 1024 || cb > s.out_cols)) cb >>= 1;
     if (tile(cb) > 200 * 1024) return KSJ_GPU_ERROR_UNSUPPORTED;
+    cb = aligned_column_block(s.grid_rows, s.col_group, cb);
   } else {
     cb = 1;
   }
