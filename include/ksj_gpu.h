@@ -107,7 +107,8 @@ typedef struct ksj_gpu_gridding_desc {
 typedef struct ksj_gpu_gridding_tuning {
   uint32_t struct_size;
   uint32_t coil_group;      /* channels accumulated per row CTA: 1, 2, 4, 8, 16 or 32 */
-  uint32_t column_block;    /* columns per column-pass tile: a power of two (1..32) */
+  uint32_t column_block;    /* columns per column-pass tile: a power of two (1..32); taken larger on grids of more
+                                than 256 rows where few coils would leave a tile's TMA boxes off 128 bytes */
   uint32_t list_capacity;   /* accepted (a power of two, 64..2048) and not used: the lists are built in order */
   uint32_t frames_per_pass; /* frames per row/column pass; passes alternate between two streams (0: two passes
                                 once there are 4 or more frames) */
